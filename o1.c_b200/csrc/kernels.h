@@ -48,6 +48,8 @@ bool gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void
 // copies the (cached) tensor map of a row-major bf16 matrix into *out; false + error text on failure
 bool cached_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                  uint32_t box_rows);
+// encodes the tensor map of a row-major bf16 matrix [rows, cols], pitch ld elements: boxes of 64 columns x box_rows rows
+bool make_tmap_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
 // sets a kernel's dynamic shared-memory limit once per device (`done`: one bit per device ordinal)
 bool func_attr_once(std::atomic<uint64_t>& done, const void* func, int smem_bytes, const char* what);
 

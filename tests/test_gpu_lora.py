@@ -100,3 +100,43 @@ def test_lora_merge_against_the_reference_python_contract(pkg, dev, golden):
         assert pkg.lib.hd_lora_merge_gpu(ents, 1, None) == 0, pkg.last_error()
         torch.cuda.synchronize()
         check_merged(torch_to_u16(wd), g[f"c{i}_merged"], w0, max_frac=1e-3)
+
+
+def merged_f64(w0, up, down, s):
+    return w0.double() + s * (up.double() @ down.double())
+
+
+@pytest.mark.parametrize("shapes", [
+    [(8, 128, 1)],                                            # one tile, eight of its rows
+    [(127, 256, 15), (129, 128, 16), (128, 384, 17)],         # a row short of a tile, a row over; one and two MMA steps
+    [(256, 128, 63), (200, 256, 64), (130, 128, 65)],         # around one chunk of ranks
+    [(300, 640, 129), (64, 128, 192), (1, 128, 8)],           # several chunks; the last one runs without tensor cores
+    [(128 * (i % 3 + 1), 128 * (i % 4 + 1), 4 + i) for i in range(37)],   # more targets than one launch takes
+    [(20000, 128, 8)],                                        # every SM walks a column of row blocks
+], ids=["one", "rows", "rank", "chunks", "many", "tall"])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_lora_merge_tile_edges(pkg, dev, shapes, shift):
+    """Edges of the merge kernel's tiles, rank chunks and launch groups against 64 bits, all targets in one call.  shift:
+    adapters that begin 4 bytes off a 16-byte boundary.  The FP32 sum of 6 R products is within R * 2^-22 of the exact
+    delta's magnitude sum, so a weight may differ from the rounded 64-bit value only where that bound crosses a rounding
+    boundary, and then by one bf16 step."""
+    g = torch.Generator(device=dev).manual_seed(len(shapes) * 2 + shift)
+    ents, keep = (pkg.LoraEntry * len(shapes))(), []
+    for e, (n, k, r) in zip(ents, shapes):
+        w = torch.empty(n + 1, k, device=dev).normal_(0, 0.02, generator=g).bfloat16()      # a canary row behind
+        up = torch.empty(n * r + shift, device=dev).normal_(0, 0.05, generator=g)[shift:]
+        down = torch.empty(r * k + shift, device=dev).normal_(0, 0.05, generator=g)[shift:]
+        ee = entry(pkg, w, up, down, r, k, n, 0.7 * r, -1.3)
+        C.memmove(C.byref(e), C.byref(ee), C.sizeof(e))
+        keep.append((w, w.clone(), up, down))
+    assert pkg.lib.hd_lora_merge_gpu(ents, len(shapes), None) == 0, pkg.last_error()
+    assert pkg.lib.o1_device_error() == 0
+    for (n, k, r), (w, w0, up, down) in zip(shapes, keep):
+        u, d = up.view(n, r), down.view(r, k)
+        want = merged_f64(w0[:n], u, d, 0.7 * -1.3)
+        bound = (u.abs().double() @ d.abs().double() + w0[:n].abs().double()) * (r + 4) * 2.0 ** -22
+        # rounding is monotonic: the result lies between the rounded ends of the interval around the exact value
+        lo, hi = (want - bound).bfloat16().double(), (want + bound).bfloat16().double()
+        got = w[:n].double()
+        assert ((got >= lo) & (got <= hi)).all(), (n, k, r, ((got < lo) | (got > hi)).sum().item())
+        assert torch.equal(w[n:].view(torch.int16), w0[n:].view(torch.int16)), "rows beyond N were written"
