@@ -540,7 +540,10 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     float* xch = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 192);
-    float* m_sh = xch + T1_XCH / 4;       // [row]: the max every stored P, partial sum and O is relative to
+    // [tile parity][row]: the max that every stored P, partial sum and O is relative to after a tile, as the unscaled bf16
+    // score it came from.  Both threads of a row read the previous tile's entry and one writes this tile's, so the two lie
+    // in different places, and all eight warps of a set arrive on m_pub: an entry is not overwritten before it is read.
+    uint16_t* m_sh = reinterpret_cast<uint16_t*>(xch + T1_XCH / 4);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -586,7 +589,7 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int s = 0; s < T1_K_STAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
         for (int s = 0; s < T1_V_STAGES; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
         for (int s = 0; s < T1_S_BUFS; ++s) { mbar_init(&s_full[s], 1); mbar_init(&p_ready[s], 8); }
-        for (int s = 0; s < 2; ++s) mbar_init(&m_pub[s], 4);
+        for (int s = 0; s < 2; ++s) mbar_init(&m_pub[s], 8);
         mbar_init(o_done, 1);
         fence_mbar_init();
     }
@@ -698,6 +701,7 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int bar_id = 1 + set;              // named barrier of the set's 256 threads
         constexpr int BAR_THREADS = 256;
         float m_mine = -INFINITY;                // max this thread's partial sum is relative to
+        uint32_t m_raw = 0xff800000u;            // the score it came from
         float l = 0.f;                           // this thread's share of the row sum
         bool ok = true;
         for (int j = set; j < n_tiles; j += 2) {
@@ -750,30 +754,30 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             }
             asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(BAR_THREADS) : "memory");
             if (!ok) continue;
-            float mx = fmaxf(__uint_as_float(mb & 0xffff0000u), __uint_as_float((uint32_t)x16[use * 256 + (half ^ 1) * 128] << 16));
+            const float mx = fmaxf(__uint_as_float(mb & 0xffff0000u), __uint_as_float((uint32_t)x16[use * 256 + (half ^ 1) * 128] << 16));
             const float m_tile = mx * a.scale_log2;
             // the max in force after the previous tile, which the other set decided
-            float m_prev = -INFINITY;
             if (j >= 1) {
                 if (!mbar_wait_warp(&m_pub[set ^ 1], ((j - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; continue; }
-                m_prev = m_sh[row];
-            }
-            if (m_prev != m_mine) {        // the other set raised it: this thread's sum follows
-                l *= ex2_approx(m_mine - m_prev);     // m_mine == -inf: l is 0 and stays 0
-                m_mine = m_prev;
+                const uint32_t raw = (uint32_t)m_sh[((j - 1) & 1) * T1_ROWS + row] << 16;
+                if (raw != m_raw) {        // the other set raised it: this thread's sum follows
+                    const float m_prev = __uint_as_float(raw) * a.scale_log2;
+                    l *= ex2_approx(m_mine - m_prev);     // m_mine == -inf: l is 0 and stays 0
+                    m_mine = m_prev;
+                    m_raw = raw;
+                }
             }
             const bool grow = (m_tile - m_mine) > 8.0f;      // also true while m_mine == -inf
             float alpha = 1.0f;
             if (grow) {
                 alpha = ex2_approx(m_mine - m_tile);         // 0 on the first tile
                 m_mine = m_tile;
+                m_raw = __float_as_uint(mx);
                 l *= alpha;
             }
-            if (half == 0) {
-                m_sh[row] = m_mine;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&m_pub[set]);
-            }
+            if (half == 0) m_sh[(j & 1) * T1_ROWS + row] = (uint16_t)(m_raw >> 16);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&m_pub[set]);
             if (j >= 1 && __any_sync(0xffffffffu, grow)) {
                 // O must hold all of PV(j-1) and nothing of PV(j): the first is what v_empty of tile j-1 reports,
                 // the second waits for this set's p_ready.  Each thread scales its own 64 output columns.
@@ -806,8 +810,12 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (ok && ((n_tiles - 1) & 1) != set) {
             if (!mbar_wait_warp(&m_pub[set ^ 1], ((n_tiles - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; }
             if (ok) {
-                const float m_fin = m_sh[row];
-                if (m_fin != m_mine) { l *= ex2_approx(m_mine - m_fin); m_mine = m_fin; }
+                const uint32_t raw = (uint32_t)m_sh[((n_tiles - 1) & 1) * T1_ROWS + row] << 16;
+                if (raw != m_raw) {
+                    const float m_fin = __uint_as_float(raw) * a.scale_log2;
+                    l *= ex2_approx(m_mine - m_fin);
+                    m_mine = m_fin;
+                }
             }
         }
         // ---- output: O / l -> bf16 -> out[row_g, h*128 + part4*32 ..]
