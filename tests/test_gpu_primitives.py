@@ -459,3 +459,31 @@ def test_gemm_on_cta_pairs_equals_single_cta_tiles(pkg, dev, M, N, K, epi):
     if epi == 2: ref = (ref.bfloat16().float() + resid.float())
     err = (outs[1].float() - ref).abs().max().item() / max(ref.abs().max().item(), 1e-6)
     assert err < 1e-2, err     # the pair form really computed the product (fp32 reference, bf16 rounding of the result)
+
+
+@pytest.mark.parametrize("sigma", [0.857, 1.0, 0.008, 1.0 / 3.0, 0.99999994, 3e-10, 1e-12, 2e9, 1e30])
+@pytest.mark.parametrize("n", [8, 4096 * 8, 1003])
+def test_fused_step_equals_the_chain_for_every_kind_of_value(pkg, dev, sigma, n):
+    """The fused guidance + Euler step shares one reciprocal of sigma among all its divisions; its bits are those of the
+    separate kernels with their IEEE divisions, also where the short division does not apply: equal operands, signed
+    zeros, tiny and huge values, infinities, NaN, and sigmas outside its range."""
+    g = torch.Generator(device=dev).manual_seed(n)
+    special = torch.tensor([0.0, -0.0, 1e-38, -1e-38, 2e-30, -3e-17, 1e20, -1e20, 3e38, float("inf"), -float("inf"), float("nan"),
+                            1.0, -1.0, 0.5, 8.0], device=dev).bfloat16()
+    z, xc, xu = (torch.empty(n, device=dev).normal_(0, s, generator=g).bfloat16() for s in (4.0, 1.0, 1.0))
+    for t in (z, xc, xu):           # a run of ordinary vectors, then specials in every combination that falls out
+        at = torch.randperm(n, device=dev, generator=g)[:max(1, n // 3)]
+        t[at] = special[torch.randint(0, 16, (at.numel(),), device=dev, generator=g)]
+    xc[:: 5] = z[:: 5]
+    fused, chain = torch.empty_like(z), torch.empty_like(z)
+    s1 = sigma * 0.9
+    assert pkg.lib.o1_sched_cfg_flow_step(pkg.ptr(z), pkg.ptr(xc), pkg.ptr(xu), sigma, s1, 5.0, pkg.ptr(fused), n) == 0
+    mc, mu, mo = (torch.empty(n, device=dev) for _ in range(3))
+    pkg.lib.hd_sched_vcond(pkg.ptr(z), pkg.ptr(xc), sigma, pkg.ptr(mc), n)
+    pkg.lib.hd_sched_vcond(pkg.ptr(z), pkg.ptr(xu), sigma, pkg.ptr(mu), n)
+    pkg.lib.hd_sched_cfg_guided(pkg.ptr(mc), pkg.ptr(mu), 5.0, pkg.ptr(mo), n)
+    pkg.lib.hd_sched_flow_match_step(pkg.ptr(z), pkg.ptr(mo), sigma, s1, pkg.ptr(chain), n)
+    done(pkg, "sched")
+    nan = chain.isnan()
+    assert torch.equal(nan, fused.isnan())
+    assert torch.equal(fused.view(torch.int16)[~nan], chain.view(torch.int16)[~nan])
