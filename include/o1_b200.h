@@ -495,11 +495,10 @@ void o1_attention_tail_ways(int ways);
  * the one-tile kernel (environment O1_ATTN_TILE_MODE sets the initial value).  Same arithmetic up to fp32 summation
  * order and the reference max of the lazy rescale. */
 void o1_attention_tile_mode(int mode);
-/* GEMM tile form for the large-M families (plain, bias, residual, SwiGLU, grouped q|k|v) when the problem has at least
- * two rounds of 256 x 256 tiles: 1 (default; environment O1_GEMM_PAIR=0 turns it off) = a cluster of two CTAs per
- * tile with cta_group::2 MMAs, each CTA holding 128 rows of A and of the accumulator and half of the B tile;
- * 0 = one CTA per 128 x 256 tile; 2 = pairs for the SwiGLU family as well (measured 1.6 % slower for that family in
- * the power-capped step, so not the default).  All forms add a row's K products in the same order: same bits.  No reference
+/* GEMM tile form of the plain, bias, residual, SwiGLU and grouped q|k|v families: 1 (default; environment O1_GEMM_PAIR=0
+ * turns it off) = where that takes the fewest rounds of tiles, a cluster of two CTAs per 256 x 256 tile with
+ * cta_group::2 MMAs, each CTA holding 128 rows of A and of the accumulator and half of the B tile; 0 = always one CTA
+ * per tile.  All forms add a row's K products in the same order: same bits.  No reference
  * counterpart (cuBLASLt picks its own kernels there, src/cuda/gemm.cu:413-461). */
 void o1_gemm_pair_mode(int mode);
 /* CTA pairs of the GEMM kernel the current device holds at once (the pair form never launches more); -1 on error. */
@@ -531,7 +530,8 @@ hd_status o1_lora_merge_static(void *base_dev, const float *up_dev, const float 
 /* One CFG denoise step on device-resident state: x_c = forward(ids_cond),
  * x_u = forward(ids_uncond), z' = cfg_flow_step(z, x_c, x_u).  Composition of
  * src/runtime/generate.c:1314-1360 with the flow-match update of :900-905.
- * timestep_dev holds t = 1 - sigma.  ws is used for both branches in turn;
+ * timestep_dev holds t = 1 - sigma.  ws is used for both branches, one after the other or,
+ * up to 2048 rows each, together (hd_forward_workspace_bytes has the room);
  * xp_scratch holds 2 * seq * 3072 bf16. */
 hd_status o1_denoise_step_cfg(const hd_forward_binding *bw, hd_forward_workspace *ws,
                               const int64_t *ids_cond, const int64_t *ids_uncond, int text_len,
@@ -555,7 +555,7 @@ hd_status o1_denoise_step_cfg_ref(const hd_forward_binding *bw, hd_forward_works
  * posd[1], seq_S_uncond; :1340-1356 runs and slices that branch at its own text length).  Padding the shorter
  * prompt instead would let image rows attend to the pad rows.  Each branch: ids [text_len] int64, pos_f32
  * [3, text_len + img_tokens], ar_len (text_len - 1 for T2I), visual (may be NULL).  ws (one workspace, used by
- * both branches in turn) must come from hd_forward_workspace_bytes of the LONGER sequence; xp_scratch holds
+ * both branches) must come from hd_forward_workspace_bytes of the LONGER sequence; xp_scratch holds
  * (S_cond + S_uncond) * 3072 bf16.  The scheduler update is the flow-match Euler step; the reference's own
  * CFG path steps with FlowUniPC (generate.c:1362-1416), which a host composes from hd_forward, hd_sched_vcond,
  * hd_sched_cfg_guided and hd_unipc_* exactly as there. */

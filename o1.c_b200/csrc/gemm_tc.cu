@@ -37,9 +37,11 @@ struct GemmArgs {
     const uint16_t* bias;
     const uint16_t* resid;
     int ldr;
-    const float* rope;     // EPI_QKNORM: cos|sin table [M,128] fp32
+    const float* rope;     // EPI_QKNORM: cos|sin table [M,128] fp32; EPI_VROPE: cos [M,72]
+    const float* rope_sin; // EPI_VROPE: sin [M,72]
     float scale;
     int num_m, num_n, group_m;
+    int prefetch;          // K blocks of weights requested into L2 ahead of their load (0: none)
     // Output column blocks: column c lives at out + (c / o_cb) * o_cb_stride + row * ldo + c % o_cb
     // (o_cb == 0: plain row-major).  Lets a projection write its head groups into per-destination
     // slabs of an all-to-all send buffer.  o_cb must be a multiple of the tile width.
@@ -88,12 +90,18 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int 
     nb = r / gm;
 }
 
-// GELU of a bf16-valued activation, as o1.c's vision kernels compute it (src/cuda/vision_kernels.cu:100-133):
-// the tanh form of the ViT block MLP or the erf form of the patch mergers, fp32 throughout, rounded by the caller
-__device__ __forceinline__ float gelu_of(float v, bool exact) {
-    if (exact) return 0.5f * v * (1.0f + erff(v * 0.7071067811865476f));
-    const float u = 0.7978845608028654f * (v + 0.044715f * v * v * v);
-    return 0.5f * v * (1.0f + tanhf(u));
+// bf16-valued activations -> GELU, as o1.c's vision kernels compute it (src/cuda/vision_kernels.cu:100-133): the tanh
+// form of the ViT block MLP or the erf form of the patch mergers, fp32 throughout, rounded by the caller.  One branch for
+// all values: with one per value nothing overlaps (a 128 x 128 tile's epilogue took 9 us longer).
+template <int N>
+__device__ __forceinline__ void gelu_all(float (&v)[N], bool exact) {
+    if (exact) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[j] = 0.5f * v[j] * (1.0f + erff(v[j] * 0.7071067811865476f));
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[j] = gelu_tanh(v[j]);
+    }
 }
 __device__ __forceinline__ void store32_bf16(uint16_t* dst, const float (&v)[32]) {
     uint4* d4 = reinterpret_cast<uint4*>(dst);
@@ -106,6 +114,10 @@ __device__ __forceinline__ void store32_bf16(uint16_t* dst, const float (&v)[32]
         o.w = pack_bf16x2(v[i * 8 + 6], v[i * 8 + 7]);
         d4[i] = o;
     }
+}
+__device__ __forceinline__ void unpack8_bf16(const uint4& o, float* v) {
+    v[0] = bf16lo(o.x); v[1] = bf16hi(o.x); v[2] = bf16lo(o.y); v[3] = bf16hi(o.y);
+    v[4] = bf16lo(o.z); v[5] = bf16hi(o.z); v[6] = bf16lo(o.w); v[7] = bf16hi(o.w);
 }
 __device__ __forceinline__ void load32_bf16(const uint16_t* src, float (&v)[32]) {
     const uint4* s4 = reinterpret_cast<const uint4*>(src);
@@ -136,14 +148,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
     uint8_t* store_stage = smem + STAGES * Cfg::STAGE_BYTES + 256;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     // a kernel that already failed on this device leaves its code in *err: do nothing then
     __shared__ int s_abort;
     if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(g.err);
     __syncthreads();
-    if (!PAIR && s_abort != 0) return;      // (a pair decides together, after its first cluster barrier)
+    if (!PAIR && s_abort != 0) { grid_dep_wait(); return; }      // (a pair decides together, after its first cluster barrier)
     const uint32_t rank = PAIR ? cluster_rank() : 0u;    // 0: the CTA that issues the pair's MMAs
 
     if (threadIdx.x == 0) {
@@ -165,6 +177,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     if (PAIR) cluster_sync_all();           // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
     bool live = true;
     if (PAIR) live = (s_abort | ld_cluster_s32(map_to_rank(smem_u32(&s_abort), rank ^ 1u))) == 0;
@@ -181,7 +195,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // nothing to do: straight to the common teardown
     } else if (warp == 0) {
         // ------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tmA);
             tma_prefetch_desc(&tmB);
             if (EPI == EPI_SWIGLU || EPI == EPI_QKV) tma_prefetch_desc(&tmB2);
@@ -248,7 +262,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp == 1) {
         // ------------------------------------------------------ MMA issuer
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             constexpr uint32_t idesc = umma_idesc_bf16(PAIR ? 2 * BM : BM, BN, 0, 0);
             int stage = 0;
             uint32_t phase = 0;
@@ -498,8 +512,31 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                 }
             } else {
+                // the residual of the next 32 columns is requested before the current ones are worked on: in the last tile
+                // of a CTA nothing else covers that latency
+                constexpr bool HAS_RESID = EPI == EPI_RESID || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID;
+                const uint16_t* rrow = HAS_RESID ? g.resid + (size_t)row * g.ldr + nb * BN : nullptr;
+                uint4 rn[4] = {};
+                if (HAS_RESID && row_ok) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) rn[i] = reinterpret_cast<const uint4*>(rrow)[i];
+                }
 #pragma unroll 1
                 for (int c = 0; c < BN / 32; ++c) {
+                    float rs[32];
+                    if (HAS_RESID) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            rs[i * 8 + 0] = bf16lo(rn[i].x); rs[i * 8 + 1] = bf16hi(rn[i].x);
+                            rs[i * 8 + 2] = bf16lo(rn[i].y); rs[i * 8 + 3] = bf16hi(rn[i].y);
+                            rs[i * 8 + 4] = bf16lo(rn[i].z); rs[i * 8 + 5] = bf16hi(rn[i].z);
+                            rs[i * 8 + 6] = bf16lo(rn[i].w); rs[i * 8 + 7] = bf16hi(rn[i].w);
+                        }
+                        if (row_ok && c + 1 < BN / 32) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) rn[i] = reinterpret_cast<const uint4*>(rrow + (c + 1) * 32)[i];
+                        }
+                    }
                     uint32_t r[32];
                     tmem_ld32(t_row + c * 32, r);
                     tmem_ld_wait();
@@ -520,7 +557,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                     for (int j = 0; j < 8; ++j) v8[j] = bf16_round(v8[j]) + b8[j];
                                     if (EPI == EPI_BIAS_GELU) {
 #pragma unroll
-                                        for (int j = 0; j < 8; ++j) v8[j] = gelu_of(bf16_round(v8[j]), g.scale != 0.f);
+                                        for (int j = 0; j < 8; ++j) v8[j] = bf16_round(v8[j]);
+                                        gelu_all(v8, g.scale != 0.f);
                                     }
                                 }
                                 uint4 o;
@@ -542,26 +580,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             for (int j = 0; j < 32; ++j) v[j] = bf16_round(v[j]) + b[j];
                             if (EPI == EPI_BIAS_GELU) {
 #pragma unroll
-                                for (int j = 0; j < 32; ++j) v[j] = gelu_of(bf16_round(v[j]), g.scale != 0.f);
+                                for (int j = 0; j < 32; ++j) v[j] = bf16_round(v[j]);
+                                gelu_all(v, g.scale != 0.f);
                             }
                         } else if (EPI == EPI_BIAS_RESID) {
                             // linear + bias stored as bf16, then the residual add of src/cuda/residual.cu:14-23
-                            float b[32], rs[32];
+                            float b[32];
                             load32_bf16(g.bias + col, b);
-                            load32_bf16(g.resid + (size_t)row * g.ldr + col, rs);
 #pragma unroll
                             for (int j = 0; j < 32; ++j) v[j] = rs[j] + bf16_round(bf16_round(v[j]) + b[j]);
                         } else if (EPI == EPI_GATE_RESID) {
-                            float gt[32], rs[32];
+                            float gt[32];
                             load32_bf16(g.bias + col, gt);
-                            load32_bf16(g.resid + (size_t)row * g.ldr + col, rs);
 #pragma unroll
                             for (int j = 0; j < 32; ++j) v[j] = rs[j] + bf16_round(gt[j] * bf16_round(v[j]));
                         } else if (EPI == EPI_RESID) {
-                            float b[32];
-                            load32_bf16(g.resid + (size_t)row * g.ldr + col, b);
 #pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = bf16_round(v[j]) + b[j];
+                            for (int j = 0; j < 32; ++j) v[j] = bf16_round(v[j]) + rs[j];
                         } else if (EPI == EPI_LORA) {
                             float b[32];
                             load32_bf16(g.out + (size_t)row * g.ldo + ocol, b);
@@ -592,38 +627,340 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
 }
 
+// ---------------------------------------------------------------- few tiles
+// A problem with few output tiles leaves most SMs idle in the persistent kernel: a 77-row projection is 32 tiles of 128
+// columns, the tower's fc2 at 520 rows 45 tiles of 68 K blocks.  This kernel takes one tile per CTA, two CTAs per SM (one's
+// epilogue runs under the other's main loop), and makes more of them in one of two ways:
+//  * narrower tiles (32 or 96 columns): the same sum for every element, for callers that rely on it;
+//  * the K blocks of a 128-column tile shared by the `ks` CTAs of a cluster.  Each accumulates its part in its own tensor
+//    memory; then CTA r takes over the 16-column units [8r/ks, 8(r+1)/ks): the others write those FP32 columns straight
+//    into its shared memory (one thread per row: consecutive 16-byte pieces, no bank conflicts) and it adds them in rank
+//    order, so the result does not depend on timing and no workspace, atomic or second launch is needed.
+static constexpr int SK_BN = 128;
+// K blocks of weights requested into L2 ahead of their load, before the wait for the previous grid to begin with: three to
+// five stages do not cover the way from memory (1152 x 4304 at 520 rows, five CTAs per tile: 21.0 -> 19.0 us; the
+// persistent kernel's six stages do, and there the requests only cost: 24 -> 32 us at 77 x 4096 x 4096).
+static constexpr int SK_PREFETCH = 24;
+template <int BN>
+struct SplitCfg {
+    static constexpr int STAGES = BN <= 32 ? 5 : 3;      // as many as leave room for a second CTA
+    static constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
+    static constexpr int TMEM_COLS = BN <= 32 ? 32 : (BN <= 128 ? 128 : 256);
+};
+// The tower's q | k | v projection takes the same kernel unsplit with tiles of 144 columns, two whole heads of 72: a
+// thread then holds both halves of its row's heads and the rotary is part of the epilogue (3456 = 24 tiles exactly).
+static constexpr int VQ_BN = 144;
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d)
+                 : "memory");
+}
+
+template <int EPI, int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 2)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g,
+                  const int ks) {
+    constexpr int SK_STAGE_BYTES = SplitCfg<BN>::STAGE_BYTES, SK_STAGES = SplitCfg<BN>::STAGES, NU = BN / 16;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + SK_STAGES * SK_STAGE_BYTES);
+    uint64_t* empty = full + SK_STAGES;
+    uint64_t* acc_done = empty + SK_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+    int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+    __shared__ uint4 bias_s[BN / 8];
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const int rank = (int)(blockIdx.x % ks), tile = (int)(blockIdx.x / ks);
+    const int nb = tile / g.num_m, mb = tile - nb * g.num_m;      // CTAs that share weights run next to each other
+
+    if (threadIdx.x == 0) {
+        *s_abort = *reinterpret_cast<volatile int*>(g.err);
+        for (int s = 0; s < SK_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(acc_done, 1);
+        fence_mbar_init();
+    }
+    if (warp == 1) { tmem_alloc(tmem_slot, SplitCfg<BN>::TMEM_COLS); tmem_relinquish(); }
+    const int kblocks = (g.K + BK - 1) / BK;
+    const int kb0 = rank * kblocks / ks, nkb = (rank + 1) * kblocks / ks - kb0;
+    const bool ahead = mb == 0 && g.prefetch > 0;     // the other row tiles find the weights in L2
+    if (ahead && warp == 0 && elect_one())
+        for (int i = 0; i < g.prefetch && i < nkb; ++i) tma_prefetch_2d(&tmB, (kb0 + i) * BK, nb * BN);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
+    const uint32_t tmem_base = *tmem_slot;
+    // a kernel that already failed on this device leaves its code in *err: no loads and no results then, but the
+    // cluster's barriers below are passed all the same (the CTAs of a cluster may read the word at different times)
+    bool ok = *s_abort == 0;
+
+    if (ok && warp == 0) {
+        if (elect_one()) {
+            tma_prefetch_desc(&tmA);
+            tma_prefetch_desc(&tmB);
+            for (int i = 0; i < nkb; ++i) {
+                const int s = i % SK_STAGES;
+                if (!mbar_wait(&empty[s], ((i / SK_STAGES) & 1) ^ 1)) { atomicExch(g.err, 51); break; }
+                if (ahead && i + g.prefetch < nkb) tma_prefetch_2d(&tmB, (kb0 + i + g.prefetch) * BK, nb * BN);
+                uint8_t* a_s = smem + s * SK_STAGE_BYTES;
+                mbar_expect_tx(&full[s], SK_STAGE_BYTES);
+                int a_c0 = (kb0 + i) * BK, a_c1 = mb * BM;
+                if (g.a_kblk > 0) {
+                    const int blk = a_c0 / g.a_kblk;
+                    a_c0 -= blk * g.a_kblk;
+                    a_c1 += blk * g.a_rows;
+                }
+                tma_load_2d(a_s, &tmA, &full[s], a_c0, a_c1);
+                tma_load_2d(a_s + BM * BK * 2, &tmB, &full[s], (kb0 + i) * BK, nb * BN);
+            }
+        }
+    } else if (ok && warp == 1) {
+        if (elect_one()) {
+            constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, 0, 0);
+            bool good = true;
+            for (int i = 0; i < nkb && good; ++i) {
+                const int s = i % SK_STAGES;
+                if (!mbar_wait(&full[s], (i / SK_STAGES) & 1)) { atomicExch(g.err, 52); good = false; break; }
+                tc_fence_after();
+                const uint32_t a_addr = smem_u32(smem + s * SK_STAGE_BYTES);
+                const uint64_t ad = umma_desc_sw128(a_addr, 16, 1024);
+                const uint64_t bd = umma_desc_sw128(a_addr + BM * BK * 2, 16, 1024);
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k) umma_ss(tmem_base, ad + 2 * k, bd + 2 * k, idesc, (i | k) != 0);
+                umma_commit(&empty[s]);
+            }
+            umma_commit(acc_done);
+        }
+    }
+    // The epilogue's other operands are requested while the main loop runs: this thread's residual row into registers, the
+    // tile's bias into shared memory (each of the eight units of a tile would otherwise wait for its own loads).
+    constexpr bool HAS_BIAS = EPI != EPI_STORE && EPI != EPI_RESID && EPI != EPI_VROPE;
+    constexpr bool HAS_RESID = EPI == EPI_RESID || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID;
+    const int q = warp & 3;       // TMEM lane quadrant this warp may access
+    const int trow = q * 32 + lane;
+    const int u0 = rank * NU / ks, u1 = (rank + 1) * NU / ks;     // this CTA's share of the tile's 16-column units
+    const int row = mb * BM + trow;
+    const bool row_ok = row < g.M;
+    uint4 res[HAS_RESID ? 2 * NU : 1];
+    if (ok && warp >= 2) {
+        if (HAS_BIAS && trow * 8 < BN) {
+            const int col = nb * BN + trow * 8;
+            bias_s[trow] = col < g.N ? *reinterpret_cast<const uint4*>(g.bias + col) : make_uint4(0, 0, 0, 0);
+        }
+        if (HAS_RESID) {
+#pragma unroll
+            for (int h = 0; h < 2 * NU; ++h) {
+                const int col = nb * BN + h * 8;
+                res[h] = row_ok && col < g.N && h >= 2 * u0 && h < 2 * u1
+                             ? *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col) : make_uint4(0, 0, 0, 0);
+            }
+        }
+        if (HAS_BIAS) asm volatile("bar.sync 1, 128;" ::: "memory");      // the four epilogue warps
+    }
+    if (ok && warp >= 2) {
+        if (!mbar_wait(acc_done, 0)) { atomicExch(g.err, 53); ok = false; }
+        ok = __all_sync(0xffffffffu, ok);
+        tc_fence_after();
+    }
+    const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
+    if constexpr (EPI == EPI_VROPE) {
+        if (ok && warp >= 2) {
+#pragma unroll 1
+            for (int hh = 0; hh < 2; ++hh) {
+                uint32_t ra[32], rb[32], rc[8];
+                tmem_ld32(t_row + hh * 72, ra);
+                tmem_ld32(t_row + hh * 72 + 32, rb);
+                tmem_ld8(t_row + hh * 72 + 64, rc);
+                tmem_ld_wait();
+                if (row < g.M) {
+                    const int col = nb * VQ_BN + hh * 72, which = col / 1152, h = (col - which * 1152) / 72;
+                    float x[72];
+#pragma unroll
+                    for (int c = 0; c < 9; ++c) {
+                        const uint4 b4 = *reinterpret_cast<const uint4*>(g.bias + col + c * 8);
+                        const float b[8] = {bf16lo(b4.x), bf16hi(b4.x), bf16lo(b4.y), bf16hi(b4.y),
+                                            bf16lo(b4.z), bf16hi(b4.z), bf16lo(b4.w), bf16hi(b4.w)};
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int d = c * 8 + j;
+                            const uint32_t r = d < 32 ? ra[d & 31] : (d < 64 ? rb[d & 31] : rc[d & 7]);
+                            x[d] = bf16_round(bf16_round(__uint_as_float(r)) + b[j]);
+                        }
+                    }
+                    if (which < 2) {     // fp32 rotary, one rounding (src/cuda/rope.cu:155-178); the table repeats after 36
+#pragma unroll
+                        for (int c = 0; c < 9; ++c) {
+                            const float4 c4 = *reinterpret_cast<const float4*>(g.rope + (size_t)row * 72 + c * 4);
+                            const float4 s4 = *reinterpret_cast<const float4*>(g.rope_sin + (size_t)row * 72 + c * 4);
+                            const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float lo = x[c * 4 + j], hi = x[c * 4 + j + 36];
+                                x[c * 4 + j] = rope_f32(lo, cs[j], -hi, sn[j]);
+                                x[c * 4 + j + 36] = rope_f32(hi, cs[j], lo, sn[j]);
+                            }
+                        }
+                    }
+                    uint4* dst = reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + (which * 16 + h) * 128);
+#pragma unroll
+                    for (int c = 0; c < 9; ++c) {
+                        uint4 o;
+                        o.x = pack_bf16x2(x[c * 8], x[c * 8 + 1]); o.y = pack_bf16x2(x[c * 8 + 2], x[c * 8 + 3]);
+                        o.z = pack_bf16x2(x[c * 8 + 4], x[c * 8 + 5]); o.w = pack_bf16x2(x[c * 8 + 6], x[c * 8 + 7]);
+                        dst[c] = o;
+                    }
+                    dst[9] = make_uint4(0, 0, 0, 0);
+                }
+            }
+        }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN>::TMEM_COLS);
+        return;
+    }
+    const int mu = (NU + ks - 1) / ks;                            // most units a CTA owns
+    if (ks > 1) {
+        // every CTA's MMAs are through with its stages, which now receive the others' columns:
+        // [source][unit][4 columns][row] of 16 bytes, at most 7 x 2 or 1 x 4 units of 8 KB
+        __syncwarp();
+        cluster_sync_all();
+        if (ok && warp >= 2) {
+            for (int dst = 0; dst < ks; ++dst) {
+                if (dst == rank) continue;
+                const uint32_t base = map_to_rank(smem_u32(smem), dst);
+                const int slot = rank < dst ? rank : rank - 1, d0 = dst * NU / ks, d1 = (dst + 1) * NU / ks;
+                for (int u = d0; u < d1; ++u) {
+                    uint32_t r[16];
+                    tmem_ld16(t_row + u * 16, r);
+                    tmem_ld_wait();
+                    const uint32_t at = base + (uint32_t)((((slot * mu + u - d0) * 4) * BM + trow) * 16);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        st_cluster_v4(at + c * BM * 16, r[c * 4], r[c * 4 + 1], r[c * 4 + 2], r[c * 4 + 3]);
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync_all();
+    }
+    if (ok && warp >= 2) {
+#pragma unroll
+        for (int u = 0; u < NU; ++u) {
+            if (u < u0 || u >= u1) continue;
+            const int col = nb * BN + u * 16;
+            // (N is a multiple of eight: a unit is whole, its first half, or outside)
+            const bool h0 = row_ok && col < g.N, h1 = row_ok && col + 8 < g.N;
+            uint32_t r[16];
+            tmem_ld16(t_row + u * 16, r);
+            tmem_ld_wait();
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = 0.f;
+            for (int src = 0; src < ks; ++src) {
+                if (src == rank) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
+                } else {
+                    const int slot = src < rank ? src : src - 1;
+                    const uint8_t* at = smem + (size_t)((((slot * mu + u - u0) * 4) * BM + trow) * 16);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float4 f = *reinterpret_cast<const float4*>(at + c * BM * 16);
+                        v[c * 4] += f.x; v[c * 4 + 1] += f.y; v[c * 4 + 2] += f.z; v[c * 4 + 3] += f.w;
+                    }
+                }
+            }
+            // the rounding points of gemm_tc_kernel's epilogues
+            float b[16], rs[16];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (HAS_BIAS) unpack8_bf16(bias_s[2 * u + h], b + h * 8);
+                if (HAS_RESID) unpack8_bf16(res[HAS_RESID ? 2 * u + h : 0], rs + h * 8);
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (EPI == EPI_BIAS) v[j] = bf16_round(v[j]) + b[j];
+                if (EPI == EPI_BIAS_GELU) v[j] = bf16_round(bf16_round(v[j]) + b[j]);
+                if (EPI == EPI_RESID) v[j] = bf16_round(v[j]) + rs[j];
+                if (EPI == EPI_BIAS_RESID) v[j] = rs[j] + bf16_round(bf16_round(v[j]) + b[j]);
+                if (EPI == EPI_GATE_RESID) v[j] = rs[j] + bf16_round(b[j] * bf16_round(v[j]));
+            }
+            if (EPI == EPI_BIAS_GELU) gelu_all(v, g.scale != 0.f);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float* w = v + h * 8;
+                uint4 o;
+                o.x = pack_bf16x2(w[0], w[1]); o.y = pack_bf16x2(w[2], w[3]);
+                o.z = pack_bf16x2(w[4], w[5]); o.w = pack_bf16x2(w[6], w[7]);
+                if (h ? h1 : h0) *reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + col + h * 8) = o;
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN>::TMEM_COLS);
+}
+
 // ---------------------------------------------------------------- SIMT path
-// One warp per output element; used for M < 8 (timestep MLP, M = 1) and
-// for shapes the tensor-core tiles do not cover (N % 128 or K % 64 != 0).
-__global__ void gemm_simt_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w,
+// For M < 8 (timestep MLP, M = 1) and for shapes the tensor-core tiles do not cover.  One warp per output column and MR
+// rows: bound by the weights' way from memory, so a weight is read once for all its rows, four 16-byte pieces of a lane at
+// a time.
+template <int MR>
+__global__ void __launch_bounds__(128)
+gemm_simt_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w,
                                  const uint16_t* __restrict__ bias, uint16_t* __restrict__ y, int M,
                                  int N, int K, int ldx, int ldy) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int warps_per_block = blockDim.x >> 5;
     const int n = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
-    const int m = blockIdx.y;
+    const int m0 = blockIdx.y * MR;
     const int lane = threadIdx.x & 31;
     if (n >= N) return;
-    const uint16_t* xr = x + (size_t)m * ldx;
+    const uint16_t* xr[MR];
+#pragma unroll
+    for (int i = 0; i < MR; ++i) xr[i] = x + (size_t)(m0 + i < M ? m0 + i : M - 1) * ldx;
     const uint16_t* wr = w + (size_t)n * K;
-    float acc = 0.f;
-    if ((K & 7) == 0 && ((((uintptr_t)xr) | ((uintptr_t)wr)) & 15) == 0) {
-        for (int k = lane * 8; k < K; k += 256) {
-            const uint4 a = *reinterpret_cast<const uint4*>(xr + k);
-            const uint4 b = *reinterpret_cast<const uint4*>(wr + k);
-            acc += bf16lo(a.x) * bf16lo(b.x); acc += bf16hi(a.x) * bf16hi(b.x);
-            acc += bf16lo(a.y) * bf16lo(b.y); acc += bf16hi(a.y) * bf16hi(b.y);
-            acc += bf16lo(a.z) * bf16lo(b.z); acc += bf16hi(a.z) * bf16hi(b.z);
-            acc += bf16lo(a.w) * bf16lo(b.w); acc += bf16hi(a.w) * bf16hi(b.w);
+    float acc[MR] = {};
+    if (((K | ldx) & 7) == 0 && ((((uintptr_t)x) | ((uintptr_t)w)) & 15) == 0) {
+        constexpr int UN = MR == 1 ? 1 : 4;
+#pragma unroll 4
+        for (int k0 = lane * 8; k0 < K; k0 += 256 * UN) {
+            uint4 b[UN];
+#pragma unroll
+            for (int u = 0; u < UN; ++u)
+                b[u] = k0 + u * 256 < K ? *reinterpret_cast<const uint4*>(wr + k0 + u * 256) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < UN; ++u) {
+                if (k0 + u * 256 >= K) break;
+#pragma unroll
+                for (int i = 0; i < MR; ++i) {
+                    const uint4 a = *reinterpret_cast<const uint4*>(xr[i] + k0 + u * 256);
+                    acc[i] += bf16lo(a.x) * bf16lo(b[u].x); acc[i] += bf16hi(a.x) * bf16hi(b[u].x);
+                    acc[i] += bf16lo(a.y) * bf16lo(b[u].y); acc[i] += bf16hi(a.y) * bf16hi(b[u].y);
+                    acc[i] += bf16lo(a.z) * bf16lo(b[u].z); acc[i] += bf16hi(a.z) * bf16hi(b[u].z);
+                    acc[i] += bf16lo(a.w) * bf16lo(b[u].w); acc[i] += bf16hi(a.w) * bf16hi(b[u].w);
+                }
+            }
         }
     } else {
-        for (int k = lane; k < K; k += 32) acc += bf16_to_f32(xr[k]) * bf16_to_f32(wr[k]);
+        for (int k = lane; k < K; k += 32)
+#pragma unroll
+            for (int i = 0; i < MR; ++i) acc[i] += bf16_to_f32(xr[i][k]) * bf16_to_f32(wr[k]);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-        float v = acc;
-        if (bias) v = bf16_round(v) + bf16_to_f32(bias[n]);
-        y[(size_t)m * ldy + n] = f32_to_bf16(v);
+    for (int i = 0; i < MR; ++i) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        if (lane == 0 && m0 + i < M) {
+            float v = acc[i];
+            if (bias) v = bf16_round(v) + bf16_to_f32(bias[n]);
+            y[(size_t)(m0 + i) * ldy + n] = f32_to_bf16(v);
+        }
     }
 }
 
@@ -702,13 +1039,13 @@ bool func_attr_once(std::atomic<uint64_t>& done, const void* func, int smem_byte
     return true;
 }
 
-// 0: single-CTA tiles only; 1 (default): 256-wide tiles of the large-M families run on CTA pairs; 2: SwiGLU family too
+// 0: single-CTA tiles only; else CTA pairs where tile_form() finds them the better form (the default)
 static int g_pair_mode = -1;
 void gemm_pair_mode(int mode) { g_pair_mode = mode; }
 static bool pair_wanted() {
     if (g_pair_mode < 0) {
         const char* e = getenv("O1_GEMM_PAIR");
-        g_pair_mode = (e && e[0] == '0') ? 0 : ((e && e[0] == '2') ? 2 : 1);
+        g_pair_mode = (e && e[0] == '0') ? 0 : 1;
     }
     return g_pair_mode != 0;
 }
@@ -745,8 +1082,8 @@ static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const C
     }
     if (pairs > tiles) pairs = tiles;
     prof_before(EPI == EPI_QKV ? (int)EPI_STORE : EPI, 2.0 * g.M * (double)g.N * g.K * (EPI == EPI_SWIGLU ? 2.0 : 1.0), st);
-    cfg.gridDim = dim3(2 * pairs);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, *tA, *tB, *tB2, tB3 ? *tB3 : *tB2, g);
+    cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 2, g.M, *tA, *tB, *tB2,
+                                   tB3 ? *tB3 : *tB2, g);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (pair): launch: %s", cudaGetErrorString(e)); return false; }
@@ -774,19 +1111,26 @@ int gemm_pair_capacity() {
     return n;
 }
 
+// Which persistent form takes the fewest (rounds of tiles) x (time of a K block): one CTA per 128 x 128 or 128 x 256 tile,
+// or a pair of CTAs per 256 x 256 tile.  The sums are the same in all of them.  A round of tiles with K = 4096 takes 15.6,
+// 29 and 25 us; measured at 4096 columns: 593 rows 32.4 / 31.7 / 30.2 us, 1280 rows 48.8 / 58.0 / 51.4, 2242 rows 72.6 /
+// 63.6 / 56.6, and at 6144 columns (q | k | v) 296 rows 24.6 / 38.6 / 40.1, 1280 rows 66.4 / 60.5 / 53.0.  Gate | up as
+// pairs instead of one CTA per 128 x 256 tile: 1280 rows 213 / 186 us, a block of 16640 rows 9.24 / 9.02 ms.
+enum TileForm { TILE_128, TILE_256, TILE_PAIR };
+static constexpr int TILE_COST[3] = {31, 58, 50};
+static TileForm tile_form(int num_m, int N, bool wide_ok, bool pair_ok) {
+    if (!wide_ok) return TILE_128;
+    const long sms = sm_count();
+    auto cost = [&](TileForm f, long tiles, long at_once) { return (tiles + at_once - 1) / at_once * TILE_COST[f]; };
+    const long c128 = cost(TILE_128, (long)num_m * (N / 128), sms), c256 = cost(TILE_256, (long)num_m * (N / 256), sms);
+    const long cp = pair_ok && pair_wanted() ? cost(TILE_PAIR, (long)((num_m + 1) / 2) * (N / 256), sms / 2) : c256 + 1;
+    if (cp <= c256 && cp <= c128) return TILE_PAIR;
+    return c256 <= c128 ? TILE_256 : TILE_128;
+}
+
 template <int EPI, int BN>
 static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2,
                       GemmArgs& g, cudaStream_t st, const CUtensorMap* tB3 = nullptr) {
-    // CTA pairs for the families that carry the large-M work, when there are at least two rounds of pair tiles.
-    // Measured at 16640 rows, stand-alone: o_proj 1306 -> 1384, down 1348 -> 1423, q|k|v 1315 -> 1391, head 1203 -> 1235
-    // TFLOP/s; gate|up + SwiGLU 1438 -> 1358, so that family keeps one CTA per tile.
-    if constexpr (BN == 256 && (EPI == EPI_STORE || EPI == EPI_BIAS || EPI == EPI_RESID || EPI == EPI_QKV)) {
-        if (pair_wanted() && ((g.num_m + 1) / 2) * g.num_n >= sm_count()) return launch_tc_pair<EPI>(tA, tB, tB2, g, st, tB3);
-    }
-    // mode 2: gate|up + SwiGLU too (in the power-capped step 1403 -> 1380 TFLOP/s for that family, step time unchanged)
-    if constexpr (BN == 256 && EPI == EPI_SWIGLU) {
-        if (pair_wanted() && g_pair_mode == 2 && ((g.num_m + 1) / 2) * g.num_n >= sm_count()) return launch_tc_pair<EPI>(tA, tB, tB2, g, st, tB3);
-    }
     using Cfg = GemmCfg<BN>;
     static std::atomic<uint64_t> attr_done{0};
     auto kern = gemm_tc_kernel<EPI, BN, false>;
@@ -795,11 +1139,63 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
     int grid = sm_count();
     if (grid > tiles) grid = tiles;
     prof_before((EPI == EPI_QKNORM || EPI == EPI_QKV) ? (int)EPI_STORE : (EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : ((EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID) ? (int)EPI_RESID : EPI)), 2.0 * g.M * (double)g.N * g.K * (EPI == EPI_SWIGLU ? 2.0 : 1.0), st);
-    kern<<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(*tA, *tB, *tB2, tB3 ? *tB3 : *tB2, g);
+    cudaError_t e = launch_chained(kern, dim3(grid), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 1, g.M, *tA, *tB, *tB2,
+                                   tB3 ? *tB3 : *tB2, g);
     prof_after(st);
-    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm: launch: %s", cudaGetErrorString(e)); return false; }
     return true;
+}
+
+// Which form of gemm_split_kernel a problem takes: tile width and CTAs per tile; width 0: the persistent kernel is the
+// better one.  Times in us, persistent kernel with 128-column tiles against this one:
+//  * 32 columns where that makes at most two CTAs per SM:    77 x 4096 x 4096 19.4 / 17.2, 520 x 1152 x 1152 11.1 / 8.7,
+//    130 x 4608 x 4608 23.9 / 20.0; beyond, the activations are read too often: 296 x 4096 x 4096 19.6 / 31.6
+//  * 96 columns where the wider tiles need a second round and these do not, and K is short: 2916 x 1152 x 1152 16.0 / 12.5,
+//    520 x 4304 x 1152 16.4 / 14.1; 593 x 4096 x 12288 86 / 84, where CTA pairs take 72
+//  * K over a cluster where even narrow tiles leave a long main loop: 520 x 1152 x 4304 23.5 / 18.7 (five CTAs, 32 columns
+//    27.2), 96 x 1152 x 4304 22.2 / 12.9 (six; 16.2); with 64 tiles and more 32 columns are as good (130 x 4096 x 4608)
+struct SplitPlan { int bn, ks; };
+static SplitPlan split_plan(int M, int N, int K, bool may_split) {
+    const int sms = sm_count(), kblocks = (K + BK - 1) / BK;
+    const long num_m = (M + BM - 1) / BM;
+    auto tiles = [&](int bn) { return num_m * ((N + bn - 1) / bn); };
+    if (may_split && kblocks >= 32 && tiles(128) * 3 <= sms) {
+        const long ks = sms * 8 / 5 / tiles(128);
+        return {128, ks > 6 ? 6 : (int)ks};
+    }
+    if (tiles(32) <= 2 * sms) return {32, 1};
+    if (K <= 2048 && tiles(128) > sms && tiles(96) <= 2 * sms) return {96, 1};
+    return {0, 0};
+}
+
+template <int EPI, int BN>
+static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmArgs& g, int ks, cudaStream_t st) {
+    static std::atomic<uint64_t> attr_done{0};
+    constexpr int SMEM = SplitCfg<BN>::SMEM;
+    auto kern = gemm_split_kernel<EPI, BN>;
+    if (!func_attr_once(attr_done, (const void*)kern, SMEM, "gemm (few tiles)")) return false;
+    g.num_n = (g.N + BN - 1) / BN;
+    g.prefetch = SK_PREFETCH;
+    prof_before((EPI == EPI_BIAS_GELU || EPI == EPI_VROPE) ? (int)EPI_BIAS
+                                                           : ((EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID) ? (int)EPI_RESID : EPI),
+                2.0 * g.M * (double)g.N * g.K, st);
+    cudaError_t e = launch_chained(kern, dim3(g.num_m * g.num_n * ks), dim3(GEMM_THREADS), SMEM, st, ks, g.M, *tA, *tB, g, ks);
+    prof_after(st);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("gemm (few tiles): launch: %s", cudaGetErrorString(e)); return false; }
+    return true;
+}
+
+template <int EPI>
+static bool launch_split(const CUtensorMap* tA, const void* w, GemmArgs& g, SplitPlan p, cudaStream_t st) {
+    CUtensorMap mB;
+    if (!cached_tmap(&mB, w, g.N, g.K, g.K, p.bn)) return false;
+    switch (p.bn) {
+        case 32: return launch_split_bn<EPI, 32>(tA, &mB, g, p.ks, st);
+        case 96: return launch_split_bn<EPI, 96>(tA, &mB, g, p.ks, st);
+        default: return launch_split_bn<EPI, 128>(tA, &mB, g, p.ks, st);
+    }
 }
 
 bool gemm_tc_supported(int M, int N, int K, int epi) {
@@ -846,12 +1242,13 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
     }
     if (!gemm_tc_supported(M, N, K, epi)) {
         if (epi != EPI_STORE && epi != EPI_BIAS) { set_error("gemm: shape unsupported for fused epilogue"); return false; }
-        dim3 block(128);
-        dim3 grid((N + 3) / 4, M);
-        gemm_simt_kernel<<<grid, block, 0, st>>>((const uint16_t*)x, (const uint16_t*)w,
-                                                 (const uint16_t*)(epi == EPI_BIAS ? bias : nullptr), (uint16_t*)y, M, N, K,
-                                                 ldx, ldy);
-        cudaError_t e = cudaGetLastError();
+        const uint16_t* b = (const uint16_t*)(epi == EPI_BIAS ? bias : nullptr);
+        const dim3 block(128);
+        const cudaError_t e =
+            M == 1 ? launch_chained(gemm_simt_kernel<1>, dim3((N + 3) / 4, 1), block, 0, st, 1, M, (const uint16_t*)x,
+                                    (const uint16_t*)w, b, (uint16_t*)y, M, N, K, ldx, ldy)
+                   : launch_chained(gemm_simt_kernel<4>, dim3((N + 3) / 4, (M + 3) / 4), block, 0, st, 1, M, (const uint16_t*)x,
+                                    (const uint16_t*)w, b, (uint16_t*)y, M, N, K, ldx, ldy);
         if (e != cudaSuccess) { set_error("gemm(simt): launch: %s", cudaGetErrorString(e)); return false; }
         return true;
     }
@@ -863,13 +1260,13 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
         set_error("gemm: the bias / gate + residual epilogues need both operands, 16-byte aligned");
         return false;
     }
-    GemmArgs g;
+    GemmArgs g = {};
     g.M = M; g.N = N; g.K = K;
     g.out = (uint16_t*)y; g.ldo = ldy;
     g.bias = (const uint16_t*)bias;
     g.resid = (const uint16_t*)resid; g.ldr = ldr;
     g.scale = scale;
-    g.rope = nullptr;
+    g.rope = g.rope_sin = nullptr;
     if (epi == EPI_QKNORM) {
         // resid carries the cos|sin table, bias the norm weight; every 128 output columns are one head
         if (!bias || !resid || (N % 128) != 0 || (o_cb && (o_cb % 128) != 0) || (((uintptr_t)bias) & 15) ||
@@ -914,22 +1311,43 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
     const CUtensorMap *tA = &mA, *tB = &mB, *tB2 = &mB2;
 
     if (epi == EPI_SWIGLU) {
+        // (2N columns of gate and up)
         g.num_n = N / 128;
+        if (force_bn <= 0 && tile_form(g.num_m, 2 * N, true, true) == TILE_PAIR)
+            return launch_tc_pair<EPI_SWIGLU>(tA, tB, tB2, g, st, nullptr);
         return launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
     }
-    int bn = 256;
-    if ((N % 256) != 0 || (o_cb && (o_cb % 256) != 0)) bn = 128;
-    else {
-        // small problems: halve the tile to fill the SMs
-        const int tiles256 = g.num_m * (N / 256);
-        if (tiles256 < 2 * sm_count()) bn = 128;
+    if (force_bn <= 0 && !o_cb && !o_tab) {
+        const SplitPlan p = split_plan(M, N, K, force_bn == GEMM_SPLIT_K);
+        if (p.bn > 0) switch (epi) {
+            case EPI_STORE: return launch_split<EPI_STORE>(tA, w, g, p, st);
+            case EPI_BIAS:  return launch_split<EPI_BIAS>(tA, w, g, p, st);
+            case EPI_RESID: return launch_split<EPI_RESID>(tA, w, g, p, st);
+            case EPI_BIAS_GELU: return launch_split<EPI_BIAS_GELU>(tA, w, g, p, st);
+            case EPI_BIAS_RESID: return launch_split<EPI_BIAS_RESID>(tA, w, g, p, st);
+            case EPI_GATE_RESID: return launch_split<EPI_GATE_RESID>(tA, w, g, p, st);
+        }
     }
+    const bool wide_ok = (N % 256) == 0 && (!o_cb || (o_cb % 256) == 0);
+    const bool pair_ok = epi == EPI_STORE || epi == EPI_BIAS || epi == EPI_RESID;
+    TileForm form = tile_form(g.num_m, N, wide_ok, pair_ok);
     if (force_bn == 128 || force_bn == 256) {
-        if (force_bn == 256 && ((N % 256) != 0 || (o_cb && (o_cb % 256) != 0))) {
+        if (force_bn == 256 && !wide_ok) {
             set_error("gemm: BN=256 needs N (and the output column block) %% 256 == 0");
             return false;
         }
-        bn = force_bn;
+        // (a forced width of 256 is the pair form where that family has two rounds of its tiles)
+        form = force_bn == 128 ? TILE_128
+                               : (pair_ok && pair_wanted() && ((g.num_m + 1) / 2) * (N / 256) >= sm_count() ? TILE_PAIR : TILE_256);
+    }
+    const int bn = form == TILE_128 ? 128 : 256;
+    if (form == TILE_PAIR) {
+        g.num_n = N / 256;
+        switch (epi) {
+            case EPI_STORE: return launch_tc_pair<EPI_STORE>(tA, tB, tB2, g, st, nullptr);
+            case EPI_BIAS:  return launch_tc_pair<EPI_BIAS>(tA, tB, tB2, g, st, nullptr);
+            default:        return launch_tc_pair<EPI_RESID>(tA, tB, tB2, g, st, nullptr);
+        }
     }
     g.num_n = (N + bn - 1) / bn;
     if (bn == 256) {
@@ -980,12 +1398,12 @@ bool gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void
         set_error("gemm_qkv: bad destination tables");
         return false;
     }
-    GemmArgs g;
+    GemmArgs g = {};
     g.M = M; g.N = N; g.K = K;
     g.out = (uint16_t*)y; g.ldo = ldy;
     g.bias = (const uint16_t*)q_norm;
     g.resid = nullptr; g.ldr = 0;
-    g.rope = cs;
+    g.rope = cs; g.rope_sin = nullptr;
     g.scale = eps;
     g.err = device_error_word();
     g.num_m = (M + BM - 1) / BM;
@@ -1015,10 +1433,30 @@ bool gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void
     // 256-wide tiles need every segment (and every destination block) to be a multiple of 256 columns
     bool wide = (qc % 256) == 0 && (kc % 256) == 0;
     if (tabs && (((qc / n_dst) % 256) != 0 || ((kc / n_dst) % 256) != 0)) wide = false;
-    if (wide && g.num_m * (N / 256) < 2 * sm_count()) wide = false;
-    const int bn = wide ? 256 : 128;
-    g.num_n = N / bn;
-    return wide ? launch_tc<EPI_QKV, 256>(&mA, &mQ, &mK, g, st, &mV) : launch_tc<EPI_QKV, 128>(&mA, &mQ, &mK, g, st, &mV);
+    const TileForm form = tile_form(g.num_m, N, wide, true);
+    g.num_n = N / (form == TILE_128 ? 128 : 256);
+    if (form == TILE_PAIR) return launch_tc_pair<EPI_QKV>(&mA, &mQ, &mK, g, st, &mV);
+    return form == TILE_256 ? launch_tc<EPI_QKV, 256>(&mA, &mQ, &mK, g, st, &mV) : launch_tc<EPI_QKV, 128>(&mA, &mQ, &mK, g, st, &mV);
+}
+
+bool gemm_vision_qkv(const void* x, const void* w, const void* b, void* y, int M, const float* cosd, const float* sind,
+                     cudaStream_t st) {
+    constexpr int K = 1152, N = 3456;
+    if (!x || !w || !b || !y || !cosd || !sind || M < 8 ||
+        ((((uintptr_t)b) | ((uintptr_t)y) | ((uintptr_t)cosd) | ((uintptr_t)sind)) & 15)) {
+        set_error("gemm_vision_qkv: bad args");
+        return false;
+    }
+    GemmArgs g = {};
+    g.M = M; g.N = N; g.K = K;
+    g.out = (uint16_t*)y; g.ldo = 3 * 16 * 128;
+    g.bias = (const uint16_t*)b;
+    g.rope = cosd; g.rope_sin = sind;
+    g.num_m = (M + BM - 1) / BM;
+    g.err = device_error_word();
+    CUtensorMap mA, mB;
+    if (!cached_tmap(&mA, x, M, K, K, 128) || !cached_tmap(&mB, w, N, K, K, VQ_BN)) return false;
+    return launch_split_bn<EPI_VROPE, VQ_BN>(&mA, &mB, g, 1, st);
 }
 
 }  // namespace o1

@@ -16,8 +16,10 @@ namespace o1 {
 // EPI_BIAS_RESID: bf16(resid + bf16(bf16(acc) + bias)): a biased projection followed by the residual add
 // EPI_GATE_RESID: bf16(resid + bf16(gate[col] * bf16(acc))), the gate vector passed as `bias` (adaLN block variant)
 // EPI_QKV: q | k | v projections in one launch (gemm_qkv): EPI_QKNORM on the q and k column tiles, EPI_STORE on the v tiles
+// EPI_VROPE: the vision tower's q | k | v projection (gemm_vision_qkv): bias, fp32 rotary on the q and k heads, heads of 72
+// columns stored 128 apart
 enum Epi { EPI_STORE = 0, EPI_BIAS = 1, EPI_RESID = 2, EPI_SWIGLU = 3, EPI_LORA = 4, EPI_QKNORM = 6, EPI_BIAS_GELU = 7,
-           EPI_BIAS_RESID = 8, EPI_GATE_RESID = 9, EPI_QKV = 10 };
+           EPI_BIAS_RESID = 8, EPI_GATE_RESID = 9, EPI_QKV = 10, EPI_VROPE = 11 };
 
 // ---- engine.cu: optional per-launch event timing of the tensor-core kernels.
 // kind: 0..4 = GEMM by epilogue (Epi), 5 = flash attention.  Costs two event
@@ -27,6 +29,11 @@ void prof_before(int kind, double work, cudaStream_t st);
 void prof_after(cudaStream_t st);
 
 // ---- gemm_tc.cu
+// force_bn: 0 = tile chosen by shape, 128 / 256 = that tile width; every output element is summed by one CTA in the order
+// of k, so that a row's result does not depend on the tile or on how many other rows the call has (the decoder's layers
+// rely on that: a row is the same in a sharded, a cached or a paired pass).  GEMM_SPLIT_K = chosen by shape, and a problem
+// of few tiles may share a tile's K among CTAs, which is another order of the FP32 sum.
+enum { GEMM_SPLIT_K = -1 };
 bool gemm_bf16(const void* x, const void* w, const void* w2, void* y, int M, int N, int K, int epi,
                const void* bias, const void* resid, float scale, int force_bn, cudaStream_t st);
 // Same, with explicit row pitches (elements) for x and y so that a GEMM can
@@ -45,6 +52,10 @@ bool gemm_tc_supported(int M, int N, int K, int epi);
 bool gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void* wv, void* y, int ldy, int M, int qc,
               int kc, int K, const void* q_norm, const void* k_norm, const float* cs, float eps, int n_dst,
               void* const* tq, void* const* tk, void* const* tv, cudaStream_t st);
+// vision tower: y[M, 3 * 16 * 128] = rotary(x wqkv^T + b) with x [M,1152], wqkv [3456,1152]; heads of 72 columns are stored
+// 128 apart, columns 72..79 as zero, 80..127 untouched; cosd / sind [M,72] fp32
+bool gemm_vision_qkv(const void* x, const void* w, const void* b, void* y, int M, const float* cosd, const float* sind,
+                     cudaStream_t st);
 // copies the (cached) tensor map of a row-major bf16 matrix into *out; false + error text on failure
 bool cached_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                  uint32_t box_rows);
@@ -62,15 +73,22 @@ bool flash_attention(const void* q, int ldq, const void* k, int ldk, const void*
                      void* out, int ldo, int S, int heads, int kv_heads, int ar_len, float scale,
                      cudaStream_t st, void* scratch = nullptr, size_t scratch_bytes = 0);
 
+// n sequences (1 or 2) behind one another, as one launch where that is possible; see attn_tc.cu
+bool flash_attention_rows(const uint16_t* qkv, int ld, void* out, int ldo, const int* rows, const int* ar_len, int n, int heads,
+                          int kv_heads, float scale, cudaStream_t st, void* scratch, size_t scratch_row);
+
 // [row_lo, row_hi): the query rows to compute and write (row_hi < 0: all rows)
 bool flash_attention_hm(const void* q, const void* k, const void* v, void* out, int S, int heads,
                         int kv_heads, int ar_len, float scale, bool out_head_major, cudaStream_t st,
                         int row_lo = 0, int row_hi = -1);
+// the vision tower's attention: 16 heads of 72 columns stored 128 apart (columns 72..79 zero) in qkv [S, 3 * 16 * 128],
+// every row sees every key; out [S, 16 * 72]
+bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cudaStream_t st);
 // tail split policy of flash_attention*: 0 = automatic, 1 = never, n = n key-range parts when they fit
 void attention_tail_ways(int ways);
 void attention_tile_mode(int mode);   // 0: by sequence length; 1: two query tiles per CTA; 2: one query tile per CTA
 int gemm_pair_capacity();
-void gemm_pair_mode(int mode);   // 0: single-CTA GEMM tiles only; 1: CTA pairs (cta_group::2) for the large-M families
+void gemm_pair_mode(int mode);   // 0: single-CTA GEMM tiles only; else CTA pairs (cta_group::2) where they are the better form
 // seq-major operands; output rows [b*out_rows, (b+1)*out_rows) go to out_tab[b] (row-major, leading
 // dimension ldo), which may be peer-mapped memory of another GPU
 bool flash_attention_tab(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,

@@ -461,6 +461,61 @@ def test_gemm_on_cta_pairs_equals_single_cta_tiles(pkg, dev, M, N, K, epi):
     assert err < 1e-2, err     # the pair form really computed the product (fp32 reference, bf16 rounding of the result)
 
 
+def check_linear_f64(y, x, w, bias, what):
+    """y against 64 bits: an FP32 sum of K products in any order is within K * 2^-23 * sum|x||w| of the exact one, and the
+    two bf16 roundings (of the sum, of the sum plus bias) are monotonic, so the result lies between the rounded ends."""
+    acc = x.double() @ w.double().t()
+    bound = (x.double().abs() @ w.double().abs().t()) * x.shape[1] * 2.0 ** -23
+    lo, hi = (acc - bound).bfloat16().double(), (acc + bound).bfloat16().double()
+    if bias is not None:
+        lo, hi = (lo + bias.double()).bfloat16().double(), (hi + bias.double()).bfloat16().double()
+    bad = ((y.double() < lo) | (y.double() > hi)).sum().item()
+    assert bad == 0, f"{what}: {bad} of {y.numel()} outside the rounding interval"
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 7, 8, 33, 127, 128, 129, 300, 517])
+@pytest.mark.parametrize("N,K", [(72, 40), (128, 64), (1032, 200), (4096, 256), (96, 4104), (1152, 1160)])
+def test_linear_of_few_tiles(pkg, dev, M, N, K):
+    """hd_linear where there are few output tiles: the row kernel below eight rows, then tiles of 32 / 64 / 96 / 128
+    columns, with a ragged last tile, a ragged last K block and fewer K blocks than stages; nothing is written behind."""
+    g = torch.Generator(device=dev).manual_seed(M * 7 + N + K)
+    x, w, b = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16() for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5)))
+    for bias in (b, None):
+        y = torch.full((M + 1, N), 777.0, dtype=torch.bfloat16, device=dev)
+        pkg.lib.hd_linear(pkg.ptr(x), pkg.ptr(w), pkg.ptr(bias), pkg.ptr(y), M, N, K, 1)
+        done(pkg, "linear")
+        check_linear_f64(y[:M], x, w, bias, f"linear {M}x{N}x{K}")
+        assert (y[M:] == 777.0).all(), "rows beyond M were written"
+    assert pkg.lib.o1_device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(96, 1152, 1152), (520, 1152, 4304), (130, 4608, 4608), (20, 4304, 1152), (9, 72, 520), (300, 128, 2048)])
+@pytest.mark.parametrize("epi", [0, 1, 2, 8, 9])
+def test_gemm_with_k_split_over_a_cluster(pkg, dev, M, N, K, epi):
+    """A tile's K shared by 1 to 8 CTAs (force_bn = -1), every epilogue that takes the form, against the whole-K tile:
+    the FP32 sums differ by their order only, so the results are equal or neighbours."""
+    if epi in (2, 8, 9) and N % 128:
+        pytest.skip("the residual epilogues take whole 128-column tiles")
+    g = torch.Generator(device=dev).manual_seed(M + N + K + epi)
+    x, w, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
+                  for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
+    ys = []
+    for bn in (-1, 0):
+        y = torch.full((M + 1, N), 777.0, dtype=torch.bfloat16, device=dev)
+        rc = pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N, M, N, K, epi, pkg.ptr(b), pkg.ptr(r), N, 0.0, bn)
+        assert rc == 0, pkg.last_error()
+        done(pkg, "gemm")
+        assert (y[M:] == 777.0).all(), "rows beyond M were written"
+        ys.append(y[:M])
+    if epi < 2:
+        check_linear_f64(ys[0], x, w, b if epi else None, "split")
+    # one bf16 step of the sum, carried through the epilogue: 2^-7 of the largest term
+    scale = (x.float() @ w.float().t()).abs() * (b.abs().float() if epi == 9 else 1.0) + b.abs().float() + r.abs().float() + 1e-3
+    assert ((ys[0].float() - ys[1].float()).abs() <= scale * 2.0 ** -6).all()
+    assert (ys[0] != ys[1]).float().mean() < 0.02
+    assert pkg.lib.o1_device_error() == 0
+
+
 @pytest.mark.parametrize("sigma", [0.857, 1.0, 0.008, 1.0 / 3.0, 0.99999994, 3e-10, 1e-12, 2e9, 1e30])
 @pytest.mark.parametrize("n", [8, 4096 * 8, 1003])
 def test_fused_step_equals_the_chain_for_every_kind_of_value(pkg, dev, sigma, n):
