@@ -37,50 +37,53 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // ------------------------------------------------------------------ RMSNorm
 // y = bf16( (w * x) * rsqrt(mean(x^2) + eps) ), fp32 inside (norm.cu:12-48).
-// One row per block; each thread keeps its slice of the row in registers
-// between the reduction and the scaling pass, so HBM sees one read + one write.
+// One row per block; each thread keeps its slice of the row and of the weight in registers, requested together before
+// the reduction, so HBM sees one read + one write and the chain of a row is one load, one barrier (every thread adds the
+// four warps' sums itself, in the order of a shuffle tree) and one store.
 template <int THREADS, int VEC_PER_THREAD>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_vec_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w,
                    uint16_t* __restrict__ y, int rows, int cols, float eps,
                    const uint16_t* __restrict__ scale, const uint16_t* __restrict__ shift) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int row = blockIdx.x;
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * cols);
     uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * cols);
     const uint4* wr = reinterpret_cast<const uint4*>(w);
     const int nvec = cols >> 3;
-    uint4 xv[VEC_PER_THREAD];
-    float sq = 0.f;
+    uint4 xv[VEC_PER_THREAD], wv[VEC_PER_THREAD];
 #pragma unroll
     for (int i = 0; i < VEC_PER_THREAD; ++i) {
         const int idx = threadIdx.x + i * THREADS;
-        if (idx < nvec) {
-            xv[i] = xr[idx];
+        if (idx < nvec) { xv[i] = xr[idx]; wv[i] = wr[idx]; }
+    }
+    float sq = 0.f;
+#pragma unroll
+    for (int i = 0; i < VEC_PER_THREAD; ++i) {
+        if (threadIdx.x + i * THREADS < nvec) {
             float f[8];
             unpack8(xv[i], f);
 #pragma unroll
             for (int j = 0; j < 8; ++j) sq += f[j] * f[j];
         }
     }
-    __shared__ float red[THREADS / 32];
-    __shared__ float inv_s;
     sq = warp_sum(sq);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float t = (threadIdx.x < THREADS / 32) ? red[threadIdx.x] : 0.f;
-        t = warp_sum(t);
-        if (threadIdx.x == 0) inv_s = rsqrtf(t / (float)cols + eps);
+    static_assert(THREADS == 32 || THREADS == 128, "one or four warps");
+    if (THREADS > 32) {
+        __shared__ float red[THREADS / 32];
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
+        __syncthreads();
+        sq = (red[0] + red[2]) + (red[1] + red[3]);
     }
-    __syncthreads();
-    const float inv = inv_s;
+    const float inv = rsqrtf(sq / (float)cols + eps);
 #pragma unroll
     for (int i = 0; i < VEC_PER_THREAD; ++i) {
         const int idx = threadIdx.x + i * THREADS;
         if (idx < nvec) {
             float f[8], g[8];
             unpack8(xv[i], f);
-            unpack8(wr[idx], g);
+            unpack8(wv[i], g);
 #pragma unroll
             for (int j = 0; j < 8; ++j) f[j] = g[j] * f[j] * inv;
             if (scale) {   // adaLN variant: the stored norm output, then * (1 + scale) + shift (NULL = o1.c's block)
@@ -124,12 +127,15 @@ bool rmsnorm_mod(const void* x, const void* w, const void* scale, const void* sh
     if (!x || !w || !y || rows <= 0 || cols <= 0 || (!scale != !shift)) { set_error("rmsnorm: bad args"); return false; }
     const bool aligned = ((((uintptr_t)x) | ((uintptr_t)y) | ((uintptr_t)w) | ((uintptr_t)scale) | ((uintptr_t)shift)) & 15) == 0;
     const uint16_t *sc = (const uint16_t*)scale, *sh = (const uint16_t*)shift;
-    if (aligned && (cols % 8) == 0 && cols <= 128 * 8 * 8 && cols > 1024) {
-        rmsnorm_vec_kernel<128, 8><<<rows, 128, 0, st>>>((const uint16_t*)x, (const uint16_t*)w,
-                                                         (uint16_t*)y, rows, cols, eps, sc, sh);
+    if (aligned && (cols % 8) == 0 && cols <= 128 * 4 * 8 && cols > 1024) {
+        launch_chained(rmsnorm_vec_kernel<128, 4>, dim3(rows), dim3(128), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
+                       (uint16_t*)y, rows, cols, eps, sc, sh);
+    } else if (aligned && (cols % 8) == 0 && cols <= 128 * 8 * 8 && cols > 1024) {
+        launch_chained(rmsnorm_vec_kernel<128, 8>, dim3(rows), dim3(128), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
+                       (uint16_t*)y, rows, cols, eps, sc, sh);
     } else if (aligned && (cols % 8) == 0 && cols <= 1024) {
-        rmsnorm_vec_kernel<32, 4><<<rows, 32, 0, st>>>((const uint16_t*)x, (const uint16_t*)w,
-                                                       (uint16_t*)y, rows, cols, eps, sc, sh);
+        launch_chained(rmsnorm_vec_kernel<32, 4>, dim3(rows), dim3(32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
+                       (uint16_t*)y, rows, cols, eps, sc, sh);
     } else {
         const int wpb = 4;
         rmsnorm_generic_kernel<<<(rows + wpb - 1) / wpb, wpb * 32, 0, st>>>(
@@ -353,6 +359,8 @@ bool mrope_cos_sin(const float* pos, int bs, int seq, const int64_t* section, in
 // Layer-invariant, so it is built once per forward instead of once per block.
 __global__ void mrope_table64_kernel(const float* __restrict__ pos, float* __restrict__ cs, int seq,
                                      float theta, int pos_stride) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int s = blockIdx.x * 4 + (threadIdx.x >> 6);
     const int kk = threadIdx.x & 63;
     if (s >= seq) return;
@@ -368,14 +376,14 @@ __global__ void mrope_table64_kernel(const float* __restrict__ pos, float* __res
 }
 bool mrope_table64(const float* pos, int seq, float theta, float* cs, cudaStream_t st) {
     if (!pos || !cs || seq <= 0) { set_error("mrope_table: bad args"); return false; }
-    mrope_table64_kernel<<<(seq + 3) / 4, 256, 0, st>>>(pos, cs, seq, theta, seq);
+    launch_chained(mrope_table64_kernel, dim3((seq + 3) / 4), dim3(256), 0, st, 1, seq, pos, cs, seq, theta, seq);
     O1_LAUNCH_CHECK("mrope_table");
     return true;
 }
 bool mrope_table64_rows(const float* pos, int pos_stride, int row0, int rows, float theta, float* cs,
                         cudaStream_t st) {
     if (!pos || !cs || rows <= 0 || row0 < 0 || row0 + rows > pos_stride) { set_error("mrope_table: bad args"); return false; }
-    mrope_table64_kernel<<<(rows + 3) / 4, 256, 0, st>>>(pos + row0, cs, rows, theta, pos_stride);
+    launch_chained(mrope_table64_kernel, dim3((rows + 3) / 4), dim3(256), 0, st, 1, rows, pos + row0, cs, rows, theta, pos_stride);
     O1_LAUNCH_CHECK("mrope_table");
     return true;
 }
