@@ -151,7 +151,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     float* xch = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 192);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
     int item = blockIdx.x, part = 0, ways = 1;
     if (item >= a.n_plain) {
@@ -163,7 +163,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const int h = item / a.nqb;
     const int q0 = (item - h * a.nqb) * AQ2;
     const int kh = h / (a.heads / a.kv_heads);
-    if (q0 + AQ2 <= a.row_lo || q0 >= a.row_hi) return;   // no row of this block is wanted (whole CTA, before any set-up)
+    if (q0 + AQ2 <= a.row_lo || q0 >= a.row_hi) { grid_dep_wait(); return; }   // no row of this block is wanted (whole CTA, before any set-up)
 
     // keys this pair of query tiles can see (the second tile's range covers the first's)
     int kv_end = a.S;
@@ -174,6 +174,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const int n_tiles = (int)((long)(part + 1) * tiles_all / ways) - j0;  // and how many it covers
     if (n_tiles <= 0) {
         // a part of a tail item that has fewer key tiles than parts: an empty partial (max -inf, sum 0), nothing else
+        grid_dep_wait();
         if (threadIdx.x < AQ2) {
             const int slot = (item - a.n_plain) * ways + part;
             *reinterpret_cast<float2*>(a.part_ml + ((size_t)slot * AQ2 + threadIdx.x) * 2) = make_float2(-INFINITY, 0.f);
@@ -188,7 +189,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         *s_abort = ab;
     }
     __syncthreads();
-    if (*s_abort != 0) return;
+    if (*s_abort != 0) { grid_dep_wait(); return; }
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -205,13 +206,15 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_S = tmem_base;         // scores of the two groups: columns [0,128) and [128,256)
     const uint32_t tmem_O = tmem_base + 256;   // output accumulators of the two groups: [256,384), [384,512)
 
     if (warp == 0) {
         // -------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tmQ);
             tma_prefetch_desc(&tmK);
             tma_prefetch_desc(&tmV);
@@ -249,7 +252,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128, 0, 0);
             constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 128, 0, 1);  // V is MN-major
             bool ok = mbar_wait(q_full, 0);
@@ -519,9 +522,22 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity));
 }
 
-__global__ void __launch_bounds__(ATTN_THREADS, 1)
-flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                  const __grid_constant__ CUtensorMap tmV, const AttnArgs a) {
+// DH: columns of a head that hold data.  72 (the vision tower; heads stored 128 apart, columns 72..79 zero) takes five of
+// the eight K steps of Q K^T and 80 of the 128 output columns; what the second panels hold beyond that is never read.
+// NSEG: sequences in one launch (the two branches of a guided step: at 296 rows each has 96 work items for 148 SMs).  The
+// first grid0 CTAs belong to the first one.
+template <int NSEG>
+struct Attn1Params {
+    CUtensorMap q[NSEG], k[NSEG], v[NSEG];
+    AttnArgs a[NSEG];
+    int grid0;
+};
+template <int DH, int NSEG>
+__global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __grid_constant__ Attn1Params<NSEG> par) {
+    const int seg = NSEG > 1 && (int)blockIdx.x >= par.grid0 ? 1 : 0;
+    const AttnArgs& a = par.a[seg];
+    const CUtensorMap &tmQ = par.q[seg], &tmK = par.k[seg], &tmV = par.v[seg];
+    constexpr int DN = (DH + 15) & ~15;      // columns the MMAs work on
     // Q | K x3 | V x3: 7 tiles of 32 KB again, the window 1024-byte aligned (checked below)
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* q_s = smem;                               // the query tile
@@ -545,9 +561,9 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // in different places, and all eight warps of a set arrive on m_pub: an entry is not overwritten before it is read.
     uint16_t* m_sh = reinterpret_cast<uint16_t*>(xch + T1_XCH / 4);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
-    int item = blockIdx.x, part = 0, ways = 1;
+    int item = (int)blockIdx.x - (seg ? par.grid0 : 0), part = 0, ways = 1;
     if (item >= a.n_plain) {
         const int t = item - a.n_plain;
         item = a.n_plain + t / a.ways;
@@ -557,7 +573,7 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int h = item / a.nqb;
     const int q0 = (item - h * a.nqb) * T1_ROWS;
     const int kh = h / (a.heads / a.kv_heads);
-    if (q0 + T1_ROWS <= a.row_lo || q0 >= a.row_hi) return;   // no row of this block is wanted (whole CTA, before any set-up)
+    if (q0 + T1_ROWS <= a.row_lo || q0 >= a.row_hi) { grid_dep_wait(); return; }   // no row of this block is wanted (whole CTA, before any set-up)
 
     // keys this query tile can see
     int kv_end = a.S;
@@ -568,6 +584,7 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int n_tiles = (int)((long)(part + 1) * tiles_all / ways) - j0;  // and how many it covers
     if (n_tiles <= 0) {
         // a part of a tail item that has fewer key tiles than parts: an empty partial (max -inf, sum 0), nothing else
+        grid_dep_wait();
         if (threadIdx.x < T1_ROWS) {
             const int slot = (item - a.n_plain) * ways + part;
             *reinterpret_cast<float2*>(a.part_ml + ((size_t)slot * T1_ROWS + threadIdx.x) * 2) = make_float2(-INFINITY, 0.f);
@@ -582,7 +599,7 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         *s_abort = ab;
     }
     __syncthreads();
-    if (*s_abort != 0) return;
+    if (*s_abort != 0) { grid_dep_wait(); return; }
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -600,13 +617,15 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_S = tmem_base;         // three score buffers: columns [0,128), [128,256), [256,384)
     const uint32_t tmem_O = tmem_base + 384;   // output accumulator: [384,512)
 
     if (warp == 0) {
         // -------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&tmQ);
             tma_prefetch_desc(&tmK);
             tma_prefetch_desc(&tmV);
@@ -641,9 +660,9 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128, 0, 0);
-            constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 128, 0, 1);  // V is MN-major
+            constexpr uint32_t idesc_pv = umma_idesc_bf16(128, DN, 0, 1);  // V is MN-major
             bool ok = mbar_wait(q_full, 0);
             if (!ok) atomicExch(a.err, 13);
             const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s), 16, 1024);
@@ -656,7 +675,7 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 const uint64_t k_desc = umma_desc_sw128(smem_u32(k_s + st * TILE_BYTES), 16, 1024);
                 const int b = j % T1_S_BUFS;
 #pragma unroll
-                for (int kk = 0; kk < AD / 16; ++kk) {
+                for (int kk = 0; kk < DN / 16; ++kk) {
                     const uint64_t off = (uint64_t)(((kk >> 2) * PANEL_BYTES + (kk & 3) * 32) >> 4);
                     umma_ss(tmem_S + b * 128, q_desc + off, k_desc + off, idesc_qk, kk != 0);
                 }
@@ -784,7 +803,7 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 if (!mbar_wait_warp(&v_empty[(j - 1) % T1_V_STAGES], ((j - 1) / T1_V_STAGES) & 1)) { atomicExch(a.err, 21); ok = false; continue; }
                 tc_fence_after();
 #pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < 4 && half * 64 + c * 16 < DN; ++c) {
                     uint32_t o[16];
                     tmem_ld16(t_o + c * 16, o);
                     tmem_ld_wait();
@@ -878,7 +897,8 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 } else if (row_g < a.row_hi && row_g >= a.row_lo) {
                     uint4* d4 = reinterpret_cast<uint4*>(a.out + (size_t)row_g * a.ldo + (size_t)h * a.out_hoff + part4 * 32);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) d4[i] = pk[i];
+                    for (int i = 0; i < 4; ++i)
+                        if (part4 * 32 + i * 8 < DH) d4[i] = pk[i];
                 }
             }
         }
@@ -893,6 +913,8 @@ flash_attn1_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // Combines the partial results of the tail items: out = sum_i O_i 2^(m_i - M) / sum_i l_i 2^(m_i - M).
 // One block per query row, one thread per output column.
 __global__ void __launch_bounds__(AD) attn_merge_kernel(const AttnArgs a, int n_tail, int AQ2 /* rows per item */) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int ti = blockIdx.x / AQ2, r = blockIdx.x - ti * AQ2;
     if (ti >= n_tail) return;
     const int item = a.n_plain + ti;
@@ -961,10 +983,19 @@ static int choose_tail_ways(int total, int nsm, int min_tiles, size_t scratch_by
     return (worth && best_cost < 0.9) ? best : 1;
 }
 
-static bool flash_attention_impl(const void* q, int ldq, const void* k, int ldk, const void* v,
+// One sequence, ready to launch.
+struct AttnSetup {
+    CUtensorMap q, k, v;
+    AttnArgs a;
+    int grid, n_tail, rows_item;
+    bool one_tile;
+    double work;
+};
+
+static bool attention_setup(AttnSetup& s, const void* q, int ldq, const void* k, int ldk, const void* v,
                                  int ldv, void* out, int ldo, int S, int heads, int kv_heads,
                                  int ar_len, float scale, bool in_head_major, bool out_head_major,
-                                 cudaStream_t st, void* const* out_tab = nullptr, int out_rows = 0,
+                                 void* const* out_tab = nullptr, int out_rows = 0,
                                  void* scratch = nullptr, size_t scratch_bytes = 0, int row_lo = 0, int row_hi = -1) {
     if (out_tab) {
         if (out_rows <= 0 || (S + out_rows - 1) / out_rows > 8 || out_head_major) { set_error("attention: bad output table"); return false; }
@@ -979,26 +1010,20 @@ static bool flash_attention_impl(const void* q, int ldq, const void* k, int ldk,
     if ((ldo % 8) != 0 || (((uintptr_t)out) & 15)) { set_error("attention: output not 16-byte aligned"); return false; }
     if (ar_len < 0) ar_len = 0;
     if (ar_len > S) ar_len = S;
-    CUtensorMap mq, mk, mv;
     bool maps_ok;
     if (in_head_major) {
-        maps_ok = cached_tmap(&mq, q, (uint64_t)heads * S, AD, AD, 128) &&
-                  cached_tmap(&mk, k, (uint64_t)kv_heads * S, AD, AD, 128) &&
-                  cached_tmap(&mv, v, (uint64_t)kv_heads * S, AD, AD, 128);
+        maps_ok = cached_tmap(&s.q, q, (uint64_t)heads * S, AD, AD, 128) &&
+                  cached_tmap(&s.k, k, (uint64_t)kv_heads * S, AD, AD, 128) &&
+                  cached_tmap(&s.v, v, (uint64_t)kv_heads * S, AD, AD, 128);
     } else {
-        maps_ok = cached_tmap(&mq, q, S, (uint64_t)heads * AD, ldq, 128) &&
-                  cached_tmap(&mk, k, S, (uint64_t)kv_heads * AD, ldk, 128) &&
-                  cached_tmap(&mv, v, S, (uint64_t)kv_heads * AD, ldv, 128);
+        maps_ok = cached_tmap(&s.q, q, S, (uint64_t)heads * AD, ldq, 128) &&
+                  cached_tmap(&s.k, k, S, (uint64_t)kv_heads * AD, ldk, 128) &&
+                  cached_tmap(&s.v, v, S, (uint64_t)kv_heads * AD, ldv, 128);
     }
     if (!maps_ok) return false;
-    const CUtensorMap *tq = &mq, *tk = &mk, *tv = &mv;
     const bool one_tile = tile_mode() == 2 || (tile_mode() == 0 && S < 8192);
     const int rows_item = one_tile ? T1_ROWS : AQ2;
-    static std::atomic<uint64_t> attr_done{0}, attr1_done{0};
-    if (one_tile) {
-        if (!func_attr_once(attr1_done, (const void*)flash_attn1_kernel, T1_SMEM, "attention (one tile)")) return false;
-    } else if (!func_attr_once(attr_done, (const void*)flash_attn_kernel, ATTN_SMEM, "attention")) return false;
-    AttnArgs a;
+    AttnArgs& a = s.a;
     a.out = (uint16_t*)out; a.ldo = ldo;
     a.S = S; a.heads = heads; a.kv_heads = kv_heads; a.ar_len = ar_len;
     a.row_lo = row_lo < 0 ? 0 : row_lo;
@@ -1040,39 +1065,120 @@ static bool flash_attention_impl(const void* q, int ldq, const void* k, int ldk,
             a.part_ml = a.part_o + (size_t)rem * w * rows_item * AD;
         }
     }
-    dim3 grid(a.n_plain + n_tail * a.ways);
-    {
-        // QK^T + PV over the keys each row can see: 4*heads*128*(ar(ar+1)/2 + (S-ar)*S)
-        const double keys = 0.5 * ar_len * (ar_len + 1.0) + (double)(S - ar_len) * S;
-        prof_before(PROF_ATTN, 4.0 * heads * 128.0 * keys, st);
+    s.grid = a.n_plain + n_tail * a.ways;
+    s.n_tail = n_tail; s.rows_item = rows_item; s.one_tile = one_tile;
+    // QK^T + PV over the keys each row can see: 4*heads*128*(ar(ar+1)/2 + (S-ar)*S)
+    s.work = 4.0 * heads * 128.0 * (0.5 * ar_len * (ar_len + 1.0) + (double)(S - ar_len) * S);
+    return true;
+}
+
+template <int NSEG>
+static cudaError_t launch_one_tile(const AttnSetup* s, cudaStream_t st) {
+    static std::atomic<uint64_t> attr_done{0};
+    auto kern = flash_attn1_kernel<AD, NSEG>;
+    if (!func_attr_once(attr_done, (const void*)kern, T1_SMEM, "attention (one tile)")) return cudaErrorInvalidValue;
+    Attn1Params<NSEG> p;
+    int grid = 0;
+    for (int i = 0; i < NSEG; ++i) {
+        p.q[i] = s[i].q; p.k[i] = s[i].k; p.v[i] = s[i].v; p.a[i] = s[i].a;
+        grid += s[i].grid;
     }
-    if (one_tile) flash_attn1_kernel<<<grid, ATTN_THREADS, T1_SMEM, st>>>(*tq, *tk, *tv, a);
-    else flash_attn_kernel<<<grid, ATTN_THREADS, ATTN_SMEM, st>>>(*tq, *tk, *tv, a);
-    if (n_tail) attn_merge_kernel<<<n_tail * rows_item, AD, 0, st>>>(a, n_tail, rows_item);
+    p.grid0 = s[0].grid;
+    return launch_chained(kern, dim3(grid), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p);
+}
+static cudaError_t launch_two_tile(const AttnSetup& s, cudaStream_t st) {
+    static std::atomic<uint64_t> attr_done{0};
+    if (!func_attr_once(attr_done, (const void*)flash_attn_kernel, ATTN_SMEM, "attention")) return cudaErrorInvalidValue;
+    return launch_chained(flash_attn_kernel, dim3(s.grid), dim3(ATTN_THREADS), ATTN_SMEM, st, 1, s.a.S, s.q, s.k, s.v, s.a);
+}
+// s[0 .. n): one launch for all of them where all take the one-tile kernel
+static bool attention_launch(const AttnSetup* s, int n, cudaStream_t st) {
+    double work = 0;
+    for (int i = 0; i < n; ++i) work += s[i].work;
+    prof_before(PROF_ATTN, work, st);
+    cudaError_t e = cudaSuccess;
+    if (n == 2 && s[0].one_tile && s[1].one_tile) e = launch_one_tile<2>(s, st);
+    else
+        for (int i = 0; i < n && e == cudaSuccess; ++i) e = s[i].one_tile ? launch_one_tile<1>(s + i, st) : launch_two_tile(s[i], st);
+    for (int i = 0; i < n && e == cudaSuccess; ++i)
+        if (s[i].n_tail)
+            e = launch_chained(attn_merge_kernel, dim3(s[i].n_tail * s[i].rows_item), dim3(AD), 0, st, 1, s[i].a.S, s[i].a, s[i].n_tail,
+                               s[i].rows_item);
     prof_after(st);
-    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("attention: launch: %s", cudaGetErrorString(e)); return false; }
     return true;
 }
 
+bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cudaStream_t st) {
+    constexpr int H = 16, DH = 72, LD = 3 * H * AD;
+    if (!qkv || !out || S <= 0 || (((uintptr_t)out) & 15)) { set_error("attention (vision): bad args"); return false; }
+    const uint16_t* q = (const uint16_t*)qkv;
+    Attn1Params<1> p = {};
+    if (!cached_tmap(&p.q[0], q, S, H * AD, LD, 128) || !cached_tmap(&p.k[0], q + H * AD, S, H * AD, LD, 128) ||
+        !cached_tmap(&p.v[0], q + 2 * H * AD, S, H * AD, LD, 128))
+        return false;
+    static std::atomic<uint64_t> attr_done{0};
+    auto kern = flash_attn1_kernel<DH, 1>;
+    if (!func_attr_once(attr_done, (const void*)kern, T1_SMEM, "attention (vision)")) return false;
+    AttnArgs& a = p.a[0];
+    a.out = (uint16_t*)out; a.ldo = H * DH; a.out_hoff = DH;
+    a.S = S; a.heads = a.kv_heads = H;
+    a.row_hi = S;
+    a.scale_log2 = scale * 1.4426950408889634f;
+    a.q_hc = a.kv_hc = AD;
+    a.err = device_error_word();
+    a.nqb = (S + T1_ROWS - 1) / T1_ROWS;
+    a.n_plain = a.nqb * H; a.ways = 1;
+    p.grid0 = a.n_plain;
+    prof_before(PROF_ATTN, 4.0 * H * DH * (double)S * S, st);
+    cudaError_t e = launch_chained(kern, dim3(a.n_plain), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p);
+    prof_after(st);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("attention (vision): launch: %s", cudaGetErrorString(e)); return false; }
+    return true;
+}
 bool flash_attention(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,
                      void* out, int ldo, int S, int heads, int kv_heads, int ar_len, float scale,
                      cudaStream_t st, void* scratch, size_t scratch_bytes) {
-    return flash_attention_impl(q, ldq, k, ldk, v, ldv, out, ldo, S, heads, kv_heads, ar_len, scale,
-                                false, false, st, nullptr, 0, scratch, scratch_bytes);
+    AttnSetup s;
+    return attention_setup(s, q, ldq, k, ldk, v, ldv, out, ldo, S, heads, kv_heads, ar_len, scale, false, false, nullptr, 0,
+                           scratch, scratch_bytes) &&
+           attention_launch(&s, 1, st);
+}
+// n sequences (1 or 2) whose rows lie behind one another in qkv [rows, q | k | v], out [rows, ldo] and scratch (scratch_row
+// bytes per row); each attends to its own rows only, with the results of a call of its own
+bool flash_attention_rows(const uint16_t* qkv, int ld, void* out, int ldo, const int* rows, const int* ar_len, int n, int heads,
+                          int kv_heads, float scale, cudaStream_t st, void* scratch, size_t scratch_row) {
+    if (n < 1 || n > 2) { set_error("attention: one or two sequences"); return false; }
+    AttnSetup s[2];
+    size_t row0 = 0;
+    for (int i = 0; i < n; ++i) {
+        const uint16_t* q = qkv + row0 * ld;
+        if (!attention_setup(s[i], q, ld, q + heads * AD, ld, q + (heads + kv_heads) * AD, ld, (uint16_t*)out + row0 * ldo, ldo,
+                             rows[i], heads, kv_heads, ar_len[i], scale, false, false, nullptr, 0,
+                             (uint8_t*)scratch + row0 * scratch_row, rows[i] * scratch_row))
+            return false;
+        row0 += rows[i];
+    }
+    return attention_launch(s, n, st);
 }
 bool flash_attention_tab(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,
                          void* const* out_tab, int out_rows, int ldo, int S, int heads, int kv_heads,
                          int ar_len, float scale, cudaStream_t st, void* scratch, size_t scratch_bytes) {
-    return flash_attention_impl(q, ldq, k, ldk, v, ldv, nullptr, ldo, S, heads, kv_heads, ar_len, scale,
-                                false, false, st, out_tab, out_rows, scratch, scratch_bytes);
+    AttnSetup s;
+    return attention_setup(s, q, ldq, k, ldk, v, ldv, nullptr, ldo, S, heads, kv_heads, ar_len, scale, false, false, out_tab,
+                           out_rows, scratch, scratch_bytes) &&
+           attention_launch(&s, 1, st);
 }
 // q [heads,S,128], k/v [kv_heads,S,128]; out head-major [heads,S,128] or seq-major [S, heads*128]
 bool flash_attention_hm(const void* q, const void* k, const void* v, void* out, int S, int heads,
                         int kv_heads, int ar_len, float scale, bool out_head_major, cudaStream_t st,
                         int row_lo, int row_hi) {
-    return flash_attention_impl(q, AD, k, AD, v, AD, out, heads * AD, S, heads, kv_heads, ar_len,
-                                scale, true, out_head_major, st, nullptr, 0, nullptr, 0, row_lo, row_hi);
+    AttnSetup s;
+    return attention_setup(s, q, AD, k, AD, v, AD, out, heads * AD, S, heads, kv_heads, ar_len, scale, true, out_head_major,
+                           nullptr, 0, nullptr, 0, row_lo, row_hi) &&
+           attention_launch(&s, 1, st);
 }
 
 }  // namespace o1

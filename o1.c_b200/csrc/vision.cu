@@ -49,6 +49,8 @@ static constexpr int LN_WARPS = 4;
 __global__ void __launch_bounds__(LN_WARPS * 32)
 layernorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, const uint16_t* __restrict__ b,
                  uint16_t* __restrict__ y, int rows, int cols, float eps, int vec) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int row = blockIdx.x * LN_WARPS + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -107,6 +109,8 @@ template <int NV>
 __global__ void __launch_bounds__(LN_WARPS * 32)
 layernorm_reg_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, const uint16_t* __restrict__ b,
                      uint16_t* __restrict__ y, int rows, int cols, float eps) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int row = blockIdx.x * LN_WARPS + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -117,6 +121,17 @@ layernorm_reg_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
     for (int k = 0; k < NV; ++k) {
         const int i = lane * 8 + k * 256;
         v[k] = i < cols ? *reinterpret_cast<const uint4*>(xr + i) : make_uint4(0, 0, 0, 0);
+    }
+    // weight and bias of a short row are requested with it: one memory latency per row, not two (5.5 us at 520 rows)
+    constexpr int PRE = NV <= 5 ? NV : 1;
+    uint4 wp[PRE], bp[PRE];
+    if (NV <= 5) {
+#pragma unroll
+        for (int k = 0; k < PRE; ++k) {
+            const int i = lane * 8 + k * 256;
+            wp[k] = i < cols ? *reinterpret_cast<const uint4*>(w + i) : make_uint4(0, 0, 0, 0);
+            bp[k] = b && i < cols ? *reinterpret_cast<const uint4*>(b + i) : make_uint4(0, 0, 0, 0);
+        }
     }
     float s = 0.f, ss = 0.f;
 #pragma unroll
@@ -138,9 +153,9 @@ layernorm_reg_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
     for (int k = 0; k < NV; ++k) {
         const int i = lane * 8 + k * 256;
         if (i < cols) {
-            const uint4 wv = *reinterpret_cast<const uint4*>(w + i);
-            uint4 bv = make_uint4(0, 0, 0, 0);
-            if (b) bv = *reinterpret_cast<const uint4*>(b + i);
+            uint4 wv, bv = make_uint4(0, 0, 0, 0);
+            if (NV <= 5) { wv = wp[k % PRE]; bv = bp[k % PRE]; }
+            else { wv = *reinterpret_cast<const uint4*>(w + i); if (b) bv = *reinterpret_cast<const uint4*>(b + i); }
             const float f[8] = {bf16lo(v[k].x), bf16hi(v[k].x), bf16lo(v[k].y), bf16hi(v[k].y),
                                 bf16lo(v[k].z), bf16hi(v[k].z), bf16lo(v[k].w), bf16hi(v[k].w)};
             const float g[8] = {bf16lo(wv.x), bf16hi(wv.x), bf16lo(wv.y), bf16hi(wv.y),
@@ -164,19 +179,19 @@ bool vision_layernorm(const void* x, const void* w, const void* b, void* y, int 
     const int vec = (cols % 8) == 0 && ((((uintptr_t)x) | ((uintptr_t)w) | ((uintptr_t)b) | ((uintptr_t)y)) & 15) == 0;
     const int grid = (rows + LN_WARPS - 1) / LN_WARPS;
     if (vec && cols <= 5 * 256) {
-        layernorm_reg_kernel<5><<<grid, LN_WARPS * 32, 0, st>>>((const uint16_t*)x, (const uint16_t*)w, (const uint16_t*)b,
-                                                               (uint16_t*)y, rows, cols, eps);
+        launch_chained(layernorm_reg_kernel<5>, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
+                       (const uint16_t*)b, (uint16_t*)y, rows, cols, eps);
         O1_VLAUNCH_CHECK("vision_layernorm");
         return true;
     }
     if (vec && cols <= 18 * 256) {
-        layernorm_reg_kernel<18><<<grid, LN_WARPS * 32, 0, st>>>((const uint16_t*)x, (const uint16_t*)w, (const uint16_t*)b,
-                                                                (uint16_t*)y, rows, cols, eps);
+        launch_chained(layernorm_reg_kernel<18>, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
+                       (const uint16_t*)b, (uint16_t*)y, rows, cols, eps);
         O1_VLAUNCH_CHECK("vision_layernorm");
         return true;
     }
-    layernorm_kernel<<<(rows + LN_WARPS - 1) / LN_WARPS, LN_WARPS * 32, 0, st>>>(
-        (const uint16_t*)x, (const uint16_t*)w, (const uint16_t*)b, (uint16_t*)y, rows, cols, eps, vec);
+    launch_chained(layernorm_kernel, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
+                   (const uint16_t*)b, (uint16_t*)y, rows, cols, eps, vec);
     O1_VLAUNCH_CHECK("vision_layernorm");
     return true;
 }
@@ -190,8 +205,7 @@ __global__ void gelu_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict
     if (exact) {
         r = 0.5f * v * (1.0f + erff(v * 0.7071067811865476f));
     } else {
-        const float u = 0.7978845608028654f * (v + 0.044715f * v * v * v);
-        r = 0.5f * v * (1.0f + tanhf(u));
+        r = gelu_tanh(v);
     }
     y[i] = f32_to_bf16(r);
 }
@@ -362,34 +376,21 @@ __global__ void split_rope_pad_kernel(const uint16_t* __restrict__ qkv, const fl
             const int half = V_D / 2;
             const float xh = bf16_to_f32(src[d < half ? d + half : d - half]);
             const float c = cosd[(size_t)s * V_D + d], sn = sind[(size_t)s * V_D + d];
-            v[j] = (d < half) ? (x0 * c - xh * sn) : (x0 * c + xh * sn);
+            v[j] = rope_f32(x0, c, d < half ? -xh : xh, sn);
         }
         o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
         o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
     }
     *reinterpret_cast<uint4*>(out + (size_t)s * 3 * V_HEADS * V_DP + (size_t)which * V_HEADS * V_DP + (size_t)h * V_DP + g * 8) = o;
 }
-// attention output [n, 16*128] (padded heads) -> [n, 16*72]
-__global__ void unpad_heads_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int n) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long total = (long)n * V_HEADS * (V_D / 8);
-    if (i >= total) return;
-    const int g = (int)(i % (V_D / 8));
-    const long r = i / (V_D / 8);
-    const int h = (int)(r % V_HEADS);
-    const long s = r / V_HEADS;
-    *reinterpret_cast<uint4*>(out + (size_t)s * V_H + h * V_D + g * 8) =
-        *reinterpret_cast<const uint4*>(in + (size_t)s * V_HEADS * V_DP + h * V_DP + g * 8);
-}
-
 // GEMM + bias (+ GELU) on the tensor-core kernel where its tiles apply, otherwise the SIMT GEMM and a GELU pass
 static bool linear_act(const void* x, const void* w, const void* b, void* y, int M, int N, int K, int act /*0 none, 1 tanh, 2 erf*/,
                        cudaStream_t st, int* launches) {
     if (act && gemm_tc_supported(M, N, K, EPI_BIAS_GELU)) {
         ++*launches;
-        return gemm_bf16(x, w, nullptr, y, M, N, K, EPI_BIAS_GELU, b, nullptr, act == 2 ? 1.0f : 0.0f, 0, st);
+        return gemm_bf16(x, w, nullptr, y, M, N, K, EPI_BIAS_GELU, b, nullptr, act == 2 ? 1.0f : 0.0f, GEMM_SPLIT_K, st);
     }
-    if (!gemm_bf16(x, w, nullptr, y, M, N, K, EPI_BIAS, b, nullptr, 0.f, 0, st)) return false;
+    if (!gemm_bf16(x, w, nullptr, y, M, N, K, EPI_BIAS, b, nullptr, 0.f, GEMM_SPLIT_K, st)) return false;
     ++*launches;
     if (act) { if (!vision_gelu(y, y, (size_t)M * N, act == 2, st)) return false; ++*launches; }
     return true;
@@ -606,7 +607,6 @@ hd_status hd_vision_forward(const hd_vision_binding* bw, hd_vision_workspace* ws
     uint16_t* fc2 = (uint16_t*)(base + o.fc2);
     uint16_t* qkvp = (uint16_t*)(base + o.q);
     uint16_t* qkv = (uint16_t*)(base + o.qkv);
-    uint16_t* attn_pad = (uint16_t*)(base + o.scores);
     uint16_t* attn_out = (uint16_t*)(base + o.attn_out);
     uint16_t* fc1 = (uint16_t*)(base + o.fc1);
     float* cosf_t = (float*)(base + o.cosf);
@@ -635,24 +635,27 @@ hd_status hd_vision_forward(const hd_vision_binding* bw, hd_vision_workspace* ws
         const hd_vision_block_binding* blk = &bw->blocks[i];
         void** s0 = i == 0 ? ws->block0_snaps : nullptr;
         VIS_TRY(vision_layernorm(cur_in, blk->norm1_w, blk->norm1_b, ln1, n, V_H, eps, st));
-        VIS_TRY(linear_act(ln1, blk->qkv_w, blk->qkv_b, qkv, n, 3 * V_H, V_H, 0, st, &launches));
-        {
+        // bias, rotary and the wider spacing of the heads ride in the projection's epilogue, and attention works on (and
+        // writes) 72 columns a head, unless a snapshot asks for the bare projection or there are too few rows for tiles
+        const bool fuse_qkv = gemm_tc_supported(n, 3 * V_H, V_H, EPI_BIAS) && !(s0 && s0[HD_B0_QKV]);
+        if (fuse_qkv) {
+            VIS_TRY(gemm_vision_qkv(ln1, blk->qkv_w, blk->qkv_b, qkvp, n, cosf_t, sinf_t, st));
+            VIS_TRY(flash_attention_vision(qkvp, attn_out, n, scaling, st));
+            launches += 2;
+        } else {
+            // (whole-K tiles, as the fused form has them: both give the same bits)
+            VIS_TRY(gemm_bf16(ln1, blk->qkv_w, nullptr, qkv, n, 3 * V_H, V_H, EPI_BIAS, blk->qkv_b, nullptr, 0.f, 0, st));
             const long total = (long)n * 3 * V_HEADS * (V_DP / 8);
             split_rope_pad_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(qkv, cosf_t, sinf_t, qkvp, n);
+            VIS_TRY(cudaGetLastError() == cudaSuccess);
+            VIS_TRY(flash_attention_vision(qkvp, attn_out, n, scaling, st));
+            launches += 2;
         }
-        VIS_TRY(flash_attention(qkvp, 3 * V_HEADS * V_DP, qkvp + V_HEADS * V_DP, 3 * V_HEADS * V_DP,
-                                qkvp + 2 * V_HEADS * V_DP, 3 * V_HEADS * V_DP, attn_pad, V_HEADS * V_DP, n, V_HEADS,
-                                V_HEADS, 0, scaling, st));
-        {
-            const long total = (long)n * V_HEADS * (V_D / 8);
-            unpad_heads_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(attn_pad, attn_out, n);
-        }
-        VIS_TRY(cudaGetLastError() == cudaSuccess);
         // the two residual adds ride in the projections' epilogues unless a snapshot asks for the bare projection
         // (or the row count is below the tensor-core tile minimum)
         const bool fuse = gemm_tc_supported(n, V_H, V_H, EPI_BIAS_RESID) && !(s0 && (s0[HD_B0_PROJ] || s0[HD_B0_FC2]));
         if (fuse) {
-            VIS_TRY(gemm_bf16(attn_out, blk->proj_w, nullptr, attn_resid, n, V_H, V_H, EPI_BIAS_RESID, blk->proj_b, cur_in, 0.f, 0, st));
+            VIS_TRY(gemm_bf16(attn_out, blk->proj_w, nullptr, attn_resid, n, V_H, V_H, EPI_BIAS_RESID, blk->proj_b, cur_in, 0.f, GEMM_SPLIT_K, st));
         } else {
             VIS_TRY(linear_act(attn_out, blk->proj_w, blk->proj_b, attn_resid, n, V_H, V_H, 0, st, &launches));
             if (s0) VIS_TRY(snap(s0[HD_B0_PROJ], attn_resid, nH, st));
@@ -661,12 +664,12 @@ hd_status hd_vision_forward(const hd_vision_binding* bw, hd_vision_workspace* ws
         VIS_TRY(vision_layernorm(attn_resid, blk->norm2_w, blk->norm2_b, ln2, n, V_H, eps, st));
         VIS_TRY(linear_act(ln2, blk->fc1_w, blk->fc1_b, fc1, n, V_I, V_H, 1, st, &launches));
         if (fuse) {
-            VIS_TRY(gemm_bf16(fc1, blk->fc2_w, nullptr, cur_out, n, V_H, V_I, EPI_BIAS_RESID, blk->fc2_b, attn_resid, 0.f, 0, st));
+            VIS_TRY(gemm_bf16(fc1, blk->fc2_w, nullptr, cur_out, n, V_H, V_I, EPI_BIAS_RESID, blk->fc2_b, attn_resid, 0.f, GEMM_SPLIT_K, st));
         } else {
             VIS_TRY(linear_act(fc1, blk->fc2_w, blk->fc2_b, fc2, n, V_H, V_I, 0, st, &launches));
             VIS_TRY(residual_add(attn_resid, fc2, cur_out, (size_t)n * V_H, st));
         }
-        launches += 7;
+        launches += fuse ? 4 : 5;      // two LayerNorms and the two fused projections, or the two residual adds as well
 
         if (s0) {
             VIS_TRY(snap(s0[HD_B0_INPUT], cur_in, nH, st) && snap(s0[HD_B0_NORM1], ln1, nH, st) &&

@@ -306,3 +306,29 @@ def test_edit_pipeline_tower_into_forward(pkg, orc, dev, tower):
     out_plain = eng.forward(torch.from_numpy(text).to(dev), pos.to(dev), u16_to_torch(vin, dev), 0.3)
     torch.cuda.synchronize()
     assert metrics(out_plain, out)[0] > 1e-2
+
+
+@pytest.mark.parametrize("gh,gw", [(4, 2), (8, 12), (12, 12), (26, 20)])
+def test_fused_projection_equals_the_separate_pass(pkg, dev, tower, gh, gw):
+    """Bias + rotary + head spacing in the q | k | v projection's epilogue == projection, then the layout pass: a snapshot
+    of the bare projection makes block 0 take the separate pass, and nothing else may change by a bit."""
+    _, _, binding = tower
+    n = gh * gw
+    px = seeded_bf16((n, 1536), 9)
+    emb, ds, outs = run_tower(pkg, dev, binding, px, gh, gw)
+    ws = pkg.VisionWorkspace()
+    space = torch.zeros(pkg.lib.hd_vision_workspace_bytes(n), dtype=torch.uint8, device=dev)
+    tables = torch.zeros(pkg.lib.hd_vision_tables_bytes(n), dtype=torch.uint8, device=dev)
+    ws.patch_out, ws.tables, ws.tables_n = space.data_ptr(), tables.data_ptr(), -1
+    qkv, b0 = empty_bf16((n, 3456), dev), empty_bf16((n, 1152), dev)
+    ws.block0_snaps[2], ws.block_out_snaps[0] = qkv.data_ptr(), b0.data_ptr()
+    assert pkg.lib.hd_vision_prepare_tables(C.byref(ws), n, gh, gw) == 0
+    emb2, ds2 = torch.empty_like(emb), torch.empty_like(ds)
+    dsp = (C.c_void_p * 3)(*[ds2[j].data_ptr() for j in range(3)])
+    pxd = u16_to_torch(px, dev)
+    assert pkg.lib.hd_vision_forward(C.byref(binding), C.byref(ws), pkg.ptr(pxd), n, gh, gw, pkg.ptr(emb2), C.byref(dsp)) == 0
+    done(pkg, "vision")
+    assert qkv.float().abs().max() > 0
+    assert torch.equal(b0.view(torch.int16), outs[0].view(torch.int16))
+    assert torch.equal(emb, emb2) and torch.equal(ds, ds2)
+    assert pkg.lib.o1_device_error() == 0
