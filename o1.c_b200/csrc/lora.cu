@@ -2,9 +2,7 @@
 // (o1.c include/hd_lora.h:10-14, src/model/lora_merge.cu:26-109, where the
 // delta is an FP32 cublasSgemm over row chunks followed by an add/cast pass).
 //
-// One persistent kernel merges up to 16 targets per launch.  The seven linears of a block at rank 64 took 1790 us with
-// a staging buffer (allocated per call), split kernels and a GEMM whose epilogue read and wrote W one row per thread
-// (five 72 us launches among them); here 300 us, the wait for the end included.  What bounds it is HBM: every weight is read once and
+// One persistent kernel merges up to 16 targets per launch.  What bounds it is HBM: every weight is read once and
 // written once, 4 bytes, while the contraction over the rank is short.  So W streams through shared memory on TMA
 // loads and stores, and the delta of a 128 x 128 tile is made on the way by the tensor core from the FP32 adapters.
 // To keep FP32-grade products on bf16 operands each adapter value is split into three bf16 terms
@@ -103,7 +101,7 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_empty + 2);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) *s_abort = *reinterpret_cast<volatile int*>(g.err);
     __syncthreads();
     if (*s_abort != 0) return;
@@ -131,7 +129,7 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
 
     if (warp == 0) {
         // ------------------------------------------------------ W stream: panels in, merged panels out
-        if (lane == 0) {
+        if (elect_one()) {
             const int panels = 2 * (tile_hi - tile_lo);
             int el = e, es = e;
             auto place = [&](int& te, int p, int& c0, int& c1) {
@@ -170,7 +168,7 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
         }
     } else if (warp == 1) {
         // ------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc_bf16(128, 128, 0, 1);     // down is MN-major
             int u = 0, te = e;
             bool ok = true;

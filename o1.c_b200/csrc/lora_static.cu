@@ -4,9 +4,10 @@
 // before the engine starts (a serving process that pre-reserves HBM for weights,
 // workspaces and other tenants), or that merges an adapter while other streams are
 // busy producing images and therefore must avoid cudaMalloc / cudaFree, which
-// stall the whole device.  hd_lora_merge_gpu allocates (and frees) a staging
-// buffer per call; this entry point keeps its scratch in a fixed array inside the
-// library image instead.
+// stall the whole device, and waits on the host.  hd_lora_merge_gpu allocates
+// nothing either, but returns only when its merge is done; this entry point
+// enqueues and returns, and keeps its scratch in a fixed array inside the library
+// image.
 //
 // Arithmetic: delta = up @ down in FP32 (rank-sequential sum), then
 // W = bf16(f32(W) + scale * delta), row chunk by row chunk through the scratch --
