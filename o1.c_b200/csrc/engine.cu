@@ -10,8 +10,8 @@
 //  * hd_forward (src/model/forward.c:190-405)
 //  * o1_denoise_step_cfg (src/runtime/generate.c:1314-1360 + :900-905)
 //  * hd_lora_merge_gpu (src/model/lora_merge.cu:35-109)
-// Nothing here allocates device memory on the forward path; the only
-// allocations are the per-device error word and LoRA staging.
+// Nothing here allocates device memory; the only allocation is the per-device
+// error word.
 #include "common.cuh"
 #include "kernels.h"
 #include "../../include/o1_b200.h"
@@ -504,10 +504,21 @@ static hd_status copy_dd(void* dst, const void* src, size_t bytes, cudaStream_t 
     return HD_OK;
 }
 
-// cs: [S,128] cos|sin table for this sequence (built once per forward).
+// Sequences whose rows lie behind one another in the activations of one pass (the two branches of a guided step): every
+// token-wise operation runs over all rows at once, attention over each sequence by itself.
+struct FwdSeg {
+    const int64_t* ids;
+    int T;                            // text rows
+    const float* pos;
+    int ar_len;
+    const hd_visual_cond* visual;
+    int row0, rows;                   // its rows among all rows
+};
+
+// cs: [S,128] cos|sin table of all rows (built once per forward).
 // mod: NULL (o1.c's block) or the six adaLN vectors [shift_msa | scale_msa | gate_msa | shift_mlp | scale_mlp |
 // gate_mlp], each [hidden] bf16: norm * (1 + scale) + shift before a branch, x + gate * branch after it.
-static hd_status block_forward(const void* in, const float* cs, int ar_len, const hd_block_binding* bw,
+static hd_status block_forward(const void* in, const float* cs, const FwdSeg* seg, int nseg, const hd_block_binding* bw,
                                void* scratch, hd_block_internals* ints, void* out, int64_t S64,
                                int heads, int kv_heads, int hidden, int ff, int hd, cudaStream_t st,
                                const uint16_t* mod = nullptr) {
@@ -539,8 +550,10 @@ static hd_status block_forward(const void* in, const float* cs, int ar_len, cons
     }
     // 7. attention, output already seq-major [S, heads*hd]
     // (the SwiGLU buffer is idle until step 11: it holds the partial results of key-split tail items)
-    BLK_TRY(flash_attention(b.qkv, ld, b.qkv + qc, ld, b.qkv + qc + kc, ld, b.attn, qc, S, heads,
-                            kv_heads, ar_len, scaling, st, b.swi, (size_t)S * ff * 2), "attention");
+    int rows[2] = {0, 0}, ar[2] = {0, 0};
+    for (int i = 0; i < nseg; ++i) { rows[i] = seg[i].rows; ar[i] = seg[i].ar_len; }
+    BLK_TRY(flash_attention_rows(b.qkv, ld, b.attn, qc, rows, ar, nseg, heads, kv_heads, scaling, st, b.swi, (size_t)ff * 2),
+            "attention");
     // 8-9. o_proj (+ residual)
     if (mod) {
         if (ints && ints->attn_hidden)
@@ -624,7 +637,8 @@ static hd_status decoder_block_entry(const void* in_dev, const float* pos_dev, c
         return HD_ERR_RUNTIME;
     }
     count();
-    return block_forward(in_dev, b.cs, ar_len, bw, scratch, ints, out_dev, seq, heads, kv_heads, hidden,
+    const FwdSeg all = {nullptr, 0, nullptr, ar_len, nullptr, 0, (int)seq};
+    return block_forward(in_dev, b.cs, &all, 1, bw, scratch, ints, out_dev, seq, heads, kv_heads, hidden,
                          ff_hidden, head_dim, g_stream, mod);
 }
 
@@ -689,13 +703,24 @@ static int64_t forward_layout(int64_t seq, int text_len, int img, int hidden, in
     return o;
 }
 
+// Up to this many rows per branch a guided step runs both branches in one pass.  Below it the GEMMs of one branch leave
+// part of the SMs idle and stream all weights for few rows (296 rows: 229 us a block, twice); from a few thousand rows on
+// one branch fills the machine, and the second set of activations would only cost memory.
+static constexpr int64_t PAIRED_ROWS = 2048;
+
 int64_t hd_forward_workspace_bytes(int64_t seq, int img_tokens, int heads, int kv_heads, int hidden,
                                    int ff_hidden, int head_dim, int64_t* block_scratch_bytes) {
     int64_t off[WS_COUNT];
     int64_t text = seq - img_tokens;
     if (text < 0) text = 0;
-    return forward_layout(seq, (int)text, img_tokens, hidden, heads, kv_heads, ff_hidden, head_dim, off,
-                          block_scratch_bytes);
+    const int64_t one = forward_layout(seq, (int)text, img_tokens, hidden, heads, kv_heads, ff_hidden, head_dim, off,
+                                       block_scratch_bytes);
+    // room for two branches of any shorter length in one pass as well: the layout of twice the rows, their text rows,
+    // and the x_embedder rows
+    const int64_t s2 = seq < PAIRED_ROWS ? seq : PAIRED_ROWS;
+    const int64_t two = forward_layout(2 * s2, 0, 0, hidden, heads, kv_heads, ff_hidden, head_dim, off, nullptr) +
+                        2 * s2 * hidden * 2 + s2 * (1024 + hidden) * 2 + 4096;
+    return one > two ? one : two;
 }
 
 int64_t hd_forward_ws_offset(const char* name, int64_t seq, int text_len, int img_tokens, int heads,
@@ -732,11 +757,14 @@ int hd_forward_num_layers(const hd_forward_binding* bw) { return bw ? bw->n_laye
     } while (0)
 
 static hd_status forward_impl(const hd_forward_binding* bw, hd_forward_workspace* ws,
-                              const int64_t* input_ids, int T, const float* pos_f32, int ar_len,
-                              const void* vinputs, int I, const hd_visual_cond* visual,
-                              const float* timestep, int S, int heads, int kv_heads, int H, int ff,
+                              const FwdSeg* seg, int nseg, const void* vinputs, int I,
+                              const float* timestep, int heads, int kv_heads, int H, int ff,
                               int hd, int tms_id, hd_forward_diagnostics* diag, void* out_dev,
                               cudaStream_t st) {
+    // (with two sequences: both carry visual conditioning or neither does, and diag is NULL)
+    int S = 0, T = 0;
+    for (int i = 0; i < nseg; ++i) { S += seg[i].rows; T += seg[i].T; }
+    const bool visual = seg[0].visual != nullptr;
     uint8_t* base = (uint8_t*)ws->hidden_a;
     int64_t off[WS_COUNT], bs_bytes;
     forward_layout(S, T, I, H, heads, kv_heads, ff, hd, off, &bs_bytes);
@@ -767,24 +795,27 @@ static hd_status forward_impl(const hd_forward_binding* bw, hd_forward_workspace
     const uint16_t* t_vec = te_hidden;
 
     // steps 1+3: text rows, with the tms row(s) replaced by t_emb
-    if (visual || (diag && diag->after_embedding)) {
-        FWD_TRY(gather_rows(bw->embed_tokens, input_ids, h_text, T, H, 151936, st), "embed");
-        if (diag) FWD_COPY(diag->after_embedding, h_text, (size_t)T * H * 2);
-        if (visual) {
-            FWD_TRY(masked_scatter(h_text, visual->visual_mask, visual->image_embeds, hidden_a, T, H, st),
-                    "masked_scatter");
-            FWD_TRY(tms_condition(input_ids, hidden_a, t_vec, hidden_a, T, H, tms_id, st), "tms");
+    for (int i = 0; i < nseg; ++i) {
+        const FwdSeg& g = seg[i];
+        uint16_t* rows = hidden_a + (size_t)g.row0 * H;
+        if (visual || (diag && diag->after_embedding)) {
+            FWD_TRY(gather_rows(bw->embed_tokens, g.ids, h_text, g.T, H, 151936, st), "embed");
+            if (diag) FWD_COPY(diag->after_embedding, h_text, (size_t)g.T * H * 2);
+            if (visual) {
+                FWD_TRY(masked_scatter(h_text, g.visual->visual_mask, g.visual->image_embeds, rows, g.T, H, st),
+                        "masked_scatter");
+                FWD_TRY(tms_condition(g.ids, rows, t_vec, rows, g.T, H, tms_id, st), "tms");
+            } else {
+                FWD_TRY(tms_condition(g.ids, h_text, t_vec, rows, g.T, H, tms_id, st), "tms");
+            }
         } else {
-            FWD_TRY(tms_condition(input_ids, h_text, t_vec, hidden_a, T, H, tms_id, st), "tms");
+            FWD_TRY(embed_text(bw->embed_tokens, g.ids, t_vec, rows, g.T, H, 151936, tms_id, st), "embed+tms");
         }
-    } else {
-        FWD_TRY(embed_text(bw->embed_tokens, input_ids, t_vec, hidden_a, T, H, 151936, tms_id, st),
-                "embed+tms");
     }
     if (diag) FWD_COPY(diag->after_timestep_conditioning, hidden_a, (size_t)T * H * 2);
 
     // steps 4+5: x_embedder over the image rows, written straight behind the text rows
-    uint16_t* img_rows = hidden_a + (size_t)T * H;
+    uint16_t* img_rows = hidden_a + (size_t)seg[0].T * H;
     int I_live = I;
     if (ws->xe_ref && ws->n_ref > 0 && ws->n_ref < I) I_live = I - ws->n_ref;
     FWD_TRY(gemm_bf16(vinputs, bw->xe1_w, nullptr, xe_stage, I_live, 1024, 3072, EPI_STORE, nullptr,
@@ -792,20 +823,23 @@ static hd_status forward_impl(const hd_forward_binding* bw, hd_forward_workspace
     FWD_TRY(gemm_bf16(xe_stage, bw->xe2_w, nullptr, img_rows, I_live, H, 1024, EPI_BIAS, bw->xe2_b,
                       nullptr, 0.f, 0, st), "x_embed2");
     if (I_live < I) FWD_COPY(img_rows + (size_t)I_live * H, ws->xe_ref, (size_t)ws->n_ref * H * 2);
+    // every sequence has the same image rows
+    for (int i = 1; i < nseg; ++i) FWD_COPY(hidden_a + (size_t)(seg[i].row0 + seg[i].T) * H, img_rows, (size_t)I * H * 2);
     if (diag) {
         FWD_COPY(diag->after_target_embedding, img_rows, (size_t)I * H * 2);
         FWD_COPY(diag->after_block_0_input, hidden_a, (size_t)S * H * 2);
     }
 
     // rotary table once per forward (the reference rebuilds it in every block)
-    FWD_TRY(mrope_table64(pos_f32, S, 5000000.0f, rope, st), "mrope_table");
+    for (int i = 0; i < nseg; ++i)
+        FWD_TRY(mrope_table64(seg[i].pos, seg[i].rows, 5000000.0f, rope + (size_t)seg[i].row0 * 128, st), "mrope_table");
 
     // step 6: decoder blocks, ping-pong
     const void* cur_in = hidden_a;
     void* cur_out = hidden_b;
     const int n = bw->n_layers;
     for (int i = 0; i < n; ++i) {
-        hd_status s = block_forward(cur_in, rope, ar_len, &bw->blocks[i], scratch, nullptr, cur_out, S,
+        hd_status s = block_forward(cur_in, rope, seg, nseg, &bw->blocks[i], scratch, nullptr, cur_out, S,
                                     heads, kv_heads, H, ff, hd, st);
         if (s != HD_OK) return s;
         if (diag) {
@@ -816,8 +850,11 @@ static hd_status forward_impl(const hd_forward_binding* bw, hd_forward_workspace
             FWD_COPY(dst, cur_out, (size_t)S * H * 2);
         }
         if (visual && i < 3) {
-            FWD_TRY(deepstack_inject(cur_out, visual->visual_mask, visual->deepstack[i], (void*)cur_in, S,
-                                     H, st), "deepstack");
+            for (int k = 0; k < nseg; ++k) {
+                const size_t off = (size_t)seg[k].row0 * H;
+                FWD_TRY(deepstack_inject((uint16_t*)cur_out + off, seg[k].visual->visual_mask, seg[k].visual->deepstack[i],
+                                         (uint16_t*)cur_in + off, seg[k].rows, H, st), "deepstack");
+            }
         } else {
             void* t = cur_out; cur_out = (void*)cur_in; cur_in = t;
         }
@@ -861,9 +898,9 @@ hd_status hd_forward(const hd_forward_binding* bw, hd_forward_workspace* ws, con
         ar_len = mask_dev ? probe_ar_len(mask_dev, seq, st) : 0;
         if (ar_len < 0) { hd_set_error("forward: mask is not prefix-causal"); return HD_ERR_UNSUPPORTED; }
     }
-    return forward_impl(bw, ws, input_ids, text_len, pos_f32, ar_len, vinputs, img_tokens, visual,
-                        timestep, seq, heads, kv_heads, hidden, ff_hidden, head_dim, tms_token_id, diag,
-                        out_dev, st);
+    const FwdSeg all = {input_ids, text_len, pos_f32, ar_len, visual, 0, seq};
+    return forward_impl(bw, ws, &all, 1, vinputs, img_tokens, timestep, heads, kv_heads, hidden, ff_hidden, head_dim,
+                        tms_token_id, diag, out_dev, st);
 }
 
 // ============================================================ added entry points
@@ -980,14 +1017,21 @@ hd_status o1_denoise_step_cfg_branches(const hd_forward_binding* bw, hd_forward_
     const int Sc = cond->text_len + img_tokens, Su = uncond->text_len + img_tokens;
     uint16_t* xc = (uint16_t*)xp_scratch;
     uint16_t* xu = xc + (size_t)Sc * 3072;
-    hd_status s = forward_impl(bw, ws, cond->ids, cond->text_len, cond->pos_f32, cond->ar_len, z, img_tokens,
-                               cond->visual, timestep_dev, Sc, heads, kv_heads, hidden, ff_hidden, head_dim,
-                               tms_token_id, nullptr, xc, g_stream);
-    if (s != HD_OK) return s;
-    s = forward_impl(bw, ws, uncond->ids, uncond->text_len, uncond->pos_f32, uncond->ar_len, z, img_tokens,
-                     uncond->visual, timestep_dev, Su, heads, kv_heads, hidden, ff_hidden, head_dim, tms_token_id,
-                     nullptr, xu, g_stream);
-    if (s != HD_OK) return s;
+    // the predictions lie behind one another in xp_scratch, as the rows of a paired pass do
+    FwdSeg seg[2] = {{cond->ids, cond->text_len, cond->pos_f32, cond->ar_len, cond->visual, 0, Sc},
+                     {uncond->ids, uncond->text_len, uncond->pos_f32, uncond->ar_len, uncond->visual, Sc, Su}};
+    if (Sc <= PAIRED_ROWS && Su <= PAIRED_ROWS && !cond->visual == !uncond->visual) {
+        const hd_status s = forward_impl(bw, ws, seg, 2, z, img_tokens, timestep_dev, heads, kv_heads, hidden, ff_hidden,
+                                         head_dim, tms_token_id, nullptr, xc, g_stream);
+        if (s != HD_OK) return s;
+    } else {
+        seg[1].row0 = 0;
+        for (int i = 0; i < 2; ++i) {
+            const hd_status s = forward_impl(bw, ws, &seg[i], 1, z, img_tokens, timestep_dev, heads, kv_heads, hidden,
+                                             ff_hidden, head_dim, tms_token_id, nullptr, i ? xu : xc, g_stream);
+            if (s != HD_OK) return s;
+        }
+    }
     // target rows start at row text_len of each prediction (generate.c:1330, :1352 slice them by a copy);
     // reference rows that follow the target in z are inputs only and are not stepped
     const size_t n = (size_t)target_tokens * 3072;

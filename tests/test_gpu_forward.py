@@ -405,3 +405,53 @@ def test_loader_against_the_reference_loader_and_converter(pkg, dev, golden, tmp
                 r.hd_weight_store_free(C.byref(theirs))
         finally:
             pkg.lib.hd_weight_store_free(C.byref(mine))
+
+
+@pytest.mark.parametrize("tc,tu,gh,gw,visual", [(24, 24, 8, 12, False), (40, 9, 7, 9, False), (9, 31, 3, 5, False),
+                                                (140, 140, 10, 13, True), (200, 77, 36, 40, False), (40, 40, 48, 43, False)])
+def test_paired_step_equals_two_forwards(pkg, dev, tc, tu, gh, gw, visual):
+    """A guided step whose branches run in one pass (up to 2048 rows each; the last case is beyond) == a forward per branch
+    and the scheduler update, bit for bit: predictions and latent, with equal and different text lengths, with and
+    without visual conditioning."""
+    from o1c_b200 import CfgBranch, VisualCond
+    I, L = gh * gw, 4 if visual else 2
+    w = pkg.Weights(n_layers=L, seed=1234, weight_set="B", device=dev)
+    z = u16_to_torch(seeded_bf16((I, 3072), 61, 0.0, 4.0), dev)
+    eng = pkg.Engine(w, max(tc, tu), I)
+    eng.ws_buf.fill_(0xA5)                                       # stale workspace contents must not matter
+    s0, s1, gd = 0.8, 0.7, 5.0
+    xs, br, keep = [], [], []
+    for k, t in enumerate((tc, tu)):
+        pos, ar = pkg.seq_t2i(t, gh, gw)
+        ids, posd = torch.from_numpy(make_ids(t, 3 + k)).to(dev), pos.to(dev)
+        vis = vc = None
+        if visual:
+            mask = np.zeros(t + I, dtype=np.uint8)
+            mask[3 + k:3 + k + 50] = 1
+            vis = (torch.from_numpy(mask).to(dev), u16_to_torch(seeded_bf16((50, 4096), 70 + k), dev),
+                   [u16_to_torch(seeded_bf16((50, 4096), 80 + 3 * k + i), dev) for i in range(3)])
+            vc = VisualCond(image_embeds=vis[1].data_ptr(), visual_mask=vis[0].data_ptr(), v_tokens=50)
+            for i in range(3):
+                vc.deepstack[i] = vis[2][i].data_ptr()
+        one = pkg.Engine(w, t, I, ar_len=ar)
+        xs.append(one.forward(ids, posd, z, 1.0 - s0, visual=vis))
+        b = CfgBranch(ids=ids.data_ptr(), text_len=t, pos_f32=posd.data_ptr(), ar_len=ar)
+        if vc:
+            b.visual = C.pointer(vc)
+        br.append(b)
+        keep.append((ids, posd, vis, vc, one))
+    want = torch.empty_like(z)
+    assert pkg.lib.o1_sched_cfg_flow_step(pkg.ptr(z), C.c_void_p(xs[0].data_ptr() + tc * 6144),
+                                          C.c_void_p(xs[1].data_ptr() + tu * 6144), s0, s1, gd, pkg.ptr(want), z.numel()) == 0
+    got = torch.empty_like(z)
+    eng.timestep.fill_(1.0 - s0)
+    d = eng.dimargs
+    rc = pkg.lib.o1_denoise_step_cfg_branches(C.byref(w.binding), C.byref(eng.ws), C.byref(br[0]), C.byref(br[1]), pkg.ptr(z),
+                                              I, I, pkg.ptr(eng.timestep), s0, s1, gd, pkg.ptr(eng.xp), pkg.ptr(got), *d, pkg.TMS_ID)
+    torch.cuda.synchronize()
+    assert rc == 0, pkg.last_error()
+    xp = eng.xp[:(tc + tu + 2 * I) * 3072].view(-1, 3072)
+    assert torch.equal(xp[:tc + I].view(torch.int16), xs[0].view(torch.int16))
+    assert torch.equal(xp[tc + I:].view(torch.int16), xs[1].view(torch.int16))
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert pkg.lib.o1_device_error() == 0
