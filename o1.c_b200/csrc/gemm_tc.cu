@@ -151,14 +151,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
-    // a kernel that already failed on this device leaves its code in *err: do nothing then
+    // a kernel that already failed on this device leaves its code in *err: do nothing then (a pair decides together, after
+    // its cluster barrier).  The word is on its way while the barriers and tensor memory are set up.
     __shared__ int s_abort;
-    if (threadIdx.x == 0) s_abort = *reinterpret_cast<volatile int*>(g.err);
-    __syncthreads();
-    if (!PAIR && s_abort != 0) { grid_dep_wait(); return; }      // (a pair decides together, after its first cluster barrier)
+    if (threadIdx.x == 64) s_abort = *reinterpret_cast<volatile int*>(g.err);
     const uint32_t rank = PAIR ? cluster_rank() : 0u;    // 0: the CTA that issues the pair's MMAs
 
     if (threadIdx.x == 0) {
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+        if (EPI == EPI_SWIGLU || EPI == EPI_QKV) tma_prefetch_desc(&tmB2);
+        if (EPI == EPI_QKV) tma_prefetch_desc(&tmB3);
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
@@ -180,7 +183,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     grid_dep_launch();
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
-    bool live = true;
+    bool live = s_abort == 0;
     if (PAIR) live = (s_abort | ld_cluster_s32(map_to_rank(smem_u32(&s_abort), rank ^ 1u))) == 0;
 
     // the pair form walks tiles of 256 rows: row tile 2 * mb2 + rank of each belongs to this CTA
@@ -196,10 +199,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     } else if (warp == 0) {
         // ------------------------------------------------------ TMA producer
         if (elect_one()) {
-            tma_prefetch_desc(&tmA);
-            tma_prefetch_desc(&tmB);
-            if (EPI == EPI_SWIGLU || EPI == EPI_QKV) tma_prefetch_desc(&tmB2);
-            if (EPI == EPI_QKV) tma_prefetch_desc(&tmB3);
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -641,10 +640,12 @@ static constexpr int SK_BN = 128;
 // five stages do not cover the way from memory (1152 x 4304 at 520 rows, five CTAs per tile: 21.0 -> 19.0 us; the
 // persistent kernel's six stages do, and there the requests only cost: 24 -> 32 us at 77 x 4096 x 4096).
 static constexpr int SK_PREFETCH = 24;
-template <int BN>
+// KPS: K blocks per stage.  Two where an SM has one CTA anyway: the trip through a stage's barriers then counts half (a K
+// block of a 32-column tile takes 290 cycles instead of 390-430; 77 x 4096 x 4096 17.8 -> 12.7 us).
+template <int BN, int KPS>
 struct SplitCfg {
-    static constexpr int STAGES = BN <= 32 ? 5 : 3;      // as many as leave room for a second CTA
-    static constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
+    static constexpr int STAGES = BN <= 32 ? 5 : 3;      // with KPS = 1 as many as leave room for a second CTA
+    static constexpr int STAGE_BYTES = KPS * (BM + BN) * BK * 2;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
     static constexpr int TMEM_COLS = BN <= 32 ? 32 : (BN <= 128 ? 128 : 256);
 };
@@ -657,11 +658,11 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a,
                  : "memory");
 }
 
-template <int EPI, int BN>
-__global__ void __launch_bounds__(GEMM_THREADS, 2)
+template <int EPI, int BN, int KPS>
+__global__ void __launch_bounds__(GEMM_THREADS, KPS == 1 ? 2 : 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g,
                   const int ks) {
-    constexpr int SK_STAGE_BYTES = SplitCfg<BN>::STAGE_BYTES, SK_STAGES = SplitCfg<BN>::STAGES, NU = BN / 16;
+    constexpr int SK_STAGE_BYTES = SplitCfg<BN, KPS>::STAGE_BYTES, SK_STAGES = SplitCfg<BN, KPS>::STAGES, NU = BN / 16;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + SK_STAGES * SK_STAGE_BYTES);
@@ -674,13 +675,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int rank = (int)(blockIdx.x % ks), tile = (int)(blockIdx.x / ks);
     const int nb = tile / g.num_m, mb = tile - nb * g.num_m;      // CTAs that share weights run next to each other
 
+    if (threadIdx.x == 64) *s_abort = *reinterpret_cast<volatile int*>(g.err);
     if (threadIdx.x == 0) {
-        *s_abort = *reinterpret_cast<volatile int*>(g.err);
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
         for (int s = 0; s < SK_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         mbar_init(acc_done, 1);
         fence_mbar_init();
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, SplitCfg<BN>::TMEM_COLS); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(tmem_slot, SplitCfg<BN, KPS>::TMEM_COLS); tmem_relinquish(); }
     const int kblocks = (g.K + BK - 1) / BK;
     const int kb0 = rank * kblocks / ks, nkb = (rank + 1) * kblocks / ks - kb0;
     const bool ahead = mb == 0 && g.prefetch > 0;     // the other row tiles find the weights in L2
@@ -698,37 +701,41 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
     if (ok && warp == 0) {
         if (elect_one()) {
-            tma_prefetch_desc(&tmA);
-            tma_prefetch_desc(&tmB);
-            for (int i = 0; i < nkb; ++i) {
-                const int s = i % SK_STAGES;
-                if (!mbar_wait(&empty[s], ((i / SK_STAGES) & 1) ^ 1)) { atomicExch(g.err, 51); break; }
-                if (ahead && i + g.prefetch < nkb) tma_prefetch_2d(&tmB, (kb0 + i + g.prefetch) * BK, nb * BN);
+            for (int i = 0, it = 0; i < nkb; i += KPS, ++it) {
+                const int s = it % SK_STAGES, n = nkb - i < KPS ? nkb - i : KPS;
+                if (!mbar_wait(&empty[s], ((it / SK_STAGES) & 1) ^ 1)) { atomicExch(g.err, 51); break; }
                 uint8_t* a_s = smem + s * SK_STAGE_BYTES;
-                mbar_expect_tx(&full[s], SK_STAGE_BYTES);
-                int a_c0 = (kb0 + i) * BK, a_c1 = mb * BM;
-                if (g.a_kblk > 0) {
-                    const int blk = a_c0 / g.a_kblk;
-                    a_c0 -= blk * g.a_kblk;
-                    a_c1 += blk * g.a_rows;
+                mbar_expect_tx(&full[s], n * (SK_STAGE_BYTES / KPS));
+                for (int u = 0; u < n; ++u) {
+                    if (ahead && i + u + g.prefetch < nkb) tma_prefetch_2d(&tmB, (kb0 + i + u + g.prefetch) * BK, nb * BN);
+                    int a_c0 = (kb0 + i + u) * BK, a_c1 = mb * BM;
+                    if (g.a_kblk > 0) {
+                        const int blk = a_c0 / g.a_kblk;
+                        a_c0 -= blk * g.a_kblk;
+                        a_c1 += blk * g.a_rows;
+                    }
+                    tma_load_2d(a_s + u * BM * BK * 2, &tmA, &full[s], a_c0, a_c1);
+                    tma_load_2d(a_s + KPS * BM * BK * 2 + u * BN * BK * 2, &tmB, &full[s], (kb0 + i + u) * BK, nb * BN);
                 }
-                tma_load_2d(a_s, &tmA, &full[s], a_c0, a_c1);
-                tma_load_2d(a_s + BM * BK * 2, &tmB, &full[s], (kb0 + i) * BK, nb * BN);
             }
         }
     } else if (ok && warp == 1) {
         if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, 0, 0);
             bool good = true;
-            for (int i = 0; i < nkb && good; ++i) {
-                const int s = i % SK_STAGES;
-                if (!mbar_wait(&full[s], (i / SK_STAGES) & 1)) { atomicExch(g.err, 52); good = false; break; }
+            for (int i = 0, it = 0; i < nkb && good; i += KPS, ++it) {
+                const int s = it % SK_STAGES;
+                if (!mbar_wait(&full[s], (it / SK_STAGES) & 1)) { atomicExch(g.err, 52); good = false; break; }
                 tc_fence_after();
                 const uint32_t a_addr = smem_u32(smem + s * SK_STAGE_BYTES);
-                const uint64_t ad = umma_desc_sw128(a_addr, 16, 1024);
-                const uint64_t bd = umma_desc_sw128(a_addr + BM * BK * 2, 16, 1024);
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k) umma_ss(tmem_base, ad + 2 * k, bd + 2 * k, idesc, (i | k) != 0);
+                for (int u = 0; u < KPS; ++u) {
+                    if (i + u >= nkb) break;
+                    const uint64_t ad = umma_desc_sw128(a_addr + u * BM * BK * 2, 16, 1024);
+                    const uint64_t bd = umma_desc_sw128(a_addr + KPS * BM * BK * 2 + u * BN * BK * 2, 16, 1024);
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma_ss(tmem_base, ad + 2 * k, bd + 2 * k, idesc, (i | u | k) != 0);
+                }
                 umma_commit(&empty[s]);
             }
             umma_commit(acc_done);
@@ -818,7 +825,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
-        if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN>::TMEM_COLS);
+        if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN, KPS>::TMEM_COLS);
         return;
     }
     const int mu = (NU + ks - 1) / ks;                            // most units a CTA owns
@@ -902,7 +909,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN>::TMEM_COLS);
+    if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN, KPS>::TMEM_COLS);
 }
 
 // ---------------------------------------------------------------- SIMT path
@@ -1149,7 +1156,7 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
 
 // Which form of gemm_split_kernel a problem takes: tile width and CTAs per tile; width 0: the persistent kernel is the
 // better one.  Times in us, persistent kernel with 128-column tiles against this one:
-//  * 32 columns where that makes at most two CTAs per SM:    77 x 4096 x 4096 19.4 / 17.2, 520 x 1152 x 1152 11.1 / 8.7,
+//  * 32 columns where that makes at most two CTAs per SM: 77 x 4096 x 4096 19.4 / 12.7, 520 x 1152 x 1152 11.1 / 8.7,
 //    130 x 4608 x 4608 23.9 / 20.0; beyond, the activations are read too often: 296 x 4096 x 4096 19.6 / 31.6
 //  * 96 columns where the wider tiles need a second round and these do not, and K is short: 2916 x 1152 x 1152 16.0 / 12.5,
 //    520 x 4304 x 1152 16.4 / 14.1; 593 x 4096 x 12288 86 / 84, where CTA pairs take 72
@@ -1169,11 +1176,11 @@ static SplitPlan split_plan(int M, int N, int K, bool may_split) {
     return {0, 0};
 }
 
-template <int EPI, int BN>
+template <int EPI, int BN, int KPS = 1>
 static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmArgs& g, int ks, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
-    constexpr int SMEM = SplitCfg<BN>::SMEM;
-    auto kern = gemm_split_kernel<EPI, BN>;
+    constexpr int SMEM = SplitCfg<BN, KPS>::SMEM;
+    auto kern = gemm_split_kernel<EPI, BN, KPS>;
     if (!func_attr_once(attr_done, (const void*)kern, SMEM, "gemm (few tiles)")) return false;
     g.num_n = (g.N + BN - 1) / BN;
     g.prefetch = SK_PREFETCH;
@@ -1192,7 +1199,9 @@ static bool launch_split(const CUtensorMap* tA, const void* w, GemmArgs& g, Spli
     CUtensorMap mB;
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, p.bn)) return false;
     switch (p.bn) {
-        case 32: return launch_split_bn<EPI, 32>(tA, &mB, g, p.ks, st);
+        case 32:
+            if (g.num_m * ((g.N + 31) / 32) <= sm_count()) return launch_split_bn<EPI, 32, 2>(tA, &mB, g, p.ks, st);
+            return launch_split_bn<EPI, 32>(tA, &mB, g, p.ks, st);
         case 96: return launch_split_bn<EPI, 96>(tA, &mB, g, p.ks, st);
         default: return launch_split_bn<EPI, 128>(tA, &mB, g, p.ks, st);
     }

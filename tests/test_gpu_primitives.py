@@ -492,7 +492,7 @@ def test_linear_of_few_tiles(pkg, dev, M, N, K):
 @pytest.mark.parametrize("M,N,K", [(96, 1152, 1152), (520, 1152, 4304), (130, 4608, 4608), (20, 4304, 1152), (9, 72, 520), (300, 128, 2048)])
 @pytest.mark.parametrize("epi", [0, 1, 2, 8, 9])
 def test_gemm_with_k_split_over_a_cluster(pkg, dev, M, N, K, epi):
-    """A tile's K shared by 1 to 8 CTAs (force_bn = -1), every epilogue that takes the form, against the whole-K tile:
+    """A tile's K shared by the CTAs of a cluster where that is chosen (force_bn = -1), every epilogue, against the whole-K tile:
     the FP32 sums differ by their order only, so the results are equal or neighbours."""
     if epi in (2, 8, 9) and N % 128:
         pytest.skip("the residual epilogues take whole 128-column tiles")
