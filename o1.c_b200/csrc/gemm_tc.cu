@@ -912,6 +912,148 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN, KPS>::TMEM_COLS);
 }
 
+// ---------------------------------------------------------------- tiles fitted to the number of SMs
+// The persistent kernel with a tile width chosen at run time, a multiple of 16 from 144 to 192 columns: where 128 or 256
+// columns leave a last round of few tiles (1280 rows x 4096 columns: 320 tiles for 148 SMs, three rounds for 2.2), some
+// width in between often makes whole rounds (144 columns: 290 tiles, two rounds).  A block of 1280 rows went from 539 to
+// 503 us, a guided step of 2 x 296 rows from 11.1 to 10.5 ms.  Same warps, same pipeline and the same sums; plain
+// row-major output with the bias or residual epilogue, 16 columns at a time.
+static constexpr int FIT_MAX_STAGES = 6, FIT_SMEM = 216 * 1024 + 1024 /*align*/ + 256 /*barriers*/;
+
+template <int EPI>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g, const int bn,
+                const int stages) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int stage_bytes = (BM + bn) * BK * 2;      // (bn is a multiple of 16: the stages stay 1024-byte aligned)
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + 216 * 1024);
+    uint64_t* empty = full + FIT_MAX_STAGES;
+    uint64_t* tfull = empty + FIT_MAX_STAGES;
+    uint64_t* tempty = tfull + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    if (threadIdx.x == 64) *s_abort = *reinterpret_cast<volatile int*>(g.err);
+    if (threadIdx.x == 0) {
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 4); }
+        fence_mbar_init();
+    }
+    if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool live = *s_abort == 0;
+    const int num_tiles = g.num_m * g.num_n, kblocks = (g.K + BK - 1) / BK;
+
+    if (live && warp == 0) {
+        if (elect_one()) {
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+                int mb, nb;
+                tile_coords(tile, g.num_m, g.num_n, g.group_m, mb, nb);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!mbar_wait(&empty[stage], phase ^ 1)) { ok = false; atomicExch(g.err, 61); break; }
+                    uint8_t* a_s = smem + stage * stage_bytes;
+                    mbar_expect_tx(&full[stage], stage_bytes);
+                    int a_c0 = kb * BK, a_c1 = mb * BM;
+                    if (g.a_kblk > 0) {
+                        const int blk = a_c0 / g.a_kblk;
+                        a_c0 -= blk * g.a_kblk;
+                        a_c1 += blk * g.a_rows;
+                    }
+                    tma_load_2d(a_s, &tmA, &full[stage], a_c0, a_c1);
+                    tma_load_2d(a_s + BM * BK * 2, &tmB, &full[stage], kb * BK, nb * bn);
+                    if (++stage == stages) { stage = 0; phase ^= 1; }
+                }
+            }
+        }
+    } else if (live && warp == 1) {
+        if (elect_one()) {
+            const uint32_t idesc = umma_idesc_bf16(BM, bn, 0, 0);
+            int stage = 0, as = 0;
+            uint32_t phase = 0, aphase = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+                if (!mbar_wait(&tempty[as], aphase ^ 1)) { atomicExch(g.err, 62); break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + as * 256;
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!mbar_wait(&full[stage], phase)) { ok = false; atomicExch(g.err, 63); break; }
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + stage * stage_bytes);
+                    const uint64_t ad = umma_desc_sw128(a_addr, 16, 1024);
+                    const uint64_t bd = umma_desc_sw128(a_addr + BM * BK * 2, 16, 1024);
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma_ss(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0);
+                    umma_commit(&empty[stage]);
+                    if (++stage == stages) { stage = 0; phase ^= 1; }
+                }
+                umma_commit(&tfull[as]);
+                if (++as == 2) { as = 0; aphase ^= 1; }
+            }
+        }
+    } else if (live) {
+        const int q = warp & 3;       // TMEM lane quadrant this warp may access
+        int as = 0;
+        uint32_t aphase = 0;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+            int mb, nb;
+            tile_coords(tile, g.num_m, g.num_n, g.group_m, mb, nb);
+            const int row = mb * BM + q * 32 + lane, col0 = nb * bn;
+            const bool row_ok = row < g.M;
+            // the operand of the next 16 columns is requested before the current ones are worked on (N is a multiple of 16)
+            const uint16_t* op = EPI == EPI_RESID ? g.resid + (size_t)row * g.ldr + col0 : g.bias + col0;
+            uint4 nx[2] = {};
+            if (row_ok) { nx[0] = reinterpret_cast<const uint4*>(op)[0]; nx[1] = reinterpret_cast<const uint4*>(op)[1]; }
+            const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase));
+            if (!got) { atomicExch(g.err, 64); break; }
+            tc_fence_after();
+            const uint32_t t_row = tmem_base + as * 256 + ((uint32_t)(q * 32) << 16);
+#pragma unroll 1
+            for (int c = 0; c < bn && col0 + c < g.N; c += 16) {
+                float o[16];
+                unpack8_bf16(nx[0], o);
+                unpack8_bf16(nx[1], o + 8);
+                if (row_ok && c + 16 < bn && col0 + c + 16 < g.N) {
+                    nx[0] = reinterpret_cast<const uint4*>(op + c + 16)[0];
+                    nx[1] = reinterpret_cast<const uint4*>(op + c + 16)[1];
+                }
+                uint32_t r[16];
+                tmem_ld16(t_row + c, r);
+                tmem_ld_wait();
+                if (row_ok) {
+                    uint4* dst = reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + col0 + c);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float v[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] = bf16_round(__uint_as_float(r[h * 8 + j])) + o[h * 8 + j];
+                        dst[h] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                                            pack_bf16x2(v[6], v[7]));
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[as]);
+            if (++as == 2) { as = 0; aphase ^= 1; }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc(tmem_base, 512);
+}
+
 // ---------------------------------------------------------------- SIMT path
 // For M < 8 (timestep MLP, M = 1) and for shapes the tensor-core tiles do not cover.  One warp per output column and MR
 // rows: bound by the weights' way from memory, so a weight is read once for all its rows, four 16-byte pieces of a lane at
@@ -1135,6 +1277,45 @@ static TileForm tile_form(int num_m, int N, bool wide_ok, bool pair_ok) {
     return c256 <= c128 ? TILE_256 : TILE_128;
 }
 
+// The fitted width for the bias and residual families, or 0 where no width beats the other forms.  A round of bn columns
+// takes about 31 (1/4 + 3/4 bn/128) of TILE_COST's units: the copies of A and the trips through the barriers do not grow
+// with the tile (nor do they shrink: widths below 128 gain nothing).
+static int fit_width(int num_m, int N) {
+    const long sms = sm_count();
+    auto cost = [&](TileForm f, long tiles, long at_once) { return (tiles + at_once - 1) / at_once * TILE_COST[f] * 512; };
+    long best = cost(TILE_128, (long)num_m * (N / 128), sms);
+    if ((N % 256) == 0) {
+        const long c256 = cost(TILE_256, (long)num_m * (N / 256), sms), cp = cost(TILE_PAIR, (long)((num_m + 1) / 2) * (N / 256), sms / 2);
+        best = c256 < best ? c256 : best;
+        if (pair_wanted() && cp < best) best = cp;
+    }
+    best -= best / 16;       // (only for a gain that shows)
+    int width = 0;
+    for (int bn = 144; bn <= 192; bn += 16) {
+        const long tiles = (long)num_m * ((N + bn - 1) / bn), c = (tiles + sms - 1) / sms * TILE_COST[TILE_128] * (128 + 3 * bn);
+        if (c < best) { best = c; width = bn; }
+    }
+    return width;
+}
+template <int EPI>
+static bool launch_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, int bn, cudaStream_t st) {
+    static std::atomic<uint64_t> attr_done{0};
+    auto kern = gemm_fit_kernel<EPI>;
+    if (!func_attr_once(attr_done, (const void*)kern, FIT_SMEM, "gemm (fitted)")) return false;
+    CUtensorMap mB;
+    if (!cached_tmap(&mB, w, g.N, g.K, g.K, bn)) return false;
+    g.num_n = (g.N + bn - 1) / bn;
+    int stages = 216 * 1024 / ((BM + bn) * BK * 2);
+    if (stages > FIT_MAX_STAGES) stages = FIT_MAX_STAGES;
+    const int tiles = g.num_m * g.num_n, grid = tiles < sm_count() ? tiles : sm_count();
+    prof_before(EPI, 2.0 * g.M * (double)g.N * g.K, st);
+    cudaError_t e = launch_chained(kern, dim3(grid), dim3(GEMM_THREADS), FIT_SMEM, st, 1, g.M, *tA, mB, g, bn, stages);
+    prof_after(st);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("gemm (fitted): launch: %s", cudaGetErrorString(e)); return false; }
+    return true;
+}
+
 template <int EPI, int BN>
 static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2,
                       GemmArgs& g, cudaStream_t st, const CUtensorMap* tB3 = nullptr) {
@@ -1336,6 +1517,11 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
             case EPI_BIAS_RESID: return launch_split<EPI_BIAS_RESID>(tA, w, g, p, st);
             case EPI_GATE_RESID: return launch_split<EPI_GATE_RESID>(tA, w, g, p, st);
         }
+    }
+    if (force_bn <= 0 && !o_cb && !o_tab && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) {
+        const int width = fit_width(g.num_m, N);
+        if (width && epi == EPI_RESID) return launch_fit<EPI_RESID>(tA, w, g, width, st);
+        if (width) return launch_fit<EPI_BIAS>(tA, w, g, width, st);
     }
     const bool wide_ok = (N % 256) == 0 && (!o_cb || (o_cb % 256) == 0);
     const bool pair_ok = epi == EPI_STORE || epi == EPI_BIAS || epi == EPI_RESID;

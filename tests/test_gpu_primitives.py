@@ -542,3 +542,26 @@ def test_fused_step_equals_the_chain_for_every_kind_of_value(pkg, dev, sigma, n)
     nan = chain.isnan()
     assert torch.equal(nan, fused.isnan())
     assert torch.equal(fused.view(torch.int16)[~nan], chain.view(torch.int16)[~nan])
+
+
+@pytest.mark.parametrize("M,N,K", [(592, 4096, 256), (513, 4096, 72), (700, 4096, 1000), (1280, 4096, 320), (1500, 4096, 128),
+                                   (1000, 3072, 448), (1664, 3072, 64), (2561, 4096, 200)])
+@pytest.mark.parametrize("epi", [1, 2])
+def test_tiles_fitted_to_the_sms(pkg, dev, M, N, K, epi):
+    """Tile widths between 128 and 256 columns (chosen where they make whole rounds of tiles) give the bits of 128-column
+    tiles: partly filled last row and column tiles, ragged K, more and fewer K blocks than stages."""
+    g = torch.Generator(device=dev).manual_seed(M + K)
+    x, w, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
+                  for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
+    ys = []
+    for bn in (0, 128):
+        y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
+        rc = pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N + 8, M, N, K, epi, pkg.ptr(b), pkg.ptr(r), N, 0.0, bn)
+        assert rc == 0, pkg.last_error()
+        done(pkg, "gemm")
+        assert (y[M:] == 777.0).all() and (y[:, N:] == 777.0).all(), "written beyond the matrix"
+        ys.append(y)
+    assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
+    if epi == 1:
+        check_linear_f64(ys[0][:M, :N], x, w, b, "fitted")
+    assert pkg.lib.o1_device_error() == 0
