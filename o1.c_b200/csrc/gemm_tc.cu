@@ -1267,9 +1267,16 @@ int gemm_pair_capacity() {
 // pairs instead of one CTA per 128 x 256 tile: 1280 rows 213 / 186 us, a block of 16640 rows 9.24 / 9.02 ms.
 enum TileForm { TILE_128, TILE_256, TILE_PAIR };
 static constexpr int TILE_COST[3] = {31, 58, 50};
-static TileForm tile_form(int num_m, int N, bool wide_ok, bool pair_ok) {
+// Those times are the main loop's; below K = 2048 the epilogue counts as much, and finer tiles are the safer choice until
+// there are two full waves of wide ones.
+static constexpr int LONG_K = 2048;
+static TileForm tile_form(int num_m, int N, int K, bool wide_ok, bool pair_ok) {
     if (!wide_ok) return TILE_128;
     const long sms = sm_count();
+    if (K < LONG_K) {
+        if ((long)num_m * (N / 256) < 2 * sms) return TILE_128;
+        return pair_ok && pair_wanted() && (long)((num_m + 1) / 2) * (N / 256) >= sms ? TILE_PAIR : TILE_256;
+    }
     auto cost = [&](TileForm f, long tiles, long at_once) { return (tiles + at_once - 1) / at_once * TILE_COST[f]; };
     const long c128 = cost(TILE_128, (long)num_m * (N / 128), sms), c256 = cost(TILE_256, (long)num_m * (N / 256), sms);
     const long cp = pair_ok && pair_wanted() ? cost(TILE_PAIR, (long)((num_m + 1) / 2) * (N / 256), sms / 2) : c256 + 1;
@@ -1280,7 +1287,8 @@ static TileForm tile_form(int num_m, int N, bool wide_ok, bool pair_ok) {
 // The fitted width for the bias and residual families, or 0 where no width beats the other forms.  A round of bn columns
 // takes about 31 (1/4 + 3/4 bn/128) of TILE_COST's units: the copies of A and the trips through the barriers do not grow
 // with the tile (nor do they shrink: widths below 128 gain nothing).
-static int fit_width(int num_m, int N) {
+static int fit_width(int num_m, int N, int K) {
+    if (K < LONG_K) return 0;
     const long sms = sm_count();
     auto cost = [&](TileForm f, long tiles, long at_once) { return (tiles + at_once - 1) / at_once * TILE_COST[f] * 512; };
     long best = cost(TILE_128, (long)num_m * (N / 128), sms);
@@ -1503,7 +1511,7 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
     if (epi == EPI_SWIGLU) {
         // (2N columns of gate and up)
         g.num_n = N / 128;
-        if (force_bn <= 0 && tile_form(g.num_m, 2 * N, true, true) == TILE_PAIR)
+        if (force_bn <= 0 && tile_form(g.num_m, 2 * N, K, true, true) == TILE_PAIR)
             return launch_tc_pair<EPI_SWIGLU>(tA, tB, tB2, g, st, nullptr);
         return launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
     }
@@ -1519,13 +1527,13 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
         }
     }
     if (force_bn <= 0 && !o_cb && !o_tab && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) {
-        const int width = fit_width(g.num_m, N);
+        const int width = fit_width(g.num_m, N, K);
         if (width && epi == EPI_RESID) return launch_fit<EPI_RESID>(tA, w, g, width, st);
         if (width) return launch_fit<EPI_BIAS>(tA, w, g, width, st);
     }
     const bool wide_ok = (N % 256) == 0 && (!o_cb || (o_cb % 256) == 0);
     const bool pair_ok = epi == EPI_STORE || epi == EPI_BIAS || epi == EPI_RESID;
-    TileForm form = tile_form(g.num_m, N, wide_ok, pair_ok);
+    TileForm form = tile_form(g.num_m, N, K, wide_ok, pair_ok);
     if (force_bn == 128 || force_bn == 256) {
         if (force_bn == 256 && !wide_ok) {
             set_error("gemm: BN=256 needs N (and the output column block) %% 256 == 0");
@@ -1628,7 +1636,7 @@ bool gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void
     // 256-wide tiles need every segment (and every destination block) to be a multiple of 256 columns
     bool wide = (qc % 256) == 0 && (kc % 256) == 0;
     if (tabs && (((qc / n_dst) % 256) != 0 || ((kc / n_dst) % 256) != 0)) wide = false;
-    const TileForm form = tile_form(g.num_m, N, wide, true);
+    const TileForm form = tile_form(g.num_m, N, K, wide, true);
     g.num_n = N / (form == TILE_128 ? 128 : 256);
     if (form == TILE_PAIR) return launch_tc_pair<EPI_QKV>(&mA, &mQ, &mK, g, st, &mV);
     return form == TILE_256 ? launch_tc<EPI_QKV, 256>(&mA, &mQ, &mK, g, st, &mV) : launch_tc<EPI_QKV, 128>(&mA, &mQ, &mK, g, st, &mV);

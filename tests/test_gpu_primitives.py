@@ -544,12 +544,12 @@ def test_fused_step_equals_the_chain_for_every_kind_of_value(pkg, dev, sigma, n)
     assert torch.equal(fused.view(torch.int16)[~nan], chain.view(torch.int16)[~nan])
 
 
-@pytest.mark.parametrize("M,N,K", [(592, 4096, 256), (513, 4096, 72), (700, 4096, 1000), (1280, 4096, 320), (1500, 4096, 128),
-                                   (1000, 3072, 448), (1664, 3072, 64), (2561, 4096, 200)])
+@pytest.mark.parametrize("M,N,K", [(592, 4096, 2048), (513, 4096, 2056), (700, 4096, 3000), (1280, 4096, 2112), (1500, 4096, 2048),
+                                   (1000, 3072, 2240), (1664, 3072, 2104), (2561, 4096, 2048), (592, 4096, 256)])
 @pytest.mark.parametrize("epi", [1, 2])
 def test_tiles_fitted_to_the_sms(pkg, dev, M, N, K, epi):
     """Tile widths between 128 and 256 columns (chosen where they make whole rounds of tiles) give the bits of 128-column
-    tiles: partly filled last row and column tiles, ragged K, more and fewer K blocks than stages."""
+    tiles: partly filled last row and column tiles, ragged K, and a K too short for the form."""
     g = torch.Generator(device=dev).manual_seed(M + K)
     x, w, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
                   for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
