@@ -1199,6 +1199,10 @@ static bool pair_wanted() {
     return g_pair_mode != 0;
 }
 
+// A launch of some hundred us counts as one of many rows (see OVERLAP_ROWS): 24576 x 4096 at 3100 rows 501 us overlapped,
+// 485 without.
+static long overlap_rows(const GemmArgs& g) { return (double)g.M * g.N * g.K > 1.5e11 ? OVERLAP_ROWS + 1 : g.M; }
+
 template <int EPI>
 static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2, GemmArgs& g,
                            cudaStream_t st, const CUtensorMap* tB3) {
@@ -1231,7 +1235,7 @@ static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const C
     }
     if (pairs > tiles) pairs = tiles;
     prof_before(EPI == EPI_QKV ? (int)EPI_STORE : EPI, 2.0 * g.M * (double)g.N * g.K * (EPI == EPI_SWIGLU ? 2.0 : 1.0), st);
-    cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 2, g.M, *tA, *tB, *tB2,
+    cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 2, overlap_rows(g), *tA, *tB, *tB2,
                                    tB3 ? *tB3 : *tB2, g);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -1266,7 +1270,7 @@ int gemm_pair_capacity() {
 // 63.6 / 56.6, and at 6144 columns (q | k | v) 296 rows 24.6 / 38.6 / 40.1, 1280 rows 66.4 / 60.5 / 53.0.  Gate | up as
 // pairs instead of one CTA per 128 x 256 tile: 1280 rows 213 / 186 us, a block of 16640 rows 9.24 / 9.02 ms.
 enum TileForm { TILE_128, TILE_256, TILE_PAIR };
-static constexpr int TILE_COST[3] = {31, 58, 50};
+static constexpr int TILE_COST[3] = {31, 66, 50};
 // Those times are the main loop's; below K = 2048 the epilogue counts as much, and finer tiles are the safer choice until
 // there are two full waves of wide ones.
 static constexpr int LONG_K = 2048;
@@ -1317,7 +1321,7 @@ static bool launch_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, int bn
     if (stages > FIT_MAX_STAGES) stages = FIT_MAX_STAGES;
     const int tiles = g.num_m * g.num_n, grid = tiles < sm_count() ? tiles : sm_count();
     prof_before(EPI, 2.0 * g.M * (double)g.N * g.K, st);
-    cudaError_t e = launch_chained(kern, dim3(grid), dim3(GEMM_THREADS), FIT_SMEM, st, 1, g.M, *tA, mB, g, bn, stages);
+    cudaError_t e = launch_chained(kern, dim3(grid), dim3(GEMM_THREADS), FIT_SMEM, st, 1, overlap_rows(g), *tA, mB, g, bn, stages);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (fitted): launch: %s", cudaGetErrorString(e)); return false; }
@@ -1335,7 +1339,7 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
     int grid = sm_count();
     if (grid > tiles) grid = tiles;
     prof_before((EPI == EPI_QKNORM || EPI == EPI_QKV) ? (int)EPI_STORE : (EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : ((EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID) ? (int)EPI_RESID : EPI)), 2.0 * g.M * (double)g.N * g.K * (EPI == EPI_SWIGLU ? 2.0 : 1.0), st);
-    cudaError_t e = launch_chained(kern, dim3(grid), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 1, g.M, *tA, *tB, *tB2,
+    cudaError_t e = launch_chained(kern, dim3(grid), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 1, overlap_rows(g), *tA, *tB, *tB2,
                                    tB3 ? *tB3 : *tB2, g);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -1441,9 +1445,12 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
     if (!gemm_tc_supported(M, N, K, epi)) {
         if (epi != EPI_STORE && epi != EPI_BIAS) { set_error("gemm: shape unsupported for fused epilogue"); return false; }
         const uint16_t* b = (const uint16_t*)(epi == EPI_BIAS ? bias : nullptr);
+        // Rows share a warp's weights where these do not fit L2 (24576 x 4096: 5 rows 144 -> 111 us); otherwise a warp per row
+        // and column is faster, the weights of the later rows coming from L2 (4096 x 12288: 5 rows 55 against 69 us).
+        const bool share_rows = M > 1 && (size_t)N * K * 2 > (126u << 20);
         const dim3 block(128);
         const cudaError_t e =
-            M == 1 ? launch_chained(gemm_simt_kernel<1>, dim3((N + 3) / 4, 1), block, 0, st, 1, M, (const uint16_t*)x,
+            !share_rows ? launch_chained(gemm_simt_kernel<1>, dim3((N + 3) / 4, M), block, 0, st, 1, M, (const uint16_t*)x,
                                     (const uint16_t*)w, b, (uint16_t*)y, M, N, K, ldx, ldy)
                    : launch_chained(gemm_simt_kernel<4>, dim3((N + 3) / 4, (M + 3) / 4), block, 0, st, 1, M, (const uint16_t*)x,
                                     (const uint16_t*)w, b, (uint16_t*)y, M, N, K, ldx, ldy);
