@@ -1266,7 +1266,7 @@ int gemm_pair_capacity() {
 
 // Which persistent form takes the fewest (rounds of tiles) x (time of a K block): one CTA per 128 x 128 or 128 x 256 tile,
 // or a pair of CTAs per 256 x 256 tile.  The sums are the same in all of them.  A round of tiles with K = 4096 takes 15.6,
-// 29 and 25 us; measured at 4096 columns: 593 rows 32.4 / 31.7 / 30.2 us, 1280 rows 48.8 / 58.0 / 51.4, 2242 rows 72.6 /
+// 29 (4096 columns) to 33 (24576) and 25 us; measured at 4096 columns: 593 rows 32.4 / 31.7 / 30.2 us, 1280 rows 48.8 / 58.0 / 51.4, 2242 rows 72.6 /
 // 63.6 / 56.6, and at 6144 columns (q | k | v) 296 rows 24.6 / 38.6 / 40.1, 1280 rows 66.4 / 60.5 / 53.0.  Gate | up as
 // pairs instead of one CTA per 128 x 256 tile: 1280 rows 213 / 186 us, a block of 16640 rows 9.24 / 9.02 ms.
 enum TileForm { TILE_128, TILE_256, TILE_PAIR };
