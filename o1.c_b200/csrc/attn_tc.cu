@@ -1083,11 +1083,16 @@ static bool attention_setup(AttnSetup& s, const void* q, int ldq, const void* k,
     return true;
 }
 
+// (a failed attribute call has left its own text)
+static bool launched(cudaError_t e) {
+    if (e != cudaSuccess) set_error("attention: launch: %s", cudaGetErrorString(e));
+    return e == cudaSuccess;
+}
 template <int NSEG>
-static cudaError_t launch_one_tile(const AttnSetup* s, cudaStream_t st) {
+static bool launch_one_tile(const AttnSetup* s, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
     auto kern = flash_attn1_kernel<AD, NSEG>;
-    if (!func_attr_once(attr_done, (const void*)kern, T1_SMEM, "attention (one tile)")) return cudaErrorInvalidValue;
+    if (!func_attr_once(attr_done, (const void*)kern, T1_SMEM, "attention (one tile)")) return false;
     Attn1Params<NSEG> p;
     int grid = 0;
     for (int i = 0; i < NSEG; ++i) {
@@ -1095,30 +1100,28 @@ static cudaError_t launch_one_tile(const AttnSetup* s, cudaStream_t st) {
         grid += s[i].grid;
     }
     p.grid0 = s[0].grid;
-    return launch_chained(kern, dim3(grid), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p);
+    return launched(launch_chained(kern, dim3(grid), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p));
 }
-static cudaError_t launch_two_tile(const AttnSetup& s, cudaStream_t st) {
+static bool launch_two_tile(const AttnSetup& s, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
-    if (!func_attr_once(attr_done, (const void*)flash_attn_kernel, ATTN_SMEM, "attention")) return cudaErrorInvalidValue;
-    return launch_chained(flash_attn_kernel, dim3(s.grid), dim3(ATTN_THREADS), ATTN_SMEM, st, 1, s.a.S, s.q, s.k, s.v, s.a);
+    if (!func_attr_once(attr_done, (const void*)flash_attn_kernel, ATTN_SMEM, "attention")) return false;
+    return launched(launch_chained(flash_attn_kernel, dim3(s.grid), dim3(ATTN_THREADS), ATTN_SMEM, st, 1, s.a.S, s.q, s.k, s.v, s.a));
 }
 // s[0 .. n): one launch for all of them where all take the one-tile kernel
 static bool attention_launch(const AttnSetup* s, int n, cudaStream_t st) {
     double work = 0;
     for (int i = 0; i < n; ++i) work += s[i].work;
     prof_before(PROF_ATTN, work, st);
-    cudaError_t e = cudaSuccess;
-    if (n == 2 && s[0].one_tile && s[1].one_tile) e = launch_one_tile<2>(s, st);
+    bool ok = true;
+    if (n == 2 && s[0].one_tile && s[1].one_tile) ok = launch_one_tile<2>(s, st);
     else
-        for (int i = 0; i < n && e == cudaSuccess; ++i) e = s[i].one_tile ? launch_one_tile<1>(s + i, st) : launch_two_tile(s[i], st);
-    for (int i = 0; i < n && e == cudaSuccess; ++i)
+        for (int i = 0; i < n && ok; ++i) ok = s[i].one_tile ? launch_one_tile<1>(s + i, st) : launch_two_tile(s[i], st);
+    for (int i = 0; i < n && ok; ++i)
         if (s[i].n_tail)
-            e = launch_chained(attn_merge_kernel, dim3(s[i].n_tail * s[i].rows_item), dim3(AD), 0, st, 1, s[i].a.S, s[i].a, s[i].n_tail,
-                               s[i].rows_item);
+            ok = launched(launch_chained(attn_merge_kernel, dim3(s[i].n_tail * s[i].rows_item), dim3(AD), 0, st, 1, s[i].a.S, s[i].a,
+                                         s[i].n_tail, s[i].rows_item));
     prof_after(st);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) { set_error("attention: launch: %s", cudaGetErrorString(e)); return false; }
-    return true;
+    return ok && launched(cudaGetLastError());
 }
 
 bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cudaStream_t st) {

@@ -90,7 +90,9 @@ inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, siz
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cfg.attrs = at; cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();     // the caller reports it: the next call's check must not find it again
+    return e;
 }
 
 // ---- process-wide state (one stream, one error buffer: the reference's

@@ -1183,7 +1183,11 @@ bool func_attr_once(std::atomic<uint64_t>& done, const void* func, int smem_byte
     const uint64_t bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return true;
     cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) { set_error("%s: smem attribute: %s", what, cudaGetErrorString(e)); return false; }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_error("%s: smem attribute: %s", what, cudaGetErrorString(e));
+        return false;
+    }
     done.fetch_or(bit, std::memory_order_release);
     return true;
 }

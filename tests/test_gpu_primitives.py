@@ -565,3 +565,19 @@ def test_tiles_fitted_to_the_sms(pkg, dev, M, N, K, epi):
     if epi == 1:
         check_linear_f64(ys[0][:M, :N], x, w, b, "fitted")
     assert pkg.lib.o1_device_error() == 0
+
+
+def test_a_refused_launch_is_reported_once(pkg, dev):
+    """A launch that CUDA refuses on the host (a grid of 70000 rows, the limit being 65535: no kernel runs) is an error of the
+    call that asked for it and of no later one."""
+    M, N, K = 70000, 9, 8
+    x, w, y = (torch.zeros(s, dtype=torch.bfloat16, device=dev) for s in ((M, K), (N, K), (M, N)))
+    assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N, M, N, K, 0, None, None, 0, 0.0, 0) != 0
+    assert "launch" in pkg.last_error()
+    pkg.lib.hd_cuda_clear_error()
+    for rows in (4, 200):           # the row kernel and a norm, which look at CUDA's last error after their launch
+        pkg.lib.hd_linear(pkg.ptr(x), pkg.ptr(w), None, pkg.ptr(y), rows, N, K, 1)
+        pkg.check_cuda_errbuf("hd_linear after a refused launch")
+    pkg.lib.hd_rmsnorm(pkg.ptr(x), pkg.ptr(w), pkg.ptr(y), 4, K, 1e-6)
+    pkg.check_cuda_errbuf("hd_rmsnorm after a refused launch")
+    assert float(torch.ones(8, device=dev).sum()) == 8.0
