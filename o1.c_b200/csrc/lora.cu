@@ -338,6 +338,7 @@ struct LoraGroup {
         return false;
     }
     bool low_rank = true;                    // up to 64 all of them, or above 64 all of them
+    bool launched = false;                   // by any launch of the call
     template <int NCH>
     bool launch_as(cudaStream_t st) {
         static std::atomic<uint64_t> attr_done{0};
@@ -350,6 +351,7 @@ struct LoraGroup {
         if (a.count == 0) return true;
         a.err = device_error_word();
         if (!(low_rank ? launch_as<1>(st) : launch_as<2>(st))) return false;
+        launched = true;
         a.count = a.tiles = 0;
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) { set_error("lora: launch: %s", cudaGetErrorString(e)); return false; }
@@ -363,7 +365,9 @@ using namespace o1;
 
 extern "C" {
 
-// Returns once the merge is done, so that the caller may release the adapters.
+// Returns once the merge is done, so that the caller may release the adapters.  HD_ERR_RUNTIME when it was not: an error of
+// the stream, or the device's error word set, in which case the kernel merges nothing (it was set before) or stops on the way
+// (one of its waits ran out).
 hd_status hd_lora_merge_gpu(hd_lora_entry* entries, size_t count, void* stream) {
     if (count == 0) return HD_OK;
     if (!entries) { set_error("lora: null entries"); return HD_ERR_MISSING; }
@@ -410,8 +414,18 @@ hd_status hd_lora_merge_gpu(hd_lora_entry* entries, size_t count, void* stream) 
     }
     // (an entry that cannot be used ends the call; the ones before it are merged)
     if (!grp.launch(st) && rc == HD_OK) rc = HD_ERR_RUNTIME;
-    cudaStreamSynchronize(st);
-    return rc;
+    int word = 0;
+    cudaError_t e = cudaSuccess;
+    if (grp.launched) e = cudaMemcpyAsync(&word, device_error_word(), sizeof(int), cudaMemcpyDeviceToHost, st);
+    const cudaError_t e2 = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = e2;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_error("lora: %s", cudaGetErrorString(e));
+    } else if (word != 0) {
+        set_error("lora: the device's error word is set (code %d): the weights are not, or not all, merged", word);
+    }
+    return rc == HD_OK && (e != cudaSuccess || word != 0) ? HD_ERR_RUNTIME : rc;
 }
 
 }  // extern "C"

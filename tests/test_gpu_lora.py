@@ -140,3 +140,27 @@ def test_lora_merge_tile_edges(pkg, dev, shapes, shift):
         got = w[:n].double()
         assert ((got >= lo) & (got <= hi)).all(), (n, k, r, ((got < lo) | (got > hi)).sum().item())
         assert torch.equal(w[n:].view(torch.int16), w0[n:].view(torch.int16)), "rows beyond N were written"
+
+
+def test_lora_merge_reports_a_device_that_has_failed(pkg, dev):
+    """After a kernel ran into its wait limit the merge kernel does nothing, and the call says so; once the error word has been
+    read, the same call merges."""
+    from latefail import late_failure
+    n, k, r = 256, 128, 8
+    g = torch.Generator(device=dev).manual_seed(3)
+    w = torch.empty(n, k, device=dev).normal_(0, 0.02, generator=g).bfloat16()
+    up = torch.empty(n, r, device=dev).normal_(0, 0.05, generator=g)
+    down = torch.empty(r, k, device=dev).normal_(0, 0.05, generator=g)
+    w0 = w.clone()
+    ents = (pkg.LoraEntry * 1)(entry(pkg, w, up, down, r, k, n, 1.0, 1.0))
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    late_failure(pkg, 99)
+    try:
+        assert pkg.lib.hd_lora_merge_gpu(ents, 1, stream) == 8            # HD_ERR_RUNTIME
+        assert "error word" in pkg.last_error()
+        assert torch.equal(w.view(torch.int16), w0.view(torch.int16))
+    finally:
+        assert pkg.lib.o1_device_error() == 99       # reads and clears the word
+    pkg.lib.hd_cuda_clear_error()
+    assert pkg.lib.hd_lora_merge_gpu(ents, 1, stream) == 0
+    assert not torch.equal(w.view(torch.int16), w0.view(torch.int16))
