@@ -414,6 +414,10 @@ hd_status hd_lora_merge_gpu(hd_lora_entry* entries, size_t count, void* stream) 
     }
     // (an entry that cannot be used ends the call; the ones before it are merged)
     if (!grp.launch(st) && rc == HD_OK) rc = HD_ERR_RUNTIME;
+    // A call whose targets all took the simple kernel may be part of a stream capture: there is nothing to wait for then.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!grp.launched && cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+    if (cap != cudaStreamCaptureStatusNone) return rc;
     int word = 0;
     cudaError_t e = cudaSuccess;
     if (grp.launched) e = cudaMemcpyAsync(&word, device_error_word(), sizeof(int), cudaMemcpyDeviceToHost, st);

@@ -164,3 +164,29 @@ def test_lora_merge_reports_a_device_that_has_failed(pkg, dev):
     pkg.lib.hd_cuda_clear_error()
     assert pkg.lib.hd_lora_merge_gpu(ents, 1, stream) == 0
     assert not torch.equal(w.view(torch.int16), w0.view(torch.int16))
+
+
+def test_lora_merge_without_tiles_can_be_captured(pkg, dev):
+    """Targets that take the simple kernel (in_dim no multiple of 128) need neither a wait nor host work between their
+    launches: the call can be captured, and each replay merges the adapter once more."""
+    n, k, r = 40, 100, 4
+    g = torch.Generator(device=dev).manual_seed(5)
+    w = torch.empty(n, k, device=dev).normal_(0, 0.02, generator=g).bfloat16()
+    up = torch.empty(n, r, device=dev).normal_(0, 0.05, generator=g)
+    down = torch.empty(r, k, device=dev).normal_(0, 0.05, generator=g)
+    w0 = w.clone()
+    ents = (pkg.LoraEntry * 1)(entry(pkg, w, up, down, r, k, n, 1.0, 1.0))
+    eager = []
+    for _ in range(2):
+        assert pkg.lib.hd_lora_merge_gpu(ents, 1, C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        eager.append(w.clone())
+    w.copy_(w0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert pkg.lib.hd_lora_merge_gpu(ents, 1, C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0, pkg.last_error()
+    assert torch.equal(w.view(torch.int16), w0.view(torch.int16))
+    for want in eager:
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(w.view(torch.int16), want.view(torch.int16))
