@@ -495,11 +495,13 @@ void o1_attention_tail_ways(int ways);
  * the one-tile kernel (environment O1_ATTN_TILE_MODE sets the initial value).  Same arithmetic up to fp32 summation
  * order and the reference max of the lazy rescale. */
 void o1_attention_tile_mode(int mode);
-/* GEMM tile form of the plain, bias, residual, SwiGLU and grouped q|k|v families: 1 (default; environment O1_GEMM_PAIR=0
- * turns it off) = where that takes the fewest rounds of tiles, a cluster of two CTAs per 256 x 256 tile with
- * cta_group::2 MMAs, each CTA holding 128 rows of A and of the accumulator and half of the B tile; 0 = always one CTA
- * per tile.  All forms add a row's K products in the same order: same bits.  No reference
- * counterpart (cuBLASLt picks its own kernels there, src/cuda/gemm.cu:413-461). */
+/* Clusters of CTAs in the GEMMs: 1 (default, as is every value but 0; environment O1_GEMM_PAIR=0 turns them off) = the plain,
+ * bias, residual, SwiGLU and grouped q|k|v families take, where that needs the fewest rounds of tiles, two CTAs per
+ * 256 x 256 tile with cta_group::2 MMAs, each CTA holding 128 rows of A and of the accumulator and half of the B tile; and a
+ * linear of the vision tower that has few tiles shares the K of a tile among up to six CTAs.  0 = always one CTA per tile, no
+ * cluster is launched.  The pairs add a row's K products in the order of single CTAs: same bits.  The shared K is another
+ * order of the fp32 sum, so the tower's outputs (hd_vision_forward) at small images depend on the mode within rounding;
+ * those of the decoder do not.  No reference counterpart (cuBLASLt picks its own kernels there, src/cuda/gemm.cu:413-461). */
 void o1_gemm_pair_mode(int mode);
 /* CTA pairs of the GEMM kernel the current device holds at once (the pair form never launches more); -1 on error. */
 int o1_gemm_pair_capacity(void);

@@ -1192,7 +1192,8 @@ bool func_attr_once(std::atomic<uint64_t>& done, const void* func, int smem_byte
     return true;
 }
 
-// 0: single-CTA tiles only; else CTA pairs where tile_form() finds them the better form (the default)
+// 0: single CTAs only, no cluster is launched; else CTA pairs where tile_form() finds them the better form and, for callers
+// that allow it, K split over a cluster (the default)
 static int g_pair_mode = -1;
 void gemm_pair_mode(int mode) { g_pair_mode = mode; }
 static bool pair_wanted() {
@@ -1527,7 +1528,7 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
         return launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
     }
     if (force_bn <= 0 && !o_cb && !o_tab) {
-        const SplitPlan p = split_plan(M, N, K, force_bn == GEMM_SPLIT_K);
+        const SplitPlan p = split_plan(M, N, K, force_bn == GEMM_SPLIT_K && pair_wanted());
         if (p.bn > 0) switch (epi) {
             case EPI_STORE: return launch_split<EPI_STORE>(tA, w, g, p, st);
             case EPI_BIAS:  return launch_split<EPI_BIAS>(tA, w, g, p, st);

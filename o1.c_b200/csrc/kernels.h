@@ -32,7 +32,8 @@ void prof_after(cudaStream_t st);
 // force_bn: 0 = tile chosen by shape, 128 / 256 = that tile width; every output element is summed by one CTA in the order
 // of k, so that a row's result does not depend on the tile or on how many other rows the call has (the decoder's layers
 // rely on that: a row is the same in a sharded, a cached or a paired pass).  GEMM_SPLIT_K = chosen by shape, and a problem
-// of few tiles may share a tile's K among CTAs, which is another order of the FP32 sum.
+// of few tiles may share a tile's K among the CTAs of a cluster, which is another order of the FP32 sum (not in mode 0 of
+// gemm_pair_mode).
 enum { GEMM_SPLIT_K = -1 };
 bool gemm_bf16(const void* x, const void* w, const void* w2, void* y, int M, int N, int K, int epi,
                const void* bias, const void* resid, float scale, int force_bn, cudaStream_t st);
@@ -88,7 +89,7 @@ bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cuda
 void attention_tail_ways(int ways);
 void attention_tile_mode(int mode);   // 0: by sequence length; 1: two query tiles per CTA; 2: one query tile per CTA
 int gemm_pair_capacity();
-void gemm_pair_mode(int mode);   // 0: single-CTA GEMM tiles only; else CTA pairs (cta_group::2) where they are the better form
+void gemm_pair_mode(int mode);   // 0: single CTAs only; else clusters (CTA pairs, K split) where they are the better form
 // seq-major operands; output rows [b*out_rows, (b+1)*out_rows) go to out_tab[b] (row-major, leading
 // dimension ldo), which may be peer-mapped memory of another GPU
 bool flash_attention_tab(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,

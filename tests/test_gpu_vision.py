@@ -332,3 +332,29 @@ def test_fused_projection_equals_the_separate_pass(pkg, dev, tower, gh, gw):
     assert torch.equal(b0.view(torch.int16), outs[0].view(torch.int16))
     assert torch.equal(emb, emb2) and torch.equal(ds, ds2)
     assert pkg.lib.o1_device_error() == 0
+
+
+@pytest.mark.parametrize("gh,gw", [(12, 8), (26, 20), (34, 18)])
+def test_no_clusters_means_no_shared_k(pkg, dev, tower, gh, gw):
+    """o1_gemm_pair_mode(0) promises one CTA per tile: the tower's linears then keep a tile's K in one CTA, so that a linear is
+    bit for bit the one of force_bn = 0, and the tower repeats itself; the default differs from it within rounding only."""
+    _, _, binding = tower
+    px = seeded_bf16((gh * gw, 1536), 21)
+    n, k = 1152, 4304
+    x, w, b = (dv(seeded_bf16(s, 31 + i, 0.0, 0.05), dev) for i, s in enumerate(((gh * gw, k), (n, k), n)))
+    try:
+        pkg.lib.o1_gemm_pair_mode(0)
+        ys = []
+        for bn in (-1, 0):
+            y = empty_bf16((gh * gw, n), dev)
+            assert pkg.lib.o1_gemm(pkg.ptr(x), k, pkg.ptr(w), None, pkg.ptr(y), n, gh * gw, n, k, 1, pkg.ptr(b), None, 0, 0.0, bn) == 0
+            ys.append(y)
+        done(pkg, "gemm")
+        assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
+        one = [run_tower(pkg, dev, binding, px, gh, gw, snaps=False)[:2] for _ in range(2)]
+    finally:
+        pkg.lib.o1_gemm_pair_mode(1)
+    two = run_tower(pkg, dev, binding, px, gh, gw, snaps=False)[:2]
+    for a, b2, c in zip(one[0], one[1], two):
+        assert torch.equal(a.view(torch.int16), b2.view(torch.int16))
+        assert_close(a, c, "V", "single CTAs against clusters")
