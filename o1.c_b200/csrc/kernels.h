@@ -87,6 +87,7 @@ bool flash_attention_hm(const void* q, const void* k, const void* v, void* out, 
 bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cudaStream_t st);
 // tail split policy of flash_attention*: 0 = automatic, 1 = never, n = n key-range parts when they fit
 void attention_tail_ways(int ways);
+bool attention_two_tile_only();       // mode 1 is set
 void attention_tile_mode(int mode);   // 0: by sequence length; 1: two query tiles per CTA; 2: one query tile per CTA
 int gemm_pair_capacity();
 void gemm_pair_mode(int mode);   // 0: single CTAs only; else clusters (CTA pairs, K split) where they are the better form

@@ -383,6 +383,16 @@ __global__ void split_rope_pad_kernel(const uint16_t* __restrict__ qkv, const fl
     }
     *reinterpret_cast<uint4*>(out + (size_t)s * 3 * V_HEADS * V_DP + (size_t)which * V_HEADS * V_DP + (size_t)h * V_DP + g * 8) = o;
 }
+// attention output [n, 16*128] (heads 128 apart) -> [n, 16*72]
+__global__ void unpad_heads_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int n) {
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;      // one 16-byte piece per thread
+    constexpr int PIECES = V_HEADS * (V_D / 8);
+    if (i >= (long)n * PIECES) return;
+    const long s = i / PIECES;
+    const int p = (int)(i - s * PIECES), h = p / (V_D / 8), c = (p - h * (V_D / 8)) * 8;
+    *reinterpret_cast<uint4*>(out + (size_t)s * V_H + h * V_D + c) =
+        *reinterpret_cast<const uint4*>(in + ((size_t)s * V_HEADS + h) * V_DP + c);
+}
 // GEMM + bias (+ GELU) on the tensor-core kernel where its tiles apply, otherwise the SIMT GEMM and a GELU pass
 static bool linear_act(const void* x, const void* w, const void* b, void* y, int M, int N, int K, int act /*0 none, 1 tanh, 2 erf*/,
                        cudaStream_t st, int* launches) {
@@ -607,6 +617,7 @@ hd_status hd_vision_forward(const hd_vision_binding* bw, hd_vision_workspace* ws
     uint16_t* fc2 = (uint16_t*)(base + o.fc2);
     uint16_t* qkvp = (uint16_t*)(base + o.q);
     uint16_t* qkv = (uint16_t*)(base + o.qkv);
+    uint16_t* attn_pad = (uint16_t*)(base + o.scores);
     uint16_t* attn_out = (uint16_t*)(base + o.attn_out);
     uint16_t* fc1 = (uint16_t*)(base + o.fc1);
     float* cosf_t = (float*)(base + o.cosf);
@@ -636,20 +647,32 @@ hd_status hd_vision_forward(const hd_vision_binding* bw, hd_vision_workspace* ws
         void** s0 = i == 0 ? ws->block0_snaps : nullptr;
         VIS_TRY(vision_layernorm(cur_in, blk->norm1_w, blk->norm1_b, ln1, n, V_H, eps, st));
         // bias, rotary and the wider spacing of the heads ride in the projection's epilogue, and attention works on (and
-        // writes) 72 columns a head, unless a snapshot asks for the bare projection or there are too few rows for tiles
-        const bool fuse_qkv = gemm_tc_supported(n, 3 * V_H, V_H, EPI_BIAS) && !(s0 && s0[HD_B0_QKV]);
+        // writes) 72 columns a head, unless a snapshot asks for the bare projection or there are too few rows for tiles.
+        // The two-tile attention kernel, where a program asks for it, works on heads zero-padded to 128 columns.
+        const bool whole_heads = attention_two_tile_only();
+        const bool fuse_qkv = !whole_heads && gemm_tc_supported(n, 3 * V_H, V_H, EPI_BIAS) && !(s0 && s0[HD_B0_QKV]);
         if (fuse_qkv) {
             VIS_TRY(gemm_vision_qkv(ln1, blk->qkv_w, blk->qkv_b, qkvp, n, cosf_t, sinf_t, st));
-            VIS_TRY(flash_attention_vision(qkvp, attn_out, n, scaling, st));
-            launches += 2;
+            ++launches;
         } else {
             // (whole-K tiles, as the fused form has them: both give the same bits)
             VIS_TRY(gemm_bf16(ln1, blk->qkv_w, nullptr, qkv, n, 3 * V_H, V_H, EPI_BIAS, blk->qkv_b, nullptr, 0.f, 0, st));
             const long total = (long)n * 3 * V_HEADS * (V_DP / 8);
             split_rope_pad_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(qkv, cosf_t, sinf_t, qkvp, n);
             VIS_TRY(cudaGetLastError() == cudaSuccess);
-            VIS_TRY(flash_attention_vision(qkvp, attn_out, n, scaling, st));
             launches += 2;
+        }
+        if (whole_heads) {
+            constexpr int LD = 3 * V_HEADS * V_DP;
+            VIS_TRY(flash_attention(qkvp, LD, qkvp + V_HEADS * V_DP, LD, qkvp + 2 * V_HEADS * V_DP, LD, attn_pad, V_HEADS * V_DP, n,
+                                    V_HEADS, V_HEADS, 0, scaling, st));
+            const long total = (long)n * V_HEADS * (V_D / 8);
+            unpad_heads_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(attn_pad, attn_out, n);
+            VIS_TRY(cudaGetLastError() == cudaSuccess);
+            launches += 2;
+        } else {
+            VIS_TRY(flash_attention_vision(qkvp, attn_out, n, scaling, st));
+            ++launches;
         }
         // the two residual adds ride in the projections' epilogues unless a snapshot asks for the bare projection
         // (or the row count is below the tensor-core tile minimum)

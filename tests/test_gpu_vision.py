@@ -358,3 +358,23 @@ def test_no_clusters_means_no_shared_k(pkg, dev, tower, gh, gw):
     for a, b2, c in zip(one[0], one[1], two):
         assert torch.equal(a.view(torch.int16), b2.view(torch.int16))
         assert_close(a, c, "V", "single CTAs against clusters")
+
+
+def test_attention_tile_mode_holds_for_the_tower(pkg, dev, tower):
+    """o1_attention_tile_mode(1) is the two-tile kernel everywhere, the tower included: other bits than the one-tile form of
+    modes 0 and 2 (another order of the sums, another reference max), the same results within rounding."""
+    _, _, binding = tower
+    gh, gw = 26, 20
+    px = seeded_bf16((gh * gw, 1536), 23)
+    out = {}
+    try:
+        for mode in (0, 1, 2):
+            pkg.lib.o1_attention_tile_mode(mode)
+            out[mode] = run_tower(pkg, dev, binding, px, gh, gw)
+    finally:
+        pkg.lib.o1_attention_tile_mode(0)
+    b0 = {m: o[2][0].view(torch.int16) for m, o in out.items()}
+    assert torch.equal(b0[0], b0[2])
+    assert not torch.equal(b0[0], b0[1])
+    assert_close(out[1][2][0], out[0][2][0], "D", "block 0 output")
+    assert_close(out[1][0], out[0][0], "V", "image_embeds")
