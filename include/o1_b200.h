@@ -401,7 +401,8 @@ typedef struct {
  * merge_fc2, ds_fc2).  q, k, v are the three 2048-column slices of one [n, 6144] buffer: head h occupies
  * columns 128h .. 128h+71 of its slice, the remaining 56 are zero, q and k are already rotated (qr = q,
  * kr = k).  `scores` is the attention output in the same padded form [n, 2048]; cosf / sinf are [n, 72] fp32;
- * mlp_resid = h_b (where the 27th block leaves its output). */
+ * mlp_resid = h_b (where the 27th block leaves its output).  After hd_vision_forward the tensors are those of the
+ * 27th block. */
 typedef struct {
     int64_t patch_out, pos_emb, rot, h_a, h_b, ln1, attn_resid, ln2, fc2, mlp_resid, q, k, v, qr, kr, qkv,
         scores, probs, mask, attn_out, fc1, cosf, sinf, merged, merge_norm, merge_fc1, merge_fc2, ds_merged,

@@ -648,8 +648,10 @@ hd_status hd_vision_forward(const hd_vision_binding* bw, hd_vision_workspace* ws
         VIS_TRY(vision_layernorm(cur_in, blk->norm1_w, blk->norm1_b, ln1, n, V_H, eps, st));
         // bias, rotary and the wider spacing of the heads ride in the projection's epilogue, and attention works on (and
         // writes) 72 columns a head, unless a snapshot asks for the bare projection or there are too few rows for tiles.
-        // The two-tile attention kernel, where a program asks for it, works on heads zero-padded to 128 columns.
-        const bool whole_heads = attention_two_tile_only();
+        // The two-tile attention kernel, where a program asks for it, works on heads zero-padded to 128 columns.  So does the
+        // last block: what the workspace then holds is what hd_vision_layout describes (q, k, v and scores padded with
+        // zeros, qkv the bare projection).
+        const bool whole_heads = attention_two_tile_only() || i == V_DEPTH - 1;
         const bool fuse_qkv = !whole_heads && gemm_tc_supported(n, 3 * V_H, V_H, EPI_BIAS) && !(s0 && s0[HD_B0_QKV]);
         if (fuse_qkv) {
             VIS_TRY(gemm_vision_qkv(ln1, blk->qkv_w, blk->qkv_b, qkvp, n, cosf_t, sinf_t, st));

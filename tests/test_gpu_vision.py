@@ -378,3 +378,41 @@ def test_attention_tile_mode_holds_for_the_tower(pkg, dev, tower):
     assert not torch.equal(b0[0], b0[1])
     assert_close(out[1][2][0], out[0][2][0], "D", "block 0 output")
     assert_close(out[1][0], out[0][0], "V", "image_embeds")
+
+
+@pytest.mark.parametrize("gh,gw", [(2, 2), (8, 12), (26, 20)])
+def test_workspace_tensors_are_those_of_the_layout(pkg, dev, tower, gh, gw):
+    """After a forward the workspace holds what hd_vision_layout describes, whatever it held before (NaN here): the bare
+    projection, q | k | v in heads of 128 columns with 56 zeros, v being the projection's, and the attention output in the
+    same padded form and in the dense one."""
+    _, _, binding = tower
+    n = gh * gw
+    off = pkg.VisionOffsets()
+    pkg.lib.hd_vision_layout(n, n // 4, C.byref(off))
+    ws = pkg.VisionWorkspace()
+    space = torch.full((pkg.lib.hd_vision_workspace_bytes(n),), 0xff, dtype=torch.uint8, device=dev)
+    tables = torch.zeros(pkg.lib.hd_vision_tables_bytes(n), dtype=torch.uint8, device=dev)
+    ws.patch_out, ws.tables, ws.tables_n = space.data_ptr(), tables.data_ptr(), -1
+    assert pkg.lib.hd_vision_prepare_tables(C.byref(ws), n, gh, gw) == 0
+    px = seeded_bf16((n, 1536), 27)
+    pxd, emb = u16_to_torch(px, dev), empty_bf16((n // 4, 4096), dev)
+    assert pkg.lib.hd_vision_forward(C.byref(binding), C.byref(ws), pkg.ptr(pxd), n, gh, gw, pkg.ptr(emb), None) == 0
+    done(pkg, "vision")
+
+    def view(at, cols):
+        return space[at:at + n * cols * 2].view(torch.bfloat16).view(n, cols)
+
+    heads = view(off.q, 3 * 16 * 128).view(n, 3, 16, 128)
+    qkv = view(off.qkv, 3 * 1152).view(n, 3, 16, 72)
+    scores, dense = view(off.scores, 16 * 128).view(n, 16, 128), view(off.attn_out, 1152).view(n, 16, 72)
+    bits = lambda t: t.contiguous().view(torch.int16)  # noqa: E731
+    assert (bits(heads[..., 72:]) == 0).all()
+    assert torch.equal(bits(heads[:, 2, :, :72]), bits(qkv[:, 2]))
+    assert torch.equal(bits(scores[..., :72]), bits(dense))
+    assert (scores[..., 72:] == 0).all()
+    # a rotation keeps the length of each pair of components
+    a, b = heads[:, :2, :, :72].float(), qkv[:, :2].float()
+    norm = lambda t: (t[..., :36] ** 2 + t[..., 36:] ** 2).sqrt()  # noqa: E731
+    assert ((norm(a) - norm(b)).abs() <= 2.0 ** -7 * norm(b) + 1e-6).all()
+    want = run_tower(pkg, dev, binding, px, gh, gw, snaps=False)[0]
+    assert torch.equal(bits(emb), bits(want))
