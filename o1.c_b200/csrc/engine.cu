@@ -703,24 +703,25 @@ static int64_t forward_layout(int64_t seq, int text_len, int img, int hidden, in
     return o;
 }
 
-// Up to this many rows per branch a guided step runs both branches in one pass.  Below it the GEMMs of one branch leave
-// part of the SMs idle and stream all weights for few rows (296 rows: 229 us a block, twice); from a few thousand rows on
-// one branch fills the machine, and the second set of activations would only cost memory.
-static constexpr int64_t PAIRED_ROWS = 2048;
+// Up to O1_PAIRED_ROWS rows per branch a guided step runs both branches in one pass, where the workspace has the room: the
+// GEMMs of one branch leave part of the SMs idle and stream all weights for few rows.  A guided step of six blocks, one after
+// the other / paired, in ms: 300 rows 2.36 / 1.55, 700 rows 3.59 / 2.93, 1040 rows 5.26 / 4.41, 1280 rows 5.83 / 4.85, 1600
+// rows 7.40 / 6.50, 2048 rows 8.97 / 8.66: the gain has run out there, and the second set of activations costs memory.
+// The room is known from block_scratch_bytes, which the host sets together with the region's size.  A region of seq rows
+// holds a pair of Sc + Su <= seq rows in all: its two branches have the same image rows, so per row they need less than
+// one sequence (text + 2 * image = Sc + Su, and a text row takes 2 * hidden bytes, an image row 2 * (1024 + hidden)
+// with hidden >= 1024).
+static bool pair_fits(const hd_forward_workspace* ws, int64_t Sc, int64_t Su, int heads, int kv_heads, int hidden, int ff, int hd) {
+    return Sc <= O1_PAIRED_ROWS && Su <= O1_PAIRED_ROWS && hidden >= 1024 &&
+           ws->block_scratch_bytes >= hd_decoder_block_scratch_bytes(Sc + Su, heads, kv_heads, hidden, ff, hd);
+}
 
 int64_t hd_forward_workspace_bytes(int64_t seq, int img_tokens, int heads, int kv_heads, int hidden,
                                    int ff_hidden, int head_dim, int64_t* block_scratch_bytes) {
     int64_t off[WS_COUNT];
     int64_t text = seq - img_tokens;
     if (text < 0) text = 0;
-    const int64_t one = forward_layout(seq, (int)text, img_tokens, hidden, heads, kv_heads, ff_hidden, head_dim, off,
-                                       block_scratch_bytes);
-    // room for two branches of any shorter length in one pass as well: the layout of twice the rows, their text rows,
-    // and the x_embedder rows
-    const int64_t s2 = seq < PAIRED_ROWS ? seq : PAIRED_ROWS;
-    const int64_t two = forward_layout(2 * s2, 0, 0, hidden, heads, kv_heads, ff_hidden, head_dim, off, nullptr) +
-                        2 * s2 * hidden * 2 + s2 * (1024 + hidden) * 2 + 4096;
-    return one > two ? one : two;
+    return forward_layout(seq, (int)text, img_tokens, hidden, heads, kv_heads, ff_hidden, head_dim, off, block_scratch_bytes);
 }
 
 int64_t hd_forward_ws_offset(const char* name, int64_t seq, int text_len, int img_tokens, int heads,
@@ -1020,7 +1021,7 @@ hd_status o1_denoise_step_cfg_branches(const hd_forward_binding* bw, hd_forward_
     // the predictions lie behind one another in xp_scratch, as the rows of a paired pass do
     FwdSeg seg[2] = {{cond->ids, cond->text_len, cond->pos_f32, cond->ar_len, cond->visual, 0, Sc},
                      {uncond->ids, uncond->text_len, uncond->pos_f32, uncond->ar_len, uncond->visual, Sc, Su}};
-    if (Sc <= PAIRED_ROWS && Su <= PAIRED_ROWS && !cond->visual == !uncond->visual) {
+    if (!cond->visual == !uncond->visual && pair_fits(ws, Sc, Su, heads, kv_heads, hidden, ff_hidden, head_dim)) {
         const hd_status s = forward_impl(bw, ws, seg, 2, z, img_tokens, timestep_dev, heads, kv_heads, hidden, ff_hidden,
                                          head_dim, tms_token_id, nullptr, xc, g_stream);
         if (s != HD_OK) return s;

@@ -22,6 +22,7 @@ SLOT_NAMES = ["q_proj", "k_proj", "v_proj", "o_proj", "input_ln", "post_ln", "ga
 GLOBAL_NAMES = ["embed_tokens", "te0_w", "te0_b", "te2_w", "te2_b", "xe1_w", "xe2_w", "xe2_b", "fl_w",
                 "fl_b", "fnorm_w"]
 NORM_NAMES = {"input_ln", "post_ln", "q_norm", "k_norm", "fnorm_w"}
+PAIRED_ROWS = 2048      # O1_PAIRED_ROWS: the most rows of a branch that runs in one pass with the other
 DEV_TIMESTEPS = [999, 987, 974, 960, 945, 929, 913, 895, 877, 857, 836, 814, 790, 764, 737, 707, 675,
                  640, 602, 560, 515, 464, 409, 347, 278, 199, 110, 8]
 
@@ -171,9 +172,10 @@ class Weights:
 
 
 class Engine:
-    """Workspace + call wrappers for one sequence geometry on one GPU."""
+    """Workspace + call wrappers for one sequence geometry on one GPU.  guided: the workspace has the room to run both branches
+    of a guided step in one pass (about twice the bytes; without it they run one after the other, with the same bits)."""
 
-    def __init__(self, weights, text_len, img_tokens, ar_len=None):
+    def __init__(self, weights, text_len, img_tokens, ar_len=None, guided=True):
         self.w = weights
         self.T, self.I, self.S = text_len, img_tokens, text_len + img_tokens
         self.ar_len = text_len - 1 if ar_len is None else ar_len
@@ -183,6 +185,8 @@ class Engine:
         bs = C.c_int64(0)
         nbytes = lib.hd_forward_workspace_bytes(self.S, self.I, *self.dimargs, C.byref(bs))
         self.block_scratch_bytes = bs.value
+        if guided and self.S <= PAIRED_ROWS:
+            nbytes = lib.hd_forward_workspace_bytes(2 * self.S, self.I, *self.dimargs, C.byref(bs))
         self.ws_buf = torch.empty(nbytes + 256, dtype=torch.uint8, device=self.device)
         self.ws = ForwardWorkspace()
         self.ws.hidden_a = self.ws_buf.data_ptr()

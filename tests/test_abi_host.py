@@ -60,6 +60,8 @@ def test_workspace_layout(pkg):
     assert len(set(offs.values())) == len(offs)
     assert offs["hidden_a"] == 0 and offs["hidden_b"] == S * 4096 * 2
     assert lib.hd_forward_ws_offset(b"nope", S, S - I, I, 32, 8, 4096, 12288, 128, None) == -1
+    # one sequence, no more: the room for a guided step's second branch is asked for by its rows
+    assert total == offs["block_scratch"] + (bs.value + 255) // 256 * 256
     # scratch grows linearly in S
     b2 = lib.hd_decoder_block_scratch_bytes(2 * S, 32, 8, 4096, 12288, 128)
     assert abs(b2 - 2 * bs.value) < 8192
@@ -299,3 +301,21 @@ def test_reference_harness_mirrors_the_seeded_arena_rules(pkg):
     assert C.sizeof(rh.ForwardWorkspace) == C.sizeof(pkg.ForwardWorkspace)
     assert C.sizeof(rh.BlockBinding) == C.sizeof(pkg.BlockBinding)
     assert C.sizeof(rh.ForwardDiagnostics) == C.sizeof(pkg.ForwardDiagnostics)
+
+
+@pytest.mark.parametrize("H,ff,heads,kv", [(4096, 12288, 32, 8), (1024, 2048, 8, 2)])
+def test_a_workspace_of_both_branches_rows_holds_the_pair(pkg, H, ff, heads, kv):
+    """A guided step runs both branches in one pass where block_scratch_bytes covers their rows together.  Whatever share of
+    image rows the region was sized with, it then holds that pass: its regions take, for Sc + Su = S rows of which two times I
+    are image rows, no more than those of one sequence of S rows."""
+    def total(seq, img):
+        return pkg.lib.hd_forward_workspace_bytes(seq, img, heads, kv, H, ff, 128, None)
+
+    for S in (16, 77, 592, 1281, 4096):
+        for img in {0, 1, S // 3, S - 1}:
+            region = total(S, img)
+            for I in {1, S // 5, (S - 2) // 2}:
+                text = S - 2 * I
+                # the pass: S rows in all activations, the text rows of both branches, the x_embedder rows once
+                pair = total(S, 0) - S * H * 2 + text * H * 2 + I * (1024 + H) * 2
+                assert pair <= region, (S, img, I)

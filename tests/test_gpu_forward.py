@@ -455,3 +455,40 @@ def test_paired_step_equals_two_forwards(pkg, dev, tc, tu, gh, gw, visual):
     assert torch.equal(xp[tc + I:].view(torch.int16), xs[1].view(torch.int16))
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     assert pkg.lib.o1_device_error() == 0
+
+
+@pytest.mark.parametrize("room", ["longer", "sum - 1", "sum"])
+def test_guided_step_stays_inside_the_workspace_it_was_given(pkg, dev, room):
+    """The branches run one after the other in a workspace sized for the longer one and together in one sized for the sum of
+    their rows (and for not a row less): the same bits, and nothing behind the workspace is written."""
+    tc, tu, gh, gw, L = 40, 9, 14, 17, 8
+    I, Sc, Su = gh * gw, 40 + 14 * 17, 9 + 14 * 17
+    w = pkg.Weights(n_layers=L, seed=1234, weight_set="B", device=dev)
+    eng = pkg.Engine(w, tc, I, guided=False)
+    rows = {"longer": Sc, "sum - 1": Sc + Su - 1, "sum": Sc + Su}[room]
+    bs = C.c_int64(0)
+    nbytes = pkg.lib.hd_forward_workspace_bytes(rows, I, *eng.dimargs, C.byref(bs))
+    if room == "longer":
+        assert eng.ws_buf.numel() < nbytes + 1024           # what the engine without the second branch's room takes
+    buf = torch.full((nbytes + (1 << 20),), 0x5A, dtype=torch.uint8, device=dev)
+    eng.ws.hidden_a, eng.ws.block_scratch_bytes = buf.data_ptr(), bs.value
+    z = u16_to_torch(seeded_bf16((I, 3072), 61, 0.0, 4.0), dev)
+    br, keep, xs = [], [], []
+    for k, t in enumerate((tc, tu)):
+        pos, ar = pkg.seq_t2i(t, gh, gw)
+        ids, posd = torch.from_numpy(make_ids(t, 3 + k)).to(dev), pos.to(dev)
+        br.append((ids, posd, ar))
+        one = pkg.Engine(w, t, I, ar_len=ar, guided=False)
+        xs.append(one.forward(ids, posd, z, 0.2))
+        keep.append(one)
+    pkg.lib.o1_launch_count(1)
+    eng.denoise_step_cfg_branches(br[0], br[1], z, 0.8, 0.7, 5.0)
+    launches = pkg.lib.o1_launch_count(0)
+    torch.cuda.synchronize()
+    # seven launches a block: one pass has fewer than two passes' blocks alone
+    one_pass = launches < 2 * 7 * L
+    assert one_pass == (room == "sum"), launches
+    assert (buf[nbytes:] == 0x5A).all(), "written behind the workspace"
+    xp = eng.xp[:(Sc + Su) * 3072].view(-1, 3072)
+    assert torch.equal(xp[:Sc].view(torch.int16), xs[0].view(torch.int16))
+    assert torch.equal(xp[Sc:].view(torch.int16), xs[1].view(torch.int16))
