@@ -182,9 +182,8 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         return;
     }
 
-    // a kernel that already failed on this device leaves its code in *err: do nothing then
     if (threadIdx.x == 0) {
-        int ab = *reinterpret_cast<volatile int*>(a.err);
+        int ab = error_word(a.err);
         if (ab == 0 && (smem_u32(smem) & 1023u) != 0) { ab = 20; atomicExch(a.err, 20); }
         *s_abort = ab;
     }
@@ -407,8 +406,10 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
         // ---- output: O / l -> bf16 -> out[row_g, h*128 + half*64 ..]
         if (ok && n_tiles > 0) {
+            const int failed = error_word(a.err);
             if (!mbar_wait(o_done, 0)) { atomicExch(a.err, 19); ok = false; }
             tc_fence_after();
+            if (failed) ok = false;
         }
         // the row sum is the two threads' shares together (same exchange slots; every thread of the
         // group reaches this barrier: a failed wait above fails for the whole group alike)
@@ -592,10 +593,9 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         return;
     }
 
-    // a kernel that already failed on this device leaves its code in *err: do nothing then
-    // (the word is on its way while the barriers and tensor memory are set up)
+    // (the error word is on its way while the barriers and tensor memory are set up)
     if (threadIdx.x == 64) {
-        int ab = *reinterpret_cast<volatile int*>(a.err);
+        int ab = error_word(a.err);
         if (ab == 0 && (smem_u32(smem) & 1023u) != 0) { ab = 20; atomicExch(a.err, 20); }
         *s_abort = ab;
     }
@@ -850,8 +850,10 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         }
         // ---- output: O / l -> bf16 -> out[row_g, h*128 + part4*32 ..]
         if (ok) {
+            const int failed = error_word(a.err);
             if (!mbar_wait_warp(o_done, 0)) { atomicExch(a.err, 19); ok = false; }
             tc_fence_after();
+            if (failed) ok = false;
         }
         // the row sum is the four threads' shares together (the exchange window as [quarter][row] floats; every
         // softmax thread reaches these barriers: a failed wait above fails for all of them alike)

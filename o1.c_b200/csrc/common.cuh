@@ -71,6 +71,11 @@ __device__ __forceinline__ float rope_f32(float x, float c, float partner, float
 // block of 1280 rows 521 / 540 us; but a block of 4352 rows 1738 / 1712 us and of 16640 rows 9.52 / 9.25 ms.
 static constexpr long OVERLAP_ROWS = 4096;
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel that has failed (a wait ran out) leaves its code in the device's error word, and those after it store nothing.
+// A chained kernel reads the word twice: early, beside its set-up, to do nothing at all after a failure that lies behind; and,
+// since the kernels before it may still be running then, once more after grid_dep_wait(), in the threads that store, where
+// the wait for the first result hides the read.
+__device__ __forceinline__ int error_word(const int* err) { return *reinterpret_cast<const volatile int*>(err); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
 inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,

@@ -151,10 +151,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
-    // a kernel that already failed on this device leaves its code in *err: do nothing then (a pair decides together, after
-    // its cluster barrier).  The word is on its way while the barriers and tensor memory are set up.
+    // (a pair decides together, after its cluster barrier; the word is on its way while barriers and tensor memory are set up)
     __shared__ int s_abort;
-    if (threadIdx.x == 64) s_abort = *reinterpret_cast<volatile int*>(g.err);
+    if (threadIdx.x == 64) s_abort = error_word(g.err);
     const uint32_t rank = PAIR ? cluster_rank() : 0u;    // 0: the CTA that issues the pair's MMAs
 
     if (threadIdx.x == 0) {
@@ -297,14 +296,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int q = warp & 3;  // TMEM lane quadrant this warp may access
         int as = 0;
         uint32_t aphase = 0;
+        const int failed = error_word(g.err);
         for (int tile = tile0; tile < num_tiles; tile += tile_step) {
             int mb, nb;
             tile_coords(tile, sched_m, g.num_n, sched_group, mb, nb);
             if (PAIR) mb = mb * 2 + (int)rank;
             if (!mbar_wait(&tfull[as], aphase)) { atomicExch(g.err, 4); break; }
             tc_fence_after();
+            const int rows = failed ? 0 : g.M;
             const int row = mb * BM + q * 32 + lane;
-            const bool row_ok = row < g.M;
+            const bool row_ok = row < rows;
             const uint32_t t_row = tmem_base + as * BN + ((uint32_t)(q * 32) << 16);
             // EPI_QKV: which segment this column tile lies in decides the epilogue (warp-uniform); everything
             // below addresses the output through (seg_col0 + column inside the segment) or the segment's tables
@@ -370,7 +371,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         const int rr = k * 4 + (lane >> 3);
                         const uint4 o = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((ch ^ (rr & 7)) * 16));
                         const int grow = mb * BM + q * 32 + rr;
-                        if (grow < g.M) *reinterpret_cast<uint4*>(obase + (size_t)grow * g.ldo + ch * 8) = o;
+                        if (grow < rows) *reinterpret_cast<uint4*>(obase + (size_t)grow * g.ldo + ch * 8) = o;
                     }
                     __syncwarp();
                 }
@@ -467,7 +468,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 const int rr = k * 4 + (lane >> 3);
                                 const uint4 o = *reinterpret_cast<const uint4*>(stg + hf * (32 * 128) + rr * 128 + ((ch ^ (rr & 7)) * 16));
                                 const int grow = mb * BM + q * 32 + rr;
-                                if (grow < g.M) *reinterpret_cast<uint4*>(obase + (size_t)grow * g.ldo + hf * 64 + ch * 8) = o;
+                                if (grow < rows) *reinterpret_cast<uint4*>(obase + (size_t)grow * g.ldo + hf * 64 + ch * 8) = o;
                             }
                         __syncwarp();
                     }
@@ -675,7 +676,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int rank = (int)(blockIdx.x % ks), tile = (int)(blockIdx.x / ks);
     const int nb = tile / g.num_m, mb = tile - nb * g.num_m;      // CTAs that share weights run next to each other
 
-    if (threadIdx.x == 64) *s_abort = *reinterpret_cast<volatile int*>(g.err);
+    if (threadIdx.x == 64) *s_abort = error_word(g.err);
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
@@ -695,9 +696,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     grid_dep_launch();
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
-    // a kernel that already failed on this device leaves its code in *err: no loads and no results then, but the
-    // cluster's barriers below are passed all the same (the CTAs of a cluster may read the word at different times)
+    // after a failure no loads and no results, but the cluster's barriers below are passed all the same (the CTAs of a cluster
+    // may read the word at different times)
     bool ok = *s_abort == 0;
+    const int failed = warp >= 2 ? error_word(g.err) : 0;
 
     if (ok && warp == 0) {
         if (elect_one()) {
@@ -771,6 +773,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
     }
+    const bool store = row_ok && !failed;
     const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
     if constexpr (EPI == EPI_VROPE) {
         if (ok && warp >= 2) {
@@ -781,7 +784,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 tmem_ld32(t_row + hh * 72 + 32, rb);
                 tmem_ld8(t_row + hh * 72 + 64, rc);
                 tmem_ld_wait();
-                if (row < g.M) {
+                if (store) {
                     const int col = nb * VQ_BN + hh * 72, which = col / 1152, h = (col - which * 1152) / 72;
                     float x[72];
 #pragma unroll
@@ -859,7 +862,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             if (u < u0 || u >= u1) continue;
             const int col = nb * BN + u * 16;
             // (N is a multiple of eight: a unit is whole, its first half, or outside)
-            const bool h0 = row_ok && col < g.N, h1 = row_ok && col + 8 < g.N;
+            const bool h0 = store && col < g.N, h1 = store && col + 8 < g.N;
             uint32_t r[16];
             tmem_ld16(t_row + u * 16, r);
             tmem_ld_wait();
@@ -934,7 +937,7 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     const int warp = warp_index(), lane = threadIdx.x & 31;
-    if (threadIdx.x == 64) *s_abort = *reinterpret_cast<volatile int*>(g.err);
+    if (threadIdx.x == 64) *s_abort = error_word(g.err);
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
@@ -1005,6 +1008,7 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int q = warp & 3;       // TMEM lane quadrant this warp may access
         int as = 0;
         uint32_t aphase = 0;
+        const int failed = error_word(g.err);
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
             int mb, nb;
             tile_coords(tile, g.num_m, g.num_n, g.group_m, mb, nb);
@@ -1030,7 +1034,7 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 uint32_t r[16];
                 tmem_ld16(t_row + c, r);
                 tmem_ld_wait();
-                if (row_ok) {
+                if (row_ok && !failed) {
                     uint4* dst = reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + col0 + c);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {

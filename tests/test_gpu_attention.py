@@ -233,3 +233,34 @@ def test_attention_eager_general_path_fills_scores_and_probs(pkg, dev, H, KV, S,
                                D ** -0.5)
     assert pkg.lib.hd_cuda_last_error() != b""
     pkg.lib.hd_cuda_clear_error()
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+def test_attention_after_a_late_failure_stores_nothing(pkg, dev, mode):
+    """The launch may start while the kernel before it still runs; if that one then fails, nothing is stored."""
+    from latefail import late_failure
+    S, H, KV = 300, 4, 2
+    q, k, v = (torch.randn(S, n * 128, device=dev).bfloat16() for n in (H, KV, KV))
+    out = torch.full((S, H * 128), 777.0, dtype=torch.bfloat16, device=dev)
+
+    def call():
+        return pkg.lib.o1_flash_attention(pkg.ptr(q), H * 128, pkg.ptr(k), KV * 128, pkg.ptr(v), KV * 128, pkg.ptr(out), H * 128,
+                                          S, H, KV, 20, 128 ** -0.5)
+
+    pkg.lib.o1_attention_tile_mode(mode)
+    try:
+        assert call() == 0, pkg.last_error()
+        out.fill_(777.0)
+        torch.cuda.synchronize()
+        late_failure(pkg, 98)
+        assert call() == 0
+        torch.cuda.synchronize()
+        assert (out == 777.0).all()
+        assert pkg.lib.o1_device_error() == 98
+        assert call() == 0
+        torch.cuda.synchronize()
+        assert not (out == 777.0).any()
+    finally:
+        torch.cuda.synchronize()
+        pkg.lib.o1_device_error()
+        pkg.lib.o1_attention_tile_mode(0)

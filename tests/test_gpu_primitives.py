@@ -581,3 +581,62 @@ def test_a_refused_launch_is_reported_once(pkg, dev):
     pkg.lib.hd_rmsnorm(pkg.ptr(x), pkg.ptr(w), pkg.ptr(y), 4, K, 1e-6)
     pkg.check_cuda_errbuf("hd_rmsnorm after a refused launch")
     assert float(torch.ones(8, device=dev).sum()) == 8.0
+
+
+LATE = [("128", 300, 512, 256, 1, 128), ("256", 300, 512, 256, 2, 256), ("fitted", 592, 4096, 2112, 1, 0), ("fitted + residual", 592, 4096, 2112, 2, 0),
+        ("pairs", 2304, 4096, 2048, 0, 0), ("SwiGLU", 300, 512, 256, 3, 0), ("32 columns", 77, 1024, 512, 2, 0), ("32 columns, one K block a stage", 300, 3136, 256, 0, 0),
+        ("96 columns", 520, 4304, 1152, 7, 0), ("shared K", 520, 1152, 4304, 8, -1)]
+
+
+@pytest.mark.parametrize("what,M,N,K,epi,bn", LATE, ids=[c[0] for c in LATE])
+def test_gemm_after_a_late_failure_stores_nothing(pkg, dev, what, M, N, K, epi, bn):
+    """A chained launch may start while the kernel before it still runs.  If that one then fails, the GEMM must not leave
+    results behind: every form looks at the error word again before it stores."""
+    from latefail import late_failure
+    g = torch.Generator(device=dev).manual_seed(7)
+    x, w, w2, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
+                      for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
+    y = torch.full((M, N), 777.0, dtype=torch.bfloat16, device=dev)
+
+    def call():
+        return pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), pkg.ptr(w2), pkg.ptr(y), N, M, N, K, epi, pkg.ptr(b), pkg.ptr(r), N, 0.0, bn)
+
+    assert call() == 0, pkg.last_error()        # (a kernel's first launch loads it, which takes longer than the failure does)
+    y.fill_(777.0)
+    torch.cuda.synchronize()
+    late_failure(pkg, 98)
+    try:
+        assert call() == 0, pkg.last_error()
+        torch.cuda.synchronize()
+        assert (y == 777.0).all(), f"{(y != 777.0).sum().item()} results stored after a failure"
+    finally:
+        torch.cuda.synchronize()
+        assert pkg.lib.o1_device_error() == 98
+    assert call() == 0
+    done(pkg, "gemm")
+    assert (y != 777.0).float().mean() > 0.99
+
+
+def test_qkv_projection_after_a_late_failure_stores_nothing(pkg, dev):
+    from latefail import late_failure
+    M, qc, kc, K = 300, 512, 128, 256
+    ld = qc + 2 * kc
+    g = torch.Generator(device=dev).manual_seed(8)
+    x, wq, wk, wv, nw = (torch.empty(s, device=dev).normal_(0, 0.1, generator=g).bfloat16() for s in ((M, K), (qc, K), (kc, K), (kc, K), (128,)))
+    tab = torch.zeros(M, 128, device=dev)
+    y = torch.full((M, ld), 777.0, dtype=torch.bfloat16, device=dev)
+    def call():
+        return pkg.lib.o1_gemm_qkv(pkg.ptr(x), K, pkg.ptr(wq), pkg.ptr(wk), pkg.ptr(wv), pkg.ptr(y), ld, M, qc, kc, K, pkg.ptr(nw),
+                                   pkg.ptr(nw), pkg.ptr(tab), 1e-6)
+
+    assert call() == 0, pkg.last_error()
+    y.fill_(777.0)
+    torch.cuda.synchronize()
+    late_failure(pkg, 98)
+    try:
+        assert call() == 0
+        torch.cuda.synchronize()
+        assert (y == 777.0).all()
+    finally:
+        torch.cuda.synchronize()
+        assert pkg.lib.o1_device_error() == 98
