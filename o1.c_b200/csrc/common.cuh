@@ -105,6 +105,7 @@ inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, siz
 cudaStream_t current_stream();
 char* errbuf();             // 512 bytes
 void set_error(const char* fmt, ...);
+int* device_failed_word();  // one int of mapped host memory per device, beside the error word (see lora.cu), or NULL
 int* device_error_word();   // per-device int set by kernels whose bounded waits ran out
 int sm_count();
 

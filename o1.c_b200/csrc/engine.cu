@@ -10,8 +10,8 @@
 //  * hd_forward (src/model/forward.c:190-405)
 //  * o1_denoise_step_cfg (src/runtime/generate.c:1314-1360 + :900-905)
 //  * hd_lora_merge_gpu (src/model/lora_merge.cu:35-109)
-// Nothing here allocates device memory; the only allocation is the per-device
-// error word.
+// Nothing here allocates device memory; the only allocations are, once per
+// device, the error word and its mirror in host memory.
 #include "common.cuh"
 #include "kernels.h"
 #include "../../include/o1_b200.h"
@@ -52,6 +52,7 @@ static void set_model_error(const char* fmt, ...) {
 
 struct DevState {
     int* err_word = nullptr;   // [0] error word of the bounded waits, [1] result slot of the mask probe
+    int* failed = nullptr;     // host memory that the device writes: the code of a merge that failed
     int sms = 0;
 };
 static DevState& dev_state() {
@@ -63,12 +64,14 @@ static DevState& dev_state() {
     DevState& s = states[dev];
     if (!s.err_word) {
         if (cudaMalloc(&s.err_word, 2 * sizeof(int)) == cudaSuccess) cudaMemset(s.err_word, 0, 2 * sizeof(int));
+        if (cudaHostAlloc(&s.failed, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) *s.failed = 0;
         cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, dev);
         if (s.sms <= 0) s.sms = 148;
     }
     return s;
 }
 int* device_error_word() { return dev_state().err_word; }
+int* device_failed_word() { return dev_state().failed; }
 int sm_count() { return dev_state().sms; }
 
 static inline void count(int n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -163,7 +166,10 @@ int o1_device_error(void) {
     cudaError_t e = cudaMemcpyAsync(&v, w, sizeof(int), cudaMemcpyDeviceToHost, g_stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g_stream);
     if (e != cudaSuccess) { set_error("device_error: %s", cudaGetErrorString(e)); return -1; }
-    if (v != 0) cudaMemsetAsync(w, 0, sizeof(int), g_stream);
+    if (v != 0) {
+        cudaMemsetAsync(w, 0, sizeof(int), g_stream);
+        if (device_failed_word()) *(volatile int*)device_failed_word() = 0;
+    }
     return v;
 }
 

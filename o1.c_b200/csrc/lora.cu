@@ -46,7 +46,12 @@ struct LoraArgs {
     LoraTarget t[L_GROUP];
     int count, tiles;
     int* err;
+    int* failed;            // host memory: set beside the error word, so that the waiting host need not copy that
 };
+__device__ __forceinline__ void lora_fail(const LoraArgs& g, int code) {
+    atomicExch(g.err, code);
+    *reinterpret_cast<volatile int*>(g.failed) = code;
+}
 
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int32_t c0, int32_t c1) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
@@ -102,7 +107,10 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) *s_abort = *reinterpret_cast<volatile int*>(g.err);
+    if (threadIdx.x == 0) {
+        *s_abort = error_word(g.err);
+        if (*s_abort != 0) *reinterpret_cast<volatile int*>(g.failed) = *s_abort;
+    }
     __syncthreads();
     if (*s_abort != 0) return;
     if (threadIdx.x == 0) {
@@ -151,7 +159,7 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
                 const int s = p % L_SLOTS;
                 if (!mbar_wait(&w_done[s], (p / L_SLOTS) & 1)) {
                     // give up, but not before the loads still under way have landed
-                    atomicExch(g.err, 41);
+                    lora_fail(g, 41);
                     for (int q = p; q < panels && q < p + L_SLOTS - (p ? 1 : 0); ++q) mbar_wait(&w_full[q % L_SLOTS], (q / L_SLOTS) & 1);
                     break;
                 }
@@ -176,11 +184,11 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
                 const int i = tile - tile_lo, as = i & 1;
                 while (te + 1 < g.count && g.t[te + 1].tile0 <= tile) ++te;
                 const int R = g.t[te].R;
-                if (!mbar_wait(&t_empty[as], ((i >> 1) & 1) ^ 1)) { atomicExch(g.err, 42); break; }
+                if (!mbar_wait(&t_empty[as], ((i >> 1) & 1) ^ 1)) { lora_fail(g, 42); break; }
                 tc_fence_after();
                 const uint32_t d = tmem_base + as * LT;
                 for (int r0 = 0; r0 < R; r0 += LRC, ++u) {
-                    if (!mbar_wait(&u_full[u % NB], (u / NB) & 1)) { atomicExch(g.err, 43); ok = false; break; }
+                    if (!mbar_wait(&u_full[u % NB], (u / NB) & 1)) { lora_fail(g, 43); ok = false; break; }
                     tc_fence_after();
                     const uint64_t ad = umma_desc_sw128(smem_u32(a_s), 16, 1024);
                     const uint64_t bd = umma_desc_sw128(smem_u32(b_s + (u % NB) * Cfg::OP_BYTES), LR * 128, 1024);
@@ -225,7 +233,7 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
                     if (rr < ks16) lora_load8(t.down + (size_t)(rc + rr) * t.K + col0 + c8 * 8, rr < nr ? 8 : 0, t.vec, f[p]);
                 }
                 // the buffer's previous unit has been consumed
-                if (!mbar_wait(&u_done[u % NB], ((u / NB) & 1) ^ 1)) { atomicExch(g.err, 44); ok = false; }
+                if (!mbar_wait(&u_done[u % NB], ((u / NB) & 1) ^ 1)) { lora_fail(g, 44); ok = false; }
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 uint8_t* b0 = b_s + (u % NB) * Cfg::OP_BYTES + (c8 >> 3) * (LR * 128);
@@ -236,7 +244,7 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
                 }
                 if (new_a) {
                     // single buffer: the unit before this one must be through with the old terms
-                    if (u > 0 && !mbar_wait(&u_done[(u - 1) % NB], ((u - 1) / NB) & 1)) { atomicExch(g.err, 45); ok = false; }
+                    if (u > 0 && !mbar_wait(&u_done[(u - 1) % NB], ((u - 1) / NB) & 1)) { lora_fail(g, 45); ok = false; }
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     const int k8 = tid & 7;
@@ -271,14 +279,14 @@ __global__ void __launch_bounds__(LORA_THREADS, 1) lora_merge_kernel(const __gri
             while (te + 1 < g.count && g.t[te + 1].tile0 <= tile) ++te;
             const float scale = g.t[te].scale;
             ok = __all_sync(0xffffffffu, mbar_wait(&t_full[as], (i >> 1) & 1));
-            if (!ok) { atomicExch(g.err, 46); break; }
+            if (!ok) { lora_fail(g, 46); break; }
             tc_fence_after();
             const uint32_t t_row = tmem_base + as * LT + ((uint32_t)(qd * 32) << 16);
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {
                 const int p = 2 * i + h, s = p % L_SLOTS;
                 ok = __all_sync(0xffffffffu, mbar_wait(&w_full[s], (p / L_SLOTS) & 1));
-                if (!ok) { atomicExch(g.err, 47); break; }
+                if (!ok) { lora_fail(g, 47); break; }
                 uint32_t r[2][32];
                 tmem_ld32(t_row + h * 64, r[0]);
                 tmem_ld32(t_row + h * 64 + 32, r[1]);
@@ -329,7 +337,7 @@ __global__ void lora_simt_kernel(uint16_t* __restrict__ w, const float* __restri
 struct LoraGroup {
     LoraArgs a;
     uintptr_t lo[L_GROUP], hi[L_GROUP];      // address ranges of their weights
-    LoraGroup() { a.count = 0; a.tiles = 0; a.err = nullptr; }
+    LoraGroup() { a.count = 0; a.tiles = 0; a.err = a.failed = nullptr; }
     // Targets of one launch are merged in no particular order, so a weight that is already in the group (a second
     // adapter for it) has to wait for the next launch: each adapter's result is rounded to bf16 before the next.
     bool clashes(uintptr_t l, uintptr_t h) const {
@@ -350,6 +358,8 @@ struct LoraGroup {
     bool launch(cudaStream_t st) {
         if (a.count == 0) return true;
         a.err = device_error_word();
+        a.failed = device_failed_word();
+        if (!a.err || !a.failed) { set_error("lora: no memory for the error word"); return false; }
         if (!(low_rank ? launch_as<1>(st) : launch_as<2>(st))) return false;
         launched = true;
         a.count = a.tiles = 0;
@@ -418,11 +428,9 @@ hd_status hd_lora_merge_gpu(hd_lora_entry* entries, size_t count, void* stream) 
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (!grp.launched && cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
     if (cap != cudaStreamCaptureStatusNone) return rc;
-    int word = 0;
-    cudaError_t e = cudaSuccess;
-    if (grp.launched) e = cudaMemcpyAsync(&word, device_error_word(), sizeof(int), cudaMemcpyDeviceToHost, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = e2;
+    const cudaError_t e = cudaStreamSynchronize(st);
+    // (a copy of the error word itself would take 7.6 us: 236 -> 244 us for the adapter of a whole block)
+    const int word = grp.launched ? *(volatile int*)device_failed_word() : 0;
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error("lora: %s", cudaGetErrorString(e));
