@@ -1062,8 +1062,9 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // For M < 8 (timestep MLP, M = 1) and for shapes the tensor-core tiles do not cover.  One warp per output column and MR
 // rows: bound by the weights' way from memory, so a weight is read once for all its rows, four 16-byte pieces of a lane at
 // a time.
+// A warp per row needs every warp an SM holds: 36 registers instead of 32, two blocks fewer, cost 10 % (4096 x 4096, 2 rows).
 template <int MR>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, MR == 1 ? 16 : 1)
 gemm_simt_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w,
                                  const uint16_t* __restrict__ bias, uint16_t* __restrict__ y, int M,
                                  int N, int K, int ldx, int ldy) {
@@ -1079,7 +1080,8 @@ gemm_simt_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w,
     for (int i = 0; i < MR; ++i) xr[i] = x + (size_t)(m0 + i < M ? m0 + i : M - 1) * ldx;
     const uint16_t* wr = w + (size_t)n * K;
     float acc[MR] = {};
-    if (((K | ldx) & 7) == 0 && ((((uintptr_t)x) | ((uintptr_t)w)) & 15) == 0) {
+    // the rows and the weights lie on 16-byte boundaries
+    if (((K | (MR == 1 ? m0 * ldx : ldx)) & 7) == 0 && ((((uintptr_t)x) | ((uintptr_t)w)) & 15) == 0) {
         constexpr int UN = MR == 1 ? 1 : 4;
 #pragma unroll 4
         for (int k0 = lane * 8; k0 < K; k0 += 256 * UN) {
@@ -1409,6 +1411,22 @@ static bool launch_split(const CUtensorMap* tA, const void* w, GemmArgs& g, Spli
     }
 }
 
+// Rows that share a warp of gemm_simt_kernel, which then reads a weight once for all of them; equal groups of at most four.
+// us with a warp per row and column against shared rows (before launches overlapped, a warp per row):
+//  * K up to 1024: a warp's work is short and what counts is the number of blocks.  4096 x 256: 5 rows 6.4 / 3.6 (6.2), 7 rows
+//    8.6 / 4.4 (7.7); 12288 x 512: 2 rows 8.4 / 6.2 (8.2), 7 rows 24.4 / 12.9 (16.4); 4096 x 1024: 2 rows 4.8 / 4.5 (6.2)
+//  * beyond, three rows and more where N alone has two waves of blocks: 12288 x 2048: 3 rows 16.9 / 15.9 (19.4), 4 rows
+//    20.6 / 17.6 (22.7), 7 rows 31.5 / 28.7 (34.8); 24576 x 1536: 6 rows 48.7 / 37.1 (47.2)
+//  * weights beyond L2, which every further row would fetch from memory again: 24576 x 4096: 4 rows 53.2 (117.9)
+//  * otherwise a warp per row: a chain of loads per warp and too few warps to hide it cost more than reading the weights from
+//    L2 again.  4096 x 4096: 2 rows 8.9 / 13.5 (10.3), 7 rows 19.5 / 23.0 (22.5); 12288 x 2048: 2 rows 13.4 / 14.8 (16.4)
+static int simt_rows(int M, int N, int K) {
+    const bool share = K <= 1024 || (M >= 3 && N >= 2 * 8 * 4 * sm_count()) || (size_t)N * K * 2 > (126u << 20);
+    if (M == 1 || M > 65535 /* no more rows than the grid takes one by one */ || !share) return 1;
+    const int groups = (M + 3) / 4;
+    return (M + groups - 1) / groups;
+}
+
 bool gemm_tc_supported(int M, int N, int K, int epi) {
     // tiny M (timestep MLP, M = 1) is a GEMV: SIMT path.  K only has to keep the rows 16-byte aligned for TMA
     // (the last K block may be ragged: both operands are zero-filled beyond K).
@@ -1454,15 +1472,10 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
     if (!gemm_tc_supported(M, N, K, epi)) {
         if (epi != EPI_STORE && epi != EPI_BIAS) { set_error("gemm: shape unsupported for fused epilogue"); return false; }
         const uint16_t* b = (const uint16_t*)(epi == EPI_BIAS ? bias : nullptr);
-        // Rows share a warp's weights where these do not fit L2 (24576 x 4096: 5 rows 144 -> 111 us); otherwise a warp per row
-        // and column is faster, the weights of the later rows coming from L2 (4096 x 12288: 5 rows 55 against 69 us).
-        const bool share_rows = M > 1 && (size_t)N * K * 2 > (126u << 20);
-        const dim3 block(128);
-        const cudaError_t e =
-            !share_rows ? launch_chained(gemm_simt_kernel<1>, dim3((N + 3) / 4, M), block, 0, st, 1, M, (const uint16_t*)x,
-                                    (const uint16_t*)w, b, (uint16_t*)y, M, N, K, ldx, ldy)
-                   : launch_chained(gemm_simt_kernel<4>, dim3((N + 3) / 4, (M + 3) / 4), block, 0, st, 1, M, (const uint16_t*)x,
-                                    (const uint16_t*)w, b, (uint16_t*)y, M, N, K, ldx, ldy);
+        const int mr = simt_rows(M, N, K);
+        auto kern = mr == 1 ? gemm_simt_kernel<1> : mr == 2 ? gemm_simt_kernel<2> : mr == 3 ? gemm_simt_kernel<3> : gemm_simt_kernel<4>;
+        const cudaError_t e = launch_chained(kern, dim3((N + 3) / 4, (M + mr - 1) / mr), dim3(128), 0, st, 1, M, (const uint16_t*)x,
+                                             (const uint16_t*)w, b, (uint16_t*)y, M, N, K, ldx, ldy);
         if (e != cudaSuccess) { set_error("gemm(simt): launch: %s", cudaGetErrorString(e)); return false; }
         return true;
     }

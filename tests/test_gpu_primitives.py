@@ -640,3 +640,27 @@ def test_qkv_projection_after_a_late_failure_stores_nothing(pkg, dev):
     finally:
         torch.cuda.synchronize()
         assert pkg.lib.o1_device_error() == 98
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 6, 7, 9, 11])
+@pytest.mark.parametrize("N,K,pad", [(9473, 1032, 0), (9473, 1032, 3), (515, 1024, 8), (515, 1024, 1), (13, 77, 0), (4097, 264, 5)])
+def test_row_kernel_groups_and_pitches(pkg, dev, M, N, K, pad):
+    """The row kernel with one to four rows to a warp, a last group that is not full, row pitches that leave the rows aligned
+    and that do not, and a K without whole 16-byte pieces; nothing is written beside the result."""
+    g = torch.Generator(device=dev).manual_seed(M + N + K + pad)
+    x, w, b = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16() for s, d in (((M, K + pad), 1.0), ((N, K), 0.05), ((N,), 0.5)))
+    ldy = N + 3
+    y = torch.full((M + 1, ldy), 777.0, dtype=torch.bfloat16, device=dev)
+    rc = pkg.lib.o1_gemm(pkg.ptr(x), K + pad, pkg.ptr(w), None, pkg.ptr(y), ldy, M, N, K, 1, pkg.ptr(b), None, 0, 0.0, 0)
+    assert rc == 0, pkg.last_error()
+    done(pkg, "rows")
+    check_linear_f64(y[:M, :N], x[:, :K], w, b, "rows")
+    assert (y[M:] == 777.0).all() and (y[:, N:] == 777.0).all(), "written beside the result"
+    if pad % 8 == 0:       # a row is the same whatever it shares a warp with (where the rows' alignment is the same)
+        one = torch.empty(M, N, dtype=torch.bfloat16, device=dev)
+        for i in range(M):
+            rc = pkg.lib.o1_gemm(C.c_void_p(x.data_ptr() + 2 * i * (K + pad)), K + pad, pkg.ptr(w), None,
+                                 C.c_void_p(one.data_ptr() + 2 * i * N), N, 1, N, K, 1, pkg.ptr(b), None, 0, 0.0, 0)
+            assert rc == 0, pkg.last_error()
+        done(pkg, "rows")
+        assert torch.equal(one.view(torch.int16), y[:M, :N].contiguous().view(torch.int16))
