@@ -13,7 +13,8 @@
 //   RESID  : bf16(bf16(acc) + resid)           (residual.cu:14-23)
 //   SWIGLU : B tile = 128 gate rows + 128 up rows of the same columns;
 //            bf16(bf16(silu(bf16 g)) * bf16 u) (act.cu:22-34)
-//   LORA   : W = bf16(f32(W) + scale*acc)      (lora_merge.cu:26-33)
+//   LORA   : W = bf16(f32(W) + scale*acc)      (lora_merge.cu:26-33), for callers of o1_gemm; hd_lora_merge_gpu has a
+//            kernel of its own (lora.cu)
 #include <cstdlib>
 #include "common.cuh"
 #include "ptx.cuh"
@@ -597,11 +598,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         } else if (EPI == EPI_RESID) {
 #pragma unroll
                             for (int j = 0; j < 32; ++j) v[j] = bf16_round(v[j]) + rs[j];
-                        } else if (EPI == EPI_LORA) {
-                            float b[32];
-                            load32_bf16(g.out + (size_t)row * g.ldo + ocol, b);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = b[j] + g.scale * v[j];
                         }
                         store32_bf16(g.out + (size_t)row * g.ldo + ocol, v);
                     }
@@ -834,7 +830,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int mu = (NU + ks - 1) / ks;                            // most units a CTA owns
     if (ks > 1) {
         // every CTA's MMAs are through with its stages, which now receive the others' columns:
-        // [source][unit][4 columns][row] of 16 bytes, at most 7 x 2 or 1 x 4 units of 8 KB
+        // [source][unit][4 columns][row] of 16 bytes: (ks - 1) x mu units of 8 KB, see split_exchange_fits()
         __syncwarp();
         cluster_sync_all();
         if (ok && warp >= 2) {
@@ -1367,13 +1363,18 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
 //  * K over a cluster where even narrow tiles leave a long main loop: 520 x 1152 x 4304 23.5 / 18.7 (five CTAs, 32 columns
 //    27.2), 96 x 1152 x 4304 22.2 / 12.9 (six; 16.2); with 64 tiles and more 32 columns are as good (130 x 4096 x 4608)
 struct SplitPlan { int bn, ks; };
+static constexpr int MAX_SPLIT = 6;
+// A CTA's stages have to hold the columns it takes over from the ks - 1 others (six CTAs: 5 x 2 units of 8 KB in 96 KB).
+static constexpr bool split_exchange_fits(int bn, int ks, int stage_total) {
+    return (ks - 1) * ((bn / 16 + ks - 1) / ks) * 8192 <= stage_total;
+}
 static SplitPlan split_plan(int M, int N, int K, bool may_split) {
     const int sms = sm_count(), kblocks = (K + BK - 1) / BK;
     const long num_m = (M + BM - 1) / BM;
     auto tiles = [&](int bn) { return num_m * ((N + bn - 1) / bn); };
     if (may_split && kblocks >= 32 && tiles(128) * 3 <= sms) {
         const long ks = sms * 8 / 5 / tiles(128);
-        return {128, ks > 6 ? 6 : (int)ks};
+        return {128, ks > MAX_SPLIT ? MAX_SPLIT : (int)ks};
     }
     if (tiles(32) <= 2 * sms) return {32, 1};
     if (K <= 2048 && tiles(128) > sms && tiles(96) <= 2 * sms) return {96, 1};
@@ -1384,6 +1385,10 @@ template <int EPI, int BN, int KPS = 1>
 static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmArgs& g, int ks, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
     constexpr int SMEM = SplitCfg<BN, KPS>::SMEM;
+    if (ks < 1 || ks > MAX_SPLIT || !split_exchange_fits(BN, ks, SplitCfg<BN, KPS>::STAGES * SplitCfg<BN, KPS>::STAGE_BYTES)) {
+        set_error("gemm (few tiles): %d CTAs cannot share a %d-column tile", ks, BN);
+        return false;
+    }
     auto kern = gemm_split_kernel<EPI, BN, KPS>;
     if (!func_attr_once(attr_done, (const void*)kern, SMEM, "gemm (few tiles)")) return false;
     g.num_n = (g.N + BN - 1) / BN;
