@@ -472,6 +472,11 @@ int64_t o1_launch_count(int reset);
  * anything else runs a SIMT kernel (epilogues 0 and 1 only).  Returns 0 on success. */
 int o1_gemm(const void *x, int ldx, const void *w, const void *w2, void *y, int ldy, int M, int N,
             int K, int epi, const void *bias, const void *resid, int ldr, float scale, int force_bn);
+/* The form o1_gemm gives a problem on the current device (no launch): 0 = a warp per column (*width: rows that share it), 1 =
+ * one CTA per tile of 128 rows x *width columns, 2 = two CTAs per 256 x 256 tile, 3 = one CTA per tile of a *width fitted to
+ * the number of SMs, 4 = the kernel for few tiles of *width columns, *ctas of a cluster sharing the K of each; -1 = not
+ * supported.  force_bn -1 (which o1_gemm takes too): as 0, and K may be shared. */
+int o1_gemm_form(int M, int N, int K, int epi, int force_bn, int *width, int *ctas);
 /* The q, k and v projections of a decoder block (src/model/block.c:257-265) with the per-head RMSNorm + rotary of
  * q and k (:266-289) as ONE launch over the three weight tensors: y [M, qc | kc | kc] (row pitch ldy) =
  * norm_rope(x wq^T) | norm_rope(x wk^T) | x wv^T.  q_norm / k_norm [128] bf16, cs [M,128] fp32 (o1_mrope_table),

@@ -918,6 +918,15 @@ int o1_gemm(const void* x, int ldx, const void* w, const void* w2, void* y, int 
     count();
     return 0;
 }
+int o1_gemm_form(int M, int N, int K, int epi, int force_bn, int* width, int* ctas) {
+    if (M <= 0 || N <= 0 || K <= 0) return -1;
+    const GemmPlan p = gemm_plan(M, N, K, epi, force_bn, true, (N % 256) == 0);
+    if (p.form == GEMM_ROWS && epi != EPI_STORE && epi != EPI_BIAS) return -1;
+    if (p.form != GEMM_ROWS && epi != EPI_SWIGLU && force_bn == 256 && (N % 256) != 0) return -1;
+    if (width) *width = p.bn;
+    if (ctas) *ctas = p.ks;
+    return p.form;
+}
 int o1_gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void* wv, void* y, int ldy, int M, int qc,
                 int kc, int K, const void* q_norm, const void* k_norm, const float* cs, float eps) {
     if (!gemm_qkv(x, ldx, wq, wk, wv, y, ldy, M, qc, kc, K, q_norm, k_norm, cs, eps, 0, nullptr, nullptr, nullptr, g_stream))

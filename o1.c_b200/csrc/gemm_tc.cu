@@ -1381,6 +1381,34 @@ static SplitPlan split_plan(int M, int N, int K, bool may_split) {
     return {0, 0};
 }
 
+static int simt_rows(int M, int N, int K);
+// The form a GEMM takes.  plain: row-major output; wide_ok: 256-column tiles fit it.
+GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok) {
+    if (!gemm_tc_supported(M, N, K, epi)) return {GEMM_ROWS, simt_rows(M, N, K), 1};
+    const int num_m = (M + BM - 1) / BM;
+    if (epi == EPI_SWIGLU) {     // (2N columns of gate and up)
+        const bool pair = force_bn <= 0 && tile_form(num_m, 2 * N, K, true, true) == TILE_PAIR;
+        return {pair ? GEMM_PAIR : GEMM_TILE, 256, pair ? 2 : 1};
+    }
+    const bool pair_ok = epi == EPI_STORE || epi == EPI_BIAS || epi == EPI_RESID;
+    if (force_bn == 128) return {GEMM_TILE, 128, 1};
+    if (force_bn == 256) {       // the pair form where that family has two rounds of its tiles
+        const bool pair = pair_ok && pair_wanted() && ((num_m + 1) / 2) * (N / 256) >= sm_count();
+        return {pair ? GEMM_PAIR : GEMM_TILE, 256, pair ? 2 : 1};
+    }
+    plain = plain && force_bn <= 0;
+    if (plain && (pair_ok || epi == EPI_BIAS_GELU || epi == EPI_BIAS_RESID || epi == EPI_GATE_RESID)) {
+        const SplitPlan p = split_plan(M, N, K, force_bn == GEMM_SPLIT_K && pair_wanted());
+        if (p.bn > 0) return {GEMM_FEW, p.bn, p.ks};
+    }
+    if (plain && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) {
+        const int width = fit_width(num_m, N, K);
+        if (width) return {GEMM_FIT, width, 1};
+    }
+    const TileForm f = tile_form(num_m, N, K, wide_ok, pair_ok);
+    return {f == TILE_PAIR ? GEMM_PAIR : GEMM_TILE, f == TILE_128 ? 128 : 256, f == TILE_PAIR ? 2 : 1};
+}
+
 template <int EPI, int BN, int KPS = 1>
 static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmArgs& g, int ks, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
@@ -1404,7 +1432,7 @@ static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmAr
 }
 
 template <int EPI>
-static bool launch_split(const CUtensorMap* tA, const void* w, GemmArgs& g, SplitPlan p, cudaStream_t st) {
+static bool launch_split(const CUtensorMap* tA, const void* w, GemmArgs& g, const GemmPlan& p, cudaStream_t st) {
     CUtensorMap mB;
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, p.bn)) return false;
     switch (p.bn) {
@@ -1542,43 +1570,27 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
     else mB2 = mB;
     const CUtensorMap *tA = &mA, *tB = &mB, *tB2 = &mB2;
 
-    if (epi == EPI_SWIGLU) {
-        // (2N columns of gate and up)
-        g.num_n = N / 128;
-        if (force_bn <= 0 && tile_form(g.num_m, 2 * N, K, true, true) == TILE_PAIR)
-            return launch_tc_pair<EPI_SWIGLU>(tA, tB, tB2, g, st, nullptr);
-        return launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
-    }
-    if (force_bn <= 0 && !o_cb && !o_tab) {
-        const SplitPlan p = split_plan(M, N, K, force_bn == GEMM_SPLIT_K && pair_wanted());
-        if (p.bn > 0) switch (epi) {
-            case EPI_STORE: return launch_split<EPI_STORE>(tA, w, g, p, st);
-            case EPI_BIAS:  return launch_split<EPI_BIAS>(tA, w, g, p, st);
-            case EPI_RESID: return launch_split<EPI_RESID>(tA, w, g, p, st);
-            case EPI_BIAS_GELU: return launch_split<EPI_BIAS_GELU>(tA, w, g, p, st);
-            case EPI_BIAS_RESID: return launch_split<EPI_BIAS_RESID>(tA, w, g, p, st);
-            case EPI_GATE_RESID: return launch_split<EPI_GATE_RESID>(tA, w, g, p, st);
-        }
-    }
-    if (force_bn <= 0 && !o_cb && !o_tab && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) {
-        const int width = fit_width(g.num_m, N, K);
-        if (width && epi == EPI_RESID) return launch_fit<EPI_RESID>(tA, w, g, width, st);
-        if (width) return launch_fit<EPI_BIAS>(tA, w, g, width, st);
-    }
     const bool wide_ok = (N % 256) == 0 && (!o_cb || (o_cb % 256) == 0);
-    const bool pair_ok = epi == EPI_STORE || epi == EPI_BIAS || epi == EPI_RESID;
-    TileForm form = tile_form(g.num_m, N, K, wide_ok, pair_ok);
-    if (force_bn == 128 || force_bn == 256) {
-        if (force_bn == 256 && !wide_ok) {
-            set_error("gemm: BN=256 needs N (and the output column block) %% 256 == 0");
-            return false;
-        }
-        // (a forced width of 256 is the pair form where that family has two rounds of its tiles)
-        form = force_bn == 128 ? TILE_128
-                               : (pair_ok && pair_wanted() && ((g.num_m + 1) / 2) * (N / 256) >= sm_count() ? TILE_PAIR : TILE_256);
+    if (epi != EPI_SWIGLU && force_bn == 256 && !wide_ok) {
+        set_error("gemm: BN=256 needs N (and the output column block) %% 256 == 0");
+        return false;
     }
-    const int bn = form == TILE_128 ? 128 : 256;
-    if (form == TILE_PAIR) {
+    const GemmPlan p = gemm_plan(M, N, K, epi, force_bn, !o_cb && !o_tab, wide_ok);
+    if (epi == EPI_SWIGLU) {
+        g.num_n = N / 128;
+        return p.form == GEMM_PAIR ? launch_tc_pair<EPI_SWIGLU>(tA, tB, tB2, g, st, nullptr) : launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
+    }
+    if (p.form == GEMM_FEW) switch (epi) {
+        case EPI_STORE: return launch_split<EPI_STORE>(tA, w, g, p, st);
+        case EPI_BIAS:  return launch_split<EPI_BIAS>(tA, w, g, p, st);
+        case EPI_RESID: return launch_split<EPI_RESID>(tA, w, g, p, st);
+        case EPI_BIAS_GELU: return launch_split<EPI_BIAS_GELU>(tA, w, g, p, st);
+        case EPI_BIAS_RESID: return launch_split<EPI_BIAS_RESID>(tA, w, g, p, st);
+        case EPI_GATE_RESID: return launch_split<EPI_GATE_RESID>(tA, w, g, p, st);
+    }
+    if (p.form == GEMM_FIT) return epi == EPI_RESID ? launch_fit<EPI_RESID>(tA, w, g, p.bn, st) : launch_fit<EPI_BIAS>(tA, w, g, p.bn, st);
+    const int bn = p.bn;
+    if (p.form == GEMM_PAIR) {
         g.num_n = N / 256;
         switch (epi) {
             case EPI_STORE: return launch_tc_pair<EPI_STORE>(tA, tB, tB2, g, st, nullptr);

@@ -35,6 +35,12 @@ void prof_after(cudaStream_t st);
 // of few tiles may share a tile's K among the CTAs of a cluster, which is another order of the FP32 sum (not in mode 0 of
 // gemm_pair_mode).
 enum { GEMM_SPLIT_K = -1 };
+// The form a problem takes: GEMM_ROWS = warps (bn: rows that share one), GEMM_TILE = one CTA per 128 x bn tile, GEMM_PAIR = two
+// per 256 x 256 tile, GEMM_FIT = one per tile of a width fitted to the SMs, GEMM_FEW = tiles for problems that have few (ctas of
+// a cluster share a tile's K).
+enum GemmForm { GEMM_ROWS = 0, GEMM_TILE = 1, GEMM_PAIR = 2, GEMM_FIT = 3, GEMM_FEW = 4 };
+struct GemmPlan { int form, bn, ks; };
+GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok);
 bool gemm_bf16(const void* x, const void* w, const void* w2, void* y, int M, int N, int K, int epi,
                const void* bias, const void* resid, float scale, int force_bn, cudaStream_t st);
 // Same, with explicit row pitches (elements) for x and y so that a GEMM can

@@ -319,3 +319,46 @@ def test_a_workspace_of_both_branches_rows_holds_the_pair(pkg, H, ff, heads, kv)
                 # the pass: S rows in all activations, the text rows of both branches, the x_embedder rows once
                 pair = total(S, 0) - S * H * 2 + text * H * 2 + I * (1024 + H) * 2
                 assert pair <= region, (S, img, I)
+
+
+def test_gemm_form_keeps_its_promises(pkg):
+    """The form of a GEMM over random shapes: no cluster in mode 0, a shared K only where the caller allows it, widths the kernels
+    exist for, and the same answer for every epilogue that adds whole sums with the same tiles."""
+    import random
+    rng = random.Random(5)
+    width, ctas = C.c_int(0), C.c_int(0)
+
+    def form(*a):
+        f = pkg.lib.o1_gemm_form(*a, C.byref(width), C.byref(ctas))
+        return f, width.value, ctas.value
+
+    seen = set()
+    try:
+        for _ in range(3000):
+            m, n, k = (int(round(2 ** rng.uniform(lo, hi))) for lo, hi in ((0, 14), (6, 14), (6, 13.6)))
+            n, k = n // 8 * 8, k // 8 * 8
+            if rng.random() < 0.7:
+                n = (n + 127) // 128 * 128
+            for epi in (0, 1, 2, 3, 7, 8, 9):
+                for bn in (0, -1, 128, 256):
+                    for mode in (1, 0):
+                        pkg.lib.o1_gemm_pair_mode(mode)
+                        f, w, c = form(m, n, k, epi, bn)
+                        if epi not in (0, 1, 7) and n % 128 or m < 8 and epi > 1 or m >= 8 and bn == 256 and epi != 3 and n % 256:
+                            assert f == -1
+                            continue
+                        assert (f == 0) == (m < 8)
+                        if f == 0:
+                            assert 1 <= w <= min(4, m) and c == 1
+                            continue
+                        seen.add((f, w, c))
+                        assert mode == 1 or c == 1, "a cluster in mode 0"
+                        assert f != 4 or c == 1 or bn == -1, "a shared K that was not asked for"
+                        if bn > 0:
+                            assert f in (1, 2) and w == (256 if epi == 3 else bn)
+                        assert {1: w in (128, 256), 2: w == 256 and c == 2, 3: w % 16 == 0 and 144 <= w <= 192 and epi in (1, 2),
+                                4: w in (32, 96) and c == 1 or w == 128 and 4 <= c <= 6}[f], (f, w, c)
+    finally:
+        pkg.lib.o1_gemm_pair_mode(1)
+    assert {(1, 128, 1), (1, 256, 1), (2, 256, 2), (3, 144, 1), (4, 32, 1), (4, 96, 1)} <= seen and any(c > 2 for _, _, c in seen)
+    assert form(0, 8, 8, 0, 0)[0] == -1 and form(8, 100, 64, 2, 0)[0] == -1

@@ -431,21 +431,28 @@ def test_qkv_projections_as_one_launch(pkg, dev, M, qc, kc, K):
     assert (torch_to_u16(one)[:, qc + 2 * kc:] == fill[:, qc + 2 * kc:]).all()
 
 
-@pytest.mark.parametrize("M,N,K,epi", [(4352, 4096, 512, 0), (4115, 4096, 256, 2), (4200, 3072, 320, 1), (8320, 4096, 192, 2)])
+@pytest.mark.parametrize("M,N,K,epi", [(4352, 4096, 512, 0), (4115, 4096, 256, 2), (4200, 3072, 320, 1), (8320, 4096, 192, 2),
+                                       (1280, 4096, 2048, 3), (1400, 4096, 2056, 3), (2304, 4096, 2048, 0), (2561, 4096, 2104, 2)])
 def test_gemm_on_cta_pairs_equals_single_cta_tiles(pkg, dev, M, N, K, epi):
     """The cta_group::2 form (two CTAs per 256 x 256 tile, each with half of the B tile) adds a row's K products in the
     same order as the one-CTA form: same bits, for an even and an odd number of row tiles, a partly filled last row
-    tile and a ragged last K block, with the epilogues that take the pair form (plain, +bias, +residual)."""
+    tile and a ragged last K block, with the epilogues that take the pair form (plain, +bias, +residual, SwiGLU), by the
+    rule for a short K and by the one from K = 2048 on."""
+    if pkg.lib.o1_sm_count() == 148:
+        assert gemm_form(pkg, M, N, K, epi, 0) == (2, 256, 2)
     x = dv(seeded_bf16((M, K), 91), dev)
     w = dv(seeded_bf16((N, K), 92, 0.0, 0.05), dev)
+    up = dv(seeded_bf16((N, K), 95, 0.0, 0.05), dev) if epi == 3 else None
     bias = dv(seeded_bf16(N, 93, 0.0, 0.5), dev) if epi == 1 else None
     resid = dv(seeded_bf16((M, N), 94), dev) if epi == 2 else None
     outs = []
     try:
         for mode in (0, 1):
             pkg.lib.o1_gemm_pair_mode(mode)
+            if mode == 0:
+                assert gemm_form(pkg, M, N, K, epi, 0)[2] == 1
             y = torch.zeros(M, N, dtype=torch.bfloat16, device=dev)
-            rc = pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N, M, N, K, epi,
+            rc = pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), pkg.ptr(up), pkg.ptr(y), N, M, N, K, epi,
                                  pkg.ptr(bias) if bias is not None else None,
                                  pkg.ptr(resid) if resid is not None else None, N, 0.0, 0)
             assert rc == 0, pkg.last_error()
@@ -457,6 +464,7 @@ def test_gemm_on_cta_pairs_equals_single_cta_tiles(pkg, dev, M, N, K, epi):
     ref = x.float() @ w.float().t()
     if epi == 1: ref = (ref.bfloat16().float() + bias.float())
     if epi == 2: ref = (ref.bfloat16().float() + resid.float())
+    if epi == 3: ref = torch.nn.functional.silu(ref.bfloat16().float()).bfloat16().float() * (x.float() @ up.float().t()).bfloat16().float()
     err = (outs[1].float() - ref).abs().max().item() / max(ref.abs().max().item(), 1e-6)
     assert err < 1e-2, err     # the pair form really computed the product (fp32 reference, bf16 rounding of the result)
 
@@ -476,7 +484,7 @@ def check_linear_f64(y, x, w, bias, what):
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 7, 8, 33, 127, 128, 129, 300, 517])
 @pytest.mark.parametrize("N,K", [(72, 40), (128, 64), (1032, 200), (4096, 256), (96, 4104), (1152, 1160)])
 def test_linear_of_few_tiles(pkg, dev, M, N, K):
-    """hd_linear where there are few output tiles: the row kernel below eight rows, then tiles of 32 / 64 / 96 / 128
+    """hd_linear where there are few output tiles: the row kernel below eight rows, then tiles of 32, 96 or 128
     columns, with a ragged last tile, a ragged last K block and fewer K blocks than stages; nothing is written behind."""
     g = torch.Generator(device=dev).manual_seed(M * 7 + N + K)
     x, w, b = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16() for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5)))
@@ -489,13 +497,55 @@ def test_linear_of_few_tiles(pkg, dev, M, N, K):
     assert pkg.lib.o1_device_error() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(96, 1152, 1152), (520, 1152, 4304), (130, 4608, 4608), (20, 4304, 1152), (9, 72, 520), (300, 128, 2048)])
-@pytest.mark.parametrize("epi", [0, 1, 2, 8, 9])
-def test_gemm_with_k_split_over_a_cluster(pkg, dev, M, N, K, epi):
-    """A tile's K shared by the CTAs of a cluster where that is chosen (force_bn = -1), every epilogue, against the whole-K tile:
-    the FP32 sums differ by their order only, so the results are equal or neighbours."""
+def gemm_form(pkg, M, N, K, epi, bn):
+    """(form, tile width or rows, CTAs that share a tile) of o1_gemm_form."""
+    width, ctas = C.c_int(0), C.c_int(0)
+    return pkg.lib.o1_gemm_form(M, N, K, epi, bn, C.byref(width), C.byref(ctas)), width.value, ctas.value
+
+
+def gelu_tanh_f64(v):
+    """0.5 v (1 + tanh u) = v / (1 + e^-2u): in 64 bits too, 1 + tanh u has no digits left where u is far below zero."""
+    return v / (1 + torch.exp(-2 * 0.7978845608028654 * (v + 0.044715 * v ** 3)))
+
+
+def check_epilogue_f64(y, x, w, b, r, epi, what):
+    """As check_linear_f64, carried through the epilogue's further roundings, each of which is monotonic; GELU is not, so there
+    its slope (at most 1.13) times the interval is allowed, the rounding to bf16 (2^-8 of the value just above a power of two)
+    and the fp32 evaluation: an exponent of up to 88 with three roundings of 2^-24, so 2^-15 of the value, and two ulp each for
+    exponential and division; 2^-14 in all."""
+    acc = x.double() @ w.double().t()
+    bound = (x.double().abs() @ w.double().abs().t()) * x.shape[1] * 2.0 ** -23
+    rnd = lambda t: t.bfloat16().double()  # noqa: E731
+    lo, hi = rnd(acc - bound), rnd(acc + bound)
+    if epi in (1, 7, 8):
+        lo, hi = rnd(lo + b.double()), rnd(hi + b.double())
+    if epi == 9:
+        ends = rnd(lo * b.double()), rnd(hi * b.double())
+        lo, hi = torch.minimum(*ends), torch.maximum(*ends)
+    if epi in (2, 8, 9):
+        lo, hi = rnd(r.double() + lo), rnd(r.double() + hi)
+    if epi == 7:
+        mid = gelu_tanh_f64((lo + hi) / 2)
+        room = 1.13 * (hi - lo) / 2 + (2.0 ** -8 + 2.0 ** -14) * mid.abs() + 1e-30
+        lo, hi = mid - room, mid + room
+    bad = (y.double() < lo) | (y.double() > hi)
+    first = [t[bad][:4].tolist() for t in (y.double(), lo, hi)]
+    assert not bad.any(), f"{what}: {bad.sum().item()} of {y.numel()} outside the rounding interval: {first}"
+
+
+@pytest.mark.parametrize("M,N,K,ctas", [(520, 1152, 4304, 5), (96, 1152, 4304, 6), (128, 4608, 4608, 6), (300, 128, 2048, 6),
+                                        (300, 1160, 2112, 6), (700, 1024, 2112, 4), (96, 1152, 1152, 1), (130, 4608, 4608, 1),
+                                        (20, 4304, 1152, 1), (9, 72, 520, 1)])
+@pytest.mark.parametrize("epi", [0, 1, 2, 7, 8, 9])
+def test_gemm_with_k_split_over_a_cluster(pkg, dev, M, N, K, ctas, epi):
+    """A tile's K shared by four to six CTAs of a cluster where force_bn = -1 chooses that (and, last, shapes where it does not),
+    every epilogue, against 64 bits and against the whole-K tile: the FP32 sums differ by their order only, so the results are
+    equal or neighbours."""
     if epi in (2, 8, 9) and N % 128:
         pytest.skip("the residual epilogues take whole 128-column tiles")
+    if pkg.lib.o1_sm_count() == 148:
+        assert gemm_form(pkg, M, N, K, epi, -1) == (4, 128 if ctas > 1 else 32, ctas)
+    assert gemm_form(pkg, M, N, K, epi, 0)[2] == 1
     g = torch.Generator(device=dev).manual_seed(M + N + K + epi)
     x, w, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
                   for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
@@ -506,9 +556,8 @@ def test_gemm_with_k_split_over_a_cluster(pkg, dev, M, N, K, epi):
         assert rc == 0, pkg.last_error()
         done(pkg, "gemm")
         assert (y[M:] == 777.0).all(), "rows beyond M were written"
+        check_epilogue_f64(y[:M], x, w, b, r, epi, f"epilogue {epi}, force_bn {bn}")
         ys.append(y[:M])
-    if epi < 2:
-        check_linear_f64(ys[0], x, w, b if epi else None, "split")
     # one bf16 step of the sum, carried through the epilogue: 2^-7 of the largest term
     scale = (x.float() @ w.float().t()).abs() * (b.abs().float() if epi == 9 else 1.0) + b.abs().float() + r.abs().float() + 1e-3
     assert ((ys[0].float() - ys[1].float()).abs() <= scale * 2.0 ** -6).all()
@@ -544,12 +593,15 @@ def test_fused_step_equals_the_chain_for_every_kind_of_value(pkg, dev, sigma, n)
     assert torch.equal(fused.view(torch.int16)[~nan], chain.view(torch.int16)[~nan])
 
 
-@pytest.mark.parametrize("M,N,K", [(592, 4096, 2048), (513, 4096, 2056), (700, 4096, 3000), (1280, 4096, 2112), (1500, 4096, 2048),
-                                   (1000, 3072, 2240), (1664, 3072, 2104), (2561, 4096, 2048), (592, 4096, 256)])
+@pytest.mark.parametrize("M,N,K,width", [(592, 4096, 2112, 144), (513, 4096, 2056, 144), (700, 4096, 3000, 176), (1280, 4096, 2112, 144),
+                                         (1500, 4096, 2048, 176), (1000, 3072, 2240, 176), (1664, 3072, 2104, 144), (2400, 4096, 2048, 192),
+                                         (2050, 3072, 2048, 192), (592, 4096, 256, 0)])
 @pytest.mark.parametrize("epi", [1, 2])
-def test_tiles_fitted_to_the_sms(pkg, dev, M, N, K, epi):
+def test_tiles_fitted_to_the_sms(pkg, dev, M, N, K, width, epi):
     """Tile widths between 128 and 256 columns (chosen where they make whole rounds of tiles) give the bits of 128-column
     tiles: partly filled last row and column tiles, ragged K, and a K too short for the form."""
+    if pkg.lib.o1_sm_count() == 148:
+        assert gemm_form(pkg, M, N, K, epi, 0) == ((3, width, 1) if width else (4, 96, 1))
     g = torch.Generator(device=dev).manual_seed(M + K)
     x, w, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
                   for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
@@ -583,13 +635,15 @@ def test_a_refused_launch_is_reported_once(pkg, dev):
     assert float(torch.ones(8, device=dev).sum()) == 8.0
 
 
-LATE = [("128", 300, 512, 256, 1, 128), ("256", 300, 512, 256, 2, 256), ("fitted", 592, 4096, 2112, 1, 0), ("fitted + residual", 592, 4096, 2112, 2, 0),
-        ("pairs", 2304, 4096, 2048, 0, 0), ("SwiGLU", 300, 512, 256, 3, 0), ("32 columns", 77, 1024, 512, 2, 0), ("32 columns, one K block a stage", 300, 3136, 256, 0, 0),
-        ("96 columns", 520, 4304, 1152, 7, 0), ("shared K", 520, 1152, 4304, 8, -1)]
+LATE = [("128 columns", 300, 512, 256, 1, 128, (1, 128)), ("256 columns", 300, 512, 256, 2, 256, (1, 256)),
+        ("SwiGLU", 300, 512, 256, 3, 0, (1, 256)), ("pairs", 2304, 4096, 2048, 0, 0, (2, 256)),
+        ("fitted, bias", 592, 4096, 2112, 1, 0, (3, 144)), ("fitted, residual", 592, 4096, 2112, 2, 0, (3, 144)),
+        ("few, two K blocks a stage", 77, 1024, 512, 2, 0, (4, 32)), ("few, one K block a stage", 300, 3136, 256, 0, 0, (4, 32)),
+        ("few, 96 columns", 520, 4304, 1152, 7, 0, (4, 96)), ("few, shared K", 520, 1152, 4304, 8, -1, (4, 128))]
 
 
-@pytest.mark.parametrize("what,M,N,K,epi,bn", LATE, ids=[c[0] for c in LATE])
-def test_gemm_after_a_late_failure_stores_nothing(pkg, dev, what, M, N, K, epi, bn):
+@pytest.mark.parametrize("what,M,N,K,epi,bn,form", LATE, ids=[c[0] for c in LATE])
+def test_gemm_after_a_late_failure_stores_nothing(pkg, dev, what, M, N, K, epi, bn, form):
     """A chained launch may start while the kernel before it still runs.  If that one then fails, the GEMM must not leave
     results behind: every form looks at the error word again before it stores."""
     from latefail import late_failure
@@ -601,6 +655,8 @@ def test_gemm_after_a_late_failure_stores_nothing(pkg, dev, what, M, N, K, epi, 
     def call():
         return pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), pkg.ptr(w2), pkg.ptr(y), N, M, N, K, epi, pkg.ptr(b), pkg.ptr(r), N, 0.0, bn)
 
+    if pkg.lib.o1_sm_count() == 148:
+        assert gemm_form(pkg, M, N, K, epi, bn)[:2] == form
     assert call() == 0, pkg.last_error()        # (a kernel's first launch loads it, which takes longer than the failure does)
     y.fill_(777.0)
     torch.cuda.synchronize()
@@ -664,3 +720,20 @@ def test_row_kernel_groups_and_pitches(pkg, dev, M, N, K, pad):
             assert rc == 0, pkg.last_error()
         done(pkg, "rows")
         assert torch.equal(one.view(torch.int16), y[:M, :N].contiguous().view(torch.int16))
+
+
+def test_gelu_is_rounded_once_for_every_bf16_value(pkg, dev):
+    """The tanh form of GELU over all finite bf16 values: the result is the 64-bit value rounded to bf16, down to the smallest
+    normal numbers (an fp32 evaluation may fall on the other side of a rounding boundary, but none of these values does; a form
+    that computes 1 + tanh u misses about 150 of them, between -3 and -10)."""
+    x = torch.arange(65536, dtype=torch.int32, device=dev).to(torch.int16).view(torch.bfloat16)
+    y = torch.empty_like(x)
+    pkg.lib.hd_vision_gelu(pkg.ptr(x), pkg.ptr(y), x.numel())
+    done(pkg, "gelu")
+    want = gelu_tanh_f64(x.double())
+    normal = torch.isfinite(x) & (want.abs() > 2.0 ** -120)
+    assert normal.sum() > 30000
+    assert torch.equal(y[normal], want[normal].bfloat16())
+    tiny = torch.isfinite(x) & ~normal & (x.abs() > 9)
+    assert (y[tiny].double().abs() <= 2.0 ** -119).all()
+    assert (y[x == float("inf")] == float("inf")).all() and y[torch.isnan(x)].isnan().all()
