@@ -1206,9 +1206,15 @@ static bool pair_wanted() {
     return g_pair_mode != 0;
 }
 
+// Activations of less than 128 KB: loads through a tensor map of so few bytes slow down with the number of CTAs that make them
+// (4096 x 4096 as 128 tiles: 15 rows 27.9 us, 16 rows 12.3, wherever the rows lie; the cause is not known).
+static bool small_rows(long M, long K) { return M * K * 2 < (128l << 10); }
 // A launch of some hundred us counts as one of many rows (see OVERLAP_ROWS): 24576 x 4096 at 3100 rows 501 us overlapped,
-// 485 without.
-static long overlap_rows(const GemmArgs& g) { return (double)g.M * g.N * g.K > 1.5e11 ? OVERLAP_ROWS + 1 : g.M; }
+// 485 without.  So does one whose loads are slow anyway, if its K is long: 12 x 12288 x 4096 38.0 / 37.1, 10 x 4096 x 4096
+// 23.4 / 22.5; but 12 x 8192 x 2048 18.3 / 20.0.
+static long overlap_rows(const GemmArgs& g) {
+    return (double)g.M * g.N * g.K > 1.5e11 || (small_rows(g.M, g.K) && g.K >= 4096) ? OVERLAP_ROWS + 1 : g.M;
+}
 
 template <int EPI>
 static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2, GemmArgs& g,
@@ -1362,6 +1368,12 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
 //    520 x 4304 x 1152 16.4 / 14.1; 593 x 4096 x 12288 86 / 84, where CTA pairs take 72
 //  * K over a cluster where even narrow tiles leave a long main loop: 520 x 1152 x 4304 23.5 / 18.7 (five CTAs, 32 columns
 //    27.2), 96 x 1152 x 4304 22.2 / 12.9 (six; 16.2); with 64 tiles and more 32 columns are as good (130 x 4096 x 4608)
+// But few rows of a long K (small_rows()) are read by at most half the SMs, in wider tiles.  Narrow / 128 columns / before there
+// were narrow ones: 10 x 4096 x 4096 27.4 / 22.5 / 24.6, 10 x 6144 x 4096 52.0 / 26.5 / 26.3, 12 x 8192 x 2048 28.7 / 18.3 /
+// 19.7, 33 x 8192 x 1024 13.7 / 9.8 / 12.3, 12 x 8192 x 512 9.5 / 6.5 / 8.5, 96 columns at 20 x 24576 x 2048 37.1 / 26.0 /
+// 32.7; but 10 x 2304 x 4096 (72 tiles) 20.5 / 18.6 / 24.6, 10 x 1024 x 4096 15.0 / 17.3 / 24.6, 33 x 4096 x 256 4.2 / 4.9 /
+// 7.8.  And K of no whole 64 columns, whose rows lie across the memory's lines, gains nothing from two CTAs per SM:
+// 640 x 1152 x 4304 27.0 / 22.5 / 26.7.
 struct SplitPlan { int bn, ks; };
 static constexpr int MAX_SPLIT = 6;
 // A CTA's stages have to hold the columns it takes over from the ks - 1 others (six CTAs: 5 x 2 units of 8 KB in 96 KB).
@@ -1376,8 +1388,12 @@ static SplitPlan split_plan(int M, int N, int K, bool may_split) {
         const long ks = sms * 8 / 5 / tiles(128);
         return {128, ks > MAX_SPLIT ? MAX_SPLIT : (int)ks};
     }
-    if (tiles(32) <= 2 * sms) return {32, 1};
-    if (K <= 2048 && tiles(128) > sms && tiles(96) <= 2 * sms) return {96, 1};
+    const bool small_a = small_rows(M, K);
+    long most = 2 * sms;
+    if ((K % 64) != 0) most = sms;
+    if (small_a && K >= 512) most = K >= 1024 ? sms / 2 : sms;
+    if (tiles(32) <= most) return {32, 1};
+    if (K <= (small_a ? 1024 : 2048) && tiles(128) > sms && tiles(96) <= 2 * sms) return {96, 1};
     return {0, 0};
 }
 

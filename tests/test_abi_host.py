@@ -362,3 +362,20 @@ def test_gemm_form_keeps_its_promises(pkg):
         pkg.lib.o1_gemm_pair_mode(1)
     assert {(1, 128, 1), (1, 256, 1), (2, 256, 2), (3, 144, 1), (4, 32, 1), (4, 96, 1)} <= seen and any(c > 2 for _, _, c in seen)
     assert form(0, 8, 8, 0, 0)[0] == -1 and form(8, 100, 64, 2, 0)[0] == -1
+
+
+def test_narrow_tiles_are_for_activations_of_some_size(pkg):
+    """Few rows, many columns: 128-column tiles below 128 KB of activations, narrow ones from there on, for short K and for few
+    columns (on 148 SMs)."""
+    if pkg.lib.o1_sm_count() != 148:
+        pytest.skip("the rule counts SMs")
+    width = C.c_int(0)
+
+    def form(m, n, k):
+        return pkg.lib.o1_gemm_form(m, n, k, 1, 0, C.byref(width), None), width.value
+
+    for n, k in ((4096, 4096), (6144, 4096), (8192, 2048), (2400, 2056), (8192, 1024)):
+        edge = (128 << 10) // (2 * k) + ((128 << 10) % (2 * k) > 0)      # the first row count of 128 KB
+        assert form(max(8, edge - 1), n, k) == (1, 128), (n, k)
+        assert form(edge, n, k) == (4, 32), (n, k)
+    assert form(10, 2304, 4096) == form(33, 4096, 256) == form(8, 1024, 4096) == (4, 32)

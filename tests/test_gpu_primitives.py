@@ -482,7 +482,7 @@ def check_linear_f64(y, x, w, bias, what):
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 7, 8, 33, 127, 128, 129, 300, 517])
-@pytest.mark.parametrize("N,K", [(72, 40), (128, 64), (1032, 200), (4096, 256), (96, 4104), (1152, 1160)])
+@pytest.mark.parametrize("N,K", [(72, 40), (128, 64), (1032, 200), (4096, 256), (96, 4104), (1152, 1160), (2400, 2056)])
 def test_linear_of_few_tiles(pkg, dev, M, N, K):
     """hd_linear where there are few output tiles: the row kernel below eight rows, then tiles of 32, 96 or 128
     columns, with a ragged last tile, a ragged last K block and fewer K blocks than stages; nothing is written behind."""
@@ -535,7 +535,7 @@ def check_epilogue_f64(y, x, w, b, r, epi, what):
 
 @pytest.mark.parametrize("M,N,K,ctas", [(520, 1152, 4304, 5), (96, 1152, 4304, 6), (128, 4608, 4608, 6), (300, 128, 2048, 6),
                                         (300, 1160, 2112, 6), (700, 1024, 2112, 4), (96, 1152, 1152, 1), (130, 4608, 4608, 1),
-                                        (20, 4304, 1152, 1), (9, 72, 520, 1)])
+                                        (64, 4304, 1152, 1), (9, 72, 520, 1)])
 @pytest.mark.parametrize("epi", [0, 1, 2, 7, 8, 9])
 def test_gemm_with_k_split_over_a_cluster(pkg, dev, M, N, K, ctas, epi):
     """A tile's K shared by four to six CTAs of a cluster where force_bn = -1 chooses that (and, last, shapes where it does not),
