@@ -1368,19 +1368,20 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
 //    520 x 4304 x 1152 16.4 / 14.1; 593 x 4096 x 12288 86 / 84, where CTA pairs take 72
 //  * K over a cluster where even narrow tiles leave a long main loop: 520 x 1152 x 4304 23.5 / 18.7 (five CTAs, 32 columns
 //    27.2), 96 x 1152 x 4304 22.2 / 12.9 (six; 16.2); with 64 tiles and more 32 columns are as good (130 x 4096 x 4608)
-// But few rows of a long K (small_rows()) are read by at most half the SMs, in wider tiles.  Narrow / 128 columns / before there
-// were narrow ones: 10 x 4096 x 4096 27.4 / 22.5 / 24.6, 10 x 6144 x 4096 52.0 / 26.5 / 26.3, 12 x 8192 x 2048 28.7 / 18.3 /
-// 19.7, 33 x 8192 x 1024 13.7 / 9.8 / 12.3, 12 x 8192 x 512 9.5 / 6.5 / 8.5, 96 columns at 20 x 24576 x 2048 37.1 / 26.0 /
-// 32.7; but 10 x 2304 x 4096 (72 tiles) 20.5 / 18.6 / 24.6, 10 x 1024 x 4096 15.0 / 17.3 / 24.6, 33 x 4096 x 256 4.2 / 4.9 /
-// 7.8.  And K of no whole 64 columns, whose rows lie across the memory's lines, gains nothing from two CTAs per SM:
-// 640 x 1152 x 4304 27.0 / 22.5 / 26.7.
+// But few rows of a long K (small_rows()) are read by fewer SMs in wider tiles: by at most half of them from K = 2048 on, by no
+// more than all from K = 512 on.  Narrow / 128 columns / before there were narrow ones: 10 x 4096 x 4096 27.4 / 22.5 / 24.6,
+// 10 x 6144 x 4096 52.0 / 26.5 / 26.3, 12 x 8192 x 2048 28.7 / 18.3 / 19.7, 33 x 8192 x 1024 13.7 / 9.8 / 12.3, 12 x 8192 x 512
+// 9.5 / 6.5 / 8.5, 96 columns at 20 x 24576 x 2048 37.1 / 26.0 / 32.7; but 10 x 2304 x 4096 (72 tiles) 20.5 / 18.6 / 24.6,
+// 10 x 1024 x 4096 15.0 / 17.3 / 24.6, 33 x 4096 x 256 4.2 / 4.9 / 7.8, and the tower of 36 patches (135 tiles, K = 1152) 1.78
+// / 1.93 / 3.15 ms.  K of no whole 64 columns, whose rows lie across the memory's lines, gains nothing from two CTAs per SM
+// (640 x 1152 x 4304 27.0 / 22.5 / 26.7) except where a residual is added (the tower of 832 patches 2.66 / 2.70 ms).
 struct SplitPlan { int bn, ks; };
 static constexpr int MAX_SPLIT = 6;
 // A CTA's stages have to hold the columns it takes over from the ks - 1 others (six CTAs: 5 x 2 units of 8 KB in 96 KB).
 static constexpr bool split_exchange_fits(int bn, int ks, int stage_total) {
     return (ks - 1) * ((bn / 16 + ks - 1) / ks) * 8192 <= stage_total;
 }
-static SplitPlan split_plan(int M, int N, int K, bool may_split) {
+static SplitPlan split_plan(int M, int N, int K, bool may_split, bool resid) {
     const int sms = sm_count(), kblocks = (K + BK - 1) / BK;
     const long num_m = (M + BM - 1) / BM;
     auto tiles = [&](int bn) { return num_m * ((N + bn - 1) / bn); };
@@ -1390,8 +1391,8 @@ static SplitPlan split_plan(int M, int N, int K, bool may_split) {
     }
     const bool small_a = small_rows(M, K);
     long most = 2 * sms;
-    if ((K % 64) != 0) most = sms;
-    if (small_a && K >= 512) most = K >= 1024 ? sms / 2 : sms;
+    if ((K % 64) != 0 && !resid) most = sms;
+    if (small_a && K >= 512) most = K >= 2048 ? sms / 2 : sms;
     if (tiles(32) <= most) return {32, 1};
     if (K <= (small_a ? 1024 : 2048) && tiles(128) > sms && tiles(96) <= 2 * sms) return {96, 1};
     return {0, 0};
@@ -1414,7 +1415,8 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
     }
     plain = plain && force_bn <= 0;
     if (plain && (pair_ok || epi == EPI_BIAS_GELU || epi == EPI_BIAS_RESID || epi == EPI_GATE_RESID)) {
-        const SplitPlan p = split_plan(M, N, K, force_bn == GEMM_SPLIT_K && pair_wanted());
+        const bool resid = epi == EPI_RESID || epi == EPI_BIAS_RESID || epi == EPI_GATE_RESID;
+        const SplitPlan p = split_plan(M, N, K, force_bn == GEMM_SPLIT_K && pair_wanted(), resid);
         if (p.bn > 0) return {GEMM_FEW, p.bn, p.ks};
     }
     if (plain && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) {

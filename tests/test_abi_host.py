@@ -374,8 +374,8 @@ def test_narrow_tiles_are_for_activations_of_some_size(pkg):
     def form(m, n, k):
         return pkg.lib.o1_gemm_form(m, n, k, 1, 0, C.byref(width), None), width.value
 
-    for n, k in ((4096, 4096), (6144, 4096), (8192, 2048), (2400, 2056), (8192, 1024)):
+    for n, k in ((4096, 4096), (6144, 4096), (8192, 2048), (2432, 2048), (8192, 1024)):
         edge = (128 << 10) // (2 * k) + ((128 << 10) % (2 * k) > 0)      # the first row count of 128 KB
         assert form(max(8, edge - 1), n, k) == (1, 128), (n, k)
         assert form(edge, n, k) == (4, 32), (n, k)
-    assert form(10, 2304, 4096) == form(33, 4096, 256) == form(8, 1024, 4096) == (4, 32)
+    assert form(10, 2304, 4096) == form(33, 4096, 256) == form(8, 1024, 4096) == form(33, 4096, 1024) == (4, 32)
