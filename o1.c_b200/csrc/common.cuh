@@ -78,7 +78,7 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ int error_word(const int* err) { return *reinterpret_cast<const volatile int*>(err); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,
+[[nodiscard]] inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,
                                   long rows, const A&... args) {
     cudaLaunchAttribute at[2];
     int n = 0;
@@ -99,6 +99,8 @@ inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, siz
     if (e != cudaSuccess) cudaGetLastError();     // the caller reports it: the next call's check must not find it again
     return e;
 }
+
+bool launch_ok(cudaError_t e, const char* what);     // sets the error text "<what>: ..." when e is one
 
 // ---- process-wide state (one stream, one error buffer: the reference's
 // primitive ABI has no stream argument and reports through a message buffer)

@@ -128,14 +128,14 @@ bool rmsnorm_mod(const void* x, const void* w, const void* scale, const void* sh
     const bool aligned = ((((uintptr_t)x) | ((uintptr_t)y) | ((uintptr_t)w) | ((uintptr_t)scale) | ((uintptr_t)shift)) & 15) == 0;
     const uint16_t *sc = (const uint16_t*)scale, *sh = (const uint16_t*)shift;
     if (aligned && (cols % 8) == 0 && cols <= 128 * 4 * 8 && cols > 1024) {
-        launch_chained(rmsnorm_vec_kernel<128, 4>, dim3(rows), dim3(128), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
-                       (uint16_t*)y, rows, cols, eps, sc, sh);
+        return launch_ok(launch_chained(rmsnorm_vec_kernel<128, 4>, dim3(rows), dim3(128), 0, st, 1, rows, (const uint16_t*)x,
+                                        (const uint16_t*)w, (uint16_t*)y, rows, cols, eps, sc, sh), "rmsnorm");
     } else if (aligned && (cols % 8) == 0 && cols <= 128 * 8 * 8 && cols > 1024) {
-        launch_chained(rmsnorm_vec_kernel<128, 8>, dim3(rows), dim3(128), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
-                       (uint16_t*)y, rows, cols, eps, sc, sh);
+        return launch_ok(launch_chained(rmsnorm_vec_kernel<128, 8>, dim3(rows), dim3(128), 0, st, 1, rows, (const uint16_t*)x,
+                                        (const uint16_t*)w, (uint16_t*)y, rows, cols, eps, sc, sh), "rmsnorm");
     } else if (aligned && (cols % 8) == 0 && cols <= 1024) {
-        launch_chained(rmsnorm_vec_kernel<32, 4>, dim3(rows), dim3(32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
-                       (uint16_t*)y, rows, cols, eps, sc, sh);
+        return launch_ok(launch_chained(rmsnorm_vec_kernel<32, 4>, dim3(rows), dim3(32), 0, st, 1, rows, (const uint16_t*)x,
+                                        (const uint16_t*)w, (uint16_t*)y, rows, cols, eps, sc, sh), "rmsnorm");
     } else {
         const int wpb = 4;
         rmsnorm_generic_kernel<<<(rows + wpb - 1) / wpb, wpb * 32, 0, st>>>(
@@ -376,16 +376,14 @@ __global__ void mrope_table64_kernel(const float* __restrict__ pos, float* __res
 }
 bool mrope_table64(const float* pos, int seq, float theta, float* cs, cudaStream_t st) {
     if (!pos || !cs || seq <= 0) { set_error("mrope_table: bad args"); return false; }
-    launch_chained(mrope_table64_kernel, dim3((seq + 3) / 4), dim3(256), 0, st, 1, seq, pos, cs, seq, theta, seq);
-    O1_LAUNCH_CHECK("mrope_table");
-    return true;
+    return launch_ok(launch_chained(mrope_table64_kernel, dim3((seq + 3) / 4), dim3(256), 0, st, 1, seq, pos, cs, seq, theta, seq),
+                     "mrope_table");
 }
 bool mrope_table64_rows(const float* pos, int pos_stride, int row0, int rows, float theta, float* cs,
                         cudaStream_t st) {
     if (!pos || !cs || rows <= 0 || row0 < 0 || row0 + rows > pos_stride) { set_error("mrope_table: bad args"); return false; }
-    launch_chained(mrope_table64_kernel, dim3((rows + 3) / 4), dim3(256), 0, st, 1, rows, pos + row0, cs, rows, theta, pos_stride);
-    O1_LAUNCH_CHECK("mrope_table");
-    return true;
+    return launch_ok(launch_chained(mrope_table64_kernel, dim3((rows + 3) / 4), dim3(256), 0, st, 1, rows, pos + row0, cs, rows, theta, pos_stride),
+                     "mrope_table");
 }
 
 // rotate-half on head-major [heads, seq, dim] (rope.cu:97-134). f32_mode = 0

@@ -43,6 +43,10 @@ void set_error(const char* fmt, ...) {
     vsnprintf(g_cuda_err, sizeof(g_cuda_err), fmt, ap);
     va_end(ap);
 }
+bool launch_ok(cudaError_t e, const char* what) {
+    if (e != cudaSuccess) set_error("%s: %s", what, cudaGetErrorString(e));
+    return e == cudaSuccess;
+}
 static void set_model_error(const char* fmt, ...) {
     va_list ap;
     va_start(ap, fmt);

@@ -232,8 +232,9 @@ bool sched_cfg_flow_step(const void* z, const void* xc, const void* xu, float si
         const size_t cap = (size_t)sm_count() * 16;
         const float y = 1.0f / sigma;
         const SharedDivisor d = {sigma, y, fmaf(-sigma, y, 1.0f) * y, sigma > 0x1p-30f && sigma < 0x1p30f};
-        launch_chained(cfg_flow_step_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(256), 0, st, 1, 0,
-                       (const uint4*)z, (const uint4*)xc, (const uint4*)xu, d, dt, g, (uint4*)z_next, nvec);
+        return launch_ok(launch_chained(cfg_flow_step_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(256), 0, st, 1, 0,
+                                        (const uint4*)z, (const uint4*)xc, (const uint4*)xu, d, dt, g, (uint4*)z_next, nvec),
+                         "sched_cfg_flow_step");
     } else {
         cfg_flow_step_scalar_kernel<<<nblocks(n), 256, 0, st>>>(
             (const uint16_t*)z, (const uint16_t*)xc, (const uint16_t*)xu, sigma, dt, g,

@@ -178,22 +178,13 @@ bool vision_layernorm(const void* x, const void* w, const void* b, void* y, int 
     if (!x || !w || !y || rows <= 0 || cols <= 0) { set_error("vision_layernorm: bad args"); return false; }
     const int vec = (cols % 8) == 0 && ((((uintptr_t)x) | ((uintptr_t)w) | ((uintptr_t)b) | ((uintptr_t)y)) & 15) == 0;
     const int grid = (rows + LN_WARPS - 1) / LN_WARPS;
-    if (vec && cols <= 5 * 256) {
-        launch_chained(layernorm_reg_kernel<5>, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
-                       (const uint16_t*)b, (uint16_t*)y, rows, cols, eps);
-        O1_VLAUNCH_CHECK("vision_layernorm");
-        return true;
-    }
-    if (vec && cols <= 18 * 256) {
-        launch_chained(layernorm_reg_kernel<18>, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
-                       (const uint16_t*)b, (uint16_t*)y, rows, cols, eps);
-        O1_VLAUNCH_CHECK("vision_layernorm");
-        return true;
-    }
-    launch_chained(layernorm_kernel, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
-                   (const uint16_t*)b, (uint16_t*)y, rows, cols, eps, vec);
-    O1_VLAUNCH_CHECK("vision_layernorm");
-    return true;
+    auto launch = [&](auto kern, auto... more) {
+        return launch_ok(launch_chained(kern, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
+                                        (const uint16_t*)b, (uint16_t*)y, rows, cols, eps, more...), "vision_layernorm");
+    };
+    if (vec && cols <= 5 * 256) return launch(layernorm_reg_kernel<5>);
+    if (vec && cols <= 18 * 256) return launch(layernorm_reg_kernel<18>);
+    return launch(layernorm_kernel, vec);
 }
 
 // GELU, tanh form (block MLP) or erf form (mergers): vision_kernels.cu:100-133

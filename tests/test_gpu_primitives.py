@@ -737,3 +737,46 @@ def test_gelu_is_rounded_once_for_every_bf16_value(pkg, dev):
     tiny = torch.isfinite(x) & ~normal & (x.abs() > 9)
     assert (y[tiny].double().abs() <= 2.0 ** -119).all()
     assert (y[x == float("inf")] == float("inf")).all() and y[torch.isnan(x)].isnan().all()
+
+
+def test_every_kind_of_launch_reports_its_refusal(pkg, dev):
+    """On a stream whose capture has become invalid CUDA refuses every launch, on the host; each entry point says so, and none
+    leaves the error to the next call of an ordinary stream."""
+    from cuda.bindings import driver
+    M, N, K = 16, 128, 128
+    x, w, y = (torch.zeros(s, dtype=torch.bfloat16, device=dev) for s in ((M, K), (N, K), (M, N)))
+    f, cs = torch.zeros(3, M, device=dev), torch.zeros(M, 128, device=dev)
+    p, lib = pkg.ptr, pkg.lib
+    calls = {
+        "rmsnorm, 32 threads a row": lambda: lib.hd_rmsnorm(p(x), p(w), p(y), M, K, 1e-6),
+        "rmsnorm, 128 threads a row": lambda: lib.hd_rmsnorm(p(x), p(w), p(y), 1, 8 * K + 8 * M, 1e-6),
+        "layernorm": lambda: lib.hd_vision_layernorm(p(x), p(w), None, p(y), M, K, 1e-6),
+        "mrope": lambda: lib.o1_mrope_table(p(f), M, 5e6, p(cs)),
+        "sched": lambda: lib.o1_sched_cfg_flow_step(p(x), p(x), p(x), 0.8, 0.7, 5.0, p(y), 256),
+        "linear, tiles": lambda: lib.hd_linear(p(x), p(w), None, p(y), M, N, K, 1),
+        "linear, rows": lambda: lib.hd_linear(p(x), p(w), None, p(y), 1, N, K, 1),
+        "attention": lambda: lib.o1_flash_attention(p(x), K, p(x), K, p(x), K, p(y), K, M, 1, 1, 0, 0.1),
+    }
+    for call in calls.values():
+        call()                       # (the kernels are loaded before the capture)
+    done(pkg, "warm-up")
+    stream = torch.cuda.Stream()
+    h = stream.cuda_stream
+    assert int(driver.cuStreamBeginCapture(h, driver.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_THREAD_LOCAL)[0]) == 0
+    lib.o1_set_stream(C.c_void_p(h))
+    said = {}
+    try:
+        assert int(driver.cuStreamSynchronize(h)[0]) != 0        # not allowed while capturing: the capture is invalid now
+        for name, call in calls.items():
+            lib.hd_cuda_clear_error()
+            call()
+            said[name] = lib.hd_cuda_last_error()
+    finally:
+        assert int(driver.cuStreamEndCapture(h)[0]) != 0
+        pkg.use_torch_stream()
+        lib.hd_cuda_clear_error()
+    assert all(said.values()), said
+    for call in calls.values():
+        call()
+        done(pkg, "afterwards")
+    assert float(torch.ones(8, device=dev).sum()) == 8.0
