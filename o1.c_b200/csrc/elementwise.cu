@@ -37,31 +37,36 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // ------------------------------------------------------------------ RMSNorm
 // y = bf16( (w * x) * rsqrt(mean(x^2) + eps) ), fp32 inside (norm.cu:12-48).
-// One row per block; each thread keeps its slice of the row and of the weight in registers, requested together before
-// the reduction, so HBM sees one read + one write and the chain of a row is one load, one barrier (every thread adds the
-// four warps' sums itself, in the order of a shuffle tree) and one store.
-template <int THREADS, int VEC_PER_THREAD>
-__global__ void __launch_bounds__(THREADS)
+// Blocks of 128 threads, a row to all of them or to each warp; each thread keeps its slice of the row and of the weight in
+// registers, requested together before the reduction, so HBM sees one read + one write and the chain of a row is one load, one
+// barrier (every thread adds the four warps' sums itself, in the order of a shuffle tree) and one store.  (EARLY_W
+// false: the weight later, for many rows of 4097 to 6144 columns, where its registers cost more warps than its latency is
+// worth: 16640 x 4608 56.9 us against 49.4; 1280 x 4608 4.4 against 6.0, 16640 x 8192 82.0 against 86.3.)
+// Short rows are bound by the number of blocks: 16640 x 128 with one warp to a block 20.6 us, 6.5 with four.
+template <int THREADS, int VEC_PER_THREAD, bool EARLY_W>
+__global__ void __launch_bounds__(128)
 rmsnorm_vec_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w,
                    uint16_t* __restrict__ y, int rows, int cols, float eps,
                    const uint16_t* __restrict__ scale, const uint16_t* __restrict__ shift) {
     grid_dep_launch();
     grid_dep_wait();
-    const int row = blockIdx.x;
+    const int tid = THREADS == 32 ? threadIdx.x & 31 : threadIdx.x;
+    const int row = THREADS == 32 ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
+    if (THREADS == 32 && row >= rows) return;
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * cols);
     uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * cols);
     const uint4* wr = reinterpret_cast<const uint4*>(w);
     const int nvec = cols >> 3;
-    uint4 xv[VEC_PER_THREAD], wv[VEC_PER_THREAD];
+    uint4 xv[VEC_PER_THREAD], wv[EARLY_W ? VEC_PER_THREAD : 1];
 #pragma unroll
     for (int i = 0; i < VEC_PER_THREAD; ++i) {
-        const int idx = threadIdx.x + i * THREADS;
-        if (idx < nvec) { xv[i] = xr[idx]; wv[i] = wr[idx]; }
+        const int idx = tid + i * THREADS;
+        if (idx < nvec) { xv[i] = xr[idx]; if (EARLY_W) wv[i] = wr[idx]; }
     }
     float sq = 0.f;
 #pragma unroll
     for (int i = 0; i < VEC_PER_THREAD; ++i) {
-        if (threadIdx.x + i * THREADS < nvec) {
+        if (tid + i * THREADS < nvec) {
             float f[8];
             unpack8(xv[i], f);
 #pragma unroll
@@ -79,11 +84,11 @@ rmsnorm_vec_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ 
     const float inv = rsqrtf(sq / (float)cols + eps);
 #pragma unroll
     for (int i = 0; i < VEC_PER_THREAD; ++i) {
-        const int idx = threadIdx.x + i * THREADS;
+        const int idx = tid + i * THREADS;
         if (idx < nvec) {
             float f[8], g[8];
             unpack8(xv[i], f);
-            unpack8(wv[i], g);
+            unpack8(EARLY_W ? wv[EARLY_W ? i : 0] : wr[idx], g);
 #pragma unroll
             for (int j = 0; j < 8; ++j) f[j] = g[j] * f[j] * inv;
             if (scale) {   // adaLN variant: the stored norm output, then * (1 + scale) + shift (NULL = o1.c's block)
@@ -127,15 +132,13 @@ bool rmsnorm_mod(const void* x, const void* w, const void* scale, const void* sh
     if (!x || !w || !y || rows <= 0 || cols <= 0 || (!scale != !shift)) { set_error("rmsnorm: bad args"); return false; }
     const bool aligned = ((((uintptr_t)x) | ((uintptr_t)y) | ((uintptr_t)w) | ((uintptr_t)scale) | ((uintptr_t)shift)) & 15) == 0;
     const uint16_t *sc = (const uint16_t*)scale, *sh = (const uint16_t*)shift;
-    if (aligned && (cols % 8) == 0 && cols <= 128 * 4 * 8 && cols > 1024) {
-        return launch_ok(launch_chained(rmsnorm_vec_kernel<128, 4>, dim3(rows), dim3(128), 0, st, 1, rows, (const uint16_t*)x,
-                                        (const uint16_t*)w, (uint16_t*)y, rows, cols, eps, sc, sh), "rmsnorm");
-    } else if (aligned && (cols % 8) == 0 && cols <= 128 * 8 * 8 && cols > 1024) {
-        return launch_ok(launch_chained(rmsnorm_vec_kernel<128, 8>, dim3(rows), dim3(128), 0, st, 1, rows, (const uint16_t*)x,
-                                        (const uint16_t*)w, (uint16_t*)y, rows, cols, eps, sc, sh), "rmsnorm");
-    } else if (aligned && (cols % 8) == 0 && cols <= 1024) {
-        return launch_ok(launch_chained(rmsnorm_vec_kernel<32, 4>, dim3(rows), dim3(32), 0, st, 1, rows, (const uint16_t*)x,
-                                        (const uint16_t*)w, (uint16_t*)y, rows, cols, eps, sc, sh), "rmsnorm");
+    if (aligned && (cols % 8) == 0 && cols <= 128 * 8 * 8) {
+        const bool early = rows <= OVERLAP_ROWS || cols > 6144;
+        auto kern = cols <= 1024 ? rmsnorm_vec_kernel<32, 4, true>
+                                 : (cols <= 4096 ? rmsnorm_vec_kernel<128, 4, true>
+                                                 : (early ? rmsnorm_vec_kernel<128, 8, true> : rmsnorm_vec_kernel<128, 8, false>));
+        return launch_ok(launch_chained(kern, dim3(cols <= 1024 ? (rows + 3) / 4 : rows), dim3(128), 0, st, 1, rows,
+                                        (const uint16_t*)x, (const uint16_t*)w, (uint16_t*)y, rows, cols, eps, sc, sh), "rmsnorm");
     } else {
         const int wpb = 4;
         rmsnorm_generic_kernel<<<(rows + wpb - 1) / wpb, wpb * 32, 0, st>>>(

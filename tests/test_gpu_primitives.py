@@ -780,3 +780,26 @@ def test_every_kind_of_launch_reports_its_refusal(pkg, dev):
         call()
         done(pkg, "afterwards")
     assert float(torch.ones(8, device=dev).sum()) == 8.0
+
+
+@pytest.mark.parametrize("rows", [1, 3, 4, 5, 130, 4096, 4097, 5000])
+@pytest.mark.parametrize("cols", [8, 128, 1024, 1032, 4096, 4104, 8192])
+def test_norms_by_rows_and_columns(pkg, dev, rows, cols):
+    """RMSNorm and LayerNorm over their forms' edges (a warp or a block to a row, few and many rows, weights requested early or
+    late) against 64 bits; rows behind the last one stay as they are.  bf16 rounding is 2^-9 of a value, an fp32 sum of `cols`
+    squares cols * 2^-24 at the most; with mean and variance as differences 2^-7 of the largest term covers both."""
+    g = torch.Generator(device=dev).manual_seed(rows + cols)
+    x, w, b = (torch.empty(s, device=dev).normal_(m, 0.5, generator=g).bfloat16() for s, m in (((rows, cols), 0.2), ((cols,), 1.0), ((cols,), 0.0)))
+    y = torch.full((rows + 1, cols), 777.0, dtype=torch.bfloat16, device=dev)
+    pkg.lib.hd_rmsnorm(pkg.ptr(x), pkg.ptr(w), pkg.ptr(y), rows, cols, 1e-6)
+    done(pkg, "rmsnorm")
+    xd = x.double()
+    want = xd * w.double() * torch.rsqrt((xd * xd).mean(-1, keepdim=True) + 1e-6)
+    assert ((y[:rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-9).all()
+    assert (y[rows:] == 777.0).all()
+    pkg.lib.hd_vision_layernorm(pkg.ptr(x), pkg.ptr(w), pkg.ptr(b), pkg.ptr(y), rows, cols, 1e-6)
+    done(pkg, "layernorm")
+    term = (xd - xd.mean(-1, keepdim=True)) * torch.rsqrt(xd.var(-1, unbiased=False, keepdim=True) + 1e-6) * w.double()
+    want = term + b.double()
+    assert ((y[:rows].double() - want).abs() <= 2.0 ** -7 * (term.abs() + b.double().abs())).all()
+    assert (y[rows:] == 777.0).all()
