@@ -105,12 +105,17 @@ layernorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w,
 // The same arithmetic with the row held in registers (rows of at most NV * 256 elements: the tower's 1152 and
 // the mergers' 4608): every element is read from memory once, all NV loads of a lane are in flight together, and
 // the sums run over the lane's elements in the same order as in layernorm_kernel, so the two agree bit for bit.
-template <int NV>
+// FEW: up to a few thousand rows, where latency counts: the launch is chained, and weight and bias of a row of at most 1280 are
+// requested with it, one memory latency per row, not two (5.5 us at 520 rows).  With many rows the registers for that cost more
+// (41600 x 128 16.5 us against 12.4).
+template <int NV, bool FEW>
 __global__ void __launch_bounds__(LN_WARPS * 32)
 layernorm_reg_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, const uint16_t* __restrict__ b,
                      uint16_t* __restrict__ y, int rows, int cols, float eps) {
-    grid_dep_launch();
-    grid_dep_wait();
+    if (FEW) {
+        grid_dep_launch();
+        grid_dep_wait();
+    }
     const int row = blockIdx.x * LN_WARPS + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -122,10 +127,10 @@ layernorm_reg_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
         const int i = lane * 8 + k * 256;
         v[k] = i < cols ? *reinterpret_cast<const uint4*>(xr + i) : make_uint4(0, 0, 0, 0);
     }
-    // weight and bias of a short row are requested with it: one memory latency per row, not two (5.5 us at 520 rows)
-    constexpr int PRE = NV <= 5 ? NV : 1;
+    constexpr bool EARLY_W = FEW && NV <= 5;
+    constexpr int PRE = EARLY_W ? NV : 1;
     uint4 wp[PRE], bp[PRE];
-    if (NV <= 5) {
+    if (EARLY_W) {
 #pragma unroll
         for (int k = 0; k < PRE; ++k) {
             const int i = lane * 8 + k * 256;
@@ -154,7 +159,7 @@ layernorm_reg_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
         const int i = lane * 8 + k * 256;
         if (i < cols) {
             uint4 wv, bv = make_uint4(0, 0, 0, 0);
-            if (NV <= 5) { wv = wp[k % PRE]; bv = bp[k % PRE]; }
+            if (EARLY_W) { wv = wp[k % PRE]; bv = bp[k % PRE]; }
             else { wv = *reinterpret_cast<const uint4*>(w + i); if (b) bv = *reinterpret_cast<const uint4*>(b + i); }
             const float f[8] = {bf16lo(v[k].x), bf16hi(v[k].x), bf16lo(v[k].y), bf16hi(v[k].y),
                                 bf16lo(v[k].z), bf16hi(v[k].z), bf16lo(v[k].w), bf16hi(v[k].w)};
@@ -178,13 +183,17 @@ bool vision_layernorm(const void* x, const void* w, const void* b, void* y, int 
     if (!x || !w || !y || rows <= 0 || cols <= 0) { set_error("vision_layernorm: bad args"); return false; }
     const int vec = (cols % 8) == 0 && ((((uintptr_t)x) | ((uintptr_t)w) | ((uintptr_t)b) | ((uintptr_t)y)) & 15) == 0;
     const int grid = (rows + LN_WARPS - 1) / LN_WARPS;
-    auto launch = [&](auto kern, auto... more) {
+    if (vec && cols <= 18 * 256) {
+        const bool few = rows <= OVERLAP_ROWS;
+        auto kern = cols <= 5 * 256 ? (few ? layernorm_reg_kernel<5, true> : layernorm_reg_kernel<5, false>)
+                                    : (few ? layernorm_reg_kernel<18, true> : layernorm_reg_kernel<18, false>);
         return launch_ok(launch_chained(kern, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows, (const uint16_t*)x, (const uint16_t*)w,
-                                        (const uint16_t*)b, (uint16_t*)y, rows, cols, eps, more...), "vision_layernorm");
-    };
-    if (vec && cols <= 5 * 256) return launch(layernorm_reg_kernel<5>);
-    if (vec && cols <= 18 * 256) return launch(layernorm_reg_kernel<18>);
-    return launch(layernorm_kernel, vec);
+                                        (const uint16_t*)b, (uint16_t*)y, rows, cols, eps), "vision_layernorm");
+    }
+    // (overlapped up to 1024 rows only: 300 x 8192 11.0 us against 12.4, but 2048 x 8192 29.4 against 15.5)
+    return launch_ok(launch_chained(layernorm_kernel, dim3(grid), dim3(LN_WARPS * 32), 0, st, 1, rows <= 1024 ? rows : OVERLAP_ROWS + 1,
+                                    (const uint16_t*)x, (const uint16_t*)w, (const uint16_t*)b, (uint16_t*)y, rows, cols, eps, vec),
+                     "vision_layernorm");
 }
 
 // GELU, tanh form (block MLP) or erf form (mergers): vision_kernels.cu:100-133
