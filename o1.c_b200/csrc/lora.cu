@@ -377,7 +377,8 @@ extern "C" {
 
 // Returns once the merge is done, so that the caller may release the adapters.  HD_ERR_RUNTIME when it was not: an error of
 // the stream, or the device's error word set, in which case the kernel merges nothing (it was set before) or stops on the way
-// (one of its waits ran out).
+// (one of its waits ran out).  A call whose targets all take the simple kernel (no whole 128-column tiles) only enqueues: it
+// takes 4 us instead of 11 and can be captured, and the adapters stay until the stream has come past it.
 hd_status hd_lora_merge_gpu(hd_lora_entry* entries, size_t count, void* stream) {
     if (count == 0) return HD_OK;
     if (!entries) { set_error("lora: null entries"); return HD_ERR_MISSING; }
@@ -424,13 +425,10 @@ hd_status hd_lora_merge_gpu(hd_lora_entry* entries, size_t count, void* stream) 
     }
     // (an entry that cannot be used ends the call; the ones before it are merged)
     if (!grp.launch(st) && rc == HD_OK) rc = HD_ERR_RUNTIME;
-    // A call whose targets all took the simple kernel may be part of a stream capture: there is nothing to wait for then.
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!grp.launched && cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-    if (cap != cudaStreamCaptureStatusNone) return rc;
+    if (!grp.launched) return rc;
     const cudaError_t e = cudaStreamSynchronize(st);
     // (a copy of the error word itself would take 7.6 us: 236 -> 244 us for the adapter of a whole block)
-    const int word = grp.launched ? *(volatile int*)device_failed_word() : 0;
+    const int word = *(volatile int*)device_failed_word();
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error("lora: %s", cudaGetErrorString(e));
