@@ -649,6 +649,7 @@ struct SplitCfg {
 // The tower's q | k | v projection takes the same kernel unsplit with tiles of 144 columns, two whole heads of 72: a
 // thread then holds both halves of its row's heads and the rotary is part of the epilogue (3456 = 24 tiles exactly).
 static constexpr int VQ_BN = 144;
+static constexpr int VQ_PITCH = 168;     // bytes of a staged row of one head: 16 lanes' 8-byte pieces meet 32 different banks
 
 __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d)
@@ -741,7 +742,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     // The epilogue's other operands are requested while the main loop runs: this thread's residual row into registers, the
     // tile's bias into shared memory (each of the eight units of a tile would otherwise wait for its own loads).
-    constexpr bool HAS_BIAS = EPI != EPI_STORE && EPI != EPI_RESID && EPI != EPI_VROPE;
+    constexpr bool HAS_BIAS = EPI != EPI_STORE && EPI != EPI_RESID;
     constexpr bool HAS_RESID = EPI == EPI_RESID || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID;
     const int q = warp & 3;       // TMEM lane quadrant this warp may access
     const int trow = q * 32 + lane;
@@ -749,7 +750,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int row = mb * BM + trow;
     const bool row_ok = row < g.M;
     uint4 res[HAS_RESID ? 2 * NU : 1];
+    float vcs[36], vsn[36];      // (EPI_VROPE)
     if (ok && warp >= 2) {
+        if (EPI == EPI_VROPE) {
+            const int r = row_ok ? row : 0;
+#pragma unroll
+            for (int c = 0; c < 9; ++c) {
+                const float4 c4 = *reinterpret_cast<const float4*>(g.rope + (size_t)r * 72 + c * 4);
+                const float4 s4 = *reinterpret_cast<const float4*>(g.rope_sin + (size_t)r * 72 + c * 4);
+                vcs[c * 4] = c4.x; vcs[c * 4 + 1] = c4.y; vcs[c * 4 + 2] = c4.z; vcs[c * 4 + 3] = c4.w;
+                vsn[c * 4] = s4.x; vsn[c * 4 + 1] = s4.y; vsn[c * 4 + 2] = s4.z; vsn[c * 4 + 3] = s4.w;
+            }
+        }
         if (HAS_BIAS && trow * 8 < BN) {
             const int col = nb * BN + trow * 8;
             bias_s[trow] = col < g.N ? *reinterpret_cast<const uint4*>(g.bias + col) : make_uint4(0, 0, 0, 0);
@@ -772,52 +784,56 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const bool store = row_ok && !failed;
     const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
     if constexpr (EPI == EPI_VROPE) {
+        // Bias, rotary and the spacing of the heads.  cos and sin of this thread's row have come into registers under the main
+        // loop; a head goes through shared memory (the stages are free now) and leaves as whole rows of 160 bytes.  With cos / sin
+        // loaded per head and every thread storing its own row, 32 lines to an instruction, this epilogue took three times the
+        // main loop's time: the launch 21.4 -> 14.6 us at 520 rows and 60.8 -> 43.8 us at 4096.
         if (ok && warp >= 2) {
+            uint8_t* stg = smem + q * (32 * VQ_PITCH);
 #pragma unroll 1
             for (int hh = 0; hh < 2; ++hh) {
-                uint32_t ra[32], rb[32], rc[8];
-                tmem_ld32(t_row + hh * 72, ra);
-                tmem_ld32(t_row + hh * 72 + 32, rb);
-                tmem_ld8(t_row + hh * 72 + 64, rc);
-                tmem_ld_wait();
-                if (store) {
-                    const int col = nb * VQ_BN + hh * 72, which = col / 1152, h = (col - which * 1152) / 72;
-                    float x[72];
+                const int col = nb * VQ_BN + hh * 72, which = col / 1152, h = (col - which * 1152) / 72;
+                const uint2* bs = reinterpret_cast<const uint2*>(bias_s) + hh * 18;
+                __syncwarp();
 #pragma unroll
-                    for (int c = 0; c < 9; ++c) {
-                        const uint4 b4 = *reinterpret_cast<const uint4*>(g.bias + col + c * 8);
-                        const float b[8] = {bf16lo(b4.x), bf16hi(b4.x), bf16lo(b4.y), bf16hi(b4.y),
-                                            bf16lo(b4.z), bf16hi(b4.z), bf16lo(b4.w), bf16hi(b4.w)};
+                for (int k = 0; k < 3; ++k) {      // twelve columns and their partners 36 further
+                    uint32_t rl[3][4], rh[3][4];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const int d = c * 8 + j;
-                            const uint32_t r = d < 32 ? ra[d & 31] : (d < 64 ? rb[d & 31] : rc[d & 7]);
-                            x[d] = bf16_round(bf16_round(__uint_as_float(r)) + b[j]);
+                    for (int i = 0; i < 3; ++i) {
+                        tmem_ld4(t_row + hh * 72 + k * 12 + i * 4, rl[i]);
+                        tmem_ld4(t_row + hh * 72 + 36 + k * 12 + i * 4, rh[i]);
+                    }
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        const uint2 bl = bs[k * 3 + i], bh = bs[9 + k * 3 + i];
+                        const float b0[4] = {bf16lo(bl.x), bf16hi(bl.x), bf16lo(bl.y), bf16hi(bl.y)};
+                        const float b1[4] = {bf16lo(bh.x), bf16hi(bh.x), bf16lo(bh.y), bf16hi(bh.y)};
+                        float lo[4], hi[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float x = bf16_round(bf16_round(__uint_as_float(rl[i][j])) + b0[j]);
+                            const float y = bf16_round(bf16_round(__uint_as_float(rh[i][j])) + b1[j]);
+                            const float c = vcs[(k * 3 + i) * 4 + j], sn = vsn[(k * 3 + i) * 4 + j];
+                            // fp32 rotary, one rounding (src/cuda/rope.cu:155-178); the table repeats after 36
+                            lo[j] = which < 2 ? rope_f32(x, c, -y, sn) : x;
+                            hi[j] = which < 2 ? rope_f32(y, c, x, sn) : y;
                         }
+                        uint2* d = reinterpret_cast<uint2*>(stg + lane * VQ_PITCH) + k * 3 + i;
+                        d[0] = make_uint2(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]));
+                        d[9] = make_uint2(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]));
                     }
-                    if (which < 2) {     // fp32 rotary, one rounding (src/cuda/rope.cu:155-178); the table repeats after 36
+                }
+                __syncwarp();
+                const int rows = failed ? 0 : g.M - mb * BM - q * 32;
+                uint16_t* out = g.out + (size_t)(mb * BM + q * 32) * g.ldo + (which * 16 + h) * 128;
 #pragma unroll
-                        for (int c = 0; c < 9; ++c) {
-                            const float4 c4 = *reinterpret_cast<const float4*>(g.rope + (size_t)row * 72 + c * 4);
-                            const float4 s4 = *reinterpret_cast<const float4*>(g.rope_sin + (size_t)row * 72 + c * 4);
-                            const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const float lo = x[c * 4 + j], hi = x[c * 4 + j + 36];
-                                x[c * 4 + j] = rope_f32(lo, cs[j], -hi, sn[j]);
-                                x[c * 4 + j + 36] = rope_f32(hi, cs[j], lo, sn[j]);
-                            }
-                        }
-                    }
-                    uint4* dst = reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + (which * 16 + h) * 128);
-#pragma unroll
-                    for (int c = 0; c < 9; ++c) {
-                        uint4 o;
-                        o.x = pack_bf16x2(x[c * 8], x[c * 8 + 1]); o.y = pack_bf16x2(x[c * 8 + 2], x[c * 8 + 3]);
-                        o.z = pack_bf16x2(x[c * 8 + 4], x[c * 8 + 5]); o.w = pack_bf16x2(x[c * 8 + 6], x[c * 8 + 7]);
-                        dst[c] = o;
-                    }
-                    dst[9] = make_uint4(0, 0, 0, 0);
+                for (int i = 0; i < 10; ++i) {
+                    const int p = i * 32 + lane, r = p / 10, c = p - r * 10;
+                    const uint2* sp = reinterpret_cast<const uint2*>(stg + r * VQ_PITCH) + c * 2;
+                    uint4 o = make_uint4(0, 0, 0, 0);          // columns 72..79
+                    if (c < 9) { const uint2 o0 = sp[0], o1 = sp[1]; o = make_uint4(o0.x, o0.y, o1.x, o1.y); }
+                    if (r < rows) *reinterpret_cast<uint4*>(out + (size_t)r * g.ldo + c * 8) = o;
                 }
             }
         }
