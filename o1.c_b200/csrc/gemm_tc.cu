@@ -5,7 +5,7 @@
 // Structure: persistent CTAs (one per SM), 128 x BN x 64 tiles.
 //   warp 0      : TMA producer  (global -> 128B-swizzled shared, 4-6 stages)
 //   warp 1      : tcgen05.mma issuer, accumulators in TMEM, double buffered
-//   warps 2..5  : epilogue (tcgen05.ld -> registers -> fused op -> global)
+//   warps 2..9  : epilogue (tcgen05.ld -> registers -> fused op -> shared memory -> global)
 // The epilogue of tile i overlaps the main loop of tile i+1.
 //
 // Fused epilogues keep the reference's bf16 rounding points:
@@ -29,7 +29,9 @@ namespace o1 {
 
 static constexpr int BM = 128;
 static constexpr int BK = 64;
-static constexpr int GEMM_THREADS = 192;
+static constexpr int EPI_WARPS = 8;                       // two per quadrant of tensor memory
+static constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
+static constexpr int SK_THREADS = 192;                    // gemm_split_kernel's 32-column and shared tiles: four epilogue warps
 
 struct GemmArgs {
     int M, N, K;
@@ -75,7 +77,7 @@ struct GemmCfg {
     static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int STAGES = PAIR ? 6 : ((BN == 256) ? 4 : 6);
-    static constexpr int STORE_STAGE_BYTES = 4 * 2 * 32 * 128;   // per epilogue warp two slices of 32 rows x 128 B (peer stores)
+    static constexpr int STORE_STAGE_BYTES = EPI_WARPS * 4096;   // epilogue staging, 4 KB per warp
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + STORE_STAGE_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;
 };
@@ -104,31 +106,189 @@ __device__ __forceinline__ void gelu_all(float (&v)[N], bool exact) {
         for (int j = 0; j < N; ++j) v[j] = gelu_tanh(v[j]);
     }
 }
-__device__ __forceinline__ void store32_bf16(uint16_t* dst, const float (&v)[32]) {
-    uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint4 o;
-        o.x = pack_bf16x2(v[i * 8 + 0], v[i * 8 + 1]);
-        o.y = pack_bf16x2(v[i * 8 + 2], v[i * 8 + 3]);
-        o.z = pack_bf16x2(v[i * 8 + 4], v[i * 8 + 5]);
-        o.w = pack_bf16x2(v[i * 8 + 6], v[i * 8 + 7]);
-        d4[i] = o;
-    }
-}
 __device__ __forceinline__ void unpack8_bf16(const uint4& o, float* v) {
     v[0] = bf16lo(o.x); v[1] = bf16hi(o.x); v[2] = bf16lo(o.y); v[3] = bf16hi(o.y);
     v[4] = bf16lo(o.z); v[5] = bf16hi(o.z); v[6] = bf16lo(o.w); v[7] = bf16hi(o.w);
 }
-__device__ __forceinline__ void load32_bf16(const uint16_t* src, float (&v)[32]) {
-    const uint4* s4 = reinterpret_cast<const uint4*>(src);
+
+// ---- epilogues.  A warp holds 32 accumulator rows, one per thread.  What it loads and stores goes through its slice of shared
+// memory, so that every access to global memory is of whole row segments of 64 bytes and more: with a thread storing its own row an
+// instruction touches 32 lines, and that, four warps instead of eight and SwiGLU's branch per value (its division) made an epilogue
+// of 11 us (SwiGLU), 15 (per-head norm) and 5 to 10 (the others) per 256-column tile.  The main loop of the next tile covers that, but
+// not a CTA's last tile: q | k | v at 592 rows was 48 us for a round of 25.
+
+// Groups of 32 columns at c_first, c_first + c_step, ... of a tile, plain row-major output (or column blocks, see GemmArgs).
+template <int EPI>
+struct PlainEpilogue {
+    static constexpr bool HAS_BIAS = EPI != EPI_STORE && EPI != EPI_RESID;
+    static constexpr bool HAS_RESID = EPI == EPI_RESID || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID;
+    uint4 rn[4] = {};        // the residual of the group that comes next, eight rows of four 16-byte pieces at a time
+    // row0: first of the warp's rows; cols: columns of the tile that exist (a multiple of eight)
+    __device__ __forceinline__ void ahead(const GemmArgs& g, int row0, int col0, int cols, int c, int lane) {
+        if (!HAS_RESID) return;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint4 o = s4[i];
-        v[i * 8 + 0] = bf16lo(o.x); v[i * 8 + 1] = bf16hi(o.x);
-        v[i * 8 + 2] = bf16lo(o.y); v[i * 8 + 3] = bf16hi(o.y);
-        v[i * 8 + 4] = bf16lo(o.z); v[i * 8 + 5] = bf16hi(o.z);
-        v[i * 8 + 6] = bf16lo(o.w); v[i * 8 + 7] = bf16hi(o.w);
+        for (int k = 0; k < 4; ++k) {
+            const int row = row0 + k * 8 + (lane >> 2), col = c + (lane & 3) * 8;
+            if (row < g.M && col < cols) rn[k] = *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col0 + col);
+        }
+    }
+    // the caller has called ahead() for c_first; stg: 2 KB of the warp's own
+    __device__ __forceinline__ void run(const GemmArgs& g, uint32_t t_row, int row0, int col0, int cols, int c_first, int c_step,
+                                        uint8_t* stg, int lane, bool failed) {
+        const int sr = lane >> 2, ch = lane & 3;
+        uint4* own = reinterpret_cast<uint4*>(stg + lane * 64);
+#pragma unroll 1
+        for (int c = c_first; c < cols; c += c_step) {
+            __syncwarp();
+            if (HAS_RESID) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    *reinterpret_cast<uint4*>(stg + (k * 8 + sr) * 64 + ((ch ^ ((sr >> 1) & 3)) * 16)) = rn[k];
+                ahead(g, row0, col0, cols, c + c_step, lane);
+                __syncwarp();
+            }
+            uint32_t r[32];
+            tmem_ld32(t_row + c, r);
+            tmem_ld_wait();
+            float v[32];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float b[8] = {}, rs[8] = {};
+                if (HAS_BIAS) {
+                    const int col = c + i * 8;
+                    unpack8_bf16(col < cols ? *reinterpret_cast<const uint4*>(g.bias + col0 + col) : make_uint4(0, 0, 0, 0), b);
+                }
+                if (HAS_RESID) unpack8_bf16(own[i ^ ((lane >> 1) & 3)], rs);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    float x = __uint_as_float(r[i * 8 + j]);
+                    if (EPI == EPI_BIAS) x = bf16_round(x) + b[j];
+                    if (EPI == EPI_BIAS_GELU) x = bf16_round(bf16_round(x) + b[j]);
+                    if (EPI == EPI_RESID) x = bf16_round(x) + rs[j];
+                    // linear + bias stored as bf16, then the residual add of src/cuda/residual.cu:14-23
+                    if (EPI == EPI_BIAS_RESID) x = rs[j] + bf16_round(bf16_round(x) + b[j]);
+                    if (EPI == EPI_GATE_RESID) x = rs[j] + bf16_round(b[j] * bf16_round(x));
+                    v[i * 8 + j] = x;
+                }
+            }
+            if (EPI == EPI_BIAS_GELU) gelu_all(v, g.scale != 0.f);
+            store_group(g, v, stg, row0, col0 + c, cols - c, lane, failed);
+        }
+    }
+    // this thread's row of 32 columns -> the warp's rows as segments of 64 bytes
+    static __device__ __forceinline__ void store_group(const GemmArgs& g, const float (&v)[32], uint8_t* stg, int row0, int col, int cols,
+                                                       int lane, bool failed) {
+        const int sr = lane >> 2, ch = lane & 3;
+        uint4* own = reinterpret_cast<uint4*>(stg + lane * 64);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float* x = v + i * 8;
+            own[i ^ ((lane >> 1) & 3)] = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]),
+                                                    pack_bf16x2(x[6], x[7]));
+        }
+        __syncwarp();
+        // (a group of 32 columns never straddles an output block)
+        uint16_t* out = g.out + (g.o_cb ? (size_t)(col / g.o_cb) * g.o_cb_stride + col % g.o_cb : (size_t)col) + ch * 8;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int row = row0 + k * 8 + sr;
+            const uint4 o = *reinterpret_cast<const uint4*>(stg + (k * 8 + sr) * 64 + ((ch ^ ((sr >> 1) & 3)) * 16));
+            if (!failed && row < g.M && ch * 8 < cols) *reinterpret_cast<uint4*>(out + (size_t)row * g.ldo) = o;
+        }
+    }
+};
+
+// SwiGLU of 32 columns: bf16(silu(g)) * u with silu(g) = g * (1 / (1 + e^-g)).  The quotient is the IEEE one, by Markstein's step from
+// the approximate reciprocal (P. Markstein, IBM J. Res. Dev. 34, 1990); the division itself, which branches for each value, is left
+// to warps that hold a gate below -80, where 1 + e^-g comes near the largest number, or a NaN.
+__device__ __forceinline__ void swiglu_all(const uint32_t (&rg)[32], const uint32_t (&ru)[32], float (&v)[32]) {
+    bool plain = true;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        v[j] = bf16_round(__uint_as_float(rg[j]));
+        plain = plain && v[j] > -80.f;
+    }
+    if (__all_sync(0xffffffffu, plain)) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const float x = 1.0f + expf(-v[j]);
+            const float y = __fdividef(1.0f, x);
+            const float sg = __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+            v[j] = bf16_round(v[j] * sg) * bf16_round(__uint_as_float(ru[j]));
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const float sg = 1.0f / (1.0f + expf(-v[j]));
+            v[j] = bf16_round(v[j] * sg) * bf16_round(__uint_as_float(ru[j]));
+        }
+    }
+}
+
+// Per-head RMSNorm + rotary on a projection's output (o1.c src/model/block.c:266-289 runs head split, hd_rmsnorm, hd_apply_rotary as
+// separate passes).  The 128 values of a head are rounded to bf16 (the projection's stored result) and pass through shared memory, 16
+// rows at a time; then eight lanes take a row: each sums 8 + 8 elements, the pairwise tree over the lanes is the order of
+// qk_norm_rope_kernel, so that both paths agree bit for bit, and cos | sin and the result are whole lines.  half_lo .. half_hi: which
+// of the warp's two groups of 16 rows; obase: the head's first column of row 0.
+__device__ __forceinline__ void head_epilogue(const GemmArgs& g, uint32_t t_head, int row0, int rows, uint16_t* obase,
+                                              const uint16_t* norm_w, int half_lo, int half_hi, uint8_t* stg, int lane) {
+    const int t = lane & 7, sub = lane >> 3;
+    float wl[8], wh[8];
+    unpack8_bf16(*reinterpret_cast<const uint4*>(norm_w + 8 * t), wl);
+    unpack8_bf16(*reinterpret_cast<const uint4*>(norm_w + 64 + 8 * t), wh);
+#pragma unroll 1
+    for (int hf = half_lo; hf < half_hi; ++hf) {
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            uint32_t r[32];
+            tmem_ld32(t_head + c * 32, r);
+            tmem_ld_wait();
+            if ((lane >> 4) == hf) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    uint4 o;
+                    o.x = pack_bf16x2(__uint_as_float(r[8 * i]), __uint_as_float(r[8 * i + 1]));
+                    o.y = pack_bf16x2(__uint_as_float(r[8 * i + 2]), __uint_as_float(r[8 * i + 3]));
+                    o.z = pack_bf16x2(__uint_as_float(r[8 * i + 4]), __uint_as_float(r[8 * i + 5]));
+                    o.w = pack_bf16x2(__uint_as_float(r[8 * i + 6]), __uint_as_float(r[8 * i + 7]));
+                    *reinterpret_cast<uint4*>(stg + (lane & 15) * 256 + (((c * 4 + i) ^ (lane & 7)) * 16)) = o;
+                }
+            }
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (int it = 0; it < 4; ++it) {
+            const int rr = it * 4 + sub, row = row0 + hf * 16 + rr;
+            const bool row_ok = row < rows;
+            const float* cs = g.rope + (size_t)(row_ok ? row : 0) * 128 + 8 * t;
+            const float4 ca = *reinterpret_cast<const float4*>(cs), cb = *reinterpret_cast<const float4*>(cs + 4);
+            const float4 sa = *reinterpret_cast<const float4*>(cs + 64), sb = *reinterpret_cast<const float4*>(cs + 68);
+            float lo[8], hi[8];
+            unpack8_bf16(*reinterpret_cast<const uint4*>(stg + rr * 256 + ((t ^ (rr & 7)) * 16)), lo);
+            unpack8_bf16(*reinterpret_cast<const uint4*>(stg + rr * 256 + (((8 + t) ^ (rr & 7)) * 16)), hi);
+            float sq = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sq = __fadd_rn(sq, __fmaf_rn(hi[j], hi[j], __fmul_rn(lo[j], lo[j])));
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) sq = __fadd_rn(sq, __shfl_xor_sync(0xffffffffu, sq, o));
+            const float inv = rsqrtf(sq / 128.0f + g.scale);
+            const float cc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+            const float ss[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+            float ol[8], oh[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float a = bf16_round(wl[j] * lo[j] * inv);
+                const float b = bf16_round(wh[j] * hi[j] * inv);
+                ol[j] = bf16_round(a * cc[j]) - bf16_round(b * ss[j]);
+                oh[j] = bf16_round(b * cc[j]) + bf16_round(a * ss[j]);
+            }
+            if (row_ok) {
+                uint16_t* o = obase + (size_t)row * g.ldo + 8 * t;
+                *reinterpret_cast<uint4*>(o) = make_uint4(pack_bf16x2(ol[0], ol[1]), pack_bf16x2(ol[2], ol[3]), pack_bf16x2(ol[4], ol[5]), pack_bf16x2(ol[6], ol[7]));
+                *reinterpret_cast<uint4*>(o + 64) = make_uint4(pack_bf16x2(oh[0], oh[1]), pack_bf16x2(oh[2], oh[3]), pack_bf16x2(oh[4], oh[5]), pack_bf16x2(oh[6], oh[7]));
+            }
+        }
     }
 }
 
@@ -168,7 +328,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&tfull[s], 1);
-            mbar_init(&tempty[s], PAIR ? 8 : 4);    // the epilogue warps of both CTAs arrive on the first CTA's
+            mbar_init(&tempty[s], PAIR ? 2 * EPI_WARPS : EPI_WARPS);    // the epilogue warps of both CTAs arrive on the first CTA's
         }
         fence_mbar_init();
     }
@@ -294,7 +454,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else {
         // ------------------------------------------------------ epilogue
-        const int q = warp & 3;  // TMEM lane quadrant this warp may access
+        const int q = warp & 3;                  // TMEM lane quadrant this warp may access
+        const int half = (warp - 2) >> 2;        // which of the quadrant's two warps
+        uint8_t* stg = store_stage + (warp - 2) * 4096;
         int as = 0;
         uint32_t aphase = 0;
         const int failed = error_word(g.err);
@@ -302,11 +464,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int mb, nb;
             tile_coords(tile, sched_m, g.num_n, sched_group, mb, nb);
             if (PAIR) mb = mb * 2 + (int)rank;
-            if (!mbar_wait(&tfull[as], aphase)) { atomicExch(g.err, 4); break; }
-            tc_fence_after();
             const int rows = failed ? 0 : g.M;
-            const int row = mb * BM + q * 32 + lane;
-            const bool row_ok = row < rows;
+            const int row0 = mb * BM + q * 32;
+            const int cols = g.N - nb * BN < BN ? g.N - nb * BN : BN;      // (plain epilogues: N may be ragged, N % 8 == 0)
+            PlainEpilogue<EPI> plain;
+            plain.ahead(g, row0, nb * BN, cols, half * 32, lane);
+            const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase));
+            if (!got) { atomicExch(g.err, 4); break; }
+            tc_fence_after();
             const uint32_t t_row = tmem_base + as * BN + ((uint32_t)(q * 32) << 16);
             // EPI_QKV: which segment this column tile lies in decides the epilogue (warp-uniform); everything
             // below addresses the output through (seg_col0 + column inside the segment) or the segment's tables
@@ -324,31 +489,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int epi_eff = (EPI == EPI_QKV) ? (seg < 2 ? (int)EPI_QKNORM : (int)EPI_STORE) : EPI;
             if (EPI == EPI_SWIGLU) {
 #pragma unroll 1
-                for (int c = 0; c < 4; ++c) {
+                for (int c = half * 32; c < 128; c += 64) {
                     uint32_t rg[32], ru[32];
-                    tmem_ld32(t_row + c * 32, rg);
-                    tmem_ld32(t_row + 128 + c * 32, ru);
+                    tmem_ld32(t_row + c, rg);
+                    tmem_ld32(t_row + 128 + c, ru);
                     tmem_ld_wait();
-                    if (row_ok) {
-                        float v[32];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const float gg = bf16_round(__uint_as_float(rg[j]));
-                            const float uu = bf16_round(__uint_as_float(ru[j]));
-                            const float sg = 1.0f / (1.0f + expf(-gg));
-                            v[j] = bf16_round(gg * sg) * uu;
-                        }
-                        store32_bf16(g.out + (size_t)row * g.ldo + nb * 128 + c * 32, v);
-                    }
+                    float v[32];
+                    swiglu_all(rg, ru, v);
+                    __syncwarp();
+                    PlainEpilogue<EPI_STORE>::store_group(g, v, stg, row0, nb * 128 + c, 32, lane, failed);
                 }
             } else if (epi_eff == EPI_STORE && g.o_tab_n) {
                 // Blocks of the output live in other GPUs' memory.  One thread per row would put 16-byte
                 // pieces of 32 different rows into every store instruction; over NVLink each piece is a
-                // packet of its own.  So 64 columns at a time go through a swizzled shared-memory slice of
+                // packet of its own.  So 64 columns at a time go through the swizzled shared-memory slice of
                 // this warp and leave as full 128-byte row segments (4 rows per instruction).
-                uint8_t* stg = store_stage + q * (2 * 32 * 128);
 #pragma unroll 1
-                for (int c2 = 0; c2 < BN / 64; ++c2) {
+                for (int c2 = half; c2 < BN / 64; c2 += 2) {
                     uint32_t r0[32], r1[32];
                     tmem_ld32(t_row + c2 * 64, r0);
                     tmem_ld32(t_row + c2 * 64 + 32, r1);
@@ -371,130 +528,43 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     for (int k = 0; k < 8; ++k) {
                         const int rr = k * 4 + (lane >> 3);
                         const uint4 o = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((ch ^ (rr & 7)) * 16));
-                        const int grow = mb * BM + q * 32 + rr;
-                        if (grow < rows) *reinterpret_cast<uint4*>(obase + (size_t)grow * g.ldo + ch * 8) = o;
+                        if (row0 + rr < rows) *reinterpret_cast<uint4*>(obase + (size_t)(row0 + rr) * g.ldo + ch * 8) = o;
                     }
                     __syncwarp();
                 }
             } else if (epi_eff == EPI_QKNORM) {
-                // Per-head RMSNorm + rotary on the projection's output row (o1.c src/model/block.c:266-289 runs
-                // head split, hd_rmsnorm, hd_apply_rotary as separate passes).  This thread owns the whole row of
-                // the tile, i.e. BN/128 complete heads: the 128 values of a head are rounded to bf16 (the
-                // projection's stored result), summed in the order of qk_norm_rope_kernel (eight partial sums of
-                // 8 + 8 elements, pairwise tree) so that both paths agree bit for bit, normalised, rotated with the
-                // partner 64 columns away, and written once.
-#pragma unroll 1
-                for (int hb = 0; hb < BN / 128; ++hb) {
-                    uint32_t r[4][32];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) tmem_ld32(t_row + hb * 128 + c * 32, r[c]);
-                    tmem_ld_wait();
-                    if (row_ok) {
-                        float part[8];
-#pragma unroll
-                        for (int t = 0; t < 8; ++t) {
-                            float acc = 0.f;
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const int e = 8 * t + j;
-                                const float lo = bf16_round(__uint_as_float(r[e >> 5][e & 31]));
-                                const float hi = bf16_round(__uint_as_float(r[2 + (e >> 5)][e & 31]));
-                                r[e >> 5][e & 31] = __float_as_uint(lo);
-                                r[2 + (e >> 5)][e & 31] = __float_as_uint(hi);
-                                acc = __fadd_rn(acc, __fmaf_rn(hi, hi, __fmul_rn(lo, lo)));
-                            }
-                            part[t] = acc;
-                        }
-                        const float sq = __fadd_rn(__fadd_rn(__fadd_rn(part[0], part[1]), __fadd_rn(part[2], part[3])),
-                                                   __fadd_rn(__fadd_rn(part[4], part[5]), __fadd_rn(part[6], part[7])));
-                        const float inv = rsqrtf(sq / 128.0f + g.scale);
-                        const int col = seg_col0 + lcol0 + hb * 128;
-                        const size_t ocol = g.o_cb ? (size_t)(col / g.o_cb) * g.o_cb_stride + (col % g.o_cb) : (size_t)col;
-                        uint16_t* orow = g.o_tab_n ? nullptr : g.out + (size_t)row * g.ldo + ocol;
-                        uint8_t* stg_row = store_stage + q * (2 * 32 * 128) + lane * 128;
-                        const float* cs = g.rope + (size_t)row * 128;
-#pragma unroll
-                        for (int t = 0; t < 8; ++t) {
-                            const uint4 wl4 = *reinterpret_cast<const uint4*>(norm_w + 8 * t);
-                            const uint4 wh4 = *reinterpret_cast<const uint4*>(norm_w + 64 + 8 * t);
-                            const float wl[8] = {bf16lo(wl4.x), bf16hi(wl4.x), bf16lo(wl4.y), bf16hi(wl4.y),
-                                                 bf16lo(wl4.z), bf16hi(wl4.z), bf16lo(wl4.w), bf16hi(wl4.w)};
-                            const float wh[8] = {bf16lo(wh4.x), bf16hi(wh4.x), bf16lo(wh4.y), bf16hi(wh4.y),
-                                                 bf16lo(wh4.z), bf16hi(wh4.z), bf16lo(wh4.w), bf16hi(wh4.w)};
-                            const float4 ca = *reinterpret_cast<const float4*>(cs + 8 * t);
-                            const float4 cb = *reinterpret_cast<const float4*>(cs + 8 * t + 4);
-                            const float4 sa = *reinterpret_cast<const float4*>(cs + 64 + 8 * t);
-                            const float4 sb = *reinterpret_cast<const float4*>(cs + 64 + 8 * t + 4);
-                            const float cc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
-                            const float ss[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
-                            float ol[8], oh[8];
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const int e = 8 * t + j;
-                                const float lo = __uint_as_float(r[e >> 5][e & 31]);
-                                const float hi = __uint_as_float(r[2 + (e >> 5)][e & 31]);
-                                const float a = bf16_round(wl[j] * lo * inv);
-                                const float b = bf16_round(wh[j] * hi * inv);
-                                ol[j] = bf16_round(a * cc[j]) - bf16_round(b * ss[j]);
-                                oh[j] = bf16_round(b * cc[j]) + bf16_round(a * ss[j]);
-                            }
-                            uint4 po, ph;
-                            po.x = pack_bf16x2(ol[0], ol[1]); po.y = pack_bf16x2(ol[2], ol[3]);
-                            po.z = pack_bf16x2(ol[4], ol[5]); po.w = pack_bf16x2(ol[6], ol[7]);
-                            ph.x = pack_bf16x2(oh[0], oh[1]); ph.y = pack_bf16x2(oh[2], oh[3]);
-                            ph.z = pack_bf16x2(oh[4], oh[5]); ph.w = pack_bf16x2(oh[6], oh[7]);
-                            if (g.o_tab_n) {
-                                // destination rows live in another GPU's memory: both 64-column halves of the
-                                // head go through this warp's two swizzled shared-memory slices first
-                                *reinterpret_cast<uint4*>(stg_row + ((t ^ (lane & 7)) * 16)) = po;
-                                *reinterpret_cast<uint4*>(stg_row + 32 * 128 + ((t ^ (lane & 7)) * 16)) = ph;
-                            } else {
-                                *reinterpret_cast<uint4*>(orow + 8 * t) = po;
-                                *reinterpret_cast<uint4*>(orow + 64 + 8 * t) = ph;
-                            }
-                        }
-                    }
-                    if (g.o_tab_n) {
-                        // leave as full 128-byte row segments, 4 rows per store instruction (a head never straddles
-                        // a destination block: o_cb % 128 == 0)
-                        __syncwarp();
-                        const int col = lcol0 + hb * 128;
-                        uint16_t* obase = tab[col / cb] + (col % cb);
-                        const uint8_t* stg = store_stage + q * (2 * 32 * 128);
-                        const int ch = lane & 7;
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) {
-                                const int rr = k * 4 + (lane >> 3);
-                                const uint4 o = *reinterpret_cast<const uint4*>(stg + hf * (32 * 128) + rr * 128 + ((ch ^ (rr & 7)) * 16));
-                                const int grow = mb * BM + q * 32 + rr;
-                                if (grow < rows) *reinterpret_cast<uint4*>(obase + (size_t)grow * g.ldo + hf * 64 + ch * 8) = o;
-                            }
-                        __syncwarp();
-                    }
+                // two heads: one for each of a quadrant's warps; one head: 16 rows each
+                const int hb = BN == 256 ? half : 0, col = lcol0 + hb * 128;
+                uint16_t* obase;
+                if (g.o_tab_n) obase = tab[col / cb] + (col % cb);       // (a head never straddles a destination block)
+                else {
+                    const int c = seg_col0 + col;
+                    obase = g.out + (g.o_cb ? (size_t)(c / g.o_cb) * g.o_cb_stride + (c % g.o_cb) : (size_t)c);
                 }
+                head_epilogue(g, t_row + hb * 128, row0, rows, obase, norm_w, BN == 256 ? 0 : half, BN == 256 ? 2 : half + 1, stg, lane);
             } else if (EPI == EPI_LORA) {
-                // In-place update of W.  The contraction is short (9 x rank), so this epilogue's read-modify-
-                // write of W bounds the kernel: all of the row's W values of four 32-column groups are requested
-                // before the first is used, which keeps about 32 KB per SM in flight instead of one load per thread.
+                // In-place update of W.  The contraction is short (9 x rank), so this epilogue's read-modify-write of W bounds
+                // the kernel: a row's W values of two 32-column groups are requested before the first is used.
+                const int row = row0 + lane;
+                const bool row_ok = row < rows;
 #pragma unroll 1
                 for (int c4 = 0; c4 < BN / 128; ++c4) {
-                    uint4 wv[4][4];
-                    const uint16_t* wrow = g.out + (size_t)row * g.ldo + nb * BN + c4 * 128;
+                    uint4 wv[2][4];
+                    const int at = c4 * 128 + half * 64;
+                    const uint16_t* wrow = g.out + (size_t)row * g.ldo + nb * BN + at;
                     if (row_ok) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
+                        for (int c = 0; c < 2; ++c)
 #pragma unroll
                             for (int i = 0; i < 4; ++i) wv[c][i] = reinterpret_cast<const uint4*>(wrow + c * 32)[i];
                     }
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
+                    for (int c = 0; c < 2; ++c) {
                         uint32_t r[32];
-                        tmem_ld32(t_row + c4 * 128 + c * 32, r);
+                        tmem_ld32(t_row + at + c * 32, r);
                         tmem_ld_wait();
                         if (row_ok) {
-                            uint4* dst = reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + nb * BN + c4 * 128 + c * 32);
+                            uint4* dst = reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + nb * BN + at + c * 32);
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
                                 const uint4 o = wv[c][i];
@@ -512,96 +582,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                 }
-            } else {
-                // the residual of the next 32 columns is requested before the current ones are worked on: in the last tile
-                // of a CTA nothing else covers that latency
-                constexpr bool HAS_RESID = EPI == EPI_RESID || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID;
-                const uint16_t* rrow = HAS_RESID ? g.resid + (size_t)row * g.ldr + nb * BN : nullptr;
-                uint4 rn[4] = {};
-                if (HAS_RESID && row_ok) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) rn[i] = reinterpret_cast<const uint4*>(rrow)[i];
-                }
-#pragma unroll 1
-                for (int c = 0; c < BN / 32; ++c) {
-                    float rs[32];
-                    if (HAS_RESID) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            rs[i * 8 + 0] = bf16lo(rn[i].x); rs[i * 8 + 1] = bf16hi(rn[i].x);
-                            rs[i * 8 + 2] = bf16lo(rn[i].y); rs[i * 8 + 3] = bf16hi(rn[i].y);
-                            rs[i * 8 + 4] = bf16lo(rn[i].z); rs[i * 8 + 5] = bf16hi(rn[i].z);
-                            rs[i * 8 + 6] = bf16lo(rn[i].w); rs[i * 8 + 7] = bf16hi(rn[i].w);
-                        }
-                        if (row_ok && c + 1 < BN / 32) {
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) rn[i] = reinterpret_cast<const uint4*>(rrow + (c + 1) * 32)[i];
-                        }
-                    }
-                    uint32_t r[32];
-                    tmem_ld32(t_row + c * 32, r);
-                    tmem_ld_wait();
-                    const int col = nb * BN + c * 32;
-                    if (row_ok && col + 32 > g.N) {
-                        // ragged right edge (N % 32 != 0, N % 8 == 0; plain, bias and bias+GELU epilogues only):
-                        // the same arithmetic, eight columns at a time, nothing read or written beyond column N
-                        if (EPI == EPI_STORE || EPI == EPI_BIAS || EPI == EPI_BIAS_GELU) {
-                            for (int c8 = 0; c8 < 4 && col + c8 * 8 < g.N; ++c8) {
-                                float v8[8];
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) v8[j] = __uint_as_float(r[c8 * 8 + j]);
-                                if (EPI != EPI_STORE) {
-                                    const uint4 b4 = *reinterpret_cast<const uint4*>(g.bias + col + c8 * 8);
-                                    const float b8[8] = {bf16lo(b4.x), bf16hi(b4.x), bf16lo(b4.y), bf16hi(b4.y),
-                                                         bf16lo(b4.z), bf16hi(b4.z), bf16lo(b4.w), bf16hi(b4.w)};
-#pragma unroll
-                                    for (int j = 0; j < 8; ++j) v8[j] = bf16_round(v8[j]) + b8[j];
-                                    if (EPI == EPI_BIAS_GELU) {
-#pragma unroll
-                                        for (int j = 0; j < 8; ++j) v8[j] = bf16_round(v8[j]);
-                                        gelu_all(v8, g.scale != 0.f);
-                                    }
-                                }
-                                uint4 o;
-                                o.x = pack_bf16x2(v8[0], v8[1]); o.y = pack_bf16x2(v8[2], v8[3]);
-                                o.z = pack_bf16x2(v8[4], v8[5]); o.w = pack_bf16x2(v8[6], v8[7]);
-                                *reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + col + c8 * 8) = o;
-                            }
-                        }
-                    } else if (row_ok) {
-                        const size_t ocol = g.o_cb ? (size_t)(col / g.o_cb) * g.o_cb_stride + (col % g.o_cb)
-                                                   : (size_t)col;
-                        float v[32];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-                        if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU) {
-                            float b[32];
-                            load32_bf16(g.bias + col, b);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = bf16_round(v[j]) + b[j];
-                            if (EPI == EPI_BIAS_GELU) {
-#pragma unroll
-                                for (int j = 0; j < 32; ++j) v[j] = bf16_round(v[j]);
-                                gelu_all(v, g.scale != 0.f);
-                            }
-                        } else if (EPI == EPI_BIAS_RESID) {
-                            // linear + bias stored as bf16, then the residual add of src/cuda/residual.cu:14-23
-                            float b[32];
-                            load32_bf16(g.bias + col, b);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = rs[j] + bf16_round(bf16_round(v[j]) + b[j]);
-                        } else if (EPI == EPI_GATE_RESID) {
-                            float gt[32];
-                            load32_bf16(g.bias + col, gt);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = rs[j] + bf16_round(gt[j] * bf16_round(v[j]));
-                        } else if (EPI == EPI_RESID) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = bf16_round(v[j]) + rs[j];
-                        }
-                        store32_bf16(g.out + (size_t)row * g.ldo + ocol, v);
-                    }
-                }
+            } else if constexpr (EPI == EPI_QKV) {
+                PlainEpilogue<EPI_STORE> v_tile;
+                v_tile.run(g, t_row, row0, nb * BN, cols, half * 32, 64, stg, lane, failed);
+            } else if constexpr (EPI != EPI_QKNORM && EPI != EPI_SWIGLU && EPI != EPI_LORA) {
+                plain.run(g, t_row, row0, nb * BN, cols, half * 32, 64, stg, lane, failed);
             }
             tc_fence_before();
             __syncwarp();
@@ -645,6 +630,7 @@ struct SplitCfg {
     static constexpr int STAGE_BYTES = KPS * (BM + BN) * BK * 2;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
     static constexpr int TMEM_COLS = BN <= 32 ? 32 : (BN <= 128 ? 128 : 256);
+    static constexpr int THREADS = BN == 96 ? GEMM_THREADS : SK_THREADS;     // (32 columns are one group for each quadrant)
 };
 // The tower's q | k | v projection takes the same kernel unsplit with tiles of 144 columns, two whole heads of 72: a
 // thread then holds both halves of its row's heads and the rotary is part of the epilogue (3456 = 24 tiles exactly).
@@ -657,7 +643,7 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a,
 }
 
 template <int EPI, int BN, int KPS>
-__global__ void __launch_bounds__(GEMM_THREADS, KPS == 1 ? 2 : 1)
+__global__ void __launch_bounds__(SplitCfg<BN, KPS>::THREADS, KPS == 1 ? 2 : 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g,
                   const int ks) {
     constexpr int SK_STAGE_BYTES = SplitCfg<BN, KPS>::STAGE_BYTES, SK_STAGES = SplitCfg<BN, KPS>::STAGES, NU = BN / 16;
@@ -739,6 +725,25 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             }
             umma_commit(acc_done);
         }
+    }
+    if constexpr (BN == 32 || BN == 96) {
+        // whole K: the epilogue of the persistent kernels, with the stages as its staging once the MMAs are through with them
+        const int row0 = mb * BM + (warp & 3) * 32, col0 = nb * BN, cols = g.N - col0 < BN ? g.N - col0 : BN;
+        const int half = (warp - 2) >> 2;        // (always 0 with 32 columns)
+        if (ok && warp >= 2) {
+            PlainEpilogue<EPI> plain;
+            plain.ahead(g, row0, col0, cols, half * 32, lane);
+            if (!mbar_wait(acc_done, 0)) { atomicExch(g.err, 53); ok = false; }
+            ok = __all_sync(0xffffffffu, ok);
+            tc_fence_after();
+            if (ok) plain.run(g, tmem_base + ((uint32_t)((warp & 3) * 32) << 16), row0, col0, cols, half * 32, 64,
+                              smem + (warp - 2) * 2048, lane, failed);
+        }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN, KPS>::TMEM_COLS);
+        return;
     }
     // The epilogue's other operands are requested while the main loop runs: this thread's residual row into registers, the
     // tile's bias into shared memory (each of the eight units of a tile would otherwise wait for its own loads).
@@ -932,8 +937,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // columns leave a last round of few tiles (1280 rows x 4096 columns: 320 tiles for 148 SMs, three rounds for 2.2), some
 // width in between often makes whole rounds (144 columns: 290 tiles, two rounds).  A block of 1280 rows went from 539 to
 // 503 us, a guided step of 2 x 296 rows from 11.1 to 10.5 ms.  Same warps, same pipeline and the same sums; plain
-// row-major output with the bias or residual epilogue, 16 columns at a time.
-static constexpr int FIT_MAX_STAGES = 6, FIT_SMEM = 216 * 1024 + 1024 /*align*/ + 256 /*barriers*/;
+// row-major output with the bias or residual epilogue.
+static constexpr int FIT_MAX_STAGES = 6, FIT_ROOM = 208 * 1024 /*stages*/, FIT_SMEM = FIT_ROOM + EPI_WARPS * 2048 + 1024 /*align*/ + 256 /*barriers*/;
 
 template <int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -942,7 +947,7 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int stage_bytes = (BM + bn) * BK * 2;      // (bn is a multiple of 16: the stages stay 1024-byte aligned)
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + 216 * 1024);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + FIT_ROOM + EPI_WARPS * 2048);
     uint64_t* empty = full + FIT_MAX_STAGES;
     uint64_t* tfull = empty + FIT_MAX_STAGES;
     uint64_t* tempty = tfull + 2;
@@ -954,7 +959,7 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
         for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 4); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], EPI_WARPS); }
         fence_mbar_init();
     }
     if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
@@ -1017,47 +1022,21 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             }
         }
     } else if (live) {
-        const int q = warp & 3;       // TMEM lane quadrant this warp may access
+        const int q = warp & 3, half = (warp - 2) >> 2;       // (as in gemm_tc_kernel)
+        uint8_t* stg = smem + FIT_ROOM + (warp - 2) * 2048;
         int as = 0;
         uint32_t aphase = 0;
         const int failed = error_word(g.err);
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
             int mb, nb;
             tile_coords(tile, g.num_m, g.num_n, g.group_m, mb, nb);
-            const int row = mb * BM + q * 32 + lane, col0 = nb * bn;
-            const bool row_ok = row < g.M;
-            // the operand of the next 16 columns is requested before the current ones are worked on (N is a multiple of 16)
-            const uint16_t* op = EPI == EPI_RESID ? g.resid + (size_t)row * g.ldr + col0 : g.bias + col0;
-            uint4 nx[2] = {};
-            if (row_ok) { nx[0] = reinterpret_cast<const uint4*>(op)[0]; nx[1] = reinterpret_cast<const uint4*>(op)[1]; }
+            const int row0 = mb * BM + q * 32, col0 = nb * bn, cols = g.N - col0 < bn ? g.N - col0 : bn;
+            PlainEpilogue<EPI> plain;
+            plain.ahead(g, row0, col0, cols, half * 32, lane);
             const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase));
             if (!got) { atomicExch(g.err, 64); break; }
             tc_fence_after();
-            const uint32_t t_row = tmem_base + as * 256 + ((uint32_t)(q * 32) << 16);
-#pragma unroll 1
-            for (int c = 0; c < bn && col0 + c < g.N; c += 16) {
-                float o[16];
-                unpack8_bf16(nx[0], o);
-                unpack8_bf16(nx[1], o + 8);
-                if (row_ok && c + 16 < bn && col0 + c + 16 < g.N) {
-                    nx[0] = reinterpret_cast<const uint4*>(op + c + 16)[0];
-                    nx[1] = reinterpret_cast<const uint4*>(op + c + 16)[1];
-                }
-                uint32_t r[16];
-                tmem_ld16(t_row + c, r);
-                tmem_ld_wait();
-                if (row_ok && !failed) {
-                    uint4* dst = reinterpret_cast<uint4*>(g.out + (size_t)row * g.ldo + col0 + c);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        float v[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] = bf16_round(__uint_as_float(r[h * 8 + j])) + o[h * 8 + j];
-                        dst[h] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
-                                            pack_bf16x2(v[6], v[7]));
-                    }
-                }
-            }
+            plain.run(g, tmem_base + as * 256 + ((uint32_t)(q * 32) << 16), row0, col0, cols, half * 32, 64, stg, lane, failed);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[as]);
@@ -1346,7 +1325,7 @@ static bool launch_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, int bn
     CUtensorMap mB;
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, bn)) return false;
     g.num_n = (g.N + bn - 1) / bn;
-    int stages = 216 * 1024 / ((BM + bn) * BK * 2);
+    int stages = FIT_ROOM / ((BM + bn) * BK * 2);
     if (stages > FIT_MAX_STAGES) stages = FIT_MAX_STAGES;
     const int tiles = g.num_m * g.num_n, grid = tiles < sm_count() ? tiles : sm_count();
     prof_before(EPI, 2.0 * g.M * (double)g.N * g.K, st);
@@ -1458,7 +1437,7 @@ static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmAr
     prof_before((EPI == EPI_BIAS_GELU || EPI == EPI_VROPE) ? (int)EPI_BIAS
                                                            : ((EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID) ? (int)EPI_RESID : EPI),
                 2.0 * g.M * (double)g.N * g.K, st);
-    cudaError_t e = launch_chained(kern, dim3(g.num_m * g.num_n * ks), dim3(GEMM_THREADS), SMEM, st, ks, g.M, *tA, *tB, g, ks);
+    cudaError_t e = launch_chained(kern, dim3(g.num_m * g.num_n * ks), dim3(SplitCfg<BN, KPS>::THREADS), SMEM, st, ks, g.M, *tA, *tB, g, ks);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (few tiles): launch: %s", cudaGetErrorString(e)); return false; }

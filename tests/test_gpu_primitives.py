@@ -803,3 +803,27 @@ def test_norms_by_rows_and_columns(pkg, dev, rows, cols):
     want = term + b.double()
     assert ((y[:rows].double() - want).abs() <= 2.0 ** -7 * (term.abs() + b.double().abs())).all()
     assert (y[rows:] == 777.0).all()
+
+
+@pytest.mark.parametrize("M", [8, 200])
+def test_fused_swiglu_equals_the_pass_for_every_gate(pkg, dev, M):
+    """gate | up + SwiGLU as one GEMM against the projections and hd_swiglu, for all bf16 gates: the epilogue's quotient is the
+    IEEE one, far below zero, at infinities and at NaN too (where a warp holds one of those it divides for all its values)."""
+    N, K = 65536, 64
+    gates = torch.arange(N, dtype=torch.int32, device=dev).to(torch.int16).view(torch.bfloat16)
+    order = torch.randperm(N, generator=torch.Generator().manual_seed(3)).to(dev)
+    x = torch.zeros(M, K, dtype=torch.bfloat16, device=dev)
+    x[:, 0] = 1
+    for mixed in (False, True):        # neighbours alike, and every group with some extreme value in it
+        wg, wu = torch.zeros(2, N, K, dtype=torch.bfloat16, device=dev)
+        wg[:, 0] = gates[order] if mixed else gates
+        wu[:, 0] = torch.linspace(-3, 3, N, device=dev).bfloat16()
+        g, u, one, two = (torch.empty(M, N, dtype=torch.bfloat16, device=dev) for _ in range(4))
+        for w, y in ((wg, g), (wu, u)):
+            assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N, M, N, K, 0, None, None, 0, 0.0, 0) == 0
+        assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(wg), pkg.ptr(wu), pkg.ptr(one), N, M, N, K, 3, None, None, 0, 0.0, 0) == 0
+        pkg.lib.hd_swiglu(pkg.ptr(g), pkg.ptr(u), pkg.ptr(two), M * N)
+        done(pkg, "swiglu")
+        nan = two.isnan()
+        assert torch.equal(nan, one.isnan())
+        assert torch.equal(one.view(torch.int16)[~nan], two.view(torch.int16)[~nan])
