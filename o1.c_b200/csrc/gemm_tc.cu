@@ -30,6 +30,7 @@ namespace o1 {
 static constexpr int BM = 128;
 static constexpr int BK = 64;
 static constexpr int EPI_WARPS = 8;                       // two per quadrant of tensor memory
+static constexpr int EPI_SLICE = 2048 + 64;               // shared memory of a warp: 32 rows x 32 columns, and their bias
 static constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
 static constexpr int SK_THREADS = 192;                    // gemm_split_kernel's 32-column and shared tiles: four epilogue warps
 
@@ -122,9 +123,12 @@ template <int EPI>
 struct PlainEpilogue {
     static constexpr bool HAS_BIAS = EPI != EPI_STORE && EPI != EPI_RESID;
     static constexpr bool HAS_RESID = EPI == EPI_RESID || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID;
-    uint4 rn[4] = {};        // the residual of the group that comes next, eight rows of four 16-byte pieces at a time
+    // what the next group needs, requested one group ahead: the residual, eight rows of four 16-byte pieces at a time, and the bias
+    // (or gate), a piece by each of four lanes
+    uint4 rn[4] = {}, bq = {};
     // row0: first of the warp's rows; cols: columns of the tile that exist (a multiple of eight)
     __device__ __forceinline__ void ahead(const GemmArgs& g, int row0, int col0, int cols, int c, int lane) {
+        if (HAS_BIAS && lane < 4 && c + lane * 8 < cols) bq = *reinterpret_cast<const uint4*>(g.bias + col0 + c + lane * 8);
         if (!HAS_RESID) return;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -132,32 +136,32 @@ struct PlainEpilogue {
             if (row < g.M && col < cols) rn[k] = *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col0 + col);
         }
     }
-    // the caller has called ahead() for c_first; stg: 2 KB of the warp's own
+    // the caller has called ahead() for c_first; stg: EPI_SLICE bytes of the warp's own
     __device__ __forceinline__ void run(const GemmArgs& g, uint32_t t_row, int row0, int col0, int cols, int c_first, int c_step,
                                         uint8_t* stg, int lane, bool failed) {
         const int sr = lane >> 2, ch = lane & 3;
-        uint4* own = reinterpret_cast<uint4*>(stg + lane * 64);
+        uint4 *own = reinterpret_cast<uint4*>(stg + lane * 64), *bias_s = reinterpret_cast<uint4*>(stg + 2048);
 #pragma unroll 1
         for (int c = c_first; c < cols; c += c_step) {
+            uint32_t r[32];
+            tmem_ld32(t_row + c, r);
             __syncwarp();
             if (HAS_RESID) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     *reinterpret_cast<uint4*>(stg + (k * 8 + sr) * 64 + ((ch ^ ((sr >> 1) & 3)) * 16)) = rn[k];
+            }
+            if (HAS_BIAS && lane < 4) bias_s[lane] = bq;
+            if (HAS_RESID || HAS_BIAS) {
                 ahead(g, row0, col0, cols, c + c_step, lane);
                 __syncwarp();
             }
-            uint32_t r[32];
-            tmem_ld32(t_row + c, r);
             tmem_ld_wait();
             float v[32];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 float b[8] = {}, rs[8] = {};
-                if (HAS_BIAS) {
-                    const int col = c + i * 8;
-                    unpack8_bf16(col < cols ? *reinterpret_cast<const uint4*>(g.bias + col0 + col) : make_uint4(0, 0, 0, 0), b);
-                }
+                if (HAS_BIAS) unpack8_bf16(bias_s[i], b);
                 if (HAS_RESID) unpack8_bf16(own[i ^ ((lane >> 1) & 3)], rs);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -737,7 +741,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             ok = __all_sync(0xffffffffu, ok);
             tc_fence_after();
             if (ok) plain.run(g, tmem_base + ((uint32_t)((warp & 3) * 32) << 16), row0, col0, cols, half * 32, 64,
-                              smem + (warp - 2) * 2048, lane, failed);
+                              smem + (warp - 2) * EPI_SLICE, lane, failed);
         }
         tc_fence_before();
         __syncthreads();
@@ -938,7 +942,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // width in between often makes whole rounds (144 columns: 290 tiles, two rounds).  A block of 1280 rows went from 539 to
 // 503 us, a guided step of 2 x 296 rows from 11.1 to 10.5 ms.  Same warps, same pipeline and the same sums; plain
 // row-major output with the bias or residual epilogue.
-static constexpr int FIT_MAX_STAGES = 6, FIT_ROOM = 208 * 1024 /*stages*/, FIT_SMEM = FIT_ROOM + EPI_WARPS * 2048 + 1024 /*align*/ + 256 /*barriers*/;
+static constexpr int FIT_MAX_STAGES = 6, FIT_ROOM = 208 * 1024 /*stages*/, FIT_SMEM = FIT_ROOM + EPI_WARPS * EPI_SLICE + 1024 /*align*/ + 256 /*barriers*/;
 
 template <int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -947,7 +951,7 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int stage_bytes = (BM + bn) * BK * 2;      // (bn is a multiple of 16: the stages stay 1024-byte aligned)
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + FIT_ROOM + EPI_WARPS * 2048);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + FIT_ROOM + EPI_WARPS * EPI_SLICE);
     uint64_t* empty = full + FIT_MAX_STAGES;
     uint64_t* tfull = empty + FIT_MAX_STAGES;
     uint64_t* tempty = tfull + 2;
@@ -1023,7 +1027,7 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     } else if (live) {
         const int q = warp & 3, half = (warp - 2) >> 2;       // (as in gemm_tc_kernel)
-        uint8_t* stg = smem + FIT_ROOM + (warp - 2) * 2048;
+        uint8_t* stg = smem + FIT_ROOM + (warp - 2) * EPI_SLICE;
         int as = 0;
         uint32_t aphase = 0;
         const int failed = error_word(g.err);
