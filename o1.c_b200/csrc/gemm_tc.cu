@@ -1053,6 +1053,129 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
+// ---------------------------------------------------------------- CTA pairs with a tile width chosen at run time
+// The pair form (256 rows over two CTAs, each with half of the B tile) for any width that is a multiple of 16, any N and every
+// epilogue with plain row-major output.  Narrower tiles pay where they make fewer or fuller rounds: a one-CTA tile of 128 x 128
+// brings 32 KB into an SM per K block and is bound by that (70 bytes a clock); half a pair tile of 256 x 128 brings 24 KB for the
+// same products.
+static constexpr int PF_MAX_STAGES = 8, PF_STAGE_ROOM = 192 * 1024, PF_STORE = EPI_WARPS * EPI_SLICE;
+static constexpr int PF_SMEM = PF_STAGE_ROOM + PF_STORE + 1024 /*align*/ + 256 /*barriers*/;
+
+template <int EPI>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_pair_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g, const int bn,
+                     const int stages) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int stage_bytes = (BM + bn / 2) * BK * 2;      // (bn is a multiple of 16: the stages stay 1024-byte aligned)
+    uint8_t* store_s = smem + PF_STAGE_ROOM;
+    uint64_t* full = reinterpret_cast<uint64_t*>(store_s + PF_STORE);
+    uint64_t* empty = full + PF_MAX_STAGES;
+    uint64_t* tfull = empty + PF_MAX_STAGES;
+    uint64_t* tempty = tfull + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    if (threadIdx.x == 64) *s_abort = error_word(g.err);
+    if (threadIdx.x == 0) {
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 2 * EPI_WARPS); }
+        fence_mbar_init();
+    }
+    if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+    const int num_m = (g.num_m + 1) / 2, group_m = (g.group_m + 1) / 2;
+    const int num_tiles = num_m * g.num_n, kblocks = (g.K + BK - 1) / BK;
+    const int tile0 = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();           // both CTAs' barriers exist before either signals the other's
+    tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool live = (*s_abort | ld_cluster_s32(map_to_rank(smem_u32(s_abort), rank ^ 1u))) == 0;
+
+    if (live && warp == 0) {
+        if (elect_one()) {
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+                int mb, nb;
+                tile_coords(tile, num_m, g.num_n, group_m, mb, nb);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!mbar_wait(&empty[stage], phase ^ 1)) { ok = false; atomicExch(g.err, 71); break; }
+                    uint8_t* a_s = smem + stage * stage_bytes;
+                    if (rank == 0) mbar_expect_tx(&full[stage], 2 * stage_bytes);      // both CTAs' halves
+                    int a_c0 = kb * BK, a_c1 = (mb * 2 + (int)rank) * BM;
+                    if (g.a_kblk > 0) {
+                        const int blk = a_c0 / g.a_kblk;
+                        a_c0 -= blk * g.a_kblk;
+                        a_c1 += blk * g.a_rows;
+                    }
+                    tma_load_2d_pair(a_s, &tmA, &full[stage], a_c0, a_c1);
+                    tma_load_2d_pair(a_s + BM * BK * 2, &tmB, &full[stage], kb * BK, nb * bn + (int)rank * (bn / 2));
+                    if (++stage == stages) { stage = 0; phase ^= 1; }
+                }
+            }
+        }
+    } else if (live && warp == 1) {
+        if (rank == 0 && elect_one()) {
+            const uint32_t idesc = umma_idesc_bf16(2 * BM, bn, 0, 0);
+            int stage = 0, as = 0;
+            uint32_t phase = 0, aphase = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+                if (!mbar_wait(&tempty[as], aphase ^ 1)) { atomicExch(g.err, 72); break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + as * 256;
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!mbar_wait(&full[stage], phase)) { ok = false; atomicExch(g.err, 73); break; }
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + stage * stage_bytes);
+                    const uint64_t ad = umma_desc_sw128(a_addr, 16, 1024);
+                    const uint64_t bd = umma_desc_sw128(a_addr + BM * BK * 2, 16, 1024);
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma_ss_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0);
+                    umma_commit_pair(&empty[stage]);
+                    if (++stage == stages) { stage = 0; phase ^= 1; }
+                }
+                umma_commit_pair(&tfull[as]);
+                if (++as == 2) { as = 0; aphase ^= 1; }
+            }
+        }
+    } else if (live) {
+        const int q = warp & 3, half = (warp - 2) >> 2;       // (as in gemm_tc_kernel)
+        uint8_t* stg = store_s + (warp - 2) * EPI_SLICE;
+        int as = 0;
+        uint32_t aphase = 0;
+        const int failed = error_word(g.err);
+        for (int tile = tile0; tile < num_tiles; tile += tile_step) {
+            int mb, nb;
+            tile_coords(tile, num_m, g.num_n, group_m, mb, nb);
+            const int row0 = (mb * 2 + (int)rank) * BM + q * 32, col0 = nb * bn, cols = g.N - col0 < bn ? g.N - col0 : bn;
+            PlainEpilogue<EPI> plain;
+            plain.ahead(g, row0, col0, cols, half * 32, lane);
+            const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase));
+            if (!got) { atomicExch(g.err, 74); break; }
+            tc_fence_after();
+            plain.run(g, tmem_base + as * 256 + ((uint32_t)(q * 32) << 16), row0, col0, cols, half * 32, 64, stg, lane, failed);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&tempty[as]), 0));
+            if (++as == 2) { as = 0; aphase ^= 1; }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still signal it or feed an MMA
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+}
+
 // ---------------------------------------------------------------- SIMT path
 // For M < 8 (timestep MLP, M = 1) and for shapes the tensor-core tiles do not cover.  One warp per output column and MR
 // rows: bound by the weights' way from memory, so a weight is read once for all its rows, four 16-byte pieces of a lane at
@@ -1215,6 +1338,29 @@ static long overlap_rows(const GemmArgs& g) {
     return (double)g.M * g.N * g.K > 1.5e11 || (small_rows(g.M, g.K) && g.K >= 4096) ? OVERLAP_ROWS + 1 : g.M;
 }
 
+// A persistent grid must be co-resident: as many pairs as the device can hold at once (a GPC with an odd number of SMs leaves one
+// without a partner), asked once per device.  (Every pair kernel fills an SM with one CTA.)
+static int pair_capacity(const void* kern, int threads, int smem) {
+    static std::atomic<int> max_pairs[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int pairs = max_pairs[dev & 63].load(std::memory_order_acquire);
+    if (pairs > 0) return pairs;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (sm_count() / 2));
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = sm_count() / 2; }
+    if (n > sm_count() / 2) n = sm_count() / 2;
+    max_pairs[dev & 63].store(n, std::memory_order_release);
+    return n;
+}
+
 template <int EPI>
 static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2, GemmArgs& g,
                            cudaStream_t st, const CUtensorMap* tB3) {
@@ -1223,28 +1369,7 @@ static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const C
     auto kern = gemm_tc_kernel<EPI, 256, true>;
     if (!func_attr_once(attr_done, (const void*)kern, Cfg::SMEM_BYTES, "gemm (pair)")) return false;
     const int tiles = ((g.num_m + 1) / 2) * g.num_n;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    // A persistent grid must be co-resident: as many pairs as the device can hold at once (a GPC with an odd number
-    // of SMs leaves one without a partner), asked once per device.
-    static std::atomic<int> max_pairs[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int pairs = max_pairs[dev & 63].load(std::memory_order_acquire);
-    if (pairs == 0) {
-        cfg.gridDim = dim3(2 * (sm_count() / 2));
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = sm_count() / 2; }
-        if (n > sm_count() / 2) n = sm_count() / 2;
-        pairs = n;
-        max_pairs[dev & 63].store(n, std::memory_order_release);
-    }
+    int pairs = pair_capacity((const void*)kern, GEMM_THREADS, Cfg::SMEM_BYTES);
     if (pairs > tiles) pairs = tiles;
     prof_before(EPI == EPI_QKV ? (int)EPI_STORE : EPI, 2.0 * g.M * (double)g.N * g.K * (EPI == EPI_SWIGLU ? 2.0 : 1.0), st);
     cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 2, overlap_rows(g), *tA, *tB, *tB2,
@@ -1252,6 +1377,28 @@ static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const C
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (pair): launch: %s", cudaGetErrorString(e)); return false; }
+    return true;
+}
+
+template <int EPI>
+static bool launch_pair_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, int bn, cudaStream_t st) {
+    static std::atomic<uint64_t> attr_done{0};
+    auto kern = gemm_pair_fit_kernel<EPI>;
+    if (!func_attr_once(attr_done, (const void*)kern, PF_SMEM, "gemm (pair, fitted)")) return false;
+    CUtensorMap mB;
+    if (!cached_tmap(&mB, w, g.N, g.K, g.K, bn / 2)) return false;
+    g.num_n = (g.N + bn - 1) / bn;
+    int stages = PF_STAGE_ROOM / ((BM + bn / 2) * BK * 2);
+    if (stages > PF_MAX_STAGES) stages = PF_MAX_STAGES;
+    const int tiles = (g.num_m + 1) / 2 * g.num_n;
+    int pairs = pair_capacity((const void*)kern, GEMM_THREADS, PF_SMEM);
+    if (pairs > tiles) pairs = tiles;
+    prof_before(EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : (EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID ? (int)EPI_RESID : EPI),
+                2.0 * g.M * (double)g.N * g.K, st);
+    cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), PF_SMEM, st, 2, overlap_rows(g), *tA, mB, g, bn, stages);
+    prof_after(st);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("gemm (pair, fitted): launch: %s", cudaGetErrorString(e)); return false; }
     return true;
 }
 
@@ -1286,9 +1433,12 @@ static constexpr int TILE_COST[3] = {31, 66, 50};
 // Those times are the main loop's; below K = 2048 the epilogue counts as much, and finer tiles are the safer choice until
 // there are two full waves of wide ones.
 static constexpr int LONG_K = 2048;
-static TileForm tile_form(int num_m, int N, int K, bool wide_ok, bool pair_ok) {
-    if (!wide_ok) return TILE_128;
+static TileForm tile_form(int num_m, int N, int K, bool wide_ok, bool pair_ok, long* units = nullptr /*cost by TILE_COST, K >= LONG_K*/) {
     const long sms = sm_count();
+    if (!wide_ok) {
+        if (units) *units = ((long)num_m * ((N + 127) / 128) + sms - 1) / sms * TILE_COST[TILE_128];
+        return TILE_128;
+    }
     if (K < LONG_K) {
         if ((long)num_m * (N / 256) < 2 * sms) return TILE_128;
         return pair_ok && pair_wanted() && (long)((num_m + 1) / 2) * (N / 256) >= sms ? TILE_PAIR : TILE_256;
@@ -1296,6 +1446,7 @@ static TileForm tile_form(int num_m, int N, int K, bool wide_ok, bool pair_ok) {
     auto cost = [&](TileForm f, long tiles, long at_once) { return (tiles + at_once - 1) / at_once * TILE_COST[f]; };
     const long c128 = cost(TILE_128, (long)num_m * (N / 128), sms), c256 = cost(TILE_256, (long)num_m * (N / 256), sms);
     const long cp = pair_ok && pair_wanted() ? cost(TILE_PAIR, (long)((num_m + 1) / 2) * (N / 256), sms / 2) : c256 + 1;
+    if (units) *units = cp <= c256 && cp <= c128 ? cp : (c256 <= c128 ? c256 : c128);
     if (cp <= c256 && cp <= c128) return TILE_PAIR;
     return c256 <= c128 ? TILE_256 : TILE_128;
 }
@@ -1303,7 +1454,7 @@ static TileForm tile_form(int num_m, int N, int K, bool wide_ok, bool pair_ok) {
 // The fitted width for the bias and residual families, or 0 where no width beats the other forms.  A round of bn columns
 // takes about 31 (1/4 + 3/4 bn/128) of TILE_COST's units: the copies of A and the trips through the barriers do not grow
 // with the tile (nor do they shrink: widths below 128 gain nothing).
-static int fit_width(int num_m, int N, int K) {
+static int fit_width(int num_m, int N, int K, double* units) {
     if (K < LONG_K) return 0;
     const long sms = sm_count();
     auto cost = [&](TileForm f, long tiles, long at_once) { return (tiles + at_once - 1) / at_once * TILE_COST[f] * 512; };
@@ -1317,6 +1468,24 @@ static int fit_width(int num_m, int N, int K) {
     int width = 0;
     for (int bn = 144; bn <= 192; bn += 16) {
         const long tiles = (long)num_m * ((N + bn - 1) / bn), c = (tiles + sms - 1) / sms * TILE_COST[TILE_128] * (128 + 3 * bn);
+        if (c < best) { best = c; width = bn; *units = c / 512.0; }
+    }
+    return width;
+}
+// The width of a pair tile for the linears of long K, or 0 where the other forms' cost `best` (TILE_COST's units) is as good.  A
+// round of bn columns takes 0.6 + 0.1 bn us at K = 4096, two of those units per us.  Other forms against this one at 4096 x 4096:
+// 300 rows 19.0 / 16.8 us (128 columns), 768 rows 25.8 / 23.2 (176), 1280 rows 37.6 / 35.5 (144), 2600 rows 85 / 76 (160), and at
+// 4096 x 12288 62 / 47, 70 / 58, 124 / 101, 265 / 236; 3072 x 4096 at 1000 rows 30.5 / 22.4 (176); where the rule leaves the others,
+// 592 rows 21.1 / 22.0, 2242 rows 60.7 / 62.5, 4352 rows 112.7 / 120.  (No linear of the model has a K between 1152 and 3072; below
+// K = 3072 the one-CTA widths stay.)
+static constexpr int PAIR_FIT_K = 3072;
+static int pair_fit_width(int num_m, int N, double best, int lo, int hi) {
+    const long pairs = sm_count() / 2;
+    int width = 0;
+    best *= 15.0 / 16;       // (only for a gain that shows)
+    for (int bn = lo; bn <= hi; bn += 16) {
+        const long tiles = (long)((num_m + 1) / 2) * ((N + bn - 1) / bn);
+        const double c = (double)((tiles + pairs - 1) / pairs) * (1.2 + 0.2 * bn);
         if (c < best) { best = c; width = bn; }
     }
     return width;
@@ -1413,16 +1582,34 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
         return {pair ? GEMM_PAIR : GEMM_TILE, 256, pair ? 2 : 1};
     }
     plain = plain && force_bn <= 0;
-    if (plain && (pair_ok || epi == EPI_BIAS_GELU || epi == EPI_BIAS_RESID || epi == EPI_GATE_RESID)) {
-        const bool resid = epi == EPI_RESID || epi == EPI_BIAS_RESID || epi == EPI_GATE_RESID;
-        const SplitPlan p = split_plan(M, N, K, force_bn == GEMM_SPLIT_K && pair_wanted(), resid);
-        if (p.bn > 0) return {GEMM_FEW, p.bn, p.ks};
+    const bool tower = force_bn == GEMM_TOWER;
+    const bool resid = epi == EPI_RESID || epi == EPI_BIAS_RESID || epi == EPI_GATE_RESID;
+    const bool small = plain && (pair_ok || resid || epi == EPI_BIAS_GELU);
+    if (small) {
+        const SplitPlan p = split_plan(M, N, K, (tower || force_bn == GEMM_SPLIT_K) && pair_wanted(), resid);
+        // the tower's long K (the MLP's second linear, the mergers): pair tiles of any width instead of narrow ones
+        if (p.ks > 1 || (p.bn > 0 && !(tower && pair_wanted() && K >= LONG_K && num_m > 2))) return {GEMM_FEW, p.bn, p.ks};
+        if (tower && pair_wanted() && K >= LONG_K && num_m > 2) {
+            long units = 0;
+            tile_form(num_m, N, K, wide_ok, pair_ok, &units);
+            const int width = pair_fit_width(num_m, N, p.bn > 0 ? 1e9 : (double)units, 96, 256);
+            if (width) return {GEMM_FIT, width, 2};
+        }
     }
-    if (plain && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) {
-        const int width = fit_width(num_m, N, K);
-        if (width) return {GEMM_FIT, width, 1};
+    long form_units = 0;
+    const TileForm f = tile_form(num_m, N, K, wide_ok, pair_ok, &form_units);
+    double units = (double)form_units;
+    int width = 0;
+    if (plain && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) width = fit_width(num_m, N, K, &units);
+    if (small && !tower && (N % 128) == 0 && K >= PAIR_FIT_K && pair_wanted() && M > BM) {
+        if (epi == EPI_RESID || epi == EPI_BIAS) {
+            const int w = pair_fit_width(num_m, N, units, 128, 192);
+            if (w) return {w == 128 ? GEMM_TILE : GEMM_FIT, w, 2};
+        } else if (pair_fit_width(num_m, N, units, 128, 128)) {
+            return {GEMM_TILE, 128, 2};
+        }
     }
-    const TileForm f = tile_form(num_m, N, K, wide_ok, pair_ok);
+    if (width) return {GEMM_FIT, width, 1};
     return {f == TILE_PAIR ? GEMM_PAIR : GEMM_TILE, f == TILE_128 ? 128 : 256, f == TILE_PAIR ? 2 : 1};
 }
 
@@ -1604,6 +1791,14 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
         case EPI_BIAS_GELU: return launch_split<EPI_BIAS_GELU>(tA, w, g, p, st);
         case EPI_BIAS_RESID: return launch_split<EPI_BIAS_RESID>(tA, w, g, p, st);
         case EPI_GATE_RESID: return launch_split<EPI_GATE_RESID>(tA, w, g, p, st);
+    }
+    if (p.ks == 2 && (p.form == GEMM_FIT || p.form == GEMM_TILE)) switch (epi) {
+        case EPI_STORE: return launch_pair_fit<EPI_STORE>(tA, w, g, p.bn, st);
+        case EPI_BIAS:  return launch_pair_fit<EPI_BIAS>(tA, w, g, p.bn, st);
+        case EPI_RESID: return launch_pair_fit<EPI_RESID>(tA, w, g, p.bn, st);
+        case EPI_BIAS_GELU: return launch_pair_fit<EPI_BIAS_GELU>(tA, w, g, p.bn, st);
+        case EPI_BIAS_RESID: return launch_pair_fit<EPI_BIAS_RESID>(tA, w, g, p.bn, st);
+        case EPI_GATE_RESID: return launch_pair_fit<EPI_GATE_RESID>(tA, w, g, p.bn, st);
     }
     if (p.form == GEMM_FIT) return epi == EPI_RESID ? launch_fit<EPI_RESID>(tA, w, g, p.bn, st) : launch_fit<EPI_BIAS>(tA, w, g, p.bn, st);
     const int bn = p.bn;

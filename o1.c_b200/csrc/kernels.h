@@ -33,11 +33,11 @@ void prof_after(cudaStream_t st);
 // of k, so that a row's result does not depend on the tile or on how many other rows the call has (the decoder's layers
 // rely on that: a row is the same in a sharded, a cached or a paired pass).  GEMM_SPLIT_K = chosen by shape, and a problem
 // of few tiles may share a tile's K among the CTAs of a cluster, which is another order of the FP32 sum (not in mode 0 of
-// gemm_pair_mode).
-enum { GEMM_SPLIT_K = -1 };
+// gemm_pair_mode).  GEMM_TOWER = the same for the vision tower's linears, whose long K takes pair tiles of any width.
+enum { GEMM_SPLIT_K = -1, GEMM_TOWER = -2 };
 // The form a problem takes: GEMM_ROWS = warps (bn: rows that share one), GEMM_TILE = one CTA per 128 x bn tile, GEMM_PAIR = two
-// per 256 x 256 tile, GEMM_FIT = one per tile of a width fitted to the SMs, GEMM_FEW = tiles for problems that have few (ctas of
-// a cluster share a tile's K).
+// per 256 x 256 tile, GEMM_FIT = one per tile of a width fitted to the SMs, GEMM_FEW = tiles for problems that have few (ks CTAs of
+// a cluster share a tile's K).  GEMM_TILE and GEMM_FIT with ks = 2: a CTA pair per 256 x bn tile.
 enum GemmForm { GEMM_ROWS = 0, GEMM_TILE = 1, GEMM_PAIR = 2, GEMM_FIT = 3, GEMM_FEW = 4 };
 struct GemmPlan { int form, bn, ks; };
 GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok);

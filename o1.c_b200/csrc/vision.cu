@@ -398,9 +398,9 @@ static bool linear_act(const void* x, const void* w, const void* b, void* y, int
                        cudaStream_t st, int* launches) {
     if (act && gemm_tc_supported(M, N, K, EPI_BIAS_GELU)) {
         ++*launches;
-        return gemm_bf16(x, w, nullptr, y, M, N, K, EPI_BIAS_GELU, b, nullptr, act == 2 ? 1.0f : 0.0f, GEMM_SPLIT_K, st);
+        return gemm_bf16(x, w, nullptr, y, M, N, K, EPI_BIAS_GELU, b, nullptr, act == 2 ? 1.0f : 0.0f, GEMM_TOWER, st);
     }
-    if (!gemm_bf16(x, w, nullptr, y, M, N, K, EPI_BIAS, b, nullptr, 0.f, GEMM_SPLIT_K, st)) return false;
+    if (!gemm_bf16(x, w, nullptr, y, M, N, K, EPI_BIAS, b, nullptr, 0.f, GEMM_TOWER, st)) return false;
     ++*launches;
     if (act) { if (!vision_gelu(y, y, (size_t)M * N, act == 2, st)) return false; ++*launches; }
     return true;
@@ -680,7 +680,7 @@ hd_status hd_vision_forward(const hd_vision_binding* bw, hd_vision_workspace* ws
         // (or the row count is below the tensor-core tile minimum)
         const bool fuse = gemm_tc_supported(n, V_H, V_H, EPI_BIAS_RESID) && !(s0 && (s0[HD_B0_PROJ] || s0[HD_B0_FC2]));
         if (fuse) {
-            VIS_TRY(gemm_bf16(attn_out, blk->proj_w, nullptr, attn_resid, n, V_H, V_H, EPI_BIAS_RESID, blk->proj_b, cur_in, 0.f, GEMM_SPLIT_K, st));
+            VIS_TRY(gemm_bf16(attn_out, blk->proj_w, nullptr, attn_resid, n, V_H, V_H, EPI_BIAS_RESID, blk->proj_b, cur_in, 0.f, GEMM_TOWER, st));
         } else {
             VIS_TRY(linear_act(attn_out, blk->proj_w, blk->proj_b, attn_resid, n, V_H, V_H, 0, st, &launches));
             if (s0) VIS_TRY(snap(s0[HD_B0_PROJ], attn_resid, nH, st));
@@ -689,7 +689,7 @@ hd_status hd_vision_forward(const hd_vision_binding* bw, hd_vision_workspace* ws
         VIS_TRY(vision_layernorm(attn_resid, blk->norm2_w, blk->norm2_b, ln2, n, V_H, eps, st));
         VIS_TRY(linear_act(ln2, blk->fc1_w, blk->fc1_b, fc1, n, V_I, V_H, 1, st, &launches));
         if (fuse) {
-            VIS_TRY(gemm_bf16(fc1, blk->fc2_w, nullptr, cur_out, n, V_H, V_I, EPI_BIAS_RESID, blk->fc2_b, attn_resid, 0.f, GEMM_SPLIT_K, st));
+            VIS_TRY(gemm_bf16(fc1, blk->fc2_w, nullptr, cur_out, n, V_H, V_I, EPI_BIAS_RESID, blk->fc2_b, attn_resid, 0.f, GEMM_TOWER, st));
         } else {
             VIS_TRY(linear_act(fc1, blk->fc2_w, blk->fc2_b, fc2, n, V_H, V_I, 0, st, &launches));
             VIS_TRY(residual_add(attn_resid, fc2, cur_out, (size_t)n * V_H, st));

@@ -827,3 +827,29 @@ def test_fused_swiglu_equals_the_pass_for_every_gate(pkg, dev, M):
         nan = two.isnan()
         assert torch.equal(nan, one.isnan())
         assert torch.equal(one.view(torch.int16)[~nan], two.view(torch.int16)[~nan])
+
+
+@pytest.mark.parametrize("M,N,K,epi,bn,width", [(1280, 4096, 4096, 2, 0, 144), (1000, 3072, 4096, 1, 0, 176), (300, 4096, 3080, 2, 0, 128),
+                                                (257, 4096, 3072, 0, 0, 128), (2600, 4096, 4160, 2, 0, 160), (300, 4096, 3072, 9, 0, 128),
+                                                (2304, 1152, 4304, 8, -2, 144), (800, 1152, 4304, 8, -2, 96), (3000, 1152, 4304, 8, -2, 192),
+                                                (520, 4608, 4608, 7, -2, 192), (1024, 4608, 4608, 7, -2, 256), (1000, 4104, 2056, 1, -2, 112),
+                                                (700, 4312, 2048, 7, -2, 192)])
+def test_pair_tiles_of_any_width(pkg, dev, M, N, K, epi, bn, width):
+    """CTA pairs with a width chosen by the rounds of tiles give the bits of 128-column tiles: partly filled last row and column
+    tiles, an odd number of row tiles, a ragged N and K, every epilogue."""
+    if pkg.lib.o1_sm_count() == 148:
+        assert gemm_form(pkg, M, N, K, epi, bn) == (1 if width == 128 and bn == 0 else 3, width, 2)
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    x, w, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
+                  for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
+    ys = []
+    for force in (bn, 128):
+        y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
+        rc = pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N + 8, M, N, K, epi, pkg.ptr(b), pkg.ptr(r), N, 0.0, force)
+        assert rc == 0, pkg.last_error()
+        done(pkg, "gemm")
+        assert (y[M:] == 777.0).all() and (y[:, N:] == 777.0).all(), "written beyond the matrix"
+        ys.append(y)
+    assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
+    check_epilogue_f64(ys[0][:M, :N], x, w, b, r, epi, "pair tiles")
+    assert pkg.lib.o1_device_error() == 0
