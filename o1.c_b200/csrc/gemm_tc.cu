@@ -730,8 +730,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             umma_commit(acc_done);
         }
     }
-    if constexpr (BN == 32 || BN == 96) {
+    if constexpr (BN == 96 || (BN == 32 && PlainEpilogue<EPI>::HAS_RESID)) {
         // whole K: the epilogue of the persistent kernels, with the stages as its staging once the MMAs are through with them
+        // (32 columns without a residual are better stored directly: 77 x 4096 x 4096 12.66 us against 12.81)
         const int row0 = mb * BM + (warp & 3) * 32, col0 = nb * BN, cols = g.N - col0 < BN ? g.N - col0 : BN;
         const int half = (warp - 2) >> 2;        // (always 0 with 32 columns)
         if (ok && warp >= 2) {
@@ -1476,8 +1477,8 @@ static int fit_width(int num_m, int N, int K, double* units) {
 // round of bn columns takes 0.6 + 0.1 bn us at K = 4096, two of those units per us.  Other forms against this one at 4096 x 4096:
 // 300 rows 19.0 / 16.8 us (128 columns), 768 rows 25.8 / 23.2 (176), 1280 rows 37.6 / 35.5 (144), 2600 rows 85 / 76 (160), and at
 // 4096 x 12288 62 / 47, 70 / 58, 124 / 101, 265 / 236; 3072 x 4096 at 1000 rows 30.5 / 22.4 (176); where the rule leaves the others,
-// 592 rows 21.1 / 22.0, 2242 rows 60.7 / 62.5, 4352 rows 112.7 / 120.  (No linear of the model has a K between 1152 and 3072; below
-// K = 3072 the one-CTA widths stay.)
+// 592 rows 21.1 / 22.0, 2242 rows 60.7 / 62.5, 4352 rows 112.7 / 120.  (The decoder's linears have K of 256, 1024, or 3072
+// and more, in whole blocks; other K keep the one-CTA widths.)
 static constexpr int PAIR_FIT_K = 3072;
 static int pair_fit_width(int num_m, int N, double best, int lo, int hi) {
     const long pairs = sm_count() / 2;
@@ -1601,7 +1602,7 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
     double units = (double)form_units;
     int width = 0;
     if (plain && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) width = fit_width(num_m, N, K, &units);
-    if (small && !tower && (N % 128) == 0 && K >= PAIR_FIT_K && pair_wanted() && M > BM) {
+    if (small && !tower && (N % 128) == 0 && K >= PAIR_FIT_K && (K % BK) == 0 && pair_wanted() && M > BM) {
         if (epi == EPI_RESID || epi == EPI_BIAS) {
             const int w = pair_fit_width(num_m, N, units, 128, 192);
             if (w) return {w == 128 ? GEMM_TILE : GEMM_FIT, w, 2};

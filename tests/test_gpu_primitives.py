@@ -829,7 +829,7 @@ def test_fused_swiglu_equals_the_pass_for_every_gate(pkg, dev, M):
         assert torch.equal(one.view(torch.int16)[~nan], two.view(torch.int16)[~nan])
 
 
-@pytest.mark.parametrize("M,N,K,epi,bn,width", [(1280, 4096, 4096, 2, 0, 144), (1000, 3072, 4096, 1, 0, 176), (300, 4096, 3080, 2, 0, 128),
+@pytest.mark.parametrize("M,N,K,epi,bn,width", [(1280, 4096, 4096, 2, 0, 144), (1000, 3072, 4096, 1, 0, 176), (300, 4096, 3136, 2, 0, 128),
                                                 (257, 4096, 3072, 0, 0, 128), (2600, 4096, 4160, 2, 0, 160), (300, 4096, 3072, 9, 0, 128),
                                                 (2304, 1152, 4304, 8, -2, 144), (800, 1152, 4304, 8, -2, 96), (3000, 1152, 4304, 8, -2, 192),
                                                 (520, 4608, 4608, 7, -2, 192), (1024, 4608, 4608, 7, -2, 256), (1000, 4104, 2056, 1, -2, 112),
