@@ -1918,6 +1918,8 @@ bool gemm_vision_qkv(const void* x, const void* w, const void* b, void* y, int M
     g.err = device_error_word();
     CUtensorMap mA, mB;
     if (!cached_tmap(&mA, x, M, K, K, 128) || !cached_tmap(&mB, w, N, K, K, VQ_BN)) return false;
+    // (with one CTA per SM, two K blocks a stage, see SplitCfg: the tower at 520 patches 2155 -> 2058 us)
+    if (g.num_m * (N / VQ_BN) <= sm_count()) return launch_split_bn<EPI_VROPE, VQ_BN, 2>(&mA, &mB, g, 1, st);
     return launch_split_bn<EPI_VROPE, VQ_BN>(&mA, &mB, g, 1, st);
 }
 
