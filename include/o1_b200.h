@@ -497,11 +497,10 @@ int o1_flash_attention_ws(const void *q, int ldq, const void *k, int ldk, const 
                           size_t scratch_bytes);
 /* Policy of that split: 0 = automatic (default), 1 = never, n > 1 = n parts whenever scratch and key count allow. */
 void o1_attention_tail_ways(int ways);
-/* Which attention kernel: 0 = by sequence length (default: one query tile of 128 rows per CTA with triple-buffered
- * scores for S < 8192, two query tiles that share the K/V tiles above), 1 = always the two-tile kernel, 2 = always
- * the one-tile kernel (environment O1_ATTN_TILE_MODE sets the initial value).  Same arithmetic up to fp32 summation
- * order and the reference max of the lazy rescale.  The vision tower has a one-tile form of its own for its heads of 72
- * columns, which modes 0 and 2 use at every length; mode 1 holds for the tower as well. */
+/* Which attention kernel: 0 (default) and 2 = one query tile of 128 rows per CTA with triple-buffered scores, 1 = two query
+ * tiles that share the K/V tiles (environment O1_ATTN_TILE_MODE sets the initial value).  Same arithmetic up to fp32
+ * summation order and the reference max of the lazy rescale.  The vision tower has a one-tile form of its own for its heads
+ * of 72 columns, which modes 0 and 2 use; mode 1 holds for the tower as well. */
 void o1_attention_tile_mode(int mode);
 /* Clusters of CTAs in the GEMMs: 1 (default, as is every value but 0; environment O1_GEMM_PAIR=0 turns them off) = the plain,
  * bias, residual, SwiGLU and grouped q|k|v families take, where that needs the fewest rounds of tiles, two CTAs per

@@ -6,7 +6,8 @@
 //   kh = h / (heads / kv_heads); mask: rows s < ar_len see keys t <= s,
 //   rows s >= ar_len see every key (o1.c src/runtime/sequence.c:120-142).
 //
-// Two kernels.  Long sequences (the benchmark's 16640 rows), flash_attn_kernel:
+// Two kernels.  flash_attn1_kernel is the one that runs: one query tile per CTA with triple-buffered scores (described at the kernel).
+// The other, where a program asks for it (attention_tile_mode), flash_attn_kernel:
 // one CTA = 256 query rows of one head: two query tiles of 128 rows that share every K/V tile
 // brought into shared memory (half the K/V fill per query row of a one-tile CTA, and the two tiles'
 // softmax and MMA phases overlap each other).  Operands stay seq-major ([S, heads*128]); head split /
@@ -22,7 +23,6 @@
 //                critical path of the kernel, which is why a row is split over two threads.
 // An accumulator is only rescaled when its running max grows by more than 2^8 (sum and
 // accumulator share the same stale max, so the final division is still exact).
-// Short sequences, flash_attn1_kernel: one query tile per CTA with triple-buffered scores (described at the kernel).
 #include <cstdlib>
 #include "common.cuh"
 #include "ptx.cuh"
@@ -501,16 +501,14 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// One query tile per CTA, scores triple-buffered: the form used for short sequences (S < 8192), where work items of
-// 256 rows are too few and too coarse for 148 SMs (S = 1280: 160 items) and the serial chain of the two-tile kernel
-// has nothing to hide behind.  Tensor memory: three score buffers of 128 columns + one output accumulator.  The MMA
+// One query tile per CTA, scores triple-buffered: work items of 128 rows fill 148 SMs at short sequences too (S = 1280: 320
+// instead of 160), and no serial chain as in the two-tile kernel.  Tensor memory: three score buffers of 128 columns + one output accumulator.  The MMA
 // thread issues S(j+3) = Q K^T right after PV(j), so the scores of the next two key tiles are always there or on their
 // way and the softmax warps never wait for a score product that waits for them.  Warps 2..9 and 10..17 are two softmax
 // sets that take alternate key tiles (two threads per row, as above); they agree on the running max through shared
 // memory: the set that takes tile j waits for the other set's decision for tile j-1 (made early in its phase) before it
-// decides for tile j.  Measured stand-alone against the two-tile kernel: S = 1280 0.048 vs 0.072 ms, S = 4352 0.312 vs
-// 0.339 ms, S = 16640 3.97 vs 3.63 ms (twice the K/V fill per query row and half as long work items cost more there
-// than the chain).
+// decides for tile j.  Measured against the two-tile kernel: see attention_tile_mode() (before the issuing threads were elected
+// that one was 9 % faster at S = 16640).
 static constexpr int T1_ROWS = 128;       // query rows per CTA and work item
 static constexpr int T1_K_STAGES = 3;
 static constexpr int T1_V_STAGES = 3;
@@ -964,8 +962,10 @@ __global__ void __launch_bounds__(AD) attn_merge_kernel(const AttnArgs a, int n_
 // with 4 or 8 tail items after 7 or 14 waves), so it is left alone.  Every part keeps at least two key tiles.
 static int g_tail_ways = 0;   // 0: choose; 1: never split; n > 1: n parts whenever they fit
 void attention_tail_ways(int ways) { g_tail_ways = ways < 0 ? 0 : ways; }
-// Which kernel: 0 = by sequence length (one query tile per CTA below 8192 keys, two from there on), 1 = always the two-tile
-// kernel, 2 = always the one-tile kernel
+// Which kernel: 0 and 2 = one query tile per CTA, 1 = two.  One is the better form at every length since its issuing threads are
+// elected (32 / 8 heads, two / one): 1280 rows 59 / 39 us, 4352 rows 340 / 317, 8192 rows 1009 / 975, 12356 rows 2350 / 2165, 16640 rows
+// 4050 / 3850; and in a block, where the power cap counts, more than that: 8210 rows 3.75 / 3.40 ms, 12356 rows 6.25 / 5.60, 16640 rows
+// 9.5 / 8.05.
 static int g_tile_mode = -1;    // -1: not yet read from the environment (O1_ATTN_TILE_MODE)
 void attention_tile_mode(int mode) { g_tile_mode = (mode < 0 || mode > 2) ? 0 : mode; }
 static int tile_mode() {
@@ -1035,7 +1035,7 @@ static bool attention_setup(AttnSetup& s, const void* q, int ldq, const void* k,
                   cached_tmap(&s.v, v, S, (uint64_t)kv_heads * AD, ldv, 128);
     }
     if (!maps_ok) return false;
-    const bool one_tile = tile_mode() == 2 || (tile_mode() == 0 && S < 8192);
+    const bool one_tile = tile_mode() != 1;
     const int rows_item = one_tile ? T1_ROWS : AQ2;
     AttnArgs& a = s.a;
     a.out = (uint16_t*)out; a.ldo = ldo;
@@ -1127,8 +1127,6 @@ static bool attention_launch(const AttnSetup* s, int n, cudaStream_t st) {
     return ok && launched(cudaGetLastError());
 }
 
-// One-tile at every length: with 72 columns it stays ahead where the general rule takes two tiles (the whole tower, with heads
-// padded for the two-tile kernel: 9216 patches 26.7 / 28.9 ms, 12288 patches 41.1 / 46.5 ms).
 bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cudaStream_t st) {
     constexpr int H = 16, DH = 72, LD = 3 * H * AD;
     if (!qkv || !out || S <= 0 || (((uintptr_t)out) & 15)) { set_error("attention (vision): bad args"); return false; }

@@ -94,7 +94,7 @@ bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cuda
 // tail split policy of flash_attention*: 0 = automatic, 1 = never, n = n key-range parts when they fit
 void attention_tail_ways(int ways);
 bool attention_two_tile_only();       // mode 1 is set
-void attention_tile_mode(int mode);   // 0: by sequence length; 1: two query tiles per CTA; 2: one query tile per CTA
+void attention_tile_mode(int mode);   // 0, 2: one query tile per CTA; 1: two
 int gemm_pair_capacity();
 void gemm_pair_mode(int mode);   // 0: single CTAs only; else clusters (CTA pairs, K split) where they are the better form
 // seq-major operands; output rows [b*out_rows, (b+1)*out_rows) go to out_tab[b] (row-major, leading
