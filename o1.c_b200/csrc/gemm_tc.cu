@@ -164,15 +164,15 @@ struct PlainEpilogue {
                 if (HAS_BIAS) unpack8_bf16(bias_s[i], b);
                 if (HAS_RESID) unpack8_bf16(own[i ^ ((lane >> 1) & 3)], rs);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    float x = __uint_as_float(r[i * 8 + j]);
-                    if (EPI == EPI_BIAS) x = bf16_round(x) + b[j];
-                    if (EPI == EPI_BIAS_GELU) x = bf16_round(bf16_round(x) + b[j]);
-                    if (EPI == EPI_RESID) x = bf16_round(x) + rs[j];
-                    // linear + bias stored as bf16, then the residual add of src/cuda/residual.cu:14-23
-                    if (EPI == EPI_BIAS_RESID) x = rs[j] + bf16_round(bf16_round(x) + b[j]);
-                    if (EPI == EPI_GATE_RESID) x = rs[j] + bf16_round(b[j] * bf16_round(x));
-                    v[i * 8 + j] = x;
+                for (int j = 0; j < 8; j += 2) {
+                    float x = __uint_as_float(r[i * 8 + j]), y = __uint_as_float(r[i * 8 + j + 1]);
+                    if (EPI != EPI_STORE) bf16_round2(x, y);
+                    if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) { x += b[j]; y += b[j + 1]; }
+                    if (EPI == EPI_GATE_RESID) { x *= b[j]; y *= b[j + 1]; }
+                    // linear + bias stored as bf16, then GELU or the residual add of src/cuda/residual.cu:14-23
+                    if (EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID) bf16_round2(x, y);
+                    if (HAS_RESID) { x += rs[j]; y += rs[j + 1]; }
+                    v[i * 8 + j] = x; v[i * 8 + j + 1] = y;
                 }
             }
             if (EPI == EPI_BIAS_GELU) gelu_all(v, g.scale != 0.f);
@@ -208,17 +208,24 @@ struct PlainEpilogue {
 __device__ __forceinline__ void swiglu_all(const uint32_t (&rg)[32], const uint32_t (&ru)[32], float (&v)[32]) {
     bool plain = true;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        v[j] = bf16_round(__uint_as_float(rg[j]));
-        plain = plain && v[j] > -80.f;
+    for (int j = 0; j < 32; j += 2) {
+        v[j] = __uint_as_float(rg[j]); v[j + 1] = __uint_as_float(rg[j + 1]);
+        bf16_round2(v[j], v[j + 1]);
+        plain = plain && fminf(v[j], v[j + 1]) > -80.f && v[j] == v[j] && v[j + 1] == v[j + 1];
     }
     if (__all_sync(0xffffffffu, plain)) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const float x = 1.0f + expf(-v[j]);
-            const float y = __fdividef(1.0f, x);
-            const float sg = __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
-            v[j] = bf16_round(v[j] * sg) * bf16_round(__uint_as_float(ru[j]));
+        for (int j = 0; j < 32; j += 2) {
+            float s[2], u[2] = {__uint_as_float(ru[j]), __uint_as_float(ru[j + 1])};
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float x = 1.0f + expf(-v[j + i]);
+                const float y = __fdividef(1.0f, x);
+                s[i] = v[j + i] * __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+            }
+            bf16_round2(s[0], s[1]);
+            bf16_round2(u[0], u[1]);
+            v[j] = s[0] * u[0]; v[j + 1] = s[1] * u[1];
         }
     } else {
 #pragma unroll
