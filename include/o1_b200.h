@@ -476,7 +476,7 @@ int o1_gemm(const void *x, int ldx, const void *w, const void *w2, void *y, int 
  * one CTA per tile of 128 rows x *width columns, 2 = two CTAs per 256 x 256 tile, 3 = one CTA per tile of a *width fitted to
  * the number of SMs, 4 = the kernel for few tiles of *width columns, *ctas of a cluster sharing the K of each; -1 = not
  * supported.  1 and 3 with *ctas = 2: a CTA pair per tile of 256 rows.  force_bn -1 (which o1_gemm takes too): as 0, and K may
- * be shared; -2: as -1, and from K = 2048 on pair tiles of any width (the vision tower's linears). */
+ * be shared; -2: as -1, and pair tiles of any width from K = 2048, or 1024 rows, on (the vision tower's linears). */
 int o1_gemm_form(int M, int N, int K, int epi, int force_bn, int *width, int *ctas);
 /* The q, k and v projections of a decoder block (src/model/block.c:257-265) with the per-head RMSNorm + rotary of
  * q and k (:266-289) as ONE launch over the three weight tensors: y [M, qc | kc | kc] (row pitch ldy) =

@@ -1597,7 +1597,9 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
         const SplitPlan p = split_plan(M, N, K, (tower || force_bn == GEMM_SPLIT_K) && pair_wanted(), resid);
         // the tower's long K (the MLP's second linear, the mergers): pair tiles of any width instead of narrow ones
         if (p.ks > 1 || (p.bn > 0 && !(tower && pair_wanted() && K >= LONG_K && num_m > 2))) return {GEMM_FEW, p.bn, p.ks};
-        if (tower && pair_wanted() && K >= LONG_K && num_m > 2) {
+        // (from 1024 rows on its K of 1152 too: the tower of 1200 / 3024 / 4096 patches 2800 / 5600 / 8100 -> 2700 / 5370 / 7820 us,
+        // but of 832 patches 2165 -> 2197)
+        if (tower && pair_wanted() && num_m > (K >= LONG_K ? 2 : 8) && (K >= LONG_K || (K >= 1024 && !wide_ok))) {
             long units = 0;
             tile_form(num_m, N, K, wide_ok, pair_ok, &units);
             const int width = pair_fit_width(num_m, N, p.bn > 0 ? 1e9 : (double)units, 96, 256);

@@ -833,7 +833,7 @@ def test_fused_swiglu_equals_the_pass_for_every_gate(pkg, dev, M):
                                                 (257, 4096, 3072, 0, 0, 128), (2600, 4096, 4160, 2, 0, 160), (300, 4096, 3072, 9, 0, 128),
                                                 (2304, 1152, 4304, 8, -2, 144), (800, 1152, 4304, 8, -2, 96), (3000, 1152, 4304, 8, -2, 192),
                                                 (520, 4608, 4608, 7, -2, 192), (1024, 4608, 4608, 7, -2, 256), (1000, 4104, 2056, 1, -2, 112),
-                                                (700, 4312, 2048, 7, -2, 192)])
+                                                (700, 4312, 2048, 7, -2, 192), (1200, 4304, 1152, 7, -2, 160), (1100, 1152, 1152, 8, -2, 96)])
 def test_pair_tiles_of_any_width(pkg, dev, M, N, K, epi, bn, width):
     """CTA pairs with a width chosen by the rounds of tiles give the bits of 128-column tiles: partly filled last row and column
     tiles, an odd number of row tiles, a ragged N and K, every epilogue."""
