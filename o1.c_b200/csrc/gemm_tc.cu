@@ -118,11 +118,17 @@ __device__ __forceinline__ void unpack8_bf16(const uint4& o, float* v) {
 // of 11 us (SwiGLU), 15 (per-head norm) and 5 to 10 (the others) per 256-column tile.  The main loop of the next tile covers that, but
 // not a CTA's last tile: q | k | v at 592 rows was 48 us for a round of 25.
 
+// What an epilogue reads per column and per element.  In the others GemmArgs::bias is null (SwiGLU, LoRA) or the norm weight of one
+// head (per-head norm), and must not be read by column.
+static constexpr bool epi_has_bias(int e) { return e == EPI_BIAS || e == EPI_BIAS_GELU || e == EPI_BIAS_RESID || e == EPI_GATE_RESID; }
+static constexpr bool epi_has_resid(int e) { return e == EPI_RESID || e == EPI_BIAS_RESID || e == EPI_GATE_RESID; }
+static constexpr bool epi_plain(int e) { return e == EPI_STORE || epi_has_bias(e) || epi_has_resid(e); }
+
 // Groups of 32 columns at c_first, c_first + c_step, ... of a tile, plain row-major output (or column blocks, see GemmArgs).
 template <int EPI>
 struct PlainEpilogue {
-    static constexpr bool HAS_BIAS = EPI != EPI_STORE && EPI != EPI_RESID;
-    static constexpr bool HAS_RESID = EPI == EPI_RESID || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID;
+    static_assert(epi_plain(EPI), "this epilogue has no operands by column and element");
+    static constexpr bool HAS_BIAS = epi_has_bias(EPI), HAS_RESID = epi_has_resid(EPI);
     // what the next group needs, requested one group ahead: the residual, eight rows of four 16-byte pieces at a time, and the bias
     // (or gate), a piece by each of four lanes
     uint4 rn[4] = {}, bq = {};
@@ -478,7 +484,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int rows = failed ? 0 : g.M;
             const int row0 = mb * BM + q * 32;
             const int cols = g.N - nb * BN < BN ? g.N - nb * BN : BN;      // (plain epilogues: N may be ragged, N % 8 == 0)
-            PlainEpilogue<EPI> plain;
+            // (v of q | k | v is stored as it is; the other epilogues do not use this one)
+            PlainEpilogue<epi_plain(EPI) ? EPI : (int)EPI_STORE> plain;
             plain.ahead(g, row0, nb * BN, cols, half * 32, lane);
             const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase));
             if (!got) { atomicExch(g.err, 4); break; }
@@ -593,10 +600,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                 }
-            } else if constexpr (EPI == EPI_QKV) {
-                PlainEpilogue<EPI_STORE> v_tile;
-                v_tile.run(g, t_row, row0, nb * BN, cols, half * 32, 64, stg, lane, failed);
-            } else if constexpr (EPI != EPI_QKNORM && EPI != EPI_SWIGLU && EPI != EPI_LORA) {
+            } else if constexpr (epi_plain(EPI) || EPI == EPI_QKV) {
                 plain.run(g, t_row, row0, nb * BN, cols, half * 32, 64, stg, lane, failed);
             }
             tc_fence_before();
@@ -737,7 +741,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             umma_commit(acc_done);
         }
     }
-    if constexpr (BN == 96 || (BN == 32 && PlainEpilogue<EPI>::HAS_RESID)) {
+    if constexpr (BN == 96 || (BN == 32 && epi_has_resid(EPI))) {
         // whole K: the epilogue of the persistent kernels, with the stages as its staging once the MMAs are through with them
         // (32 columns without a residual are better stored directly: 77 x 4096 x 4096 12.66 us against 12.81)
         const int row0 = mb * BM + (warp & 3) * 32, col0 = nb * BN, cols = g.N - col0 < BN ? g.N - col0 : BN;
@@ -759,8 +763,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     // The epilogue's other operands are requested while the main loop runs: this thread's residual row into registers, the
     // tile's bias into shared memory (each of the eight units of a tile would otherwise wait for its own loads).
-    constexpr bool HAS_BIAS = EPI != EPI_STORE && EPI != EPI_RESID;
-    constexpr bool HAS_RESID = EPI == EPI_RESID || EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID;
+    constexpr bool HAS_BIAS = epi_has_bias(EPI) || EPI == EPI_VROPE, HAS_RESID = epi_has_resid(EPI);
     const int q = warp & 3;       // TMEM lane quadrant this warp may access
     const int trow = q * 32 + lane;
     const int u0 = rank * NU / ks, u1 = (rank + 1) * NU / ks;     // this CTA's share of the tile's 16-column units
@@ -1591,7 +1594,7 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
     }
     plain = plain && force_bn <= 0;
     const bool tower = force_bn == GEMM_TOWER;
-    const bool resid = epi == EPI_RESID || epi == EPI_BIAS_RESID || epi == EPI_GATE_RESID;
+    const bool resid = epi_has_resid(epi);
     const bool small = plain && (pair_ok || resid || epi == EPI_BIAS_GELU);
     if (small) {
         const SplitPlan p = split_plan(M, N, K, (tower || force_bn == GEMM_SPLIT_K) && pair_wanted(), resid);

@@ -379,3 +379,18 @@ def test_narrow_tiles_are_for_activations_of_some_size(pkg):
         assert form(max(8, edge - 1), n, k) == (1, 128), (n, k)
         assert form(edge, n, k) == (4, 32), (n, k)
     assert form(10, 2304, 4096) == form(33, 4096, 256) == form(8, 1024, 4096) == form(33, 4096, 1024) == (4, 32)
+
+
+def test_only_plain_epilogues_read_operands_by_column(tmp_path):
+    """GemmArgs::bias is null or a norm weight of 128 values in the SwiGLU, LoRA, per-head-norm, q|k|v and vision epilogues: the part
+    that reads bias and residual by column must not compile for them (a build without optimization would make those reads)."""
+    import subprocess
+    from __graft_entry__ import _load_build_module
+    b = _load_build_module()
+    src = tmp_path / "plain.cu"
+    others = ("EPI_SWIGLU", "EPI_LORA", "EPI_QKNORM", "EPI_QKV", "EPI_VROPE")
+    src.write_text('#include "gemm_tc.cu"\nnamespace o1 {\n' + "".join(f"template struct PlainEpilogue<{e}>;\n" for e in others) + "}\n")
+    r = subprocess.run([b._nvcc()] + b.NVCC_FLAGS + ["-I", b.CSRC, "-cubin", "-o", str(tmp_path / "plain.cubin"), str(src)],
+                       capture_output=True, text=True)
+    assert r.returncode != 0
+    assert r.stderr.count("error: static assertion failed") == len(others), r.stderr[-2000:]
