@@ -340,7 +340,7 @@ def test_gemm_form_keeps_its_promises(pkg):
             if rng.random() < 0.7:
                 n = (n + 127) // 128 * 128
             for epi in (0, 1, 2, 3, 7, 8, 9):
-                for bn in (0, -1, 128, 256):
+                for bn in (0, -1, -2, 128, 256):
                     for mode in (1, 0):
                         pkg.lib.o1_gemm_pair_mode(mode)
                         f, w, c = form(m, n, k, epi, bn)
@@ -353,14 +353,24 @@ def test_gemm_form_keeps_its_promises(pkg):
                             continue
                         seen.add((f, w, c))
                         assert mode == 1 or c == 1, "a cluster in mode 0"
-                        assert f != 4 or c == 1 or bn == -1, "a shared K that was not asked for"
+                        if bn == -2 and mode == 0:
+                            assert (f, w, c) == form(m, n, k, epi, 0), "the tower's rule differs from the general one without clusters"
+                        assert f != 4 or c == 1 or bn in (-1, -2), "a shared K that was not asked for"
                         if bn > 0:
                             assert f in (1, 2) and w == (256 if epi == 3 else bn)
-                        assert {1: w in (128, 256), 2: w == 256 and c == 2, 3: w % 16 == 0 and 144 <= w <= 192 and epi in (1, 2),
-                                4: w in (32, 96) and c == 1 or w == 128 and 4 <= c <= 6}[f], (f, w, c)
+                        # a CTA pair per 256 rows (c == 2): 128 to 192 columns, the tower's 96 to 256; one CTA per tile only with
+                        # the bias or the residual epilogue
+                        fitted = w % 16 == 0 and ((96 <= w <= 256 and epi in (0, 1, 2, 7, 8, 9)) if bn == -2 and c == 2 else
+                                                  (144 <= w <= 192 and epi in (1, 2)))
+                        assert {1: c == 1 and w in (128, 256) or (c, w) == (2, 128) and epi in (0, 1, 2, 7, 8, 9), 2: w == 256 and c == 2,
+                                3: c in (1, 2) and fitted, 4: w in (32, 96) and c == 1 or w == 128 and 4 <= c <= 6}[f], (f, w, c)
+                        # the kernel's tile needs whole units of 16 columns for each CTA's half, and a second row tile
+                        assert f not in (1, 3) or c == 1 or (m > 128 and w % 16 == 0)
     finally:
         pkg.lib.o1_gemm_pair_mode(1)
     assert {(1, 128, 1), (1, 256, 1), (2, 256, 2), (3, 144, 1), (4, 32, 1), (4, 96, 1)} <= seen and any(c > 2 for _, _, c in seen)
+    if pkg.lib.o1_sm_count() == 148:
+        assert {(1, 128, 2), (3, 144, 2), (3, 96, 2), (3, 256, 2)} <= seen
     assert form(0, 8, 8, 0, 0)[0] == -1 and form(8, 100, 64, 2, 0)[0] == -1
 
 
