@@ -63,8 +63,8 @@ struct AttnArgs {
     // (accumulator, running max, row sum) in part_o / part_ml for attn_merge_kernel, so that the last,
     // partly filled wave of CTAs is short.  ways == 1: no tail.
     int nqb, n_plain, ways;
-    float* part_o;      // [slot][256 rows][128] fp32, slot = (item - n_plain) * ways + part
-    float* part_ml;     // [slot][256 rows][2]: max (exp2 domain) the partial is relative to, row sum
+    float* part_o;      // [slot][rows of an item][128] fp32, slot = (item - n_plain) * ways + part
+    float* part_ml;     // [slot][rows of an item][2]: max (exp2 domain) the partial is relative to, row sum
 };
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -507,14 +507,16 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // way and the softmax warps never wait for a score product that waits for them.  Warps 2..9 and 10..17 are two softmax
 // sets that take alternate key tiles (two threads per row, as above); they agree on the running max through shared
 // memory: the set that takes tile j waits for the other set's decision for tile j-1 (made early in its phase) before it
-// decides for tile j.  Measured against the two-tile kernel: see attention_tile_mode() (before the issuing threads were elected
-// that one was 9 % faster at S = 16640).
+// decides for tile j.  The reference max is a row's exact score, as in the two-tile kernel, so that P of that key is exactly 1:
+// with a max rounded up to bf16 (half the exchange) the error against 64 bits was 6 % larger, 2.20e-3 against 2.06e-3 at
+// 16640 rows and alike from 592 rows on, and it was no faster (600 to 4500 rows 1 % slower, elsewhere the same).
+// Measured against the two-tile kernel: see attention_tile_mode().
 static constexpr int T1_ROWS = 128;       // query rows per CTA and work item
 static constexpr int T1_K_STAGES = 3;
 static constexpr int T1_V_STAGES = 3;
 static constexpr int T1_S_BUFS = 3;       // score buffers in tensor memory
-static constexpr int T1_XCH = 2048;       // row-max exchange ([set][use][half][row] bf16), at the end [quarter][row] float sums
-static constexpr int T1_SMEM = TILE_BYTES * (1 + T1_K_STAGES + T1_V_STAGES) + 192 + T1_XCH + 512;
+static constexpr int T1_XCH = 2048;       // row-max exchange ([set][half][row] floats), at the end [quarter][row] sums
+static constexpr int T1_SMEM = TILE_BYTES * (1 + T1_K_STAGES + T1_V_STAGES) + 192 + T1_XCH;
 
 // bounded wait with one outcome for the whole warp (the code behind it issues warp-wide tensor-memory accesses)
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
@@ -555,10 +557,6 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     float* xch = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 192);
-    // [tile parity][row]: the max that every stored P, partial sum and O is relative to after a tile, as the unscaled bf16
-    // score it came from.  Both threads of a row read the previous tile's entry and one writes this tile's, so the two lie
-    // in different places, and all eight warps of a set arrive on m_pub: an entry is not overwritten before it is read.
-    uint16_t* m_sh = reinterpret_cast<uint16_t*>(xch + T1_XCH / 4);
 
     const int warp = warp_index();
     const int lane = threadIdx.x & 31;
@@ -715,23 +713,33 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         const bool tile_has_causal = q0 < a.ar_len;
         const bool row_causal = row_g < a.ar_len;
         const uint32_t t_o = tmem_O + half * 64 + lane_off;
-        // row-max exchange slots of the two threads of a row: [set][use parity][half][row] bf16
-        uint16_t* x16 = reinterpret_cast<uint16_t*>(xch) + set * 512 + row;
+        // The max of a row's scores in a tile, half a row by each of the two threads: [set][half][row].  Its two threads read both
+        // halves, and so do those of the other set, which follow this set's decision by the same arithmetic.  All eight
+        // warps of a set arrive on m_pub once they have read; a set writes again after the other's arrival for the tile in between,
+        // which comes after its own for the tile before, so an entry is not overwritten before all four threads have it.
+        float *x_mine = xch + set * 256 + half * 128 + row, *x_half = xch + set * 256 + (half ^ 1) * 128 + row;
+        const float* x_set = xch + (set ^ 1) * 256 + row;
         const int bar_id = 1 + set;              // named barrier of the set's 256 threads
         constexpr int BAR_THREADS = 256;
         float m_mine = -INFINITY;                // max this thread's partial sum is relative to
-        uint32_t m_raw = 0xff800000u;            // the score it came from
         float l = 0.f;                           // this thread's share of the row sum
         bool ok = true;
+        // the max in force after a tile of the other set: the sum follows where that set raised it
+        auto follow = [&] {
+            const float m_tile = fmaxf(x_set[0], x_set[128]) * a.scale_log2;
+            if ((m_tile - m_mine) > 8.0f) {
+                l *= ex2_approx(m_mine - m_tile);     // m_mine == -inf: l is 0 and stays 0
+                m_mine = m_tile;
+            }
+        };
         for (int j = set; j < n_tiles; j += 2) {
             const int b = j % T1_S_BUFS;
-            const int use = (j >> 1) & 1;
             const int kv0 = (j0 + j) * AKV + half * 64;
             const uint32_t t_s = tmem_S + b * 128 + lane_off;
             // A thread whose wait ran out keeps taking part in the set's named barrier (one per tile) and does
             // nothing else, so that no partner is left waiting at a barrier that has no time limit.
             uint32_t r[2][32];
-            uint32_t mb = 0;
+            float mx = -INFINITY;
             if (ok && !mbar_wait_warp(&s_full[b], (j / T1_S_BUFS) & 1)) { atomicExch(a.err, 17); ok = false; }
             if (ok) {
             tc_fence_after();
@@ -759,7 +767,6 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
                         if (!allow) r[c][i] = 0xff800000u;   // -inf
                     }
             }
-            float mx;
             {
                 // three-input max: 64 scores in 32 instructions, four independent chains
                 float mxa = -INFINITY, mxb = -INFINITY, mxc = -INFINITY, mxd = -INFINITY;
@@ -772,38 +779,22 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
                 }
                 mx = max3(mxa, mxb, fmaxf(mxc, mxd));
             }
-            // Row max over both halves: the partner thread's value comes through shared memory.  The reference
-            // value only has to be the same for both threads and not below the true max, so it travels as a
-            // bf16 rounded toward +inf.  A slot is rewritten two uses later, after a barrier the partner only
-            // reaches once it has read this use's value.
-            mb = __float_as_uint(mx);
-            mb = ((int32_t)mb >= 0) ? (mb + 0xffffu) : mb;     // +inf / NaN cannot occur in a score
-            x16[use * 256 + half * 128] = (uint16_t)(mb >> 16);
+            // row max over both halves; the other set has decided for the previous tile
+            if (j >= 1 && !mbar_wait_warp(&m_pub[set ^ 1], ((j - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; }
+            if (ok) *x_mine = mx;
             }
             asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(BAR_THREADS) : "memory");
             if (!ok) continue;
-            const float mx = fmaxf(__uint_as_float(mb & 0xffff0000u), __uint_as_float((uint32_t)x16[use * 256 + (half ^ 1) * 128] << 16));
+            mx = fmaxf(mx, *x_half);
             const float m_tile = mx * a.scale_log2;
-            // the max in force after the previous tile, which the other set decided
-            if (j >= 1) {
-                if (!mbar_wait_warp(&m_pub[set ^ 1], ((j - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; continue; }
-                const uint32_t raw = (uint32_t)m_sh[((j - 1) & 1) * T1_ROWS + row] << 16;
-                if (raw != m_raw) {        // the other set raised it: this thread's sum follows
-                    const float m_prev = __uint_as_float(raw) * a.scale_log2;
-                    l *= ex2_approx(m_mine - m_prev);     // m_mine == -inf: l is 0 and stays 0
-                    m_mine = m_prev;
-                    m_raw = raw;
-                }
-            }
+            if (j >= 1) follow();
             const bool grow = (m_tile - m_mine) > 8.0f;      // also true while m_mine == -inf
             float alpha = 1.0f;
             if (grow) {
                 alpha = ex2_approx(m_mine - m_tile);         // 0 on the first tile
                 m_mine = m_tile;
-                m_raw = __float_as_uint(mx);
                 l *= alpha;
             }
-            if (half == 0) m_sh[(j & 1) * T1_ROWS + row] = (uint16_t)(m_raw >> 16);
             __syncwarp();
             if (lane == 0) mbar_arrive(&m_pub[set]);
             if (j >= 1 && __any_sync(0xffffffffu, grow)) {
@@ -837,14 +828,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         // ---- the sums of the set that did not take the last tile follow its max
         if (ok && ((n_tiles - 1) & 1) != set) {
             if (!mbar_wait_warp(&m_pub[set ^ 1], ((n_tiles - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; }
-            if (ok) {
-                const uint32_t raw = (uint32_t)m_sh[((n_tiles - 1) & 1) * T1_ROWS + row] << 16;
-                if (raw != m_raw) {
-                    const float m_fin = __uint_as_float(raw) * a.scale_log2;
-                    l *= ex2_approx(m_mine - m_fin);
-                    m_mine = m_fin;
-                }
-            }
+            if (ok) follow();
         }
         // ---- output: O / l -> bf16 -> out[row_g, h*128 + part4*32 ..]
         if (ok) {
@@ -963,9 +947,11 @@ __global__ void __launch_bounds__(AD) attn_merge_kernel(const AttnArgs a, int n_
 static int g_tail_ways = 0;   // 0: choose; 1: never split; n > 1: n parts whenever they fit
 void attention_tail_ways(int ways) { g_tail_ways = ways < 0 ? 0 : ways; }
 // Which kernel: 0 and 2 = one query tile per CTA, 1 = two.  One is the better form at every length since its issuing threads are
-// elected (32 / 8 heads, two / one): 1280 rows 59 / 39 us, 4352 rows 340 / 317, 8192 rows 1009 / 975, 12356 rows 2350 / 2165, 16640 rows
-// 4050 / 3850; and in a block, where the power cap counts, more than that: 8210 rows 3.75 / 3.40 ms, 12356 rows 6.25 / 5.60, 16640 rows
-// 9.5 / 8.05.
+// elected.  Two / one in turn in one process, us: 32 / 8 heads 8192 rows 1077 / 892, 10496 rows 1737 / 1471, 12356 rows 2538 / 2017,
+// 16640 rows 4402 / 3476, all rows causal 2301 / 1927; a rank of a sharded forward, whose output leaves through the table (here into
+// this GPU's memory), 8192 / 16640 rows: 16 / 4 heads 574 / 426 and 2310 / 1763, 8 / 2 heads 330 / 229 and 1032 / 819, 4 / 1 heads
+// 195 / 117 and 676 / 465.  (The row segments it stores there are of 64 bytes where the two-tile kernel's are of 128: a rank
+// of eight stores 15 MB in those 465 us, 4 % of what a link carries.)
 static int g_tile_mode = -1;    // -1: not yet read from the environment (O1_ATTN_TILE_MODE)
 void attention_tile_mode(int mode) { g_tile_mode = (mode < 0 || mode > 2) ? 0 : mode; }
 static int tile_mode() {

@@ -14,8 +14,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(params=[1, 2], ids=["two-tile", "one-tile"])
 def tile_mode(request, pkg):
-    """Both attention kernels take every case of this module: 1 = two query tiles per CTA (what long sequences get),
-    2 = one query tile per CTA with triple-buffered scores (what S < 8192 gets by default)."""
+    """Both attention kernels take every case of this module: 1 = two query tiles per CTA (on request only),
+    2 = one query tile per CTA with triple-buffered scores (what every length gets by default)."""
     pkg.lib.o1_attention_tile_mode(request.param)
     yield request.param
     pkg.lib.o1_attention_tile_mode(0)
@@ -145,6 +145,43 @@ def test_flash_attention_full_size_sampled_rows(pkg, orc, dev, tile_mode):
     hi = vmax.reshape(KV, 128)[kvh] * 1.01 + 0.02
     lo = vmin.reshape(KV, 128)[kvh] * 1.01 - 0.02
     assert bool(((o <= hi) & (o >= lo)).all()) and bool(torch.isfinite(o).all())
+
+
+@pytest.mark.parametrize("S,ar", [(8192, 255), (8211, 8211), (16640, 255)])
+def test_long_sequences_repeat_and_are_as_exact_as_with_two_tiles(pkg, dev, S, ar):
+    """The default kernel at long sequences: the same bits from call to call, and the two-tile kernel's results but for the order of the
+    row sum.  Both keep the same exact score as a row's reference max, so every P and O is the same number; a row sum that differs by
+    some 1e-6 (16640 terms of 32 bits) turns the last rounding of 1e-6 / 2^-9, 5e-4 of the results, each by 2^-8: 1e-4 in the
+    2-norm.  (With a reference max rounded to bf16 the key it came from was no longer exactly 1: 2.7e-3 away, and 7 % further from 64 bits.)"""
+    H, KV = 4, 1
+    ld = (H + 2 * KV) * 128
+    d = torch.empty(S, ld, dtype=torch.bfloat16, device=dev)
+    assert pkg.lib.o1_fill_normal_bf16(pkg.ptr(d), S * ld, 4243, 0.0, 1.0) == 0
+
+    def call(mode):
+        out = torch.full((S, H * 128), 777.0, dtype=torch.bfloat16, device=dev)
+        pkg.lib.o1_attention_tile_mode(mode)
+        try:
+            assert pkg.lib.o1_flash_attention(C.c_void_p(d.data_ptr()), ld, C.c_void_p(d.data_ptr() + H * 256), ld,
+                                              C.c_void_p(d.data_ptr() + (H + KV) * 256), ld, pkg.ptr(out), H * 128, S, H, KV, ar,
+                                              128 ** -0.5) == 0, pkg.last_error()
+            torch.cuda.synchronize()
+        finally:
+            pkg.lib.o1_attention_tile_mode(0)
+        return out
+
+    one, two = call(0), call(1)
+    for _ in range(3):
+        assert torch.equal(call(0).view(torch.int16), one.view(torch.int16))
+    rows = torch.arange(7, S, S // 400, device=dev)
+    x = d.double()
+    q, k, v = x[rows, :H * 128].view(-1, H, 128), x[:, H * 128:(H + 1) * 128], x[:, (H + 1) * 128:]
+    sc = torch.einsum("rhd,kd->rhk", q, k) * 128 ** -0.5
+    hidden = (rows < ar)[:, None] & (torch.arange(S, device=dev)[None] > rows[:, None])
+    want = (torch.softmax(sc.masked_fill(hidden[:, None], -float("inf")), -1) @ v).reshape(rows.numel(), H * 128)
+    err = [float((o[rows].double() - want).norm() / want.norm()) for o in (one, two)]
+    assert float((one.double() - two.double()).norm() / two.double().norm()) < 1e-4
+    assert err[0] <= 1.01 * err[1], err        # (a difference of 1e-5 beside errors of 2e-3)
 
 
 @pytest.mark.parametrize("S,H,KV,ar,ways", [(1280, 32, 8, 255, 0), (2304, 20, 4, 18, 0), (2304, 20, 4, 18, 9),
