@@ -488,9 +488,10 @@ int o1_gemm_qkv(const void *x, int ldx, const void *wq, const void *wk, const vo
  * v [S, ldv], out [S, ldo]; head h at columns [128h, 128h+128). */
 int o1_flash_attention(const void *q, int ldq, const void *k, int ldk, const void *v, int ldv,
                        void *out, int ldo, int S, int heads, int kv_heads, int ar_len, float scale);
-/* Same with device scratch (16-byte aligned) for key-split tail items: when the number of (256 query rows,
- * head) items is not a multiple of the SM count, the items of the last, partly filled wave are cut along the
- * keys into several CTAs whose fp32 partial results (133,120 bytes each) a merge kernel combines.  The forward
+/* Same with device scratch (16-byte aligned) for key-split tail items: when the number of (128 query rows,
+ * head) items is not a multiple of the SM count, the items of the last, partly filled wave may be cut along the
+ * keys into several CTAs whose fp32 partial results (66,560 bytes each; twice that and 256 rows with
+ * o1_attention_tile_mode(1)) a merge kernel combines.  The forward
  * and the SP stages pass the idle SwiGLU buffer.  Too little scratch only reduces or disables the split. */
 int o1_flash_attention_ws(const void *q, int ldq, const void *k, int ldk, const void *v, int ldv, void *out,
                           int ldo, int S, int heads, int kv_heads, int ar_len, float scale, void *scratch,

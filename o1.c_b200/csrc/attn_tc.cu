@@ -939,11 +939,14 @@ __global__ void __launch_bounds__(AD) attn_merge_kernel(const AttnArgs a, int n_
 
 // Number of key-range parts for the tail items: the last (total % SMs) items would otherwise occupy a wave
 // of CTAs alone.  Cost of the tail in item durations: rounds of CTAs it needs, ceil(rem * w / SMs), times the
-// duration of a part, 1/w plus a fixed share for its prologue, Q load and fp32 epilogue (about four key
-// tiles' worth).  Measured on B200: the split pays when the tail is a sizeable part of a wave (76 of 148 SMs
-// at 8 heads and S = 16640: -13 %) or when at most one full wave precedes it (S = 1280: -20 %); after many
-// full waves the SMs have drifted apart and a tail of a few items costs next to nothing (no gain measured
-// with 4 or 8 tail items after 7 or 14 waves), so it is left alone.  Every part keeps at least two key tiles.
+// duration of a part, 1/w plus a fixed share for its prologue, Q load, fp32 epilogue and the merge launch, fourteen key
+// tiles' worth with 128-row items (4 heads, 5500 rows: 24 tail items of 43 key tiles; a key tile is 0.95 us, a wave of items
+// 40, the tail 40 unsplit and 29 in six parts of 7 tiles).  Unsplit / split, us: 4 heads 5500 rows 81 / 70, 6000 rows 84 / 75, 10496
+// rows (32 tail items after two waves) 243 / 203; 8 heads 5500 rows 125 / 120, 12356 rows (36 after five) 591 / 544; 32 heads 5500
+// rows 474 / 466; and left alone: 16 heads 1280 rows 20.5 / 27.0, 1600 rows 31.6 / 38.7, 6000 rows of 8 heads 142 / 154, 3157
+// rows of 32 heads 164 / 169, 8 heads 16640 rows (4 items after seven waves) 957 / 944.
+// After full waves the SMs have drifted apart and a tail of a few items costs next to nothing: split from a fifth of a wave on, or
+// after one wave at most.  (Two-tile items of 256 rows: four key tiles' worth.)  Every part keeps at least two key tiles.
 static int g_tail_ways = 0;   // 0: choose; 1: never split; n > 1: n parts whenever they fit
 void attention_tail_ways(int ways) { g_tail_ways = ways < 0 ? 0 : ways; }
 // Which kernel: 0 and 2 = one query tile per CTA, 1 = two.  One is the better form at every length since its issuing threads are
@@ -971,7 +974,7 @@ static int choose_tail_ways(int total, int nsm, int min_tiles, size_t scratch_by
         const bool fits = g_tail_ways * 2 <= min_tiles && (size_t)rem * g_tail_ways * part_bytes <= scratch_bytes;
         return fits ? g_tail_ways : 1;
     }
-    const double fixed = 4.0 / min_tiles;
+    const double fixed = (rows_item == T1_ROWS ? 14.0 : 4.0) / min_tiles;
     int best = 1;
     double best_cost = 1.0;
     for (int w = 2; w <= 32 && w * 2 <= min_tiles; ++w) {
@@ -979,7 +982,7 @@ static int choose_tail_ways(int total, int nsm, int min_tiles, size_t scratch_by
         const double cost = (double)((rem * w + nsm - 1) / nsm) * (1.0 / w + fixed) + 0.02;
         if (cost < best_cost - 1e-9) { best_cost = cost; best = w; }
     }
-    const bool worth = rem * 4 >= nsm || total / nsm <= 1;
+    const bool worth = rem * 5 >= nsm || total / nsm <= 1;
     return (worth && best_cost < 0.9) ? best : 1;
 }
 

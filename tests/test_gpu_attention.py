@@ -223,6 +223,32 @@ def test_flash_attention_key_split_tail(pkg, orc, dev, tile_mode, S, H, KV, ar, 
     assert torch.equal(small.view(torch.int16), plain.view(torch.int16))
 
 
+@pytest.mark.parametrize("S,H,KV,split", [(1280, 16, 4, False), (1600, 16, 4, False), (3157, 32, 8, False), (6000, 8, 2, False),
+                                          (5500, 4, 1, True), (5500, 8, 2, True), (10496, 4, 1, True), (12356, 8, 2, True)])
+def test_tail_is_split_where_that_is_faster(pkg, dev, S, H, KV, split):
+    """The automatic choice on 148 SMs: a tail is cut along the keys only where the parts, with the fixed time of each and the merge
+    launch, are shorter than a wave of whole items."""
+    if pkg.lib.o1_sm_count() != 148:
+        pytest.skip("the rule counts SMs")
+    ld = (H + 2 * KV) * 128
+    d = torch.empty(S, ld, dtype=torch.bfloat16, device=dev)
+    assert pkg.lib.o1_fill_normal_bf16(pkg.ptr(d), S * ld, 4244, 0.0, 1.0) == 0
+    scratch = torch.empty(S * H * 128 * 6, dtype=torch.uint8, device=dev)       # a rank's idle SwiGLU buffer
+    outs = []
+    for ways in (0, 1):
+        outs.append(torch.empty(S, H * 128, dtype=torch.bfloat16, device=dev))
+        pkg.lib.o1_attention_tail_ways(ways)
+        try:
+            assert pkg.lib.o1_flash_attention_ws(C.c_void_p(d.data_ptr()), ld, C.c_void_p(d.data_ptr() + H * 256), ld,
+                                                 C.c_void_p(d.data_ptr() + (H + KV) * 256), ld, pkg.ptr(outs[-1]), H * 128, S, H, KV, 255,
+                                                 128 ** -0.5, pkg.ptr(scratch), scratch.numel()) == 0, pkg.last_error()
+            torch.cuda.synchronize()
+        finally:
+            pkg.lib.o1_attention_tail_ways(0)
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16)) != split
+    assert_close(outs[0], outs[1], "C", "split vs unsplit")
+
+
 def _eager_numpy(q, k, v, mask, scaling):
     """softmax(q k^T * scaling + mask) v in fp64 with the probabilities rounded to bf16 (o1.c src/cuda/attn.cu:22-113);
     q [H,S,D], k/v [KV,S,D] as float arrays; returns probs [H,S,S], out [S,H,D]."""
