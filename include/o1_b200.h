@@ -476,7 +476,8 @@ int o1_gemm(const void *x, int ldx, const void *w, const void *w2, void *y, int 
  * one CTA per tile of 128 rows x *width columns, 2 = two CTAs per 256 x 256 tile, 3 = one CTA per tile of a *width fitted to
  * the number of SMs, 4 = the kernel for few tiles of *width columns, *ctas of a cluster sharing the K of each; -1 = not
  * supported.  1 and 3 with *ctas = 2: a CTA pair per tile of 256 rows.  force_bn -1 (which o1_gemm takes too): as 0, and K may
- * be shared; -2: as -1, and pair tiles of any width from K = 2048, or 1024 rows, on (the vision tower's linears). */
+ * be shared; -2 (the vision tower's linears): as -1, and a pair tile of 96 to 256 columns from 257 rows on where K >= 2048 (in
+ * place of narrow tiles), from 1025 rows on where 1024 <= K < 2048 and N is no multiple of 256, if that takes fewer rounds. */
 int o1_gemm_form(int M, int N, int K, int epi, int force_bn, int *width, int *ctas);
 /* The q, k and v projections of a decoder block (src/model/block.c:257-265) with the per-head RMSNorm + rotary of
  * q and k (:266-289) as ONE launch over the three weight tensors: y [M, qc | kc | kc] (row pitch ldy) =
@@ -499,14 +500,15 @@ int o1_flash_attention_ws(const void *q, int ldq, const void *k, int ldk, const 
 /* Policy of that split: 0 = automatic (default), 1 = never, n > 1 = n parts whenever scratch and key count allow. */
 void o1_attention_tail_ways(int ways);
 /* Which attention kernel: 0 (default) and 2 = one query tile of 128 rows per CTA with triple-buffered scores, 1 = two query
- * tiles that share the K/V tiles (environment O1_ATTN_TILE_MODE sets the initial value).  Same arithmetic up to fp32
- * summation order and the reference max of the lazy rescale.  The vision tower has a one-tile form of its own for its heads
+ * tiles that share the K/V tiles (environment O1_ATTN_TILE_MODE sets the initial value).  Same arithmetic up to the
+ * order in which a row's probabilities are added in fp32.  The vision tower has a one-tile form of its own for its heads
  * of 72 columns, which modes 0 and 2 use; mode 1 holds for the tower as well. */
 void o1_attention_tile_mode(int mode);
-/* Clusters of CTAs in the GEMMs: 1 (default, as is every value but 0; environment O1_GEMM_PAIR=0 turns them off) = the plain,
- * bias, residual, SwiGLU and grouped q|k|v families take, where that needs the fewest rounds of tiles, two CTAs per
- * 256 x 256 tile with cta_group::2 MMAs, each CTA holding 128 rows of A and of the accumulator and half of the B tile; and a
- * linear of the vision tower that has few tiles shares the K of a tile among up to six CTAs.  0 = always one CTA per tile, no
+/* Clusters of CTAs in the GEMMs: 1 (default, as is every value but 0; environment O1_GEMM_PAIR=0 turns them off) = where that
+ * needs the fewest rounds of tiles, two CTAs per tile of 256 rows with cta_group::2 MMAs, each CTA holding 128 rows of A and
+ * of the accumulator and half of the B tile: 256 columns in the plain, bias, residual, SwiGLU and grouped q|k|v families, 96
+ * to 256 (see o1_gemm_form) in every epilogue of one weight matrix but the per-head norm and LoRA; and a
+ * linear of the vision tower that has few tiles shares the K of a tile among up to six CTAs. 0 = always one CTA per tile, no
  * cluster is launched.  The pairs add a row's K products in the order of single CTAs: same bits.  The shared K is another
  * order of the fp32 sum, so the tower's outputs (hd_vision_forward) at small images depend on the mode within rounding;
  * those of the decoder do not.  No reference counterpart (cuBLASLt picks its own kernels there, src/cuda/gemm.cu:413-461). */

@@ -1487,8 +1487,14 @@ static int fit_width(int num_m, int N, int K, double* units) {
 // round of bn columns takes 0.6 + 0.1 bn us at K = 4096, two of those units per us.  Other forms against this one at 4096 x 4096:
 // 300 rows 19.0 / 16.8 us (128 columns), 768 rows 25.8 / 23.2 (176), 1280 rows 37.6 / 35.5 (144), 2600 rows 85 / 76 (160), and at
 // 4096 x 12288 62 / 47, 70 / 58, 124 / 101, 265 / 236; 3072 x 4096 at 1000 rows 30.5 / 22.4 (176); where the rule leaves the others,
-// 592 rows 21.1 / 22.0, 2242 rows 60.7 / 62.5, 4352 rows 112.7 / 120.  (The decoder's linears have K of 256, 1024, or 3072
-// and more, in whole blocks; other K keep the one-CTA widths.)
+// 592 rows 21.1 / 22.0, 2242 rows 60.7 / 62.5, 4352 rows 112.7 / 120.
+// Epilogues that also have the 256 x 256 pair form go up to 192 columns, the others (GELU, bias or gate + residual) up to 256.
+// Form without a pair width / with it, in turn: plain store 592 x 4096 x 4096 29.5 / 21.5 (176), 3000 x 1024 x 3072 23.5 / 17.5; GELU at
+// 4096 x 4096: 592 rows 34 / 24.0 (176), 1600 rows 53 / 47.6 (208), 3000 rows 96 / 80.6 (176), 8192 rows 222 / 193 (256; with 128
+// columns 230); K in no whole blocks: 300 x 4096 x 3080 22.4 / 18.7 (128), 700 x 4096 x 3080 + residual 29.8 / 24.3 (176),
+// 1280 x 4096 x 3080 63.8 / 37.2 (144).  From K = 2048 on pairs would be ahead too (592 x 4096 x 2560 20.2 / 15.1, 1280 x 2048 x 2048
+// + residual 16.1 / 13.0), but there the one-CTA widths and the narrow tiles are the rule, as the 128-column tiles are
+// for a ragged K or N where 256 does not divide N: only the vision tower's linears, which ask for it (GEMM_TOWER), take pairs.
 static constexpr int PAIR_FIT_K = 3072;
 static int pair_fit_width(int num_m, int N, double best, int lo, int hi) {
     const long pairs = sm_count() / 2;
@@ -1598,10 +1604,12 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
     const bool small = plain && (pair_ok || resid || epi == EPI_BIAS_GELU);
     if (small) {
         const SplitPlan p = split_plan(M, N, K, (tower || force_bn == GEMM_SPLIT_K) && pair_wanted(), resid);
-        // the tower's long K (the MLP's second linear, the mergers): pair tiles of any width instead of narrow ones
+        // the tower's long K (the MLP's second linear, the mergers): pair tiles of any width instead of narrow ones, from 257 rows on
         if (p.ks > 1 || (p.bn > 0 && !(tower && pair_wanted() && K >= LONG_K && num_m > 2))) return {GEMM_FEW, p.bn, p.ks};
-        // (from 1024 rows on its K of 1152 too: the tower of 1200 / 3024 / 4096 patches 2800 / 5600 / 8100 -> 2700 / 5370 / 7820 us,
-        // but of 832 patches 2165 -> 2197)
+        // (From 1025 rows on a K of 1024 and more too: the tower of 1200 / 3024 / 4096 patches 2800 / 5600 / 8100 -> 2700 / 5370 / 7820
+        // us, but of 832 patches 2165 -> 2197.  Only where 256 does not divide N: with the 256-column forms to choose from, a
+        // pair width loses as often as it gains, 1600 x 2304 x 1152 13.5 / 14.5, 1100 x 4096 x 1024 12.6 / 13.7, 4096 rows
+        // 36.3 / 40.7, but 1280 rows 14.9 / 12.2.)
         if (tower && pair_wanted() && num_m > (K >= LONG_K ? 2 : 8) && (K >= LONG_K || (K >= 1024 && !wide_ok))) {
             long units = 0;
             tile_form(num_m, N, K, wide_ok, pair_ok, &units);
@@ -1614,13 +1622,9 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
     double units = (double)form_units;
     int width = 0;
     if (plain && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) width = fit_width(num_m, N, K, &units);
-    if (small && !tower && (N % 128) == 0 && K >= PAIR_FIT_K && (K % BK) == 0 && pair_wanted() && M > BM) {
-        if (epi == EPI_RESID || epi == EPI_BIAS) {
-            const int w = pair_fit_width(num_m, N, units, 128, 192);
-            if (w) return {w == 128 ? GEMM_TILE : GEMM_FIT, w, 2};
-        } else if (pair_fit_width(num_m, N, units, 128, 128)) {
-            return {GEMM_TILE, 128, 2};
-        }
+    if (small && !tower && K >= PAIR_FIT_K && (wide_ok || ((N % 128) == 0 && (K % BK) == 0)) && pair_wanted() && M > BM) {
+        const int w = pair_fit_width(num_m, N, units, 128, pair_ok ? 192 : 256);
+        if (w) return {w == 128 ? GEMM_TILE : GEMM_FIT, w, 2};
     }
     if (width) return {GEMM_FIT, width, 1};
     return {f == TILE_PAIR ? GEMM_PAIR : GEMM_TILE, f == TILE_128 ? 128 : 256, f == TILE_PAIR ? 2 : 1};

@@ -358,10 +358,10 @@ def test_gemm_form_keeps_its_promises(pkg):
                         assert f != 4 or c == 1 or bn in (-1, -2), "a shared K that was not asked for"
                         if bn > 0:
                             assert f in (1, 2) and w == (256 if epi == 3 else bn)
-                        # a CTA pair per 256 rows (c == 2): 128 to 192 columns, the tower's 96 to 256; one CTA per tile only with
-                        # the bias or the residual epilogue
+                        # a CTA pair per 256 rows (c == 2): 128 to 192 columns, to 256 where there is no 256 x 256 pair form, the
+                        # tower's 96 to 256; one CTA per tile only with the bias or the residual epilogue
                         fitted = w % 16 == 0 and ((96 <= w <= 256 and epi in (0, 1, 2, 7, 8, 9)) if bn == -2 and c == 2 else
-                                                  (144 <= w <= 192 and epi in (1, 2)))
+                                                  (144 <= w <= (192 if epi in (0, 1, 2) else 256) and (c == 2 or epi in (1, 2))))
                         assert {1: c == 1 and w in (128, 256) or (c, w) == (2, 128) and epi in (0, 1, 2, 7, 8, 9), 2: w == 256 and c == 2,
                                 3: c in (1, 2) and fitted, 4: w in (32, 96) and c == 1 or w == 128 and 4 <= c <= 6}[f], (f, w, c)
                         # the kernel's tile needs whole units of 16 columns for each CTA's half, and a second row tile
@@ -372,6 +372,23 @@ def test_gemm_form_keeps_its_promises(pkg):
     if pkg.lib.o1_sm_count() == 148:
         assert {(1, 128, 2), (3, 144, 2), (3, 96, 2), (3, 256, 2)} <= seen
     assert form(0, 8, 8, 0, 0)[0] == -1 and form(8, 100, 64, 2, 0)[0] == -1
+
+
+def test_pair_widths_begin_where_the_header_says(pkg):
+    """The first row counts and K of the pair tiles of any width (on 148 SMs): 257 rows at K >= 2048 and 1025 rows from K = 1024 on for
+    the vision tower's linears, K = 3072, whole 64s or not, for the others."""
+    if pkg.lib.o1_sm_count() != 148:
+        pytest.skip("the rule counts SMs")
+    ctas = C.c_int(0)
+
+    def pairs(*a):
+        return pkg.lib.o1_gemm_form(*a, None, C.byref(ctas)) in (1, 3) and ctas.value == 2
+
+    for a, b in (((256, 4608, 4608, 7, -2), (257, 4608, 4608, 7, -2)), ((1024, 1152, 1152, 8, -2), (1025, 1152, 1152, 8, -2)),
+                 ((1024, 4304, 1152, 7, -2), (1025, 4304, 1152, 7, -2)), ((2000, 4096, 1152, 1, -2), (2000, 4104, 1152, 1, -2)),
+                 ((1025, 1152, 1016, 8, -2), (1025, 1152, 1024, 8, -2)), ((300, 4096, 3064, 2, 0), (300, 4096, 3072, 2, 0)),
+                 ((300, 4096, 3064, 0, -1), (300, 4096, 3080, 0, -1)), ((128, 8192, 3080, 9, 0), (300, 4096, 3080, 9, 0))):
+        assert not pairs(*a) and pairs(*b), (a, b)
 
 
 def test_narrow_tiles_are_for_activations_of_some_size(pkg):

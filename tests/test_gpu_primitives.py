@@ -833,7 +833,10 @@ def test_fused_swiglu_equals_the_pass_for_every_gate(pkg, dev, M):
                                                 (257, 4096, 3072, 0, 0, 128), (2600, 4096, 4160, 2, 0, 160), (300, 4096, 3072, 9, 0, 128),
                                                 (2304, 1152, 4304, 8, -2, 144), (800, 1152, 4304, 8, -2, 96), (3000, 1152, 4304, 8, -2, 192),
                                                 (520, 4608, 4608, 7, -2, 192), (1024, 4608, 4608, 7, -2, 256), (1000, 4104, 2056, 1, -2, 112),
-                                                (700, 4312, 2048, 7, -2, 192), (1200, 4304, 1152, 7, -2, 160), (1100, 1152, 1152, 8, -2, 96)])
+                                                (700, 4312, 2048, 7, -2, 192), (1200, 4304, 1152, 7, -2, 160), (1100, 1152, 1152, 8, -2, 96),
+                                                (300, 4096, 3080, 2, 0, 128), (592, 4096, 3072, 0, 0, 176), (3000, 4096, 3080, 7, 0, 176),
+                                                (1700, 4096, 3072, 9, 0, 208), (2242, 4096, 3072, 8, 0, 256), (1700, 2176, 3136, 8, 0, 224),
+                                                (257, 4608, 4608, 7, -2, 128), (1025, 1152, 1152, 8, -2, 96)])
 def test_pair_tiles_of_any_width(pkg, dev, M, N, K, epi, bn, width):
     """CTA pairs with a width chosen by the rounds of tiles give the bits of 128-column tiles: partly filled last row and column
     tiles, an odd number of row tiles, a ragged N and K, every epilogue."""
@@ -853,3 +856,24 @@ def test_pair_tiles_of_any_width(pkg, dev, M, N, K, epi, bn, width):
     assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
     check_epilogue_f64(ys[0][:M, :N], x, w, b, r, epi, "pair tiles")
     assert pkg.lib.o1_device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K,epi", [(520, 4608, 4608, 7), (2304, 1152, 4304, 8), (1100, 4304, 1152, 7), (77, 1152, 1152, 8)])
+def test_the_towers_linears_keep_their_bits_without_clusters(pkg, dev, M, N, K, epi):
+    """force_bn -2 (the vision tower's linears) in pair mode 0: one CTA per tile, and where no K is shared the same bits."""
+    g = torch.Generator(device=dev).manual_seed(M)
+    x, w, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
+                  for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
+    ys = []
+    try:
+        for mode in (1, 0):
+            pkg.lib.o1_gemm_pair_mode(mode)
+            form = gemm_form(pkg, M, N, K, epi, -2)
+            assert form[2] == 1 if mode == 0 else form[2] <= 2      # (a shared K takes four CTAs and more)
+            y = torch.empty(M, N, dtype=torch.bfloat16, device=dev)
+            assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N, M, N, K, epi, pkg.ptr(b), pkg.ptr(r), N, 0.0, -2) == 0
+            done(pkg, "gemm")
+            ys.append(y)
+    finally:
+        pkg.lib.o1_gemm_pair_mode(1)
+    assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
