@@ -1436,8 +1436,8 @@ int gemm_pair_capacity() {
 
 // Which persistent form takes the fewest (rounds of tiles) x (time of a K block): one CTA per 128 x 128 or 128 x 256 tile,
 // or a pair of CTAs per 256 x 256 tile.  The sums are the same in all of them.  A round of tiles with K = 4096 takes 15.6,
-// 29 (4096 columns) to 33 (24576) and 25 us; measured at 4096 columns: 593 rows 32.4 / 31.7 / 30.2 us, 1280 rows 48.8 / 58.0 / 51.4, 2242 rows 72.6 /
-// 63.6 / 56.6, and at 6144 columns (q | k | v) 296 rows 24.6 / 38.6 / 40.1, 1280 rows 66.4 / 60.5 / 53.0.  Gate | up as
+// 29 (4096 columns) to 33 (24576) and 25 us; measured at 4096 columns: 592 rows 33.3 / 31.6 / 30.5 us, 1280 rows 51.4 / 60.3 / 54.5, 2242
+// rows 73.7 / 64.7 / 59.2, 8192 rows 255 / 197 / 197, and at 6144 columns (q | k | v) 296 rows 24.6 / 38.6 / 40.1, 1280 rows 66.4 / 60.5 / 53.0.  Gate | up as
 // pairs instead of one CTA per 128 x 256 tile: 1280 rows 213 / 186 us, a block of 16640 rows 9.24 / 9.02 ms.
 enum TileForm { TILE_128, TILE_256, TILE_PAIR };
 static constexpr int TILE_COST[3] = {31, 66, 50};
@@ -1460,6 +1460,15 @@ static TileForm tile_form(int num_m, int N, int K, bool wide_ok, bool pair_ok, l
     if (units) *units = cp <= c256 && cp <= c128 ? cp : (c256 <= c128 ? c256 : c128);
     if (cp <= c256 && cp <= c128) return TILE_PAIR;
     return c256 <= c128 ? TILE_256 : TILE_128;
+}
+
+// Below K = 2048, the plain, bias and residual families: two rounds of pairs against four of 128 columns.  128 columns / pairs:
+// 2048 x 4096 x 1024 21.3 / 18.5, with residual 24.4 / 21.4, 1000 x 8192 x 1024 24.6 / 21.7, 4096 x 2048 x 1536 32.5 / 28.0,
+// 2242 x 4096 x 512 12.6 / 11.7, but K = 256 9.8 / 9.9; three rounds against four 1100 x 8192 x 1024 24.9 / 27.4, one against two 1000 x
+// 4096 x 1024 11.4 / 11.4, K = 512 7.8 / 8.5.  (Their epilogue is short; q | k | v with K = 1024 would be slower, 1300 rows 23.0 / 24.7.)
+static bool two_rounds_of_pairs(int num_m, int N, int K) {
+    const long sms = sm_count(), pair_tiles = (long)((num_m + 1) / 2) * (N / 256);
+    return K >= 512 && K < LONG_K && pair_tiles <= sms / 2 * 2 && (long)num_m * (N / 128) > 3 * sms;
 }
 
 // The fitted width for the bias and residual families, or 0 where no width beats the other forms.  A round of bn columns
@@ -1618,7 +1627,8 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
         }
     }
     long form_units = 0;
-    const TileForm f = tile_form(num_m, N, K, wide_ok, pair_ok, &form_units);
+    TileForm f = tile_form(num_m, N, K, wide_ok, pair_ok, &form_units);
+    if (small && pair_ok && wide_ok && pair_wanted() && two_rounds_of_pairs(num_m, N, K)) f = TILE_PAIR;
     double units = (double)form_units;
     int width = 0;
     if (plain && (N % 128) == 0 && (epi == EPI_RESID || epi == EPI_BIAS)) width = fit_width(num_m, N, K, &units);

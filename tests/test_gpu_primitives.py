@@ -432,7 +432,8 @@ def test_qkv_projections_as_one_launch(pkg, dev, M, qc, kc, K):
 
 
 @pytest.mark.parametrize("M,N,K,epi", [(4352, 4096, 512, 0), (4115, 4096, 256, 2), (4200, 3072, 320, 1), (8320, 4096, 192, 2),
-                                       (1280, 4096, 2048, 3), (1400, 4096, 2056, 3), (2304, 4096, 2048, 0), (2561, 4096, 2104, 2)])
+                                       (1280, 4096, 2048, 3), (1400, 4096, 2056, 3), (2304, 4096, 2048, 0), (2561, 4096, 2104, 2),
+                                       (2048, 4096, 512, 1), (1921, 4096, 1032, 2), (2304, 4096, 1024, 0)])
 def test_gemm_on_cta_pairs_equals_single_cta_tiles(pkg, dev, M, N, K, epi):
     """The cta_group::2 form (two CTAs per 256 x 256 tile, each with half of the B tile) adds a row's K products in the
     same order as the one-CTA form: same bits, for an even and an odd number of row tiles, a partly filled last row
