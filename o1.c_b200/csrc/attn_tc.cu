@@ -507,16 +507,21 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // way and the softmax warps never wait for a score product that waits for them.  Warps 2..9 and 10..17 are two softmax
 // sets that take alternate key tiles (two threads per row, as above); they agree on the running max through shared
 // memory: the set that takes tile j waits for the other set's decision for tile j-1 (made early in its phase) before it
-// decides for tile j.  The reference max is a row's exact score, as in the two-tile kernel, so that P of that key is exactly 1:
-// with a max rounded up to bf16 (half the exchange) the error against 64 bits was 6 % larger, 2.20e-3 against 2.06e-3 at
-// 16640 rows and alike from 592 rows on, and it was no faster (600 to 4500 rows 1 % slower, elsewhere the same).
+// decides for tile j.
+// EXACT: the reference max is a row's exact score, as in the two-tile kernel, so that P of that key is exactly 1; from T1_EXACT_ROWS
+// rows on, where that kernel used to run.  Else the max is rounded up to bf16 (half the exchange): the error against 64 bits is 6 %
+// larger (16640 rows 2.20e-3 against 2.06e-3, alike from 592 rows on).  The time is the same, 600 to 4500 rows 1 % longer; shorter
+// sequences keep it because 36 blocks carry a change of single roundings as far as 4e-2 (2-norm), and their results stay
+// what they have always been.
 // Measured against the two-tile kernel: see attention_tile_mode().
 static constexpr int T1_ROWS = 128;       // query rows per CTA and work item
 static constexpr int T1_K_STAGES = 3;
 static constexpr int T1_V_STAGES = 3;
 static constexpr int T1_S_BUFS = 3;       // score buffers in tensor memory
-static constexpr int T1_XCH = 2048;       // row-max exchange ([set][half][row] floats), at the end [quarter][row] sums
-static constexpr int T1_SMEM = TILE_BYTES * (1 + T1_K_STAGES + T1_V_STAGES) + 192 + T1_XCH;
+static constexpr int T1_EXACT_ROWS = 8192;
+// row-max exchange ([set][use][half][row] bf16, EXACT: [set][half][row] floats), at the end [quarter][row] float sums
+static constexpr int T1_XCH = 2048;
+static constexpr int T1_SMEM = TILE_BYTES * (1 + T1_K_STAGES + T1_V_STAGES) + 192 + T1_XCH + 512;
 
 // bounded wait with one outcome for the whole warp (the code behind it issues warp-wide tensor-memory accesses)
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
@@ -533,7 +538,7 @@ struct Attn1Params {
     AttnArgs a[NSEG];
     int grid0;
 };
-template <int DH, int NSEG>
+template <int DH, int NSEG, bool EXACT>
 __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __grid_constant__ Attn1Params<NSEG> par) {
     const int seg = NSEG > 1 && (int)blockIdx.x >= par.grid0 ? 1 : 0;
     const AttnArgs& a = par.a[seg];
@@ -713,27 +718,46 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         const bool tile_has_causal = q0 < a.ar_len;
         const bool row_causal = row_g < a.ar_len;
         const uint32_t t_o = tmem_O + half * 64 + lane_off;
-        // The max of a row's scores in a tile, half a row by each of the two threads: [set][half][row].  Its two threads read both
-        // halves, and so do those of the other set, which follow this set's decision by the same arithmetic.  All eight
-        // warps of a set arrive on m_pub once they have read; a set writes again after the other's arrival for the tile in between,
-        // which comes after its own for the tile before, so an entry is not overwritten before all four threads have it.
+        // The max of a row's scores in a tile, half a row by each of its two threads, in shared memory.
+        // EXACT, [set][half][row]: the two threads read both halves, and so do those of the other set, which follow this set's decision
+        // by the same arithmetic.  All eight warps of a set arrive on m_pub once they have read; a set writes again after the other's
+        // arrival for the tile in between, which comes after its own for the tile before, so an entry is not overwritten
+        // before all four threads have it.
+        // Else [set][use parity][half][row] in bf16, beside it [tile parity][row] the max in force after a tile (every stored P, partial
+        // sum and O is relative to it) as the unscaled score it came from.  Both threads of a row read the previous tile's
+        // entry and one writes this tile's, so the two lie in different places, and all eight warps of a set
+        // arrive on m_pub: an entry is not overwritten before it is read.
         float *x_mine = xch + set * 256 + half * 128 + row, *x_half = xch + set * 256 + (half ^ 1) * 128 + row;
         const float* x_set = xch + (set ^ 1) * 256 + row;
+        uint16_t* x16 = reinterpret_cast<uint16_t*>(xch) + set * 512 + row;
+        uint16_t* m_sh = reinterpret_cast<uint16_t*>(xch + T1_XCH / 4);
         const int bar_id = 1 + set;              // named barrier of the set's 256 threads
         constexpr int BAR_THREADS = 256;
         float m_mine = -INFINITY;                // max this thread's partial sum is relative to
+        uint32_t m_raw = 0xff800000u;            // (not EXACT) the score it came from
         float l = 0.f;                           // this thread's share of the row sum
         bool ok = true;
-        // the max in force after a tile of the other set: the sum follows where that set raised it
-        auto follow = [&] {
-            const float m_tile = fmaxf(x_set[0], x_set[128]) * a.scale_log2;
-            if ((m_tile - m_mine) > 8.0f) {
+        // the max in force after the other set's tile j: the sum follows where that set raised it
+        auto follow = [&](int j) {
+            float m_tile;
+            bool raised;
+            if constexpr (EXACT) {
+                m_tile = fmaxf(x_set[0], x_set[128]) * a.scale_log2;
+                raised = (m_tile - m_mine) > 8.0f;
+            } else {
+                const uint32_t raw = (uint32_t)m_sh[(j & 1) * T1_ROWS + row] << 16;
+                m_tile = __uint_as_float(raw) * a.scale_log2;
+                raised = raw != m_raw;
+                m_raw = raw;
+            }
+            if (raised) {
                 l *= ex2_approx(m_mine - m_tile);     // m_mine == -inf: l is 0 and stays 0
                 m_mine = m_tile;
             }
         };
         for (int j = set; j < n_tiles; j += 2) {
             const int b = j % T1_S_BUFS;
+            const int use = (j >> 1) & 1;
             const int kv0 = (j0 + j) * AKV + half * 64;
             const uint32_t t_s = tmem_S + b * 128 + lane_off;
             // A thread whose wait ran out keeps taking part in the set's named barrier (one per tile) and does
@@ -779,22 +803,37 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
                 }
                 mx = max3(mxa, mxb, fmaxf(mxc, mxd));
             }
-            // row max over both halves; the other set has decided for the previous tile
-            if (j >= 1 && !mbar_wait_warp(&m_pub[set ^ 1], ((j - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; }
-            if (ok) *x_mine = mx;
+            // Row max over both halves: the partner thread's value comes through shared memory.
+            if constexpr (EXACT) {
+                if (j >= 1 && !mbar_wait_warp(&m_pub[set ^ 1], ((j - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; }
+                if (ok) *x_mine = mx;
+            } else {
+                // The reference value only has to be the same for both threads and not below the true max, so it travels as a
+                // bf16 rounded toward +inf (+inf / NaN cannot occur in a score).  A slot is rewritten two uses later, after a
+                // barrier the partner only reaches once it has read this use's value.
+                const uint32_t mb = __float_as_uint(mx);
+                mx = __uint_as_float(((int32_t)mb >= 0 ? mb + 0xffffu : mb) & 0xffff0000u);
+                x16[use * 256 + half * 128] = (uint16_t)(__float_as_uint(mx) >> 16);
+            }
             }
             asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(BAR_THREADS) : "memory");
             if (!ok) continue;
-            mx = fmaxf(mx, *x_half);
+            mx = fmaxf(mx, EXACT ? *x_half : __uint_as_float((uint32_t)x16[use * 256 + (half ^ 1) * 128] << 16));
             const float m_tile = mx * a.scale_log2;
-            if (j >= 1) follow();
+            // the max in force after the previous tile, which the other set decided
+            if (j >= 1) {
+                if (!EXACT && !mbar_wait_warp(&m_pub[set ^ 1], ((j - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; continue; }
+                follow(j - 1);
+            }
             const bool grow = (m_tile - m_mine) > 8.0f;      // also true while m_mine == -inf
             float alpha = 1.0f;
             if (grow) {
                 alpha = ex2_approx(m_mine - m_tile);         // 0 on the first tile
                 m_mine = m_tile;
+                m_raw = __float_as_uint(mx);
                 l *= alpha;
             }
+            if (!EXACT && half == 0) m_sh[(j & 1) * T1_ROWS + row] = (uint16_t)(m_raw >> 16);
             __syncwarp();
             if (lane == 0) mbar_arrive(&m_pub[set]);
             if (j >= 1 && __any_sync(0xffffffffu, grow)) {
@@ -828,7 +867,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         // ---- the sums of the set that did not take the last tile follow its max
         if (ok && ((n_tiles - 1) & 1) != set) {
             if (!mbar_wait_warp(&m_pub[set ^ 1], ((n_tiles - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; }
-            if (ok) follow();
+            if (ok) follow(n_tiles - 1);
         }
         // ---- output: O / l -> bf16 -> out[row_g, h*128 + part4*32 ..]
         if (ok) {
@@ -939,14 +978,17 @@ __global__ void __launch_bounds__(AD) attn_merge_kernel(const AttnArgs a, int n_
 
 // Number of key-range parts for the tail items: the last (total % SMs) items would otherwise occupy a wave
 // of CTAs alone.  Cost of the tail in item durations: rounds of CTAs it needs, ceil(rem * w / SMs), times the
-// duration of a part, 1/w plus a fixed share for its prologue, Q load, fp32 epilogue and the merge launch, fourteen key
-// tiles' worth with 128-row items (4 heads, 5500 rows: 24 tail items of 43 key tiles; a key tile is 0.95 us, a wave of items
-// 40, the tail 40 unsplit and 29 in six parts of 7 tiles).  Unsplit / split, us: 4 heads 5500 rows 81 / 70, 6000 rows 84 / 75, 10496
-// rows (32 tail items after two waves) 243 / 203; 8 heads 5500 rows 125 / 120, 12356 rows (36 after five) 591 / 544; 32 heads 5500
-// rows 474 / 466; and left alone: 16 heads 1280 rows 20.5 / 27.0, 1600 rows 31.6 / 38.7, 6000 rows of 8 heads 142 / 154, 3157
-// rows of 32 heads 164 / 169, 8 heads 16640 rows (4 items after seven waves) 957 / 944.
-// After full waves the SMs have drifted apart and a tail of a few items costs next to nothing: split from a fifth of a wave on, or
-// after one wave at most.  (Two-tile items of 256 rows: four key tiles' worth.)  Every part keeps at least two key tiles.
+// duration of a part, 1/w plus a fixed share for its prologue, Q load, fp32 epilogue and the merge launch.  With 128-row items that
+// share is some twelve key tiles' worth (4 heads, 5500 rows: a key tile is 0.95 us, a wave of items of 43 key tiles 40, the tail of 24
+// items 40 unsplit and 29 in parts of 7 key tiles).  After full waves the SMs have drifted apart and a tail of a few items costs
+// next to nothing: split from a fifth of a wave on, or after one wave at most.  Unsplit / split, us: 4 heads 10496
+// rows (32 tail items after two waves) 231 / 194, 16640 rows (76 after three, two rounds of parts) 509 / 501, 8 heads 8192 rows
+// 270 / 252, 12356 rows (36 after five) 585 / 541, 16 heads 12356 rows 1082 / 1061; left alone: 8 heads 16640 rows (4 after
+// seven) 933 / 937, 16 heads 8192 rows 485 / 522.
+// Below T1_EXACT_ROWS rows the share is four key tiles, as measured with the two-tile kernel's 256-row items (which keep it),
+// and the tail a quarter of a wave: like the max there, the choice decides the bits of a forward.  The figure above would be the
+// better one there too, 16 heads 1280 rows 27.0 / 20.5 us, 32 heads 3157 rows 169 / 164, 8 heads 6000 rows 154 / 142.
+// Every part keeps at least two key tiles.
 static int g_tail_ways = 0;   // 0: choose; 1: never split; n > 1: n parts whenever they fit
 void attention_tail_ways(int ways) { g_tail_ways = ways < 0 ? 0 : ways; }
 // Which kernel: 0 and 2 = one query tile per CTA, 1 = two.  One is the better form at every length since its issuing threads are
@@ -966,7 +1008,7 @@ static int tile_mode() {
 }
 bool attention_two_tile_only() { return tile_mode() == 1; }
 
-static int choose_tail_ways(int total, int nsm, int min_tiles, size_t scratch_bytes, int rows_item) {
+static int choose_tail_ways(int total, int nsm, int min_tiles, size_t scratch_bytes, int rows_item, int S) {
     const int rem = total % nsm;
     if (rem == 0) return 1;
     const size_t part_bytes = (size_t)rows_item * AD * 4 + (size_t)rows_item * 2 * 4;
@@ -974,7 +1016,8 @@ static int choose_tail_ways(int total, int nsm, int min_tiles, size_t scratch_by
         const bool fits = g_tail_ways * 2 <= min_tiles && (size_t)rem * g_tail_ways * part_bytes <= scratch_bytes;
         return fits ? g_tail_ways : 1;
     }
-    const double fixed = (rows_item == T1_ROWS ? 14.0 : 4.0) / min_tiles;
+    const bool long_one = rows_item == T1_ROWS && S >= T1_EXACT_ROWS;
+    const double fixed = (long_one ? 12.0 : 4.0) / min_tiles;
     int best = 1;
     double best_cost = 1.0;
     for (int w = 2; w <= 32 && w * 2 <= min_tiles; ++w) {
@@ -982,7 +1025,7 @@ static int choose_tail_ways(int total, int nsm, int min_tiles, size_t scratch_by
         const double cost = (double)((rem * w + nsm - 1) / nsm) * (1.0 / w + fixed) + 0.02;
         if (cost < best_cost - 1e-9) { best_cost = cost; best = w; }
     }
-    const bool worth = rem * 5 >= nsm || total / nsm <= 1;
+    const bool worth = rem * (long_one ? 5 : 4) >= nsm || total / nsm <= 1;
     return (worth && best_cost < 0.9) ? best : 1;
 }
 
@@ -1059,7 +1102,7 @@ static bool attention_setup(AttnSetup& s, const void* q, int ldq, const void* k,
             // the number of parts, and parts of theirs that get no key tile leave an empty partial)
             if (t >= 4 && t < min_tiles) min_tiles = t;
         }
-        const int w = (rem && min_tiles < (1 << 30)) ? choose_tail_ways(total, nsm, min_tiles, scratch_bytes, rows_item) : 1;
+        const int w = (rem && min_tiles < (1 << 30)) ? choose_tail_ways(total, nsm, min_tiles, scratch_bytes, rows_item, S) : 1;
         if (w > 1) {
             n_tail = rem;
             a.n_plain = total - rem;
@@ -1080,10 +1123,10 @@ static bool launched(cudaError_t e) {
     if (e != cudaSuccess) set_error("attention: launch: %s", cudaGetErrorString(e));
     return e == cudaSuccess;
 }
-template <int NSEG>
+template <int NSEG, bool EXACT>
 static bool launch_one_tile(const AttnSetup* s, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
-    auto kern = flash_attn1_kernel<AD, NSEG>;
+    auto kern = flash_attn1_kernel<AD, NSEG, EXACT>;
     if (!func_attr_once(attr_done, (const void*)kern, T1_SMEM, "attention (one tile)")) return false;
     Attn1Params<NSEG> p;
     int grid = 0;
@@ -1099,15 +1142,17 @@ static bool launch_two_tile(const AttnSetup& s, cudaStream_t st) {
     if (!func_attr_once(attr_done, (const void*)flash_attn_kernel, ATTN_SMEM, "attention")) return false;
     return launched(launch_chained(flash_attn_kernel, dim3(s.grid), dim3(ATTN_THREADS), ATTN_SMEM, st, 1, s.a.S, s.q, s.k, s.v, s.a));
 }
-// s[0 .. n): one launch for all of them where all take the one-tile kernel
+// s[0 .. n): one launch for all of them where all take the one-tile kernel of short sequences
 static bool attention_launch(const AttnSetup* s, int n, cudaStream_t st) {
     double work = 0;
     for (int i = 0; i < n; ++i) work += s[i].work;
     prof_before(PROF_ATTN, work, st);
     bool ok = true;
-    if (n == 2 && s[0].one_tile && s[1].one_tile) ok = launch_one_tile<2>(s, st);
+    auto exact = [&](int i) { return s[i].a.S >= T1_EXACT_ROWS; };
+    if (n == 2 && s[0].one_tile && s[1].one_tile && !exact(0) && !exact(1)) ok = launch_one_tile<2, false>(s, st);
     else
-        for (int i = 0; i < n && ok; ++i) ok = s[i].one_tile ? launch_one_tile<1>(s + i, st) : launch_two_tile(s[i], st);
+        for (int i = 0; i < n && ok; ++i)
+            ok = !s[i].one_tile ? launch_two_tile(s[i], st) : exact(i) ? launch_one_tile<1, true>(s + i, st) : launch_one_tile<1, false>(s + i, st);
     for (int i = 0; i < n && ok; ++i)
         if (s[i].n_tail)
             ok = launched(launch_chained(attn_merge_kernel, dim3(s[i].n_tail * s[i].rows_item), dim3(AD), 0, st, 1, s[i].a.S, s[i].a,
@@ -1125,7 +1170,7 @@ bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cuda
         !cached_tmap(&p.v[0], q + 2 * H * AD, S, H * AD, LD, 128))
         return false;
     static std::atomic<uint64_t> attr_done{0};
-    auto kern = flash_attn1_kernel<DH, 1>;
+    auto kern = flash_attn1_kernel<DH, 1, false>;
     if (!func_attr_once(attr_done, (const void*)kern, T1_SMEM, "attention (vision)")) return false;
     AttnArgs& a = p.a[0];
     a.out = (uint16_t*)out; a.ldo = H * DH; a.out_hoff = DH;

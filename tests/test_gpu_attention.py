@@ -223,8 +223,7 @@ def test_flash_attention_key_split_tail(pkg, orc, dev, tile_mode, S, H, KV, ar, 
     assert torch.equal(small.view(torch.int16), plain.view(torch.int16))
 
 
-@pytest.mark.parametrize("S,H,KV,split", [(1280, 16, 4, False), (1600, 16, 4, False), (3157, 32, 8, False), (6000, 8, 2, False),
-                                          (5500, 4, 1, True), (5500, 8, 2, True), (10496, 4, 1, True), (12356, 8, 2, True)])
+@pytest.mark.parametrize("S,H,KV,split", [(8192, 16, 4, False), (16640, 8, 2, False), (8192, 8, 2, True), (10496, 4, 1, True), (12356, 8, 2, True), (16640, 4, 1, True)])
 def test_tail_is_split_where_that_is_faster(pkg, dev, S, H, KV, split):
     """The automatic choice on 148 SMs: a tail is cut along the keys only where the parts, with the fixed time of each and the merge
     launch, are shorter than a wave of whole items."""
