@@ -952,7 +952,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // columns leave a last round of few tiles (1280 rows x 4096 columns: 320 tiles for 148 SMs, three rounds for 2.2), some
 // width in between often makes whole rounds (144 columns: 290 tiles, two rounds).  A block of 1280 rows went from 539 to
 // 503 us, a guided step of 2 x 296 rows from 11.1 to 10.5 ms.  Same warps, same pipeline and the same sums; plain
-// row-major output with the bias or residual epilogue.
+// row-major output with the bias or residual epilogue.  (The epilogue's slices take 17 KB: 160 columns have five stages where six
+// would fit without, 800 x 3072 x 4096 23.7 us with six, 23.6 with five.)
 static constexpr int FIT_MAX_STAGES = 6, FIT_ROOM = 208 * 1024 /*stages*/, FIT_SMEM = FIT_ROOM + EPI_WARPS * EPI_SLICE + 1024 /*align*/ + 256 /*barriers*/;
 
 template <int EPI>
@@ -1561,7 +1562,11 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
 //  * 96 columns where the wider tiles need a second round and these do not, and K is short: 2916 x 1152 x 1152 16.0 / 12.5,
 //    520 x 4304 x 1152 16.4 / 14.1; 593 x 4096 x 12288 86 / 84, where CTA pairs take 72
 //  * K over a cluster where even narrow tiles leave a long main loop: 520 x 1152 x 4304 23.5 / 18.7 (five CTAs, 32 columns
-//    27.2), 96 x 1152 x 4304 22.2 / 12.9 (six; 16.2); with 64 tiles and more 32 columns are as good (130 x 4096 x 4608)
+//    27.2), 96 x 1152 x 4304 22.2 / 12.9 (six; 16.2); with 64 tiles and more 32 columns are as good (130 x 4096 x 4608).
+//    (Narrow tiles have become faster since, with two K blocks a stage and the epilogue through shared memory: where there is at most
+//    one for each SM they are ahead of the shared K, 160 to 512 x 1152 x 4304 15 / 18-19, 128 x 4608 x 4608 15.1 / 19.2,
+//    256 x 2048 x 4096 11.9 / 17.0; not with one row tile of 36 narrow ones, 96 x 1152 x 4304 14.0 / 12.2, nor beyond one per SM,
+//    520 x 1152 x 4304 26.8 / 18.7.  The order of those sums, hence the tower's bits, hangs on this rule.)
 // But few rows of a long K (small_rows()) are read by fewer SMs in wider tiles: by at most half of them from K = 2048 on, by no
 // more than all from K = 512 on.  Narrow / 128 columns / before there were narrow ones: 10 x 4096 x 4096 27.4 / 22.5 / 24.6,
 // 10 x 6144 x 4096 52.0 / 26.5 / 26.3, 12 x 8192 x 2048 28.7 / 18.3 / 19.7, 33 x 8192 x 1024 13.7 / 9.8 / 12.3, 12 x 8192 x 512
