@@ -43,6 +43,18 @@ static constexpr int ATTN_THREADS = 576;   // TMA warp, MMA warp, two softmax gr
 static constexpr int ATTN_XCH = 2 * 2 * 128 * 4;   // [group][column half][row] floats
 static constexpr int ATTN_SMEM = TILE_BYTES * (2 + K_STAGES + V_STAGES) + 192 + ATTN_XCH;
 
+// n / d for 0 <= n < 2^31 without a division (Granlund and Montgomery, PLDI 1994: multiply by 2^32 (2^s - d) / d + 1, add n, shift
+// by s = ceil(log2 d)): a work unit takes four divisions, some 150 cycles each, before its first copy can start.
+struct FastDiv {
+    uint32_t mul, shift;
+    void set(int d) {
+        shift = 0;
+        while ((1ll << shift) < d) ++shift;
+        mul = (uint32_t)((((1ull << shift) - (uint64_t)d) << 32) / (uint64_t)d + 1);
+    }
+    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift); }
+};
+
 struct AttnArgs {
     uint16_t* out;
     int ldo;
@@ -63,6 +75,11 @@ struct AttnArgs {
     // (accumulator, running max, row sum) in part_o / part_ml for attn_merge_kernel, so that the last,
     // partly filled wave of CTAs is short.  ways == 1: no tail.
     int nqb, n_plain, ways;
+    // One-tile kernel (unit_at()): query blocks [qb0, qb0 + nqb), the first nc of them all causal; n_full of the plain items see every
+    // key, n_long work units with the parts of the tail, and n_short causal items.
+    int qb0, nc, n_full, n_long, n_short;
+    int hf, hr;         // the plain items are hf whole heads and the first hr query blocks of another
+    FastDiv by_full, by_nqb, by_ways, by_hf, by_hf1, by_group;    // nqb - nc, nqb, ways, hf, hf + 1, query heads per key head
     float* part_o;      // [slot][rows of an item][128] fp32, slot = (item - n_plain) * ways + part
     float* part_ml;     // [slot][rows of an item][2]: max (exp2 domain) the partial is relative to, row sum
 };
@@ -501,27 +518,37 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// One query tile per CTA, scores triple-buffered: work items of 128 rows fill 148 SMs at short sequences too (S = 1280: 320
+// One query tile at a time, scores triple-buffered: work items of 128 rows fill 148 SMs at short sequences too (S = 1280: 320
 // instead of 160), and no serial chain as in the two-tile kernel.  Tensor memory: three score buffers of 128 columns + one output accumulator.  The MMA
-// thread issues S(j+3) = Q K^T right after PV(j), so the scores of the next two key tiles are always there or on their
+// thread issues S(g+3) = Q K^T right after PV(g), so the scores of the next two key tiles are always there or on their
 // way and the softmax warps never wait for a score product that waits for them.  Warps 2..9 and 10..17 are two softmax
 // sets that take alternate key tiles (two threads per row, as above); they agree on the running max through shared
-// memory: the set that takes tile j waits for the other set's decision for tile j-1 (made early in its phase) before it
-// decides for tile j.
+// memory: the set that takes tile g waits for the other set's decision for tile g-1 (made early in its phase) before it
+// decides for tile g.
+// A CTA stays on its SM and takes one work unit after the other (unit_at()): the key tiles of its units are ONE stream, counted by g,
+// that copies, score products and softmax sets run through without a stop.  The next unit's Q, K and first three score products are
+// there before this one's last PV, the set that did not take the last key tile goes on with the next unit at once, and the other one
+// normalises and stores this unit's rows under it.  What stays between two units is the accumulator, which PV of the
+// next one may only overwrite once it has been read.  With a CTA for each item (barriers, tensor memory, first copies and the way out
+// for each) / with units in a stream, 32 / 8 heads, us: 592 rows 18.8 / 16.0, 1280 rows 39.2 / 34.2, 3157 rows 157 / 148, 4352 rows
+// 302 / 290, 16640 rows 3821 / 3781 (power cap), all rows causal 1280 rows 29.7 / 22.4, 3157 rows 118 / 95; the tower's 16 heads of
+// 72 at 4096 patches 118 / 107; one unit for each CTA (200 rows) 7.5 / 7.4.  The same bits.
 // EXACT: the reference max is a row's exact score, as in the two-tile kernel, so that P of that key is exactly 1; from T1_EXACT_ROWS
 // rows on, where that kernel used to run.  Else the max is rounded up to bf16 (half the exchange): the error against 64 bits is 6 %
 // larger (16640 rows 2.20e-3 against 2.06e-3, alike from 592 rows on).  The time is the same, 600 to 4500 rows 1 % longer; shorter
 // sequences keep it because 36 blocks carry a change of single roundings as far as 4e-2 (2-norm), and their results stay
 // what they have always been.
 // Measured against the two-tile kernel: see attention_tile_mode().
-static constexpr int T1_ROWS = 128;       // query rows per CTA and work item
-static constexpr int T1_K_STAGES = 3;
+static constexpr int T1_ROWS = 128;       // query rows per work item
+static constexpr int T1_Q_STAGES = 2;
+static constexpr int T1_K_STAGES = 2;
 static constexpr int T1_V_STAGES = 3;
 static constexpr int T1_S_BUFS = 3;       // score buffers in tensor memory
 static constexpr int T1_EXACT_ROWS = 8192;
-// row-max exchange ([set][use][half][row] bf16, EXACT: [set][half][row] floats), at the end [quarter][row] float sums
+static constexpr int T1_BARS = 256, T1_UNITS = 4;     // (unit table: see T1_UNITS x 32 bytes behind the barriers)
+// row-max exchange ([set][use][half][row] bf16, EXACT: [set][half][row] floats); behind it (not EXACT) the max in force, [tile parity][row]
 static constexpr int T1_XCH = 2048;
-static constexpr int T1_SMEM = TILE_BYTES * (1 + T1_K_STAGES + T1_V_STAGES) + 192 + T1_XCH + 512;
+static constexpr int T1_SMEM = TILE_BYTES * (T1_Q_STAGES + T1_K_STAGES + T1_V_STAGES) + T1_BARS + T1_UNITS * 32 + T1_XCH + 512;
 
 // bounded wait with one outcome for the whole warp (the code behind it issues warp-wide tensor-memory accesses)
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
@@ -530,92 +557,207 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
 
 // DH: columns of a head that hold data.  72 (the vision tower; heads stored 128 apart, columns 72..79 zero) takes five of
 // the eight K steps of Q K^T and 80 of the 128 output columns; what the second panels hold beyond that is never read.
-// NSEG: sequences in one launch (the two branches of a guided step: at 296 rows each has 96 work items for 148 SMs).  The
-// first grid0 CTAs belong to the first one.
+// NSEG: sequences in one launch (the two branches of a guided step: at 296 rows each has 96 work items for 148 SMs).
 template <int NSEG>
 struct Attn1Params {
     CUtensorMap q[NSEG], k[NSEG], v[NSEG];
     AttnArgs a[NSEG];
-    int grid0;
 };
+
+// A work unit: a query tile of a head with all the keys it sees, or one of the parts of a tail item.
+struct alignas(16) AttnUnit {
+    int h, q0;       // head (-1: no unit, the CTA is done), first query row
+    int kv_c, kv_r;  // tensor-map coordinates of its first key tile
+    int j0, n;       // first key tile, and how many (0: a part of an item that has fewer key tiles than parts)
+    int slot;        // where a part's results go; -1: a whole item
+    int seg;         // sequence
+};
+// Unit u of a launch.  CTA b takes the units b, b + grid, ...: those that see every key (and the parts) come first, those of causal
+// query tiles, which stop at the diagonal, after them with the longest in front, so that the rounds' sums are even (1280
+// rows, of which 256 causal, 32 heads: at most 22 key tiles for a CTA; in the order of the heads 30).
+template <int NSEG>
+__device__ __forceinline__ AttnUnit unit_at(const Attn1Params<NSEG>& par, int u) {
+    int seg = 0;
+    if (NSEG > 1) {
+        const int l0 = par.a[0].n_long, l1 = par.a[NSEG - 1].n_long, s0 = par.a[0].n_short;
+        if (u >= l0 + l1) {
+            u -= l1;
+            if (u >= l0 + s0) { u += l1 - l0 - s0; seg = 1; }
+        } else if (u >= l0) { u -= l0; seg = 1; }
+    }
+    const AttnArgs& a = par.a[seg];
+    AttnUnit un;
+    un.seg = seg;
+    int qb, part = 0;
+    un.slot = -1;
+    if (u < a.n_full) {
+        un.h = a.by_full.div(u);
+        qb = a.nc + u - un.h * (a.nqb - a.nc);
+    } else if (u < a.n_long) {
+        un.slot = u - a.n_full;
+        const int i = a.by_ways.div(un.slot), item = a.n_plain + i;
+        part = un.slot - i * a.ways;
+        un.h = a.by_nqb.div(item);
+        qb = item - un.h * a.nqb;
+    } else {
+        // hf causal tiles of each number from hr on, one more of each below
+        int v = u - a.n_long, top = a.nc;
+        if (top > a.hr && v >= (top - a.hr) * a.hf) { v -= (top - a.hr) * a.hf; top = a.hr; }
+        const int cnt = a.hf + (top <= a.hr), c = top <= a.hr ? a.by_hf1.div(v) : a.by_hf.div(v);
+        un.h = v - c * cnt;
+        qb = top - 1 - c;
+    }
+    un.q0 = (a.qb0 + qb) * T1_ROWS;
+    // keys this query tile can see
+    int kv_end = a.S;
+    if (un.q0 + T1_ROWS - 1 < a.ar_len) kv_end = un.q0 + T1_ROWS;   // all rows causal: keys <= last row
+    if (kv_end > a.S) kv_end = a.S;
+    const int tiles = (kv_end + AKV - 1) / AKV;
+    un.j0 = 0;
+    un.n = tiles;
+    if (un.slot >= 0) {
+        un.j0 = a.by_ways.div(part * tiles);
+        un.n = a.by_ways.div((part + 1) * tiles) - un.j0;
+    }
+    const int kh = a.by_group.div(un.h);
+    un.kv_c = kh * a.kv_hc;
+    un.kv_r = kh * a.kv_hr + un.j0 * AKV;
+    return un;
+}
+// The end of a unit: the rows of one of its storing warps, O / l -> bf16 -> out[row, h*128 + half*64 ..].  stg: 4 KB of the warp's
+// own, at their beginning the shares of the rows' sums.  A function of its own, called once a unit: inlined, the compiler
+// puts values of the loop over the key tiles into local memory for it.  (It gets no reference to the kernel's parameters: through one they
+// come by loads of some 700 cycles each, one after the other.)
+struct AttnRows {
+    uint16_t* out;               // row 0
+    size_t col;                  // of the head, this half
+    int ldo, r0, row_lo, row_hi; // first row of the warp, rows that are wanted
+    float *part_o, *part_ml;     // a part: where its rows' results go (null: a whole item)
+    const AttnArgs* tab;         // rows that go to a table (null: to `out`)
+};
+template <int DH>
+__device__ __noinline__ void attn_store_rows(const AttnRows w, uint8_t* stg, uint32_t t_o, uint64_t* o_free, uint64_t* q_empty, float m_used,
+                                             int half, bool failed) {
+    const int lane = threadIdx.x & 31;
+    const float* sh = reinterpret_cast<const float*>(stg) + lane;
+    const float lsum = (sh[0] + sh[32]) + (sh[64] + sh[96]);
+    const float inv_l = 1.0f / lsum;
+    // partial result of a key range: accumulator as it is (relative to the max), max and row sum
+    if (w.part_ml && !failed && half == 0) *reinterpret_cast<float2*>(w.part_ml + lane * 2) = make_float2(m_used, lsum);
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        uint32_t o[16];
+        tmem_ld16(t_o + c * 16, o);
+        tmem_ld_wait();
+        if (c == 3) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(o_free);
+        }
+        if (!w.part_o) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                uint4 pk;
+                pk.x = cvt_bf16x2(__uint_as_float(o[i * 8 + 0]) * inv_l, __uint_as_float(o[i * 8 + 1]) * inv_l);
+                pk.y = cvt_bf16x2(__uint_as_float(o[i * 8 + 2]) * inv_l, __uint_as_float(o[i * 8 + 3]) * inv_l);
+                pk.z = cvt_bf16x2(__uint_as_float(o[i * 8 + 4]) * inv_l, __uint_as_float(o[i * 8 + 5]) * inv_l);
+                pk.w = cvt_bf16x2(__uint_as_float(o[i * 8 + 6]) * inv_l, __uint_as_float(o[i * 8 + 7]) * inv_l);
+                *reinterpret_cast<uint4*>(stg + lane * 128 + (((c * 2 + i) ^ (lane & 7)) * 16)) = pk;
+            }
+        } else if (!failed) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<uint4*>(w.part_o + lane * AD + c * 16 + i * 4) = make_uint4(o[i * 4], o[i * 4 + 1], o[i * 4 + 2], o[i * 4 + 3]);
+        }
+    }
+    // The Q tile's place is filled again by a copy, which must not come before what the warp writes there.  (Behind the stores to
+    // global memory the fence would wait for them, some 2000 cycles.)
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (!w.part_o) {
+        // Rows leave as segments of 128 bytes (4 rows per store instruction) instead of 16-byte pieces of 32 rows: they may go to
+        // other GPUs' memory.
+        const int ch = lane & 7;
+#pragma unroll 4
+        for (int k = 0; k < 8; ++k) {
+            const int rr = k * 4 + (lane >> 3), rg = w.r0 + rr;
+            const uint4 v = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((ch ^ (rr & 7)) * 16));
+            if (!failed && half * 64 + ch * 8 < DH && rg < w.row_hi && rg >= w.row_lo) {
+                uint16_t* dst = w.out + (size_t)rg * w.ldo;
+                if (w.tab) {
+                    const int blk = rg / w.tab->out_rows;
+                    dst = w.tab->out_tab[blk] + (size_t)(rg - blk * w.tab->out_rows) * w.ldo;
+                }
+                *reinterpret_cast<uint4*>(dst + w.col + ch * 8) = v;
+            }
+        }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(q_empty);
+}
+
 template <int DH, int NSEG, bool EXACT>
 __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __grid_constant__ Attn1Params<NSEG> par) {
-    const int seg = NSEG > 1 && (int)blockIdx.x >= par.grid0 ? 1 : 0;
-    const AttnArgs& a = par.a[seg];
-    const CUtensorMap &tmQ = par.q[seg], &tmK = par.k[seg], &tmV = par.v[seg];
     constexpr int DN = (DH + 15) & ~15;      // columns the MMAs work on
-    // Q | K x3 | V x3: 7 tiles of 32 KB again, the window 1024-byte aligned (checked below)
+    // Q x2 | K x2 | V x3: 7 tiles of 32 KB again, the window 1024-byte aligned (checked below)
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* q_s = smem;                               // the query tile
-    uint8_t* k_s = q_s + TILE_BYTES;
+    uint8_t* q_s = smem;
+    uint8_t* k_s = q_s + T1_Q_STAGES * TILE_BYTES;
     uint8_t* v_s = k_s + T1_K_STAGES * TILE_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + T1_V_STAGES * TILE_BYTES);
-    uint64_t* q_full = bars;                // 1
-    uint64_t* k_full = bars + 1;            // T1_K_STAGES
+    uint64_t* q_full = bars;                   // T1_Q_STAGES, by unit
+    uint64_t* q_empty = q_full + T1_Q_STAGES;  // T1_Q_STAGES: the unit's score products are done and its rows have left
+    uint64_t* k_full = q_empty + T1_Q_STAGES;  // T1_K_STAGES, by tile
     uint64_t* k_empty = k_full + T1_K_STAGES;
     uint64_t* v_full = k_empty + T1_K_STAGES;  // T1_V_STAGES
     uint64_t* v_empty = v_full + T1_V_STAGES;
     uint64_t* s_full = v_empty + T1_V_STAGES;  // T1_S_BUFS (one per score buffer)
     uint64_t* p_ready = s_full + T1_S_BUFS;    // T1_S_BUFS
     uint64_t* m_pub = p_ready + T1_S_BUFS;     // 2 (one per softmax set)
-    uint64_t* o_done = m_pub + 2;           // 1
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
+    uint64_t* l_full = m_pub + 2;              // 2, by unit: all shares of the row sums are there
+    uint64_t* o_free = l_full + 2;             // 1: the accumulator has been read
+    uint64_t* u_full = o_free + 1;             // T1_UNITS: the unit stands in the table
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(u_full + T1_UNITS);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
-    float* xch = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 192);
+    // The CTA's units as the producer comes to them, the last entry with n = 0.  It is at most three ahead of the unit whose rows
+    // are being stored: it waits for a place for Q.
+    AttnUnit* units = reinterpret_cast<AttnUnit*>(reinterpret_cast<uint8_t*>(bars) + T1_BARS);
+    float* xch = reinterpret_cast<float*>(units + T1_UNITS);
 
     const int warp = warp_index();
     const int lane = threadIdx.x & 31;
-    int item = (int)blockIdx.x - (seg ? par.grid0 : 0), part = 0, ways = 1;
-    if (item >= a.n_plain) {
-        const int t = item - a.n_plain;
-        item = a.n_plain + t / a.ways;
-        part = t - (t / a.ways) * a.ways;
-        ways = a.ways;
-    }
-    const int h = item / a.nqb;
-    const int q0 = (item - h * a.nqb) * T1_ROWS;
-    const int kh = h / (a.heads / a.kv_heads);
-    if (q0 + T1_ROWS <= a.row_lo || q0 >= a.row_hi) { grid_dep_wait(); return; }   // no row of this block is wanted (whole CTA, before any set-up)
+    int* const err = par.a[0].err;
 
-    // keys this query tile can see
-    int kv_end = a.S;
-    if (q0 + T1_ROWS - 1 < a.ar_len) kv_end = q0 + T1_ROWS;   // all rows causal: keys <= last row
-    if (kv_end > a.S) kv_end = a.S;
-    const int tiles_all = (kv_end + AKV - 1) / AKV;
-    const int j0 = (int)((long)part * tiles_all / ways);                  // first key tile of this CTA
-    const int n_tiles = (int)((long)(part + 1) * tiles_all / ways) - j0;  // and how many it covers
-    if (n_tiles <= 0) {
-        // a part of a tail item that has fewer key tiles than parts: an empty partial (max -inf, sum 0), nothing else
-        grid_dep_wait();
-        if (threadIdx.x < T1_ROWS) {
-            const int slot = (item - a.n_plain) * ways + part;
-            *reinterpret_cast<float2*>(a.part_ml + ((size_t)slot * T1_ROWS + threadIdx.x) * 2) = make_float2(-INFINITY, 0.f);
-        }
-        return;
-    }
-
-    // (the error word is on its way while the barriers and tensor memory are set up)
-    if (threadIdx.x == 64) {
-        int ab = error_word(a.err);
-        if (ab == 0 && (smem_u32(smem) & 1023u) != 0) { ab = 20; atomicExch(a.err, 20); }
+    // (the error word and the descriptors are on their way while the barriers and tensor memory are set up)
+    if (threadIdx.x == 96) {
+        int ab = error_word(err);
+        if (ab == 0 && (smem_u32(smem) & 1023u) != 0) { ab = 20; atomicExch(err, 20); }
         *s_abort = ab;
     }
     if (threadIdx.x == 0) {
-        tma_prefetch_desc(&tmQ);
-        tma_prefetch_desc(&tmK);
-        tma_prefetch_desc(&tmV);
-        mbar_init(q_full, 1);
+#pragma unroll
+        for (int i = 0; i < NSEG; ++i) {
+            tma_prefetch_desc(&par.q[i]);
+            tma_prefetch_desc(&par.k[i]);
+            tma_prefetch_desc(&par.v[i]);
+        }
+    }
+    if (threadIdx.x == 64) {
+        for (int s = 0; s < T1_Q_STAGES; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1 + 8); }
         for (int s = 0; s < T1_K_STAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
         for (int s = 0; s < T1_V_STAGES; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
         for (int s = 0; s < T1_S_BUFS; ++s) { mbar_init(&s_full[s], 1); mbar_init(&p_ready[s], 8); }
-        for (int s = 0; s < 2; ++s) mbar_init(&m_pub[s], 8);
-        mbar_init(o_done, 1);
+        for (int s = 0; s < 2; ++s) { mbar_init(&m_pub[s], 8); mbar_init(&l_full[s], 16); }
+        mbar_init(o_free, 8);
+        for (int s = 0; s < T1_UNITS; ++s) mbar_init(&u_full[s], 1);
         fence_mbar_init();
     }
     if (warp == 1) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
     }
+    AttnUnit un;                 // (the producer's first one: known before the kernel in front of this one has ended)
+    if (warp == 0) un = unit_at<NSEG>(par, blockIdx.x);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -632,33 +774,64 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
     if (warp == 0) {
         // -------------------------------------------------------- TMA producer
         if (elect_one()) {
-            mbar_expect_tx(q_full, TILE_BYTES);
-            tma_load_2d(q_s, &tmQ, q_full, h * a.q_hc, h * a.q_hr + q0);
-            tma_load_2d(q_s + PANEL_BYTES, &tmQ, q_full, h * a.q_hc + 64, h * a.q_hr + q0);
-            auto load_k = [&](int j) -> bool {
-                const int st = j % T1_K_STAGES;
-                if (!mbar_wait(&k_empty[st], ((j / T1_K_STAGES) & 1) ^ 1)) { atomicExch(a.err, 11); return false; }
-                mbar_expect_tx(&k_full[st], TILE_BYTES);
-                tma_load_2d(k_s + st * TILE_BYTES, &tmK, &k_full[st], kh * a.kv_hc, kh * a.kv_hr + (j0 + j) * AKV);
-                tma_load_2d(k_s + st * TILE_BYTES + PANEL_BYTES, &tmK, &k_full[st], kh * a.kv_hc + 64,
-                            kh * a.kv_hr + (j0 + j) * AKV);
-                return true;
+            auto tile = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
+                mbar_expect_tx(bar, TILE_BYTES);
+                tma_load_2d(dst, map, bar, c0, c1);
+                tma_load_2d(dst + PANEL_BYTES, map, bar, c0 + 64, c1);
             };
-            auto load_v = [&](int j) -> bool {
-                const int st = j % T1_V_STAGES;
-                if (!mbar_wait(&v_empty[st], ((j / T1_V_STAGES) & 1) ^ 1)) { atomicExch(a.err, 12); return false; }
-                mbar_expect_tx(&v_full[st], TILE_BYTES);
-                tma_load_2d(v_s + st * TILE_BYTES, &tmV, &v_full[st], kh * a.kv_hc, kh * a.kv_hr + (j0 + j) * AKV);
-                tma_load_2d(v_s + st * TILE_BYTES + PANEL_BYTES, &tmV, &v_full[st], kh * a.kv_hc + 64,
-                            kh * a.kv_hr + (j0 + j) * AKV);
-                return true;
-            };
-            // load order follows the consumer: K0 .. K(T1_S_BUFS-1), then per tile V(j), K(j+T1_S_BUFS)
-            bool ok = true;
-            for (int j = 0; j < T1_S_BUFS && j < n_tiles && ok; ++j) ok = load_k(j);
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                ok = load_v(j);
-                if (ok && j + T1_S_BUFS < n_tiles) ok = load_k(j + T1_S_BUFS);
+            int u = blockIdx.x, ki = 0, jk = 0, i = 0;       // K: unit, its number among this CTA's, key tile in it, tile of the stream
+            int vi = 0, jv = 0, vn = 0;
+            bool more = true, first = true;
+            if (un.n > 0) {
+                // (the first two copies by themselves: nothing else to do in front of them)
+                const AttnArgs& a = par.a[NSEG > 1 ? un.seg : 0];
+                tile(q_s, &par.q[NSEG > 1 ? un.seg : 0], &q_full[0], un.h * a.q_hc, un.h * a.q_hr + un.q0);
+                tile(k_s, &par.k[NSEG > 1 ? un.seg : 0], &k_full[0], un.kv_c, un.kv_r);
+                units[0] = un;
+                mbar_arrive(&u_full[0]);
+                first = false;
+                i = 1;
+                if (un.n == 1) ki = 1; else jk = 1;
+            }
+            AttnUnit vun = un;
+            int total = 0;
+            for (int k = 0; k < NSEG; ++k) total += par.a[k].n_long + par.a[k].n_short;
+            // the stream: K0 K1 V0 K2 V1 K3 ..; a unit's first K waits for a place for its Q, and V must not wait with it
+            for (;; ++i) {
+                if (i >= 2) {
+                    const int g = i - 2, st = g % T1_V_STAGES;
+                    if (jv == 0) { vun = units[vi % T1_UNITS]; vn = vun.n; }
+                    if (vn == 0) break;
+                    if (!mbar_wait(&v_empty[st], ((g / T1_V_STAGES) & 1) ^ 1)) { atomicExch(err, 12); break; }
+                    tile(v_s + st * TILE_BYTES, &par.v[NSEG > 1 ? vun.seg : 0], &v_full[st], vun.kv_c, vun.kv_r + jv * AKV);
+                    if (++jv == vn) { jv = 0; ++vi; }
+                }
+                if (!more) continue;
+                if (jk == 0) {
+                    while (true) {
+                        if (!first) {
+                            u += (int)gridDim.x;
+                            if (u < total) un = unit_at<NSEG>(par, u);
+                            else { un.n = 0; un.h = -1; }
+                        }
+                        first = false;
+                        if (un.n > 0 || un.h < 0) break;
+                        // a part of a tail item without key tiles: an empty partial (max -inf, sum 0), nothing else
+                        for (int r = 0; r < T1_ROWS; ++r)
+                            *reinterpret_cast<float2*>(par.a[NSEG > 1 ? un.seg : 0].part_ml + ((size_t)un.slot * T1_ROWS + r) * 2) = make_float2(-INFINITY, 0.f);
+                    }
+                    units[ki % T1_UNITS] = un;
+                    mbar_arrive(&u_full[ki % T1_UNITS]);
+                    if (un.n == 0) { more = false; continue; }
+                    const int st = ki & 1;
+                    if (!mbar_wait(&q_empty[st], ((ki >> 1) & 1) ^ 1)) { atomicExch(err, 10); break; }
+                    const AttnArgs& a = par.a[NSEG > 1 ? un.seg : 0];
+                    tile(q_s + st * TILE_BYTES, &par.q[NSEG > 1 ? un.seg : 0], &q_full[st], un.h * a.q_hc, un.h * a.q_hr + un.q0);
+                }
+                const int st = i % T1_K_STAGES;
+                if (!mbar_wait(&k_empty[st], ((i / T1_K_STAGES) & 1) ^ 1)) { atomicExch(err, 11); break; }
+                tile(k_s + st * TILE_BYTES, &par.k[NSEG > 1 ? un.seg : 0], &k_full[st], un.kv_c, un.kv_r + jk * AKV);
+                if (++jk == un.n) { jk = 0; ++ki; }
             }
         }
     } else if (warp == 1) {
@@ -666,57 +839,65 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         if (elect_one()) {
             constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128, 0, 0);
             constexpr uint32_t idesc_pv = umma_idesc_bf16(128, DN, 0, 1);  // V is MN-major
-            bool ok = mbar_wait(q_full, 0);
-            if (!ok) atomicExch(a.err, 13);
-            const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s), 16, 1024);
-            // S(j) = Q K_j^T into score buffer j % T1_S_BUFS; one descriptor per operand tile, the eight K steps
-            // only move its 16-byte-unit address field
-            auto issue_qk = [&](int j) -> bool {
-                const int st = j % T1_K_STAGES;
-                if (!mbar_wait(&k_full[st], (j / T1_K_STAGES) & 1)) { atomicExch(a.err, 14); return false; }
-                tc_fence_after();
-                const uint64_t k_desc = umma_desc_sw128(smem_u32(k_s + st * TILE_BYTES), 16, 1024);
-                const int b = j % T1_S_BUFS;
+            int gq = 0, qi = 0, jq = 0, qn = 0;      // score products: tile of the stream, unit, tile in it, tiles it has
+            int pi = 0, jp = 0, pn = 0;              // the same of P V
+            bool ok = true, more = true;
+            // Per key tile g: S = Q K^T up to g + T1_S_BUFS - 1, the last of them into the buffer P(g - 1) leaves (MMAs of one
+            // thread execute in issue order), then O += P(g) V_g.  The scores of the next T1_S_BUFS - 1 tiles are already there
+            // or on their way, so the softmax warps never wait for a score product that waits for them.
+            for (int g = 0; ok; ++g) {
+                while (more && gq < g + T1_S_BUFS) {
+                    const int qs = qi & 1, st = gq % T1_K_STAGES, b = gq % T1_S_BUFS;
+                    if (jq == 0) {
+                        // A unit's first product waits for the place for Q of the unit two before it, which is free once that one's
+                        // rows have left, so that one's last P V has to be on its way (units of a single key tile).
+                        if (qi >= pi + 2) break;
+                        if (!mbar_wait(&u_full[qi % T1_UNITS], (qi / T1_UNITS) & 1)) { atomicExch(err, 23); ok = false; break; }
+                        qn = units[qi % T1_UNITS].n;
+                        if (qn == 0) { more = false; break; }
+                        if (!mbar_wait(&q_full[qs], (qi >> 1) & 1)) { atomicExch(err, 13); ok = false; break; }
+                    }
+                    if (!mbar_wait(&k_full[st], (gq / T1_K_STAGES) & 1)) { atomicExch(err, 14); ok = false; break; }
+                    tc_fence_after();
+                    // one descriptor per operand tile, the eight K steps only move its 16-byte-unit address field
+                    const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s + qs * TILE_BYTES), 16, 1024);
+                    const uint64_t k_desc = umma_desc_sw128(smem_u32(k_s + st * TILE_BYTES), 16, 1024);
 #pragma unroll
-                for (int kk = 0; kk < DN / 16; ++kk) {
-                    const uint64_t off = (uint64_t)(((kk >> 2) * PANEL_BYTES + (kk & 3) * 32) >> 4);
-                    umma_ss(tmem_S + b * 128, q_desc + off, k_desc + off, idesc_qk, kk != 0);
+                    for (int kk = 0; kk < DN / 16; ++kk) {
+                        const uint64_t off = (uint64_t)(((kk >> 2) * PANEL_BYTES + (kk & 3) * 32) >> 4);
+                        umma_ss(tmem_S + b * 128, q_desc + off, k_desc + off, idesc_qk, kk != 0);
+                    }
+                    umma_commit(&s_full[b]);
+                    umma_commit(&k_empty[st]);
+                    ++gq;
+                    if (++jq == qn) { umma_commit(&q_empty[qs]); jq = 0; ++qi; }
                 }
-                umma_commit(&s_full[b]);
-                umma_commit(&k_empty[st]);
-                return true;
-            };
-            for (int j = 0; j < T1_S_BUFS && j < n_tiles && ok; ++j) ok = issue_qk(j);
-            // Per key tile j: O += P(j) V_j, then S(j + T1_S_BUFS) = Q K^T into the buffer P(j) leaves (MMAs of one
-            // thread execute in issue order).  The scores of the next T1_S_BUFS - 1 tiles are already there or on
-            // their way, so the softmax warps never wait for a score product that waits for them.
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                const int vst = j % T1_V_STAGES;
-                const int b = j % T1_S_BUFS;
-                if (!mbar_wait(&v_full[vst], (j / T1_V_STAGES) & 1)) { atomicExch(a.err, 15); ok = false; break; }
+                if (!ok) break;
+                const int vst = g % T1_V_STAGES, b = g % T1_S_BUFS;
+                if (jp == 0) {
+                    if (qi == pi && jq == 0) break;      // the stream has ended
+                    pn = units[pi % T1_UNITS].n;
+                    if (pi > 0 && !mbar_wait(o_free, (pi - 1) & 1)) { atomicExch(err, 22); break; }
+                }
+                if (!mbar_wait(&v_full[vst], (g / T1_V_STAGES) & 1)) { atomicExch(err, 15); break; }
                 const uint64_t v_desc = umma_desc_sw128(smem_u32(v_s + vst * TILE_BYTES), PANEL_BYTES, 1024);
-                if (!mbar_wait(&p_ready[b], (j / T1_S_BUFS) & 1)) { atomicExch(a.err, 16); ok = false; break; }
+                if (!mbar_wait(&p_ready[b], (g / T1_S_BUFS) & 1)) { atomicExch(err, 16); break; }
                 tc_fence_after();
                 const uint32_t p_tmem = tmem_S + b * 128;   // bf16 P in the first 64 columns of the buffer
 #pragma unroll
                 for (int kk = 0; kk < AKV / 16; ++kk)       // 16 keys down per step, 128 B per key row
-                    umma_ts(tmem_O, p_tmem + kk * 8, v_desc + (uint64_t)((kk * 16 * 128) >> 4), idesc_pv, (j | kk) != 0);
+                    umma_ts(tmem_O, p_tmem + kk * 8, v_desc + (uint64_t)((kk * 16 * 128) >> 4), idesc_pv, (jp | kk) != 0);
                 umma_commit(&v_empty[vst]);
-                if (j + T1_S_BUFS < n_tiles) ok = issue_qk(j + T1_S_BUFS);
+                if (++jp == pn) { jp = 0; ++pi; }
             }
-            umma_commit(o_done);
         }
     } else {
         // -------------------------------------------------------- softmax sets + output
-        const int set = (warp - 2) >> 3;         // set 0 takes the even key tiles, set 1 the odd ones
-        const int half = ((warp - 2) >> 2) & 1;  // which 64 score columns of the row
-        const int part4 = (warp - 2) >> 2;       // which 32 output columns of the row (epilogue)
+        const int set = (warp - 2) >> 3;         // set 0 takes the stream's even key tiles, set 1 the odd ones
+        const int half = ((warp - 2) >> 2) & 1;  // which 64 score / output columns of the row
         const int qd = warp & 3;                 // TMEM lane quadrant this warp may access
         const int row = qd * 32 + lane;          // row within the query tile
-        const int row_g = q0 + row;              // global query index
         const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
-        const bool tile_has_causal = q0 < a.ar_len;
-        const bool row_causal = row_g < a.ar_len;
         const uint32_t t_o = tmem_O + half * 64 + lane_off;
         // The max of a row's scores in a tile, half a row by each of its two threads, in shared memory.
         // EXACT, [set][half][row]: the two threads read both halves, and so do those of the other set, which follow this set's decision
@@ -727,26 +908,47 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         // sum and O is relative to it) as the unscaled score it came from.  Both threads of a row read the previous tile's
         // entry and one writes this tile's, so the two lie in different places, and all eight warps of a set
         // arrive on m_pub: an entry is not overwritten before it is read.
+        // Each set waits for every tile of the other one, a unit's last one included, so this holds from unit to unit.
         float *x_mine = xch + set * 256 + half * 128 + row, *x_half = xch + set * 256 + (half ^ 1) * 128 + row;
         const float* x_set = xch + (set ^ 1) * 256 + row;
         uint16_t* x16 = reinterpret_cast<uint16_t*>(xch) + set * 512 + row;
         uint16_t* m_sh = reinterpret_cast<uint16_t*>(xch + T1_XCH / 4);
         const int bar_id = 1 + set;              // named barrier of the set's 256 threads
         constexpr int BAR_THREADS = 256;
+        const float scale_log2 = par.a[0].scale_log2;      // (of all sequences)
+        bool ok = true;
+        int g = 0;                               // the unit's first tile in the stream
+        for (int index = 0;; ++index) {
+        const AttnUnit* unit = units + index % T1_UNITS;
+        {
+            // the set goes on to a unit, or stops, as one
+            uint32_t got = mbar_wait(&u_full[index % T1_UNITS], (index / T1_UNITS) & 1);
+            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %0, 0;\n\tbarrier.cta.red.and.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                         : "+r"(got) : "r"(bar_id), "n"(BAR_THREADS) : "memory");
+            if (!got) { atomicExch(err, 24); break; }
+        }
+        const int g_end = g + unit->n;
+        if (g_end == g) break;
+        // last key this row sees, counted from the unit's first key tile
+        int k_last;
+        {
+            const AttnArgs& a = par.a[NSEG > 1 ? unit->seg : 0];
+            const int row_g = unit->q0 + row;
+            k_last = (row_g < a.ar_len && row_g < a.S ? row_g : a.S - 1) - unit->j0 * AKV;
+        }
         float m_mine = -INFINITY;                // max this thread's partial sum is relative to
         uint32_t m_raw = 0xff800000u;            // (not EXACT) the score it came from
         float l = 0.f;                           // this thread's share of the row sum
-        bool ok = true;
-        // the max in force after the other set's tile j: the sum follows where that set raised it
-        auto follow = [&](int j) {
+        // the max in force after the other set's tile gj: the sum follows where that set raised it
+        auto follow = [&](int gj) {
             float m_tile;
             bool raised;
             if constexpr (EXACT) {
-                m_tile = fmaxf(x_set[0], x_set[128]) * a.scale_log2;
+                m_tile = fmaxf(x_set[0], x_set[128]) * scale_log2;
                 raised = (m_tile - m_mine) > 8.0f;
             } else {
-                const uint32_t raw = (uint32_t)m_sh[(j & 1) * T1_ROWS + row] << 16;
-                m_tile = __uint_as_float(raw) * a.scale_log2;
+                const uint32_t raw = (uint32_t)m_sh[(gj & 1) * T1_ROWS + row] << 16;
+                m_tile = __uint_as_float(raw) * scale_log2;
                 raised = raw != m_raw;
                 m_raw = raw;
             }
@@ -755,41 +957,28 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
                 m_mine = m_tile;
             }
         };
-        for (int j = set; j < n_tiles; j += 2) {
-            const int b = j % T1_S_BUFS;
-            const int use = (j >> 1) & 1;
-            const int kv0 = (j0 + j) * AKV + half * 64;
+        for (int gj = g + ((g ^ set) & 1); gj < g_end; gj += 2) {
+            const int b = gj % T1_S_BUFS;
+            const int use = (gj >> 1) & 1;
             const uint32_t t_s = tmem_S + b * 128 + lane_off;
             // A thread whose wait ran out keeps taking part in the set's named barrier (one per tile) and does
             // nothing else, so that no partner is left waiting at a barrier that has no time limit.
             uint32_t r[2][32];
             float mx = -INFINITY;
-            if (ok && !mbar_wait_warp(&s_full[b], (j / T1_S_BUFS) & 1)) { atomicExch(a.err, 17); ok = false; }
+            if (ok && !mbar_wait_warp(&s_full[b], (gj / T1_S_BUFS) & 1)) { atomicExch(err, 17); ok = false; }
             if (ok) {
             tc_fence_after();
-            const bool need_mask = (kv0 + 64 > a.S) || (tile_has_causal && kv0 + 63 > q0);
             // this thread's 64 fp32 scores go to registers with one wait
             tmem_ld32(t_s + half * 64, r[0]);
             tmem_ld32(t_s + half * 64 + 32, r[1]);
             tmem_ld_wait();
-            if (need_mask && kv0 > q0 + 127 && kv0 + 64 <= a.S) {
-                // right of the diagonal for every row of the tile: a causal row sees none of these keys, another row all
-                // (element by element this took 1560 cycles per key tile of such a query tile, now 280 as without a mask)
-                if (row_causal) {
-#pragma unroll
-                    for (int c = 0; c < 2; ++c)
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) r[c][i] = 0xff800000u;
-                }
-            } else if (need_mask) {
+            const int seen = k_last + 1 - ((gj - g) * AKV + half * 64);      // how many of the 64 keys the row sees
+            if (__any_sync(0xffffffffu, seen < 64)) {
 #pragma unroll
                 for (int c = 0; c < 2; ++c)
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int key = kv0 + c * 32 + i;
-                        const bool allow = key < a.S && (!row_causal || key <= row_g);
-                        if (!allow) r[c][i] = 0xff800000u;   // -inf
-                    }
+                    for (int i = 0; i < 32; ++i)
+                        if (c * 32 + i >= seen) r[c][i] = 0xff800000u;   // -inf
             }
             {
                 // three-input max: 64 scores in 32 instructions, four independent chains
@@ -805,7 +994,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
             }
             // Row max over both halves: the partner thread's value comes through shared memory.
             if constexpr (EXACT) {
-                if (j >= 1 && !mbar_wait_warp(&m_pub[set ^ 1], ((j - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; }
+                if (gj > g && !mbar_wait_warp(&m_pub[set ^ 1], ((gj - 1) >> 1) & 1)) { atomicExch(err, 18); ok = false; }
                 if (ok) *x_mine = mx;
             } else {
                 // The reference value only has to be the same for both threads and not below the true max, so it travels as a
@@ -819,11 +1008,11 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
             asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(BAR_THREADS) : "memory");
             if (!ok) continue;
             mx = fmaxf(mx, EXACT ? *x_half : __uint_as_float((uint32_t)x16[use * 256 + (half ^ 1) * 128] << 16));
-            const float m_tile = mx * a.scale_log2;
+            const float m_tile = mx * scale_log2;
             // the max in force after the previous tile, which the other set decided
-            if (j >= 1) {
-                if (!EXACT && !mbar_wait_warp(&m_pub[set ^ 1], ((j - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; continue; }
-                follow(j - 1);
+            if (gj > g) {
+                if (!EXACT && !mbar_wait_warp(&m_pub[set ^ 1], ((gj - 1) >> 1) & 1)) { atomicExch(err, 18); ok = false; continue; }
+                follow(gj - 1);
             }
             const bool grow = (m_tile - m_mine) > 8.0f;      // also true while m_mine == -inf
             float alpha = 1.0f;
@@ -833,13 +1022,13 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
                 m_raw = __float_as_uint(mx);
                 l *= alpha;
             }
-            if (!EXACT && half == 0) m_sh[(j & 1) * T1_ROWS + row] = (uint16_t)(m_raw >> 16);
+            if (!EXACT && half == 0) m_sh[(gj & 1) * T1_ROWS + row] = (uint16_t)(m_raw >> 16);
             __syncwarp();
             if (lane == 0) mbar_arrive(&m_pub[set]);
-            if (j >= 1 && __any_sync(0xffffffffu, grow)) {
-                // O must hold all of PV(j-1) and nothing of PV(j): the first is what v_empty of tile j-1 reports,
+            if (gj > g && __any_sync(0xffffffffu, grow)) {
+                // O must hold all of PV(gj-1) and nothing of PV(gj): the first is what v_empty of tile gj-1 reports,
                 // the second waits for this set's p_ready.  Each thread scales its own 64 output columns.
-                if (!mbar_wait_warp(&v_empty[(j - 1) % T1_V_STAGES], ((j - 1) / T1_V_STAGES) & 1)) { atomicExch(a.err, 21); ok = false; continue; }
+                if (!mbar_wait_warp(&v_empty[(gj - 1) % T1_V_STAGES], ((gj - 1) / T1_V_STAGES) & 1)) { atomicExch(err, 21); ok = false; continue; }
                 tc_fence_after();
 #pragma unroll 1
                 for (int c = 0; c < 4 && half * 64 + c * 16 < DN; ++c) {
@@ -858,83 +1047,48 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
             // in this tile and none before: m is still -inf then and every score is masked; 0 keeps
             // exp2(-inf + 0) = 0 instead of exp2(-inf + inf)
             const float neg_m = (m_mine == -INFINITY) ? 0.f : -m_mine;
-            const uint64_t scale2 = pack_f32x2(a.scale_log2, a.scale_log2), negm2 = pack_f32x2(neg_m, neg_m);
+            const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2), negm2 = pack_f32x2(neg_m, neg_m);
             l += softmax_exp_store(r, scale2, negm2, t_s + half * 32);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_ready[b]);
         }
-        // ---- the sums of the set that did not take the last tile follow its max
-        if (ok && ((n_tiles - 1) & 1) != set) {
-            if (!mbar_wait_warp(&m_pub[set ^ 1], ((n_tiles - 1) >> 1) & 1)) { atomicExch(a.err, 18); ok = false; }
-            if (ok) follow(n_tiles - 1);
+        const int gl = g_end - 1;                // the unit's last tile
+        const bool mine = (gl & 1) == set;       // the set that took it stores the unit's rows
+        g = g_end;
+        // ---- the sums of the other set follow its max
+        if (ok && !mine) {
+            if (!mbar_wait_warp(&m_pub[set ^ 1], (gl >> 1) & 1)) { atomicExch(err, 18); ok = false; }
+            if (ok) follow(gl);
         }
-        // ---- output: O / l -> bf16 -> out[row_g, h*128 + part4*32 ..]
-        if (ok) {
-            const int failed = error_word(a.err);
-            if (!mbar_wait_warp(o_done, 0)) { atomicExch(a.err, 19); ok = false; }
-            tc_fence_after();
-            if (failed) ok = false;
-        }
-        // the row sum is the four threads' shares together (the exchange window as [quarter][row] floats; every
-        // softmax thread reaches these barriers: a failed wait above fails for all of them alike)
-        asm volatile("bar.sync 3, 512;" ::: "memory");
-        xch[part4 * 128 + row] = l;
-        asm volatile("bar.sync 3, 512;" ::: "memory");
-        const float lsum = (xch[row] + xch[128 + row]) + (xch[256 + row] + xch[384 + row]);
-        if (ok) {
-            uint32_t o[32];
-            tmem_ld32(tmem_O + part4 * 32 + lane_off, o);
-            tmem_ld_wait();
-            if (ways > 1) {
-                // partial result of a key range: accumulator as it is (relative to the max), max and row sum
-                const int slot = (item - a.n_plain) * ways + part;
-                float* po = a.part_o + ((size_t)slot * T1_ROWS + row) * AD + part4 * 32;
-                if (part4 == 0) {
-                    float2 ml = make_float2(m_mine, lsum);
-                    *reinterpret_cast<float2*>(a.part_ml + ((size_t)slot * T1_ROWS + row) * 2) = ml;
-                }
+        if (!ok) continue;
+        // The row sum is the four threads' shares together.  They meet in the unit's Q tile, which no MMA reads any more (the scores
+        // of the last tile are there), in the 4 KB that each storing warp has for its rows: [set, half][lane], behind l_full.
+        // The shares of unit i and of unit i + 2 go through the same barrier: before a warp comes to the second it has seen the
+        // other set decide on a tile behind the first.
+        uint8_t* slices = q_s + (index & 1) * TILE_BYTES + qd * 4096;
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    *reinterpret_cast<uint4*>(po + i * 4) = make_uint4(o[i * 4], o[i * 4 + 1], o[i * 4 + 2], o[i * 4 + 3]);
-            } else {
-                const float inv_l = 1.0f / lsum;
-                uint4 pk[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    pk[i].x = cvt_bf16x2(__uint_as_float(o[i * 8 + 0]) * inv_l, __uint_as_float(o[i * 8 + 1]) * inv_l);
-                    pk[i].y = cvt_bf16x2(__uint_as_float(o[i * 8 + 2]) * inv_l, __uint_as_float(o[i * 8 + 3]) * inv_l);
-                    pk[i].z = cvt_bf16x2(__uint_as_float(o[i * 8 + 4]) * inv_l, __uint_as_float(o[i * 8 + 5]) * inv_l);
-                    pk[i].w = cvt_bf16x2(__uint_as_float(o[i * 8 + 6]) * inv_l, __uint_as_float(o[i * 8 + 7]) * inv_l);
-                }
-                if (a.out_rows > 0) {
-                    // Row blocks of the output live in other GPUs' memory: leave as 64-byte row segments (8 rows
-                    // per store instruction) instead of 16-byte pieces of 32 rows.  The staging slice is this
-                    // warp's 2 KB of the Q tile, which no MMA reads any more once o_done has completed.
-                    uint8_t* stg = q_s + (warp - 2) * (32 * 64);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(stg + lane * 64 + ((i ^ (lane & 3)) * 16)) = pk[i];
-                    __syncwarp();
-                    const int ch = lane & 3;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int rr = k * 8 + (lane >> 2);
-                        const uint4 v = *reinterpret_cast<const uint4*>(stg + rr * 64 + ((ch ^ (rr & 3)) * 16));
-                        const int rg = q0 + qd * 32 + rr;
-                        if (rg < a.row_hi && rg >= a.row_lo) {
-                            const int blk = rg / a.out_rows;
-                            uint16_t* dst = a.out_tab[blk] + (size_t)(rg - blk * a.out_rows) * a.ldo + (size_t)h * a.out_hoff +
-                                            part4 * 32 + ch * 8;
-                            *reinterpret_cast<uint4*>(dst) = v;
-                        }
-                    }
-                } else if (row_g < a.row_hi && row_g >= a.row_lo) {
-                    uint4* d4 = reinterpret_cast<uint4*>(a.out + (size_t)row_g * a.ldo + (size_t)h * a.out_hoff + part4 * 32);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (part4 * 32 + i * 8 < DH) d4[i] = pk[i];
-                }
-            }
+        for (int hh = 0; hh < 2; ++hh)
+            *reinterpret_cast<float*>(slices + hh * 4 * 4096 + (set * 2 + half) * 128 + lane * 4) = l;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&l_full[index & 1]);
+        if (!mine) continue;
+        // ---- output: O / l -> bf16 -> out[row, h*128 + half*64 ..]
+        const int failed = error_word(err);
+        // (v_empty of the last tile: its PV is done)
+        if (!mbar_wait_warp(&l_full[index & 1], (index >> 1) & 1) ||
+            !mbar_wait_warp(&v_empty[gl % T1_V_STAGES], (gl / T1_V_STAGES) & 1)) { atomicExch(err, 19); ok = false; continue; }
+        tc_fence_after();
+        const AttnArgs& a = par.a[NSEG > 1 ? unit->seg : 0];
+        AttnRows w;
+        w.out = a.out;
+        w.col = (size_t)unit->h * a.out_hoff + half * 64;
+        w.ldo = a.ldo; w.r0 = unit->q0 + qd * 32; w.row_lo = a.row_lo; w.row_hi = a.row_hi;
+        const size_t prow = (size_t)unit->slot * T1_ROWS + qd * 32;
+        w.part_o = unit->slot >= 0 ? a.part_o + prow * AD + half * 64 : nullptr;
+        w.part_ml = unit->slot >= 0 ? a.part_ml + prow * 2 : nullptr;
+        w.tab = a.out_rows > 0 ? &a : nullptr;
+        attn_store_rows<DH>(w, slices + half * 4 * 4096, tmem_O + half * 64 + lane_off, o_free, &q_empty[index & 1], m_mine, half, failed != 0);
         }
     }
 
@@ -1029,6 +1183,24 @@ static int choose_tail_ways(int total, int nsm, int min_tiles, size_t scratch_by
     return (worth && best_cost < 0.9) ? best : 1;
 }
 
+// The one-tile kernel's work units: those of the plain items, sorted by how many keys they see, and `parts` of the tail items.
+static void set_units(AttnArgs& a, int parts) {
+    int nc = a.ar_len / T1_ROWS - a.qb0;       // query blocks whose rows are all causal
+    nc = nc < 0 ? 0 : (nc > a.nqb ? a.nqb : nc);
+    a.nc = nc;
+    a.hf = a.nqb ? a.n_plain / a.nqb : 0;
+    a.hr = a.n_plain - a.hf * a.nqb;
+    a.n_full = a.hf * (a.nqb - nc) + (a.hr > nc ? a.hr - nc : 0);
+    a.by_full.set(a.nqb - nc > 0 ? a.nqb - nc : 1);
+    a.by_nqb.set(a.nqb > 0 ? a.nqb : 1);
+    a.by_ways.set(a.ways);
+    a.by_hf.set(a.hf > 0 ? a.hf : 1);
+    a.by_hf1.set(a.hf + 1);
+    a.by_group.set(a.heads / a.kv_heads);
+    a.n_long = a.n_full + parts;
+    a.n_short = a.n_plain - a.n_full;
+}
+
 // One sequence, ready to launch.
 struct AttnSetup {
     CUtensorMap q, k, v;
@@ -1085,6 +1257,12 @@ static bool attention_setup(AttnSetup& s, const void* q, int ldq, const void* k,
     for (int i = 0; i < 8; ++i) a.out_tab[i] = nullptr;
     if (out_tab) for (int i = 0; i < (S + out_rows - 1) / out_rows; ++i) a.out_tab[i] = (uint16_t*)out_tab[i];
     a.nqb = (S + rows_item - 1) / rows_item;
+    a.qb0 = 0;
+    if (one_tile) {       // (the two-tile kernel leaves query blocks out on the device)
+        a.qb0 = a.row_lo / rows_item;
+        a.nqb = (a.row_hi + rows_item - 1) / rows_item - a.qb0;
+        if (a.row_hi <= a.row_lo) a.nqb = 0;
+    }
     const int total = a.nqb * heads;
     a.n_plain = total; a.ways = 1; a.part_o = nullptr; a.part_ml = nullptr;
     int n_tail = 0;
@@ -1112,6 +1290,7 @@ static bool attention_setup(AttnSetup& s, const void* q, int ldq, const void* k,
         }
     }
     s.grid = a.n_plain + n_tail * a.ways;
+    set_units(a, n_tail * a.ways);
     s.n_tail = n_tail; s.rows_item = rows_item; s.one_tile = one_tile;
     // QK^T + PV over the keys each row can see: 4*heads*128*(ar(ar+1)/2 + (S-ar)*S)
     s.work = 4.0 * heads * 128.0 * (0.5 * ar_len * (ar_len + 1.0) + (double)(S - ar_len) * S);
@@ -1134,7 +1313,8 @@ static bool launch_one_tile(const AttnSetup* s, cudaStream_t st) {
         p.q[i] = s[i].q; p.k[i] = s[i].k; p.v[i] = s[i].v; p.a[i] = s[i].a;
         grid += s[i].grid;
     }
-    p.grid0 = s[0].grid;
+    if (grid == 0) return true;       // an empty range of rows
+    if (grid > sm_count()) grid = sm_count();
     return launched(launch_chained(kern, dim3(grid), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p));
 }
 static bool launch_two_tile(const AttnSetup& s, cudaStream_t st) {
@@ -1181,9 +1361,10 @@ bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cuda
     a.err = device_error_word();
     a.nqb = (S + T1_ROWS - 1) / T1_ROWS;
     a.n_plain = a.nqb * H; a.ways = 1;
-    p.grid0 = a.n_plain;
+    set_units(a, 0);
+    const int grid = a.n_plain < sm_count() ? a.n_plain : sm_count();
     prof_before(PROF_ATTN, 4.0 * H * DH * (double)S * S, st);
-    cudaError_t e = launch_chained(kern, dim3(a.n_plain), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p);
+    cudaError_t e = launch_chained(kern, dim3(grid), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("attention (vision): launch: %s", cudaGetErrorString(e)); return false; }

@@ -326,3 +326,36 @@ def test_attention_after_a_late_failure_stores_nothing(pkg, dev, mode):
         torch.cuda.synchronize()
         pkg.lib.o1_device_error()
         pkg.lib.o1_attention_tile_mode(0)
+
+
+@pytest.mark.parametrize("S,H,KV,ar", [(100, 600, 200, 0), (100, 450, 150, 100), (256, 320, 80, 256), (384, 200, 50, 130),
+                                       (300, 240, 60, 300), (513, 120, 30, 260), (640, 149, 149, 127)])
+def test_many_items_for_each_cta(pkg, orc, dev, S, H, KV, ar):
+    """A CTA of the one-tile kernel takes several items in one stream of key tiles: items of one and two key tiles (the next
+    one's query tile, score products and accumulator have to wait for the one before), odd and even numbers of tiles, causal items behind
+    those that see every key.  Against the oracle (class D), twice for the same bits, and in halves of the heads: an item's
+    result does not depend on what its CTA did before."""
+    ld = (H + 2 * KV) * 128
+    qkv = seeded_bf16((S, ld), 53, 0.0, 1.5)
+    d = u16_to_torch(qkv, dev)
+
+    def run(h0, n):
+        out = torch.zeros(S, n * 128, dtype=torch.bfloat16, device=dev)
+        kv0, kvn = h0 // (H // KV), max(1, n // (H // KV))
+        rc = pkg.lib.o1_flash_attention(C.c_void_p(d.data_ptr() + h0 * 256), ld, C.c_void_p(d.data_ptr() + (H + kv0) * 256), ld,
+                                        C.c_void_p(d.data_ptr() + (H + KV + kv0) * 256), ld, pkg.ptr(out), n * 128, S, n, kvn, ar,
+                                        128 ** -0.5)
+        assert rc == 0, pkg.last_error()
+        torch.cuda.synchronize()
+        return out
+
+    out = run(0, H)
+    ref = np.zeros((S, H * 128), dtype=np.uint16)
+    orc.orc_attention_rows(np_ptr(qkv), ld, np_ptr(qkv[:, H * 128:]), ld, np_ptr(qkv[:, (H + KV) * 128:]), ld,
+                           np_ptr(ref), H * 128, H, KV, S, 128, 128 ** -0.5, ar, None, 0)
+    assert_close(torch_to_u16(out), ref, "D", "items in a stream")
+    assert torch.equal(out.view(torch.int16), run(0, H).view(torch.int16))
+    g = H // KV
+    for h0, n in [(0, g), (H - g, g), (H // 2 // g * g, (H // 3 // g + 1) * g)]:
+        part = run(h0, n)
+        assert torch.equal(part.view(torch.int16), out[:, h0 * 128:(h0 + n) * 128].contiguous().view(torch.int16)), (h0, n)
