@@ -78,6 +78,7 @@ struct AttnArgs {
     // One-tile kernel (unit_at()): query blocks [qb0, qb0 + nqb), the first nc of them all causal; n_full of the plain items see every
     // key, n_long work units with the parts of the tail, and n_short causal items.
     int qb0, nc, n_full, n_long, n_short;
+    int out_copy;       // all rows go to `out`: they leave through a tensor map
     int hf, hr;         // the plain items are hf whole heads and the first hr query blocks of another
     FastDiv by_full, by_nqb, by_ways, by_hf, by_hf1, by_group;    // nqb - nc, nqb, ways, hf, hf + 1, query heads per key head
     float* part_o;      // [slot][rows of an item][128] fp32, slot = (item - n_plain) * ways + part
@@ -528,11 +529,13 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // A CTA stays on its SM and takes one work unit after the other (unit_at()): the key tiles of its units are ONE stream, counted by g,
 // that copies, score products and softmax sets run through without a stop.  The next unit's Q, K and first three score products are
 // there before this one's last PV, the set that did not take the last key tile goes on with the next unit at once, and the other one
-// normalises and stores this unit's rows under it.  What stays between two units is the accumulator, which PV of the
-// next one may only overwrite once it has been read.  With a CTA for each item (barriers, tensor memory, first copies and the way out
-// for each) / with units in a stream, 32 / 8 heads, us: 592 rows 18.8 / 16.0, 1280 rows 39.2 / 34.2, 3157 rows 157 / 148, 4352 rows
-// 302 / 290, 16640 rows 3821 / 3781 (power cap), all rows causal 1280 rows 29.7 / 22.4, 3157 rows 118 / 95; the tower's 16 heads of
-// 72 at 4096 patches 118 / 107; one unit for each CTA (200 rows) 7.5 / 7.4.  The same bits.
+// leaves this unit's rows in its Q tile, from where another warp takes them to memory.  What stays between two units is the
+// accumulator, which PV of the next one may only overwrite once it has been read.
+// A CTA for each item (barriers, tensor memory, first copies and the way out for each) / units in a stream, 32 / 8 heads, us: 592
+// rows 18.8 / 14.9, 1280 rows 39.2 / 31.9, 3157 rows 175 / 152, 8000 rows 960 / 852, 16640 rows 3853 / 3721 (power cap), all rows
+// causal 1280 rows 29.6 / 20.5, 3157 rows 115 / 88; the tower's 16 heads of 72 at 4096 patches 124 / 107; one unit for each CTA (200
+// rows) 6.5 / 6.5.  The same bits.  A key tile takes 1340 to 1410 cycles (1560 before), 1250 of which shared memory needs for the
+// operands (160 KB: Q and K 64, V 32, the copies 64); storing the rows by the set itself cost 2 to 5 % of these times.
 // EXACT: the reference max is a row's exact score, as in the two-tile kernel, so that P of that key is exactly 1; from T1_EXACT_ROWS
 // rows on, where that kernel used to run.  Else the max is rounded up to bf16 (half the exchange): the error against 64 bits is 6 %
 // larger (16640 rows 2.20e-3 against 2.06e-3, alike from 592 rows on).  The time is the same, 600 to 4500 rows 1 % longer; shorter
@@ -540,6 +543,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // what they have always been.
 // Measured against the two-tile kernel: see attention_tile_mode().
 static constexpr int T1_ROWS = 128;       // query rows per work item
+static constexpr int T1_THREADS = ATTN_THREADS + 32;    // (and the store warp)
 static constexpr int T1_Q_STAGES = 2;
 static constexpr int T1_K_STAGES = 2;
 static constexpr int T1_V_STAGES = 3;
@@ -560,7 +564,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
 // NSEG: sequences in one launch (the two branches of a guided step: at 296 rows each has 96 work items for 148 SMs).
 template <int NSEG>
 struct Attn1Params {
-    CUtensorMap q[NSEG], k[NSEG], v[NSEG];
+    CUtensorMap q[NSEG], k[NSEG], v[NSEG], o[NSEG];
     AttnArgs a[NSEG];
 };
 
@@ -624,26 +628,18 @@ __device__ __forceinline__ AttnUnit unit_at(const Attn1Params<NSEG>& par, int u)
     un.kv_r = kh * a.kv_hr + un.j0 * AKV;
     return un;
 }
-// The end of a unit: the rows of one of its storing warps, O / l -> bf16 -> out[row, h*128 + half*64 ..].  stg: 4 KB of the warp's
-// own, at their beginning the shares of the rows' sums.  A function of its own, called once a unit: inlined, the compiler
-// puts values of the loop over the key tiles into local memory for it.  (It gets no reference to the kernel's parameters: through one they
-// come by loads of some 700 cycles each, one after the other.)
-struct AttnRows {
-    uint16_t* out;               // row 0
-    size_t col;                  // of the head, this half
-    int ldo, r0, row_lo, row_hi; // first row of the warp, rows that are wanted
-    float *part_o, *part_ml;     // a part: where its rows' results go (null: a whole item)
-    const AttnArgs* tab;         // rows that go to a table (null: to `out`)
-};
-template <int DH>
-__device__ __noinline__ void attn_store_rows(const AttnRows w, uint8_t* stg, uint32_t t_o, uint64_t* o_free, uint64_t* q_empty, float m_used,
-                                             int half, bool failed) {
+// The end of a unit: the rows of one of its warps, O / l -> bf16 -> the unit's Q tile, from where the store warp takes them (a part's
+// results go out from here).  stg: 4 KB of the warp's own (32 rows of half a head, 128-byte swizzle), at their beginning the shares
+// of the rows' sums.  (16 columns at a time: with 32 the compiler puts values of the loop over the key tiles into local memory, and
+// with all but a few KB of the SM's memory taken by tiles that made the whole kernel 1.5 times as slow.)
+__device__ __forceinline__ void attn_stage_rows(uint8_t* stg, uint32_t t_o, uint64_t* o_free, uint64_t* o_staged, float m_used, float* part_o,
+                                             float* part_ml /* of the warp's first row; null: a whole item, or not wanted */, bool whole) {
     const int lane = threadIdx.x & 31;
     const float* sh = reinterpret_cast<const float*>(stg) + lane;
     const float lsum = (sh[0] + sh[32]) + (sh[64] + sh[96]);
     const float inv_l = 1.0f / lsum;
     // partial result of a key range: accumulator as it is (relative to the max), max and row sum
-    if (w.part_ml && !failed && half == 0) *reinterpret_cast<float2*>(w.part_ml + lane * 2) = make_float2(m_used, lsum);
+    if (part_ml) *reinterpret_cast<float2*>(part_ml + lane * 2) = make_float2(m_used, lsum);
 #pragma unroll 1
     for (int c = 0; c < 4; ++c) {
         uint32_t o[16];
@@ -654,7 +650,7 @@ __device__ __noinline__ void attn_store_rows(const AttnRows w, uint8_t* stg, uin
             __syncwarp();
             if (lane == 0) mbar_arrive(o_free);
         }
-        if (!w.part_o) {
+        if (whole) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 uint4 pk;
@@ -664,40 +660,20 @@ __device__ __noinline__ void attn_store_rows(const AttnRows w, uint8_t* stg, uin
                 pk.w = cvt_bf16x2(__uint_as_float(o[i * 8 + 6]) * inv_l, __uint_as_float(o[i * 8 + 7]) * inv_l);
                 *reinterpret_cast<uint4*>(stg + lane * 128 + (((c * 2 + i) ^ (lane & 7)) * 16)) = pk;
             }
-        } else if (!failed) {
+        } else if (part_o) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                *reinterpret_cast<uint4*>(w.part_o + lane * AD + c * 16 + i * 4) = make_uint4(o[i * 4], o[i * 4 + 1], o[i * 4 + 2], o[i * 4 + 3]);
+                *reinterpret_cast<uint4*>(part_o + lane * AD + c * 16 + i * 4) = make_uint4(o[i * 4], o[i * 4 + 1], o[i * 4 + 2], o[i * 4 + 3]);
         }
     }
-    // The Q tile's place is filled again by a copy, which must not come before what the warp writes there.  (Behind the stores to
-    // global memory the fence would wait for them, some 2000 cycles.)
+    // (for the copy that takes the rows out, and the one that fills the place again)
     fence_proxy_async_smem();
     __syncwarp();
-    if (!w.part_o) {
-        // Rows leave as segments of 128 bytes (4 rows per store instruction) instead of 16-byte pieces of 32 rows: they may go to
-        // other GPUs' memory.
-        const int ch = lane & 7;
-#pragma unroll 4
-        for (int k = 0; k < 8; ++k) {
-            const int rr = k * 4 + (lane >> 3), rg = w.r0 + rr;
-            const uint4 v = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((ch ^ (rr & 7)) * 16));
-            if (!failed && half * 64 + ch * 8 < DH && rg < w.row_hi && rg >= w.row_lo) {
-                uint16_t* dst = w.out + (size_t)rg * w.ldo;
-                if (w.tab) {
-                    const int blk = rg / w.tab->out_rows;
-                    dst = w.tab->out_tab[blk] + (size_t)(rg - blk * w.tab->out_rows) * w.ldo;
-                }
-                *reinterpret_cast<uint4*>(dst + w.col + ch * 8) = v;
-            }
-        }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(q_empty);
+    if (lane == 0) mbar_arrive(o_staged);
 }
 
 template <int DH, int NSEG, bool EXACT>
-__global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __grid_constant__ Attn1Params<NSEG> par) {
+__global__ void __launch_bounds__(T1_THREADS, 1) flash_attn1_kernel(const __grid_constant__ Attn1Params<NSEG> par) {
     constexpr int DN = (DH + 15) & ~15;      // columns the MMAs work on
     // Q x2 | K x2 | V x3: 7 tiles of 32 KB again, the window 1024-byte aligned (checked below)
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -717,7 +693,8 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
     uint64_t* l_full = m_pub + 2;              // 2, by unit: all shares of the row sums are there
     uint64_t* o_free = l_full + 2;             // 1: the accumulator has been read
     uint64_t* u_full = o_free + 1;             // T1_UNITS: the unit stands in the table
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(u_full + T1_UNITS);
+    uint64_t* o_staged = u_full + T1_UNITS;    // 2, by unit: its rows lie in its Q tile
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_staged + 2);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     // The CTA's units as the producer comes to them, the last entry with n = 0.  It is at most three ahead of the unit whose rows
     // are being stored: it waits for a place for Q.
@@ -740,14 +717,15 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
             tma_prefetch_desc(&par.q[i]);
             tma_prefetch_desc(&par.k[i]);
             tma_prefetch_desc(&par.v[i]);
+            if (par.a[i].out_copy) tma_prefetch_desc(&par.o[i]);
         }
     }
     if (threadIdx.x == 64) {
-        for (int s = 0; s < T1_Q_STAGES; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1 + 8); }
+        for (int s = 0; s < T1_Q_STAGES; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 2); }
         for (int s = 0; s < T1_K_STAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
         for (int s = 0; s < T1_V_STAGES; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
         for (int s = 0; s < T1_S_BUFS; ++s) { mbar_init(&s_full[s], 1); mbar_init(&p_ready[s], 8); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&m_pub[s], 8); mbar_init(&l_full[s], 16); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&m_pub[s], 8); mbar_init(&l_full[s], 16); mbar_init(&o_staged[s], 8); }
         mbar_init(o_free, 8);
         for (int s = 0; s < T1_UNITS; ++s) mbar_init(&u_full[s], 1);
         fence_mbar_init();
@@ -891,6 +869,46 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
                 if (++jp == pn) { jp = 0; ++pi; }
             }
         }
+    } else if (warp == T1_THREADS / 32 - 1) {
+        // -------------------------------------------------------- store warp
+        // The unit's rows leave its Q tile: as one copy for each half of the head, or, where a range of rows is wanted or they go to
+        // other GPUs' memory, as segments of 128 bytes (4 rows per store instruction).
+        for (int index = 0;; ++index) {
+            if (!mbar_wait_warp(&u_full[index % T1_UNITS], (index / T1_UNITS) & 1)) { atomicExch(err, 25); break; }
+            const AttnUnit w = units[index % T1_UNITS];
+            if (w.n == 0) break;
+            const int failed = error_word(err);
+            if (!mbar_wait_warp(&o_staged[index & 1], (index >> 1) & 1)) { atomicExch(err, 26); break; }
+            const AttnArgs& a = par.a[NSEG > 1 ? w.seg : 0];
+            const uint8_t* rows_s = q_s + (index & 1) * TILE_BYTES;
+            if (w.slot < 0 && !failed) {
+                if (a.out_copy) {
+                    if (elect_one()) {
+                        tma_store_3d(&par.o[NSEG > 1 ? w.seg : 0], rows_s, 0, w.q0, w.h);
+                        tma_store_3d(&par.o[NSEG > 1 ? w.seg : 0], rows_s + PANEL_BYTES, 64, w.q0, w.h);
+                        bulk_commit();
+                        bulk_wait_read();
+                    }
+                } else {
+                    const int ch = lane & 7;
+                    for (int k = lane >> 3; k < 2 * T1_ROWS; k += 4) {
+                        const int hf = k / T1_ROWS, rr = k - hf * T1_ROWS, rg = w.q0 + rr;
+                        const uint4 v = *reinterpret_cast<const uint4*>(rows_s + hf * PANEL_BYTES + rr * 128 + ((ch ^ (rr & 7)) * 16));
+                        if (hf * 64 + ch * 8 < DH && rg < a.row_hi && rg >= a.row_lo) {
+                            uint16_t* dst = a.out + (size_t)rg * a.ldo;
+                            if (a.out_rows > 0) {
+                                const int blk = rg / a.out_rows;
+                                dst = a.out_tab[blk] + (size_t)(rg - blk * a.out_rows) * a.ldo;
+                            }
+                            *reinterpret_cast<uint4*>(dst + (size_t)w.h * a.out_hoff + hf * 64 + ch * 8) = v;
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&q_empty[index & 1]);
+        }
+        bulk_wait_all();
     } else {
         // -------------------------------------------------------- softmax sets + output
         const int set = (warp - 2) >> 3;         // set 0 takes the stream's even key tiles, set 1 the odd ones
@@ -1079,16 +1097,12 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) flash_attn1_kernel(const __gr
         if (!mbar_wait_warp(&l_full[index & 1], (index >> 1) & 1) ||
             !mbar_wait_warp(&v_empty[gl % T1_V_STAGES], (gl / T1_V_STAGES) & 1)) { atomicExch(err, 19); ok = false; continue; }
         tc_fence_after();
+        const int slot = unit->slot;
         const AttnArgs& a = par.a[NSEG > 1 ? unit->seg : 0];
-        AttnRows w;
-        w.out = a.out;
-        w.col = (size_t)unit->h * a.out_hoff + half * 64;
-        w.ldo = a.ldo; w.r0 = unit->q0 + qd * 32; w.row_lo = a.row_lo; w.row_hi = a.row_hi;
-        const size_t prow = (size_t)unit->slot * T1_ROWS + qd * 32;
-        w.part_o = unit->slot >= 0 ? a.part_o + prow * AD + half * 64 : nullptr;
-        w.part_ml = unit->slot >= 0 ? a.part_ml + prow * 2 : nullptr;
-        w.tab = a.out_rows > 0 ? &a : nullptr;
-        attn_store_rows<DH>(w, slices + half * 4 * 4096, tmem_O + half * 64 + lane_off, o_free, &q_empty[index & 1], m_mine, half, failed != 0);
+        const size_t prow = (size_t)slot * T1_ROWS + qd * 32;
+        attn_stage_rows(slices + half * 4 * 4096, tmem_O + half * 64 + lane_off, o_free, &o_staged[index & 1], m_mine,
+                        slot >= 0 && !failed ? a.part_o + prow * AD + half * 64 : nullptr,
+                        slot >= 0 && !failed && half == 0 ? a.part_ml + prow * 2 : nullptr, slot < 0);
         }
     }
 
@@ -1203,7 +1217,7 @@ static void set_units(AttnArgs& a, int parts) {
 
 // One sequence, ready to launch.
 struct AttnSetup {
-    CUtensorMap q, k, v;
+    CUtensorMap q, k, v, o;
     AttnArgs a;
     int grid, n_tail, rows_item;
     bool one_tile;
@@ -1289,6 +1303,8 @@ static bool attention_setup(AttnSetup& s, const void* q, int ldq, const void* k,
             a.part_ml = a.part_o + (size_t)rem * w * rows_item * AD;
         }
     }
+    a.out_copy = one_tile && !out_tab && a.row_lo == 0 && a.row_hi == S;
+    if (a.out_copy && !cached_tmap_heads(&s.o, out, AD, S, heads, a.ldo, a.out_hoff, T1_ROWS)) return false;
     s.grid = a.n_plain + n_tail * a.ways;
     set_units(a, n_tail * a.ways);
     s.n_tail = n_tail; s.rows_item = rows_item; s.one_tile = one_tile;
@@ -1310,12 +1326,12 @@ static bool launch_one_tile(const AttnSetup* s, cudaStream_t st) {
     Attn1Params<NSEG> p;
     int grid = 0;
     for (int i = 0; i < NSEG; ++i) {
-        p.q[i] = s[i].q; p.k[i] = s[i].k; p.v[i] = s[i].v; p.a[i] = s[i].a;
+        p.q[i] = s[i].q; p.k[i] = s[i].k; p.v[i] = s[i].v; p.o[i] = s[i].o; p.a[i] = s[i].a;
         grid += s[i].grid;
     }
     if (grid == 0) return true;       // an empty range of rows
     if (grid > sm_count()) grid = sm_count();
-    return launched(launch_chained(kern, dim3(grid), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p));
+    return launched(launch_chained(kern, dim3(grid), dim3(T1_THREADS), T1_SMEM, st, 1, p.a[0].S, p));
 }
 static bool launch_two_tile(const AttnSetup& s, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
@@ -1361,10 +1377,12 @@ bool flash_attention_vision(const void* qkv, void* out, int S, float scale, cuda
     a.err = device_error_word();
     a.nqb = (S + T1_ROWS - 1) / T1_ROWS;
     a.n_plain = a.nqb * H; a.ways = 1;
+    a.out_copy = 1;
+    if (!cached_tmap_heads(&p.o[0], out, DH, S, H, a.ldo, DH, T1_ROWS)) return false;
     set_units(a, 0);
     const int grid = a.n_plain < sm_count() ? a.n_plain : sm_count();
     prof_before(PROF_ATTN, 4.0 * H * DH * (double)S * S, st);
-    cudaError_t e = launch_chained(kern, dim3(grid), dim3(ATTN_THREADS), T1_SMEM, st, 1, p.a[0].S, p);
+    cudaError_t e = launch_chained(kern, dim3(grid), dim3(T1_THREADS), T1_SMEM, st, 1, p.a[0].S, p);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("attention (vision): launch: %s", cudaGetErrorString(e)); return false; }

@@ -1288,28 +1288,51 @@ bool make_tmap_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
     return true;
 }
 
+// [heads][rows][cols] with pitches ld and hoff (elements), boxes of 64 columns x box_rows rows of one head, same swizzle: rows and columns
+// of a box that a head does not have are left out of a store
+static bool make_tmap_heads(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t heads, uint64_t ld, uint64_t hoff,
+                            uint32_t box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) { set_error("tensor map: cuTensorMapEncodeTiled entry point unavailable"); return false; }
+    if ((((uintptr_t)base) & 15) || ((ld * 2) & 15) || ((hoff * 2) & 15)) { set_error("tensor map: base/pitch not 16-byte aligned"); return false; }
+    cuuint64_t dims[3] = {cols, rows, heads};
+    cuuint64_t strides[2] = {ld * 2, hoff * 2};
+    cuuint32_t box[3] = {64, box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { set_error("tensor map: encode failed (%d)", (int)r); return false; }
+    return true;
+}
+
 struct TmapKey {
-    const void* p; uint64_t rows, cols, ld; uint32_t box;
+    const void* p; uint64_t rows, cols, ld, heads, hoff; uint32_t box;     // heads == 0: a plain matrix
     bool operator<(const TmapKey& o) const {
-        return std::tie(p, rows, cols, ld, box) < std::tie(o.p, o.rows, o.cols, o.ld, o.box);
+        return std::tie(p, rows, cols, ld, heads, hoff, box) < std::tie(o.p, o.rows, o.cols, o.ld, o.heads, o.hoff, o.box);
     }
 };
 // Encoding a tensor map costs a few microseconds on the host; weights and
 // workspace buffers repeat every block and step, so cache by (ptr, shape).
 // The map is copied out under the lock: the cache may be emptied by a later
 // call (or another thread) while the caller still holds its copy.
-bool cached_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                 uint32_t box_rows) {
+static bool cached(CUtensorMap* out, const TmapKey& k) {
     static std::map<TmapKey, CUtensorMap> cache;
     static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
-    TmapKey k{base, rows, cols, ld, box_rows};
     auto it = cache.find(k);
     if (it != cache.end()) { *out = it->second; return true; }
     if (cache.size() > 8192) cache.clear();
-    if (!make_tmap_bf16(out, base, rows, cols, ld, box_rows)) return false;
+    if (!(k.heads ? make_tmap_heads(out, k.p, k.cols, k.rows, k.heads, k.ld, k.hoff, k.box) : make_tmap_bf16(out, k.p, k.rows, k.cols, k.ld, k.box)))
+        return false;
     cache.emplace(k, *out);
     return true;
+}
+bool cached_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
+    return cached(out, TmapKey{base, rows, cols, ld, 0, 0, box_rows});
+}
+bool cached_tmap_heads(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t heads, uint64_t ld, uint64_t hoff,
+                       uint32_t box_rows) {
+    return cached(out, TmapKey{base, rows, cols, ld, heads, hoff, box_rows});
 }
 
 // cudaFuncSetAttribute is per device: remember, per kernel instantiation, on which devices it was done.

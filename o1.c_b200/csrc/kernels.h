@@ -66,6 +66,9 @@ bool gemm_vision_qkv(const void* x, const void* w, const void* b, void* y, int M
 // copies the (cached) tensor map of a row-major bf16 matrix into *out; false + error text on failure
 bool cached_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                  uint32_t box_rows);
+// the same of [heads][rows][cols], pitches ld and hoff elements, boxes of 64 columns x box_rows rows of one head
+bool cached_tmap_heads(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t heads, uint64_t ld, uint64_t hoff,
+                       uint32_t box_rows);
 // encodes the tensor map of a row-major bf16 matrix [rows, cols], pitch ld elements: boxes of 64 columns x box_rows rows
 bool make_tmap_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
 // sets a kernel's dynamic shared-memory limit once per device (`done`: one bit per device ordinal)
