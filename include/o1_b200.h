@@ -473,7 +473,8 @@ int64_t o1_launch_count(int reset);
 int o1_gemm(const void *x, int ldx, const void *w, const void *w2, void *y, int ldy, int M, int N,
             int K, int epi, const void *bias, const void *resid, int ldr, float scale, int force_bn);
 /* The form o1_gemm gives a problem on the current device (no launch): 0 = a warp per column (*width: rows that share it), 1 =
- * one CTA per tile of 128 rows x *width columns, 2 = two CTAs per 256 x 256 tile, 3 = one CTA per tile of a *width fitted to
+ * one CTA per tile of 128 rows x *width columns, 2 = two CTAs per 256 x 256 tile (SwiGLU from K = 2048 on also per 256 weight
+ * rows x 64 to 256 rows of x, as many as fit their number), 3 = one CTA per tile of a *width fitted to
  * the number of SMs, 4 = the kernel for few tiles of *width columns, *ctas of a cluster sharing the K of each; -1 = not
  * supported.  1 and 3 with *ctas = 2: a CTA pair per tile of 256 rows.  force_bn -1 (which o1_gemm takes too): as 0, and K may
  * be shared; -2 (the vision tower's linears): as -1, and a pair tile of 96 to 256 columns from 257 rows on where K >= 2048 (in
@@ -506,7 +507,8 @@ void o1_attention_tail_ways(int ways);
 void o1_attention_tile_mode(int mode);
 /* Clusters of CTAs in the GEMMs: 1 (default, as is every value but 0; environment O1_GEMM_PAIR=0 turns them off) = where that
  * needs the fewest rounds of tiles, two CTAs per tile of 256 rows with cta_group::2 MMAs, each CTA holding 128 rows of A and
- * of the accumulator and half of the B tile: 256 columns in the plain, bias, residual, SwiGLU and grouped q|k|v families, 96
+ * of the accumulator and half of the B tile: 256 columns in the plain, bias, residual, SwiGLU and grouped q|k|v families (in
+ * the last two also 256 weight rows by a fitted number of rows), 96
  * to 256 (see o1_gemm_form) in every epilogue of one weight matrix but the per-head norm and LoRA; and a
  * linear of the vision tower that has few tiles shares the K of a tile among up to six CTAs. 0 = always one CTA per tile, no
  * cluster is launched.  The pairs add a row's K products in the order of single CTAs: same bits.  The shared K is another

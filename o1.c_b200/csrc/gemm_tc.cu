@@ -211,18 +211,15 @@ struct PlainEpilogue {
 // SwiGLU of 32 columns: bf16(silu(g)) * u with silu(g) = g * (1 / (1 + e^-g)).  The quotient is the IEEE one, by Markstein's step from
 // the approximate reciprocal (P. Markstein, IBM J. Res. Dev. 34, 1990); the division itself, which branches for each value, is left
 // to warps that hold a gate below -80, where 1 + e^-g comes near the largest number, or a NaN.
-__device__ __forceinline__ void swiglu_all(const uint32_t (&rg)[32], const uint32_t (&ru)[32], float (&v)[32]) {
+template <int N>       // v: gates, then results; u: what they multiply; all of them bf16 values, results to be rounded by the caller
+__device__ __forceinline__ void swiglu_vals(float (&v)[N], const float (&u)[N]) {
     bool plain = true;
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-        v[j] = __uint_as_float(rg[j]); v[j + 1] = __uint_as_float(rg[j + 1]);
-        bf16_round2(v[j], v[j + 1]);
-        plain = plain && fminf(v[j], v[j + 1]) > -80.f && v[j] == v[j] && v[j + 1] == v[j + 1];
-    }
+    for (int j = 0; j < N; j += 2) plain = plain && fminf(v[j], v[j + 1]) > -80.f && v[j] == v[j] && v[j + 1] == v[j + 1];
     if (__all_sync(0xffffffffu, plain)) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-            float s[2], u[2] = {__uint_as_float(ru[j]), __uint_as_float(ru[j + 1])};
+        for (int j = 0; j < N; j += 2) {
+            float s[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const float x = 1.0f + expf(-v[j + i]);
@@ -230,18 +227,60 @@ __device__ __forceinline__ void swiglu_all(const uint32_t (&rg)[32], const uint3
                 s[i] = v[j + i] * __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
             }
             bf16_round2(s[0], s[1]);
-            bf16_round2(u[0], u[1]);
-            v[j] = s[0] * u[0]; v[j + 1] = s[1] * u[1];
+            v[j] = s[0] * u[j]; v[j + 1] = s[1] * u[j + 1];
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < N; ++j) {
             const float sg = 1.0f / (1.0f + expf(-v[j]));
-            v[j] = bf16_round(v[j] * sg) * bf16_round(__uint_as_float(ru[j]));
+            v[j] = bf16_round(v[j] * sg) * u[j];
         }
     }
 }
+__device__ __forceinline__ void swiglu_all(const uint32_t (&rg)[32], const uint32_t (&ru)[32], float (&v)[32]) {
+    float u[32];
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+        v[j] = __uint_as_float(rg[j]); v[j + 1] = __uint_as_float(rg[j + 1]);
+        u[j] = __uint_as_float(ru[j]); u[j + 1] = __uint_as_float(ru[j + 1]);
+        bf16_round2(v[j], v[j + 1]);
+        bf16_round2(u[j], u[j + 1]);
+    }
+    swiglu_vals(v, u);
+}
 
+// (head_epilogue()'s arithmetic for one row, by eight lanes, in gemm_rows_kernel; as a function that one uses too it costs its launches
+// 0.5 us.)  Each lane takes 8 + 8 of its bf16 values from shared memory, from column 8 t and 64 + 8 t on.
+__device__ __forceinline__ void head_row(const GemmArgs& g, const uint8_t* s_lo, const uint8_t* s_hi, const float (&wl)[8], const float (&wh)[8],
+                                         int row, bool row_ok, uint16_t* obase, int t) {
+    const float* cs = g.rope + (size_t)(row_ok ? row : 0) * 128 + 8 * t;
+    const float4 ca = *reinterpret_cast<const float4*>(cs), cb = *reinterpret_cast<const float4*>(cs + 4);
+    const float4 sa = *reinterpret_cast<const float4*>(cs + 64), sb = *reinterpret_cast<const float4*>(cs + 68);
+    float lo[8], hi[8];
+    unpack8_bf16(*reinterpret_cast<const uint4*>(s_lo), lo);
+    unpack8_bf16(*reinterpret_cast<const uint4*>(s_hi), hi);
+    float sq = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sq = __fadd_rn(sq, __fmaf_rn(hi[j], hi[j], __fmul_rn(lo[j], lo[j])));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) sq = __fadd_rn(sq, __shfl_xor_sync(0xffffffffu, sq, o));
+    const float inv = rsqrtf(sq / 128.0f + g.scale);
+    const float cc[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+    const float ss[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+    float ol[8], oh[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float a = bf16_round(wl[j] * lo[j] * inv);
+        const float b = bf16_round(wh[j] * hi[j] * inv);
+        ol[j] = bf16_round(a * cc[j]) - bf16_round(b * ss[j]);
+        oh[j] = bf16_round(b * cc[j]) + bf16_round(a * ss[j]);
+    }
+    if (row_ok) {
+        uint16_t* o = obase + (size_t)row * g.ldo + 8 * t;
+        *reinterpret_cast<uint4*>(o) = make_uint4(pack_bf16x2(ol[0], ol[1]), pack_bf16x2(ol[2], ol[3]), pack_bf16x2(ol[4], ol[5]), pack_bf16x2(ol[6], ol[7]));
+        *reinterpret_cast<uint4*>(o + 64) = make_uint4(pack_bf16x2(oh[0], oh[1]), pack_bf16x2(oh[2], oh[3]), pack_bf16x2(oh[4], oh[5]), pack_bf16x2(oh[6], oh[7]));
+    }
+}
 // Per-head RMSNorm + rotary on a projection's output (o1.c src/model/block.c:266-289 runs head split, hd_rmsnorm, hd_apply_rotary as
 // separate passes).  The 128 values of a head are rounded to bf16 (the projection's stored result) and pass through shared memory, 16
 // rows at a time; then eight lanes take a row: each sums 8 + 8 elements, the pairwise tree over the lanes is the order of
@@ -1188,6 +1227,184 @@ gemm_pair_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
+// ---------------------------------------------------------------- CTA pairs fitted to the number of rows
+// Gate | up + SwiGLU and q | k | v have epilogues that fix the columns of a tile, so the pair kernel pays whole 256s of rows: 592 rows
+// as 768.  Here the operands change places: 256 rows of WEIGHTS are the M of the MMA (128 in each CTA: 64 gate rows and the 64
+// up rows of the same columns, or one head), and the tokens its N, any multiple of 16 up to 256: 592 rows as three tiles of 208.
+// The products and the order of their sums are the same, so the bits are.  An accumulator holds a column of the output per lane; 16
+// tokens at a time go through shared memory as bf16 (the first rounding of both epilogues) and come back by token, from four warps.
+// The rule, and both sides' times: rows_width().
+static constexpr int RW_TOK = 16;                          // tokens of a group
+static constexpr int RW_STAGE = RW_TOK * 256;              // their 128 columns
+static constexpr int RW_STORE = 2 * 2 * RW_STAGE;          // two groups of four warps, two buffers each
+static constexpr int RW_SMEM = PF_STAGE_ROOM + RW_STORE + 1024 /*align*/ + 256 /*barriers*/;
+
+template <int EPI>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
+                 const __grid_constant__ CUtensorMap tmW3, const GemmArgs g, const int bn, const int stages) {
+    static_assert(EPI == EPI_SWIGLU || EPI == EPI_QKV, "the other epilogues have tiles of any number of columns");
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int stage_bytes = (BM + bn / 2) * BK * 2;      // (bn is a multiple of 16: the stages stay 1024-byte aligned)
+    uint8_t* store_s = smem + PF_STAGE_ROOM;
+    uint64_t* full = reinterpret_cast<uint64_t*>(store_s + RW_STORE);
+    uint64_t* empty = full + PF_MAX_STAGES;
+    uint64_t* tfull = empty + PF_MAX_STAGES;
+    uint64_t* tempty = tfull + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    if (threadIdx.x == 64) *s_abort = error_word(g.err);
+    if (threadIdx.x == 0) {
+        tma_prefetch_desc(&tmX);
+        tma_prefetch_desc(&tmW);
+        tma_prefetch_desc(&tmW2);
+        if (EPI == EPI_QKV) tma_prefetch_desc(&tmW3);
+        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 2 * EPI_WARPS); }
+        fence_mbar_init();
+    }
+    if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+    const int num_tiles = g.num_m * g.num_n, kblocks = (g.K + BK - 1) / BK;
+    const int tile0 = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();           // both CTAs' barriers exist before either signals the other's
+    tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool live = (*s_abort | ld_cluster_s32(map_to_rank(smem_u32(s_abort), rank ^ 1u))) == 0;
+    // q | k | v: the weight tensor of this CTA's head and the head's first column in it
+    auto segment = [&](int nb, int& lcol0) {
+        const int col0 = nb * 256 + (int)rank * 128;
+        const int seg = col0 >= g.seg_n[0] + g.seg_n[1] ? 2 : (col0 >= g.seg_n[0] ? 1 : 0);
+        lcol0 = col0 - (seg == 2 ? g.seg_n[0] + g.seg_n[1] : (seg == 1 ? g.seg_n[0] : 0));
+        return seg;
+    };
+
+    if (live && warp == 0) {
+        if (elect_one()) {
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+                int mb, nb, lrow = 0;
+                tile_coords(tile, g.num_m, g.num_n, g.group_m, mb, nb);
+                const int seg = EPI == EPI_QKV ? segment(nb, lrow) : 0;
+                const CUtensorMap* mW = seg == 0 ? &tmW : (seg == 1 ? &tmW2 : &tmW3);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!mbar_wait(&empty[stage], phase ^ 1)) { ok = false; atomicExch(g.err, 81); break; }
+                    uint8_t* a_s = smem + stage * stage_bytes;
+                    if (rank == 0) mbar_expect_tx(&full[stage], 2 * stage_bytes);      // both CTAs' halves
+                    if (EPI == EPI_SWIGLU) {
+                        tma_load_2d_pair(a_s, &tmW, &full[stage], kb * BK, nb * 128 + (int)rank * 64);
+                        tma_load_2d_pair(a_s + 64 * BK * 2, &tmW2, &full[stage], kb * BK, nb * 128 + (int)rank * 64);
+                    } else {
+                        tma_load_2d_pair(a_s, mW, &full[stage], kb * BK, lrow);
+                    }
+                    tma_load_2d_pair(a_s + BM * BK * 2, &tmX, &full[stage], kb * BK, mb * bn + (int)rank * (bn / 2));
+                    if (++stage == stages) { stage = 0; phase ^= 1; }
+                }
+            }
+        }
+    } else if (live && warp == 1) {
+        if (rank == 0 && elect_one()) {
+            const uint32_t idesc = umma_idesc_bf16(2 * BM, bn, 0, 0);
+            int stage = 0, as = 0;
+            uint32_t phase = 0, aphase = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+                if (!mbar_wait(&tempty[as], aphase ^ 1)) { atomicExch(g.err, 82); break; }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + as * 256;
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!mbar_wait(&full[stage], phase)) { ok = false; atomicExch(g.err, 83); break; }
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + stage * stage_bytes);
+                    const uint64_t ad = umma_desc_sw128(a_addr, 16, 1024);
+                    const uint64_t bd = umma_desc_sw128(a_addr + BM * BK * 2, 16, 1024);
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma_ss_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0);
+                    umma_commit_pair(&empty[stage]);
+                    if (++stage == stages) { stage = 0; phase ^= 1; }
+                }
+                umma_commit_pair(&tfull[as]);
+                if (++as == 2) { as = 0; aphase ^= 1; }
+            }
+        }
+    } else if (live) {
+        const int q = warp & 3, grp = (warp - 2) >> 2;       // quadrant of tensor memory, which of the two groups of four warps
+        const int tid = q * 32 + lane, tok = tid >> 3, t = tid & 7;      // by token: eight lanes each
+        uint8_t* stg = store_s + grp * 2 * RW_STAGE;
+        int as = 0, buf = 0;
+        uint32_t aphase = 0;
+        const int failed = error_word(g.err);
+        bool ok = true;       // (a warp whose wait ran out goes on through its group's barriers, and does nothing else)
+        for (int tile = tile0; tile < num_tiles; tile += tile_step) {
+            int mb, nb, lcol0 = 0;
+            tile_coords(tile, g.num_m, g.num_n, g.group_m, mb, nb);
+            const int row0 = mb * bn, rows = g.M - row0 < bn ? g.M - row0 : bn;
+            const int seg = EPI == EPI_QKV ? segment(nb, lcol0) : 0;
+            uint16_t* obase = g.out + (EPI == EPI_SWIGLU ? nb * 128 + (int)rank * 64 : nb * 256 + (int)rank * 128);
+            float wl[8], wh[8];
+            if (EPI == EPI_QKV && seg < 2) {
+                unpack8_bf16(*reinterpret_cast<const uint4*>(g.seg_norm[seg] + 8 * t), wl);
+                unpack8_bf16(*reinterpret_cast<const uint4*>(g.seg_norm[seg] + 64 + 8 * t), wh);
+            }
+            if (ok && !__all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase))) { atomicExch(g.err, 84); ok = false; }
+            tc_fence_after();
+            const uint32_t t_row = tmem_base + as * 256 + ((uint32_t)(q * 32) << 16);
+#pragma unroll 1
+            for (int c = grp * RW_TOK; c < rows; c += 2 * RW_TOK, buf ^= 1) {
+                uint8_t* st = stg + buf * RW_STAGE;
+                if (ok) {
+                    uint32_t r[RW_TOK];
+                    tmem_ld16(t_row + c, r);
+                    tmem_ld_wait();
+                    // this lane's column of 16 tokens: a warp writes 64 bytes of each
+#pragma unroll
+                    for (int j = 0; j < RW_TOK; j += 2) {
+                        const uint32_t p = pack_bf16x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+                        *reinterpret_cast<uint16_t*>(st + j * 256 + tid * 2) = (uint16_t)p;
+                        *reinterpret_cast<uint16_t*>(st + (j + 1) * 256 + tid * 2) = (uint16_t)(p >> 16);
+                    }
+                }
+                // (one barrier a group: a buffer is written again behind the next one, when all four warps have read it)
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+                const int row = row0 + c + tok;
+                const bool row_ok = ok && !failed && c + tok < rows;
+                const uint4* in = reinterpret_cast<const uint4*>(st + tok * 256) + t;
+                if (EPI == EPI_SWIGLU) {
+                    float v[8], u[8];
+                    unpack8_bf16(in[0], v);
+                    unpack8_bf16(in[8], u);
+                    swiglu_vals(v, u);
+                    if (row_ok) *reinterpret_cast<uint4*>(obase + (size_t)row * g.ldo + 8 * t) =
+                        make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+                } else if (seg < 2) {
+                    head_row(g, reinterpret_cast<const uint8_t*>(in), reinterpret_cast<const uint8_t*>(in + 8), wl, wh, row, row_ok, obase, t);
+                } else if (row_ok) {
+                    uint4* o = reinterpret_cast<uint4*>(obase + (size_t)row * g.ldo) + t;
+                    o[0] = in[0];
+                    o[8] = in[8];
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (ok && lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&tempty[as]), 0));
+            if (++as == 2) { as = 0; aphase ^= 1; }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still signal it or feed an MMA
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+}
+
 // ---------------------------------------------------------------- SIMT path
 // For M < 8 (timestep MLP, M = 1) and for shapes the tensor-core tiles do not cover.  One warp per output column and MR
 // rows: bound by the weights' way from memory, so a weight is read once for all its rows, four 16-byte pieces of a lane at
@@ -1437,6 +1654,31 @@ static bool launch_pair_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, i
     return true;
 }
 
+// x [M, K] (row pitch ldx) against the weights of `num_n` tiles: gate and up, or q, k and v
+template <int EPI>
+static bool launch_rows(const void* x, int ldx, const CUtensorMap* mW, const CUtensorMap* mW2, const CUtensorMap* mW3, GemmArgs& g, int bn,
+                        cudaStream_t st) {
+    static std::atomic<uint64_t> attr_done{0};
+    auto kern = gemm_rows_kernel<EPI>;
+    if (!func_attr_once(attr_done, (const void*)kern, RW_SMEM, "gemm (pair, rows)")) return false;
+    CUtensorMap mX;
+    if (!cached_tmap(&mX, x, g.M, g.K, ldx, bn / 2)) return false;
+    g.num_m = (g.M + bn - 1) / bn;
+    g.num_n = g.N / (EPI == EPI_SWIGLU ? 128 : 256);
+    g.group_m = (g.group_m * BM + bn - 1) / bn;
+    int stages = PF_STAGE_ROOM / ((BM + bn / 2) * BK * 2);
+    if (stages > PF_MAX_STAGES) stages = PF_MAX_STAGES;
+    const int tiles = g.num_m * g.num_n;
+    int pairs = pair_capacity((const void*)kern, GEMM_THREADS, RW_SMEM);
+    if (pairs > tiles) pairs = tiles;
+    prof_before(EPI == EPI_QKV ? (int)EPI_STORE : EPI, 2.0 * g.M * (double)g.N * g.K * (EPI == EPI_SWIGLU ? 2.0 : 1.0), st);
+    cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), RW_SMEM, st, 2, overlap_rows(g), mX, *mW, *mW2, *mW3, g, bn, stages);
+    prof_after(st);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("gemm (pair, rows): launch: %s", cudaGetErrorString(e)); return false; }
+    return true;
+}
+
 // CTA pairs of the GEMM kernel the current device can hold at once (what the pair form's grid is clamped to)
 int gemm_pair_capacity() {
     using Cfg = GemmCfg<256, true>;
@@ -1540,6 +1782,26 @@ static int pair_fit_width(int num_m, int N, double best, int lo, int hi) {
     }
     return width;
 }
+// The number of tokens of a tile of gemm_rows_kernel, or 0 where the other forms' cost `best` (TILE_COST's units) is as good.  tiles_w:
+// tiles of 256 weight rows.  A round takes as long as one of pair_fit_width()'s columns.  The other forms / this one, us, gate | up with
+// SwiGLU (12288 columns of each, K = 4096): 129 rows 61 / 46, 256 rows 73 / 55, 296 rows 75 / 68, 513 rows 117 / 85, 592 rows 120 / 100, 785
+// rows 171 / 131, 1030 rows 197 / 157, 1600 rows 273 / 239, 2070 rows 337 / 299; q | k | v of 4096 + 2 x 1024 columns: 64 rows
+// 29.6 / 23.5, 256 rows 21.4 / 18.7, 392 rows 34.3 / 23.4, 592 rows 36.3 / 31.3, 925 rows 58.7 / 42.6, 1280 rows 62.9 / 56.3, 1690 rows
+// 81.7 / 68.2, 2450 rows 110 / 97, 3970 rows 166 / 147.  Up to 128 rows gate | up is read from memory at 5 TB/s either way (77 rows 40.6
+// / 40.5, 100 rows 41.1 / 45.5): swiglu_rows_width().  Whole 256s, and what is near them, stay with the others (2242, 4352 rows).
+static int rows_width(int M, int tiles_w, int K, double best) {
+    if (K < LONG_K || !pair_wanted()) return 0;
+    const long pairs = sm_count() / 2;
+    int width = 0;
+    best *= 15.0 / 16;       // (only for a gain that shows)
+    for (int t = (M + 255) / 256; t <= (M + 255) / 256 + 3; ++t) {
+        const int bn = ((M + t - 1) / t + 15) / 16 * 16;
+        if (bn < 64) break;
+        const double c = (double)((t * tiles_w + pairs - 1) / pairs) * (1.2 + 0.2 * bn);
+        if (c < best) { best = c; width = bn; }
+    }
+    return width;
+}
 template <int EPI>
 static bool launch_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, int bn, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
@@ -1620,13 +1882,18 @@ static SplitPlan split_plan(int M, int N, int K, bool may_split, bool resid) {
     return {0, 0};
 }
 
+static int swiglu_rows_width(int M, int N, int K) {
+    long units = 0;
+    tile_form((M + BM - 1) / BM, 2 * N, K, true, true, &units);
+    return M <= BM || K < LONG_K ? 0 : rows_width(M, N / 128, K, (double)units);
+}
 static int simt_rows(int M, int N, int K);
 // The form a GEMM takes.  plain: row-major output; wide_ok: 256-column tiles fit it.
 GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok) {
     if (!gemm_tc_supported(M, N, K, epi)) return {GEMM_ROWS, simt_rows(M, N, K), 1};
     const int num_m = (M + BM - 1) / BM;
-    if (epi == EPI_SWIGLU) {     // (2N columns of gate and up)
-        const bool pair = force_bn <= 0 && tile_form(num_m, 2 * N, K, true, true) == TILE_PAIR;
+    if (epi == EPI_SWIGLU) {     // (2N columns of gate and up; pairs of 256 x 256 or gemm_rows_kernel's of 256 x any)
+        const bool pair = force_bn <= 0 && (tile_form(num_m, 2 * N, K, true, true) == TILE_PAIR || (force_bn == 0 && swiglu_rows_width(M, N, K)));
         return {pair ? GEMM_PAIR : GEMM_TILE, 256, pair ? 2 : 1};
     }
     const bool pair_ok = epi == EPI_STORE || epi == EPI_BIAS || epi == EPI_RESID;
@@ -1836,6 +2103,12 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
     }
     const GemmPlan p = gemm_plan(M, N, K, epi, force_bn, !o_cb && !o_tab, wide_ok);
     if (epi == EPI_SWIGLU) {
+        const int bn = force_bn == 0 && !a_kblk ? swiglu_rows_width(M, N, K) : 0;
+        if (bn) {
+            CUtensorMap mG, mU;
+            if (!cached_tmap(&mG, w, N, K, K, 64) || !cached_tmap(&mU, w2, N, K, K, 64)) return false;
+            return launch_rows<EPI_SWIGLU>(x, ldx, &mG, &mU, &mU, g, bn, st);
+        }
         g.num_n = N / 128;
         return p.form == GEMM_PAIR ? launch_tc_pair<EPI_SWIGLU>(tA, tB, tB2, g, st, nullptr) : launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
     }
@@ -1949,7 +2222,10 @@ bool gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void
     // 256-wide tiles need every segment (and every destination block) to be a multiple of 256 columns
     bool wide = (qc % 256) == 0 && (kc % 256) == 0;
     if (tabs && (((qc / n_dst) % 256) != 0 || ((kc / n_dst) % 256) != 0)) wide = false;
-    const TileForm form = tile_form(g.num_m, N, K, wide, true);
+    long units = 0;
+    const TileForm form = tile_form(g.num_m, N, K, wide, true, &units);
+    const int bn = !tabs && (N % 256) == 0 && K >= LONG_K && (ldy % 8) == 0 && (((uintptr_t)y) & 15) == 0 ? rows_width(M, N / 256, K, (double)units) : 0;
+    if (bn) return launch_rows<EPI_QKV>(x, ldx, &mQ, &mK, &mV, g, bn, st);
     g.num_n = N / (form == TILE_128 ? 128 : 256);
     if (form == TILE_PAIR) return launch_tc_pair<EPI_QKV>(&mA, &mQ, &mK, g, st, &mV);
     return form == TILE_256 ? launch_tc<EPI_QKV, 256>(&mA, &mQ, &mK, g, st, &mV) : launch_tc<EPI_QKV, 128>(&mA, &mQ, &mK, g, st, &mV);

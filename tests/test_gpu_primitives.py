@@ -470,6 +470,41 @@ def test_gemm_on_cta_pairs_equals_single_cta_tiles(pkg, dev, M, N, K, epi):
     assert err < 1e-2, err     # the pair form really computed the product (fp32 reference, bf16 rounding of the result)
 
 
+@pytest.mark.parametrize("M", [77, 129, 144, 257, 296, 513, 592, 785, 1030, 1300])
+@pytest.mark.parametrize("K", [2048, 2104])
+def test_pairs_with_tokens_as_columns(pkg, dev, M, K):
+    """gate | up + SwiGLU and q | k | v with the weights as the MMA's rows (tiles of 256 weight rows and a number of tokens that fits)
+    give the bits of one-CTA tiles: partly filled token tiles, fewer and more than a round of tiles, a ragged last K block, q, k and v tiles of
+    one launch; nothing is written beside the result."""
+    N, qc, kc = 1536, 512, 256
+    x, wg, wu = (dv(seeded_bf16((r, K), 60 + i, 0.0, 1.0 if i == 0 else 0.05), dev) for i, r in enumerate((M, N, N)))
+    ys = []
+    for bn in (0, 256):
+        y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
+        assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(wg), pkg.ptr(wu), pkg.ptr(y), N + 8, M, N, K, 3, None, None, 0, 0.0, bn) == 0, pkg.last_error()
+        done(pkg, "swiglu")
+        assert (y[M:] == 777.0).all() and (y[:, N:] == 777.0).all(), "written beside the matrix"
+        ys.append(y)
+    assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
+    g, u = ((x.float() @ w.float().t()).bfloat16().float() for w in (wg, wu))
+    ref = torch.nn.functional.silu(g).bfloat16().float() * u
+    assert (ys[0][:M, :N].float() - ref).abs().max().item() < 1e-2 * ref.abs().max().item()
+    wq, wk, wv = (dv(seeded_bf16((n, K), 70 + i, 0.0, 0.05), dev) for i, n in enumerate((qc, kc, kc)))
+    nq, nk = dv(seeded_bf16(128, 75, 1.0, 0.1), dev), dv(seeded_bf16(128, 76, 1.0, 0.1), dev)
+    tab = torch.empty(M, 128, device=dev).uniform_(-1, 1)
+    ld = qc + 2 * kc + 8
+    one, three = (torch.full((M + 1, ld), 777.0, dtype=torch.bfloat16, device=dev) for _ in range(2))
+    assert pkg.lib.o1_gemm_qkv(pkg.ptr(x), K, pkg.ptr(wq), pkg.ptr(wk), pkg.ptr(wv), pkg.ptr(one), ld, M, qc, kc, K, pkg.ptr(nq),
+                               pkg.ptr(nk), pkg.ptr(tab), 1e-6) == 0, pkg.last_error()
+    at = lambda off: C.c_void_p(three.data_ptr() + off * 2)  # noqa: E731
+    assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(wq), None, at(0), ld, M, qc, K, 6, pkg.ptr(nq), pkg.ptr(tab), 0, 1e-6, 128) == 0
+    assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(wk), None, at(qc), ld, M, kc, K, 6, pkg.ptr(nk), pkg.ptr(tab), 0, 1e-6, 128) == 0
+    assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(wv), None, at(qc + kc), ld, M, kc, K, 0, None, None, 0, 0.0, 128) == 0
+    done(pkg, "qkv")
+    assert torch.equal(one.view(torch.int16), three.view(torch.int16))
+    assert pkg.lib.o1_device_error() == 0
+
+
 def check_linear_f64(y, x, w, bias, what):
     """y against 64 bits: an FP32 sum of K products in any order is within K * 2^-23 * sum|x||w| of the exact one, and the
     two bf16 roundings (of the sum, of the sum plus bias) are monotonic, so the result lies between the rounded ends."""
