@@ -986,6 +986,107 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN, KPS>::TMEM_COLS);
 }
 
+// ---------------------------------------------------------------- narrow tiles on CTA pairs
+// The 32-column form with two CTAs to a tile of 128 rows x 64 columns: each has 64 rows of the activations, 32 of the weights and,
+// in its tensor memory, 64 rows of the result; and four K blocks to a copy.  What bounds the narrow tiles is the thread that issues the
+// copies, some 145 cycles for each whatever its size (two for a K block, and one for L2), and shared memory: an MMA of 128 x 32 x 16
+// reads 5 KB while the copies write as much, the pair's of 128 x 64 x 16 reads and writes 3 KB on an SM.  Same order of the
+// sum, so the same bits.  fewpair_pays() has both sides' times.
+static constexpr int FP_KPS = 4, FP_STAGES = 4, FP_ROWS = 64, FP_COLS = 32;      // K blocks a stage and copy; rows and columns of a CTA
+static constexpr int FP_STAGE_BYTES = FP_KPS * (FP_ROWS + FP_COLS) * BK * 2;
+static constexpr int FP_SMEM = FP_STAGES * FP_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+
+template <int EPI>
+__global__ void __launch_bounds__(SK_THREADS, 1)
+gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + FP_STAGES * FP_STAGE_BYTES);
+    uint64_t* empty = full + FP_STAGES;
+    uint64_t* acc_done = empty + FP_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+    int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int tile = (int)(blockIdx.x >> 1);
+    const int nb = tile / g.num_m, mb = tile - nb * g.num_m;      // CTAs that share weights run next to each other
+    const int a_row = mb * BM + (int)rank * FP_ROWS, b_row = nb * 2 * FP_COLS + (int)rank * FP_COLS;
+
+    if (threadIdx.x == 64) *s_abort = error_word(g.err);
+    if (threadIdx.x == 96) {
+        for (int s = 0; s < FP_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(acc_done, 1);
+        fence_mbar_init();
+    }
+    if (warp == 1) { tmem_alloc_pair(tmem_slot, 32); tmem_relinquish_pair(); }
+    const int kblocks = (g.K + BK - 1) / BK;
+    const bool ahead = mb == 0 && g.prefetch > 0;     // the other row tiles find the weights in L2
+    if (warp == 0 && elect_one()) {
+        tma_prefetch_desc(&tmB);
+        tma_prefetch_desc(&tmA);
+        if (ahead) for (int i = 0; i < g.prefetch && i < kblocks; i += FP_KPS) tma_prefetch_3d(&tmB, 0, b_row, i);
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();           // both CTAs' barriers exist before either signals the other's
+    tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool live = (*s_abort | ld_cluster_s32(map_to_rank(smem_u32(s_abort), rank ^ 1u))) == 0;
+
+    if (live && warp == 0) {
+        if (elect_one()) {
+            for (int i = 0, it = 0; i < kblocks; i += FP_KPS, ++it) {
+                const int s = it % FP_STAGES;
+                if (!mbar_wait(&empty[s], ((it / FP_STAGES) & 1) ^ 1)) { atomicExch(g.err, 91); break; }
+                uint8_t* a_s = smem + s * FP_STAGE_BYTES;
+                if (rank == 0) mbar_expect_tx(&full[s], 2 * FP_STAGE_BYTES);      // both CTAs' halves
+                tma_load_3d_pair(a_s, &tmA, &full[s], 0, a_row, i);
+                tma_load_3d_pair(a_s + FP_KPS * FP_ROWS * BK * 2, &tmB, &full[s], 0, b_row, i);
+            }
+        }
+    } else if (live && warp == 1) {
+        if (rank == 0 && elect_one()) {
+            constexpr uint32_t idesc = umma_idesc_bf16(2 * FP_ROWS, 2 * FP_COLS, 0, 0);
+            bool good = true;
+            for (int i = 0, it = 0; i < kblocks && good; i += FP_KPS, ++it) {
+                const int s = it % FP_STAGES;
+                if (!mbar_wait(&full[s], (it / FP_STAGES) & 1)) { atomicExch(g.err, 92); good = false; break; }
+                tc_fence_after();
+                const uint32_t a_addr = smem_u32(smem + s * FP_STAGE_BYTES);
+#pragma unroll
+                for (int u = 0; u < FP_KPS; ++u) {
+                    if (i + u >= kblocks) break;
+                    const uint64_t ad = umma_desc_sw128(a_addr + u * FP_ROWS * BK * 2, 16, 1024);
+                    const uint64_t bd = umma_desc_sw128(a_addr + FP_KPS * FP_ROWS * BK * 2 + u * FP_COLS * BK * 2, 16, 1024);
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma_ss_pair(tmem_base, ad + 2 * k, bd + 2 * k, idesc, (i | u | k) != 0);
+                }
+                umma_commit_pair(&empty[s]);
+            }
+            umma_commit_pair(acc_done);
+        }
+    } else if (live) {
+        // With 64 rows to a CTA the lanes 0..63 of its tensor memory hold the tile's first 32 columns, 64..127 the other 32 of the same rows.
+        const int q = warp & 3, failed = error_word(g.err);
+        const int row0 = a_row + (q & 1) * 32, col0 = nb * 2 * FP_COLS + (q >> 1) * FP_COLS, cols = g.N - col0 < FP_COLS ? g.N - col0 : FP_COLS;
+        PlainEpilogue<EPI> plain;
+        if (cols > 0) plain.ahead(g, row0, col0, cols, 0, lane);
+        bool ok = mbar_wait(acc_done, 0);
+        if (!ok) atomicExch(g.err, 93);
+        ok = __all_sync(0xffffffffu, ok);
+        tc_fence_after();
+        // (all MMAs are through with the stages, which serve as staging)
+        if (ok && cols > 0) plain.run(g, tmem_base + ((uint32_t)(q * 32) << 16), row0, col0, cols, 0, FP_COLS, smem + (warp - 2) * EPI_SLICE, lane, failed);
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still signal it or feed an MMA
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 32);
+}
+
 // ---------------------------------------------------------------- tiles fitted to the number of SMs
 // The persistent kernel with a tile width chosen at run time, a multiple of 16 from 144 to 192 columns: where 128 or 256
 // columns leave a last round of few tiles (1280 rows x 4096 columns: 320 tiles for 148 SMs, three rounds for 2.2), some
@@ -1522,8 +1623,24 @@ static bool make_tmap_heads(CUtensorMap* out, const void* base, uint64_t cols, u
     return true;
 }
 
+// A row-major matrix [rows, cols], cols a multiple of 64, as [cols / 64][rows][64]: boxes of `blocks` K blocks, each box_rows rows of 128 bytes,
+// land one behind the other.  (The extents are exactly the matrix's.)
+static bool make_tmap_kblocks(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t blocks) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) { set_error("tensor map: cuTensorMapEncodeTiled entry point unavailable"); return false; }
+    if ((((uintptr_t)base) & 15) || ((ld * 2) & 15) || (cols % 64)) { set_error("tensor map: base/pitch not 16-byte aligned"); return false; }
+    cuuint64_t dims[3] = {64, rows, cols / 64};
+    cuuint64_t strides[2] = {ld * 2, 128};
+    cuuint32_t box[3] = {64, box_rows, blocks};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { set_error("tensor map: encode failed (%d)", (int)r); return false; }
+    return true;
+}
+
 struct TmapKey {
-    const void* p; uint64_t rows, cols, ld, heads, hoff; uint32_t box;     // heads == 0: a plain matrix
+    const void* p; uint64_t rows, cols, ld, heads, hoff; uint32_t box;     // heads == 0: a plain matrix; hoff == 0: K blocks, heads of them a box
     bool operator<(const TmapKey& o) const {
         return std::tie(p, rows, cols, ld, heads, hoff, box) < std::tie(o.p, o.rows, o.cols, o.ld, o.heads, o.hoff, o.box);
     }
@@ -1539,13 +1656,16 @@ static bool cached(CUtensorMap* out, const TmapKey& k) {
     auto it = cache.find(k);
     if (it != cache.end()) { *out = it->second; return true; }
     if (cache.size() > 8192) cache.clear();
-    if (!(k.heads ? make_tmap_heads(out, k.p, k.cols, k.rows, k.heads, k.ld, k.hoff, k.box) : make_tmap_bf16(out, k.p, k.rows, k.cols, k.ld, k.box)))
+    if (!(k.heads && !k.hoff ? make_tmap_kblocks(out, k.p, k.rows, k.cols, k.ld, k.box, (uint32_t)k.heads) : k.heads ? make_tmap_heads(out, k.p, k.cols, k.rows, k.heads, k.ld, k.hoff, k.box) : make_tmap_bf16(out, k.p, k.rows, k.cols, k.ld, k.box)))
         return false;
     cache.emplace(k, *out);
     return true;
 }
 bool cached_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
     return cached(out, TmapKey{base, rows, cols, ld, 0, 0, box_rows});
+}
+static bool cached_tmap_kblocks(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t blocks) {
+    return cached(out, TmapKey{base, rows, cols, ld, blocks, 0, box_rows});
 }
 bool cached_tmap_heads(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t heads, uint64_t ld, uint64_t hoff,
                        uint32_t box_rows) {
@@ -1957,12 +2077,38 @@ static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmAr
     return true;
 }
 
+// Narrow tiles on CTA pairs: whole K blocks, from 256 columns on.  One CTA per 32 columns / pairs of 64 (and, before several K blocks to
+// a copy, pairs alone), us: 77 x 4096 x 4096 13.2 / 11.25 (12.7), 16 x 4096 x 4096 13.0 / 11.0 (12.5), 77 x 1024 x 4096 11.5 / 7.8 (11.4), 300 x 1024
+// x 4096 11.9 / 8.9, 128 x 3072 x 4096 13.2 / 10.5, 77 x 1024 x 3072 9.5 / 6.7, 16 x 4096 x 1024 9.0 / 6.3, 77 x 4096 x 1024 5.9 / 6.0, 77 x 4096 x
+// 256 5.9 / 6.0.  Eight K blocks to a copy and two stages 12.3 / 8.8 (the first two of these), two and eight 11.7 / 9.7.
+static bool fewpair_pays(const GemmArgs& g) {
+    return pair_wanted() && g.num_m * ((g.N + 31) / 32) <= sm_count() && g.K >= 256 && g.K % BK == 0 && !g.a_kblk;
+}
 template <int EPI>
-static bool launch_split(const CUtensorMap* tA, const void* w, GemmArgs& g, const GemmPlan& p, cudaStream_t st) {
+static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, cudaStream_t st) {
+    static std::atomic<uint64_t> attr_done{0};
+    auto kern = gemm_few_pair_kernel<EPI>;
+    if (!func_attr_once(attr_done, (const void*)kern, FP_SMEM, "gemm (few tiles, pairs)")) return false;
+    CUtensorMap mA, mB;
+    if (!cached_tmap_kblocks(&mA, x, g.M, g.K, ldx, FP_ROWS, FP_KPS) || !cached_tmap_kblocks(&mB, w, g.N, g.K, g.K, FP_COLS, FP_KPS)) return false;
+    g.num_n = (g.N + 2 * FP_COLS - 1) / (2 * FP_COLS);
+    g.prefetch = SK_PREFETCH;
+    prof_before(EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : (EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID ? (int)EPI_RESID : EPI),
+                2.0 * g.M * (double)g.N * g.K, st);
+    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(SK_THREADS), FP_SMEM, st, 2, g.M, mA, mB, g);
+    prof_after(st);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("gemm (few tiles, pairs): launch: %s", cudaGetErrorString(e)); return false; }
+    return true;
+}
+
+template <int EPI>
+static bool launch_split(const CUtensorMap* tA, const void* x, int ldx, const void* w, GemmArgs& g, const GemmPlan& p, cudaStream_t st) {
     CUtensorMap mB;
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, p.bn)) return false;
     switch (p.bn) {
         case 32:
+            if (fewpair_pays(g)) return launch_few_pair<EPI>(x, ldx, w, g, st);
             if (g.num_m * ((g.N + 31) / 32) <= sm_count()) return launch_split_bn<EPI, 32, 2>(tA, &mB, g, p.ks, st);
             return launch_split_bn<EPI, 32>(tA, &mB, g, p.ks, st);
         case 96: return launch_split_bn<EPI, 96>(tA, &mB, g, p.ks, st);
@@ -2113,12 +2259,12 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
         return p.form == GEMM_PAIR ? launch_tc_pair<EPI_SWIGLU>(tA, tB, tB2, g, st, nullptr) : launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
     }
     if (p.form == GEMM_FEW) switch (epi) {
-        case EPI_STORE: return launch_split<EPI_STORE>(tA, w, g, p, st);
-        case EPI_BIAS:  return launch_split<EPI_BIAS>(tA, w, g, p, st);
-        case EPI_RESID: return launch_split<EPI_RESID>(tA, w, g, p, st);
-        case EPI_BIAS_GELU: return launch_split<EPI_BIAS_GELU>(tA, w, g, p, st);
-        case EPI_BIAS_RESID: return launch_split<EPI_BIAS_RESID>(tA, w, g, p, st);
-        case EPI_GATE_RESID: return launch_split<EPI_GATE_RESID>(tA, w, g, p, st);
+        case EPI_STORE: return launch_split<EPI_STORE>(tA, x, ldx, w, g, p, st);
+        case EPI_BIAS:  return launch_split<EPI_BIAS>(tA, x, ldx, w, g, p, st);
+        case EPI_RESID: return launch_split<EPI_RESID>(tA, x, ldx, w, g, p, st);
+        case EPI_BIAS_GELU: return launch_split<EPI_BIAS_GELU>(tA, x, ldx, w, g, p, st);
+        case EPI_BIAS_RESID: return launch_split<EPI_BIAS_RESID>(tA, x, ldx, w, g, p, st);
+        case EPI_GATE_RESID: return launch_split<EPI_GATE_RESID>(tA, x, ldx, w, g, p, st);
     }
     if (p.ks == 2 && (p.form == GEMM_FIT || p.form == GEMM_TILE)) switch (epi) {
         case EPI_STORE: return launch_pair_fit<EPI_STORE>(tA, w, g, p.bn, st);

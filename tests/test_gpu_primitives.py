@@ -539,6 +539,35 @@ def gemm_form(pkg, M, N, K, epi, bn):
     return pkg.lib.o1_gemm_form(M, N, K, epi, bn, C.byref(width), C.byref(ctas)), width.value, ctas.value
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 72, 256), (77, 4096, 320), (16, 1032, 4096), (64, 1024, 576), (65, 3072, 512), (128, 4608, 1152),
+                                   (129, 2048, 448), (300, 1024, 4096), (520, 896, 2048), (1000, 512, 1024)])
+@pytest.mark.parametrize("epi", [0, 1, 2, 7, 8, 9])
+def test_narrow_tiles_on_pairs_give_the_bits_of_single_ctas(pkg, dev, M, N, K, epi):
+    """The 32-column form with two CTAs per 128 x 64 tile and four K blocks to a copy against the one-CTA form (pair mode 0), every
+    epilogue: row tiles whose second half has no rows or few, a ragged last column tile, K blocks that are no whole number of copies."""
+    if epi in (2, 8, 9) and N % 128:
+        pytest.skip("the residual epilogues take whole 128-column tiles")
+    g = torch.Generator(device=dev).manual_seed(M + N + K + epi)
+    x, w, b, r = (torch.empty(s, device=dev).normal_(0, d, generator=g).bfloat16()
+                  for s, d in (((M, K), 1.0), ((N, K), 0.05), ((N,), 0.5), ((M, N), 1.0)))
+    ys = []
+    try:
+        for mode in (1, 0):
+            pkg.lib.o1_gemm_pair_mode(mode)
+            if pkg.lib.o1_sm_count() == 148:
+                assert gemm_form(pkg, M, N, K, epi, 0) == (4, 32, 1)
+            y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
+            assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N + 8, M, N, K, epi, pkg.ptr(b), pkg.ptr(r), N, 0.0, 0) == 0, pkg.last_error()
+            done(pkg, "narrow tiles")
+            assert (y[M:] == 777.0).all() and (y[:, N:] == 777.0).all(), "written beyond the matrix"
+            ys.append(y)
+    finally:
+        pkg.lib.o1_gemm_pair_mode(1)
+    assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
+    check_epilogue_f64(ys[0][:M, :N], x, w, b, r, epi, "narrow tiles")
+    assert pkg.lib.o1_device_error() == 0
+
+
 def gelu_tanh_f64(v):
     """0.5 v (1 + tanh u) = v / (1 + e^-2u): in 64 bits too, 1 + tanh u has no digits left where u is far below zero."""
     return v / (1 + torch.exp(-2 * 0.7978845608028654 * (v + 0.044715 * v ** 3)))
