@@ -125,13 +125,15 @@ static constexpr bool epi_has_resid(int e) { return e == EPI_RESID || e == EPI_B
 static constexpr bool epi_plain(int e) { return e == EPI_STORE || epi_has_bias(e) || epi_has_resid(e); }
 
 // Groups of 32 columns at c_first, c_first + c_step, ... of a tile, plain row-major output (or column blocks, see GemmArgs).
-template <int EPI>
+// LIMIT: rows from row_end on are another CTA's (row_end <= M).
+template <int EPI, bool LIMIT = false>
 struct PlainEpilogue {
     static_assert(epi_plain(EPI), "this epilogue has no operands by column and element");
     static constexpr bool HAS_BIAS = epi_has_bias(EPI), HAS_RESID = epi_has_resid(EPI);
     // what the next group needs, requested one group ahead: the residual, eight rows of four 16-byte pieces at a time, and the bias
     // (or gate), a piece by each of four lanes
     uint4 rn[4] = {}, bq = {};
+    int row_end = 0;
     // row0: first of the warp's rows; cols: columns of the tile that exist (a multiple of eight)
     __device__ __forceinline__ void ahead(const GemmArgs& g, int row0, int col0, int cols, int c, int lane) {
         if (HAS_BIAS && lane < 4 && c + lane * 8 < cols) bq = *reinterpret_cast<const uint4*>(g.bias + col0 + c + lane * 8);
@@ -139,7 +141,7 @@ struct PlainEpilogue {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int row = row0 + k * 8 + (lane >> 2), col = c + (lane & 3) * 8;
-            if (row < g.M && col < cols) rn[k] = *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col0 + col);
+            if (row < (LIMIT ? row_end : g.M) && col < cols) rn[k] = *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col0 + col);
         }
     }
     // the caller has called ahead() for c_first; stg: EPI_SLICE bytes of the warp's own
@@ -182,12 +184,12 @@ struct PlainEpilogue {
                 }
             }
             if (EPI == EPI_BIAS_GELU) gelu_all(v, g.scale != 0.f);
-            store_group(g, v, stg, row0, col0 + c, cols - c, lane, failed);
+            store_group(g, v, stg, row0, col0 + c, cols - c, lane, failed, row_end);
         }
     }
     // this thread's row of 32 columns -> the warp's rows as segments of 64 bytes
     static __device__ __forceinline__ void store_group(const GemmArgs& g, const float (&v)[32], uint8_t* stg, int row0, int col, int cols,
-                                                       int lane, bool failed) {
+                                                       int lane, bool failed, int row_end = 0) {
         const int sr = lane >> 2, ch = lane & 3;
         uint4* own = reinterpret_cast<uint4*>(stg + lane * 64);
 #pragma unroll
@@ -203,7 +205,7 @@ struct PlainEpilogue {
         for (int k = 0; k < 4; ++k) {
             const int row = row0 + k * 8 + sr;
             const uint4 o = *reinterpret_cast<const uint4*>(stg + (k * 8 + sr) * 64 + ((ch ^ ((sr >> 1) & 3)) * 16));
-            if (!failed && row < g.M && ch * 8 < cols) *reinterpret_cast<uint4*>(out + (size_t)row * g.ldo) = o;
+            if (!failed && row < (LIMIT ? row_end : g.M) && ch * 8 < cols) *reinterpret_cast<uint4*>(out + (size_t)row * g.ldo) = o;
         }
     }
 };
@@ -992,29 +994,35 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // copies, some 145 cycles for each whatever its size (two for a K block, and one for L2), and shared memory: an MMA of 128 x 32 x 16
 // reads 5 KB while the copies write as much, the pair's of 128 x 64 x 16 reads and writes 3 KB on an SM.  Same order of the
 // sum, so the same bits.  fewpair_pays() has both sides' times.
-static constexpr int FP_KPS = 4, FP_STAGES = 4, FP_ROWS = 64, FP_COLS = 32;      // K blocks a stage and copy; rows and columns of a CTA
-static constexpr int FP_STAGE_BYTES = FP_KPS * (FP_ROWS + FP_COLS) * BK * 2;
-static constexpr int FP_SMEM = FP_STAGES * FP_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+// How many bytes of weights are on their way decides the time (77 x 4096 x 4096: two stages of four K blocks 16.6 us, four 11.3), so a stage
+// holds no more rows of the activations than there are: a tile of up to 128 rows is shared evenly, `ra` rows (a multiple of eight)
+// to a CTA.  The MMA reads 64, the others from whatever lies behind: their results are not used.
+static constexpr int FP_KPS = 4, FP_COLS = 32;      // K blocks a stage and copy; columns of a CTA
+static constexpr int FP_MAX_STAGES = 12, FP_ROOM = 216 * 1024;
+static constexpr int FP_SMEM = FP_ROOM + 1024 /*align*/ + 256 /*barriers*/;
+static constexpr int fp_stage_bytes(int ra) { return FP_KPS * (ra + FP_COLS) * BK * 2; }
 
 template <int EPI>
 __global__ void __launch_bounds__(SK_THREADS, 1)
-gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g) {
+gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g,
+                     const int ra, const int stages) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + FP_STAGES * FP_STAGE_BYTES);
-    uint64_t* empty = full + FP_STAGES;
-    uint64_t* acc_done = empty + FP_STAGES;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + FP_ROOM);
+    uint64_t* empty = full + FP_MAX_STAGES;
+    uint64_t* acc_done = empty + FP_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int tile = (int)(blockIdx.x >> 1);
     const int nb = tile / g.num_m, mb = tile - nb * g.num_m;      // CTAs that share weights run next to each other
-    const int a_row = mb * BM + (int)rank * FP_ROWS, b_row = nb * 2 * FP_COLS + (int)rank * FP_COLS;
+    const int stage_bytes = fp_stage_bytes(ra), a_bytes = ra * BK * 2;
+    const int a_row = mb * 2 * ra + (int)rank * ra, b_row = nb * 2 * FP_COLS + (int)rank * FP_COLS;
 
     if (threadIdx.x == 64) *s_abort = error_word(g.err);
     if (threadIdx.x == 96) {
-        for (int s = 0; s < FP_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         mbar_init(acc_done, 1);
         fence_mbar_init();
     }
@@ -1037,41 +1045,45 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
     if (live && warp == 0) {
         if (elect_one()) {
-            for (int i = 0, it = 0; i < kblocks; i += FP_KPS, ++it) {
-                const int s = it % FP_STAGES;
-                if (!mbar_wait(&empty[s], ((it / FP_STAGES) & 1) ^ 1)) { atomicExch(g.err, 91); break; }
-                uint8_t* a_s = smem + s * FP_STAGE_BYTES;
-                if (rank == 0) mbar_expect_tx(&full[s], 2 * FP_STAGE_BYTES);      // both CTAs' halves
+            uint32_t phase = 0;
+            for (int i = 0, s = 0; i < kblocks; i += FP_KPS) {
+                if (!mbar_wait(&empty[s], phase ^ 1)) { atomicExch(g.err, 91); break; }
+                uint8_t* a_s = smem + s * stage_bytes;
+                if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes);      // both CTAs' halves
                 tma_load_3d_pair(a_s, &tmA, &full[s], 0, a_row, i);
-                tma_load_3d_pair(a_s + FP_KPS * FP_ROWS * BK * 2, &tmB, &full[s], 0, b_row, i);
+                tma_load_3d_pair(a_s + FP_KPS * a_bytes, &tmB, &full[s], 0, b_row, i);
+                if (++s == stages) { s = 0; phase ^= 1; }
             }
         }
     } else if (live && warp == 1) {
         if (rank == 0 && elect_one()) {
-            constexpr uint32_t idesc = umma_idesc_bf16(2 * FP_ROWS, 2 * FP_COLS, 0, 0);
+            constexpr uint32_t idesc = umma_idesc_bf16(BM, 2 * FP_COLS, 0, 0);
             bool good = true;
-            for (int i = 0, it = 0; i < kblocks && good; i += FP_KPS, ++it) {
-                const int s = it % FP_STAGES;
-                if (!mbar_wait(&full[s], (it / FP_STAGES) & 1)) { atomicExch(g.err, 92); good = false; break; }
+            uint32_t phase = 0;
+            for (int i = 0, s = 0; i < kblocks && good; i += FP_KPS) {
+                if (!mbar_wait(&full[s], phase)) { atomicExch(g.err, 92); good = false; break; }
                 tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + s * FP_STAGE_BYTES);
+                const uint32_t a_addr = smem_u32(smem + s * stage_bytes);
 #pragma unroll
                 for (int u = 0; u < FP_KPS; ++u) {
                     if (i + u >= kblocks) break;
-                    const uint64_t ad = umma_desc_sw128(a_addr + u * FP_ROWS * BK * 2, 16, 1024);
-                    const uint64_t bd = umma_desc_sw128(a_addr + FP_KPS * FP_ROWS * BK * 2 + u * FP_COLS * BK * 2, 16, 1024);
+                    const uint64_t ad = umma_desc_sw128(a_addr + u * a_bytes, 16, 1024);
+                    const uint64_t bd = umma_desc_sw128(a_addr + FP_KPS * a_bytes + u * FP_COLS * BK * 2, 16, 1024);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) umma_ss_pair(tmem_base, ad + 2 * k, bd + 2 * k, idesc, (i | u | k) != 0);
                 }
                 umma_commit_pair(&empty[s]);
+                if (++s == stages) { s = 0; phase ^= 1; }
             }
             umma_commit_pair(acc_done);
         }
     } else if (live) {
         // With 64 rows to a CTA the lanes 0..63 of its tensor memory hold the tile's first 32 columns, 64..127 the other 32 of the same rows.
         const int q = warp & 3, failed = error_word(g.err);
-        const int row0 = a_row + (q & 1) * 32, col0 = nb * 2 * FP_COLS + (q >> 1) * FP_COLS, cols = g.N - col0 < FP_COLS ? g.N - col0 : FP_COLS;
-        PlainEpilogue<EPI> plain;
+        const int row0 = a_row + (q & 1) * 32;
+        const int col0 = nb * 2 * FP_COLS + (q >> 1) * FP_COLS, cols = g.N - col0 < FP_COLS ? g.N - col0 : FP_COLS;
+        PlainEpilogue<EPI, true> plain;
+        plain.row_end = a_row + ra < g.M ? a_row + ra : g.M;
         if (cols > 0) plain.ahead(g, row0, col0, cols, 0, lane);
         bool ok = mbar_wait(acc_done, 0);
         if (!ok) atomicExch(g.err, 93);
@@ -2077,10 +2089,11 @@ static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmAr
     return true;
 }
 
-// Narrow tiles on CTA pairs: whole K blocks, from 256 columns on.  One CTA per 32 columns / pairs of 64 (and, before several K blocks to
-// a copy, pairs alone), us: 77 x 4096 x 4096 13.2 / 11.25 (12.7), 16 x 4096 x 4096 13.0 / 11.0 (12.5), 77 x 1024 x 4096 11.5 / 7.8 (11.4), 300 x 1024
-// x 4096 11.9 / 8.9, 128 x 3072 x 4096 13.2 / 10.5, 77 x 1024 x 3072 9.5 / 6.7, 16 x 4096 x 1024 9.0 / 6.3, 77 x 4096 x 1024 5.9 / 6.0, 77 x 4096 x
-// 256 5.9 / 6.0.  Eight K blocks to a copy and two stages 12.3 / 8.8 (the first two of these), two and eight 11.7 / 9.7.
+// Narrow tiles on CTA pairs: whole K blocks, from 256 columns on.  One CTA per 32 columns / pairs of 64 with stages of 128 rows / of the rows
+// there are, us: 77 x 4096 x 4096 13.2 / 11.2 / 10.4, 16 x 4096 x 4096 13.0 / 11.0 / 10.0, 128 x 4096 x 4096 13.4 / 11.3 / 11.3, 77 x 1024 x 4096
+// 11.5 / 7.8 / 7.8, 300 x 1024 x 4096 11.9 / 8.8, 77 x 3072 x 4096 12.8 / 10.4 / 9.9, 8 x 1024 x 4096 13.5 / 8.2 / 7.6, 77 x 1024 x 3072 9.4 / 6.7, 16 x
+// 4096 x 1024 8.3 / 6.2 / 5.0, 77 x 4096 x 1024 6.1 / 6.1, 77 x 4096 x 256 6.1 / 6.0.  Pairs with a copy for each K block 12.7 and 11.4 (the first and
+// the fourth of these); eight K blocks to a copy and two stages 12.3 and 8.8, two and eight 11.7 and 9.7.
 static bool fewpair_pays(const GemmArgs& g) {
     return pair_wanted() && g.num_m * ((g.N + 31) / 32) <= sm_count() && g.K >= 256 && g.K % BK == 0 && !g.a_kblk;
 }
@@ -2090,12 +2103,15 @@ static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, 
     auto kern = gemm_few_pair_kernel<EPI>;
     if (!func_attr_once(attr_done, (const void*)kern, FP_SMEM, "gemm (few tiles, pairs)")) return false;
     CUtensorMap mA, mB;
-    if (!cached_tmap_kblocks(&mA, x, g.M, g.K, ldx, FP_ROWS, FP_KPS) || !cached_tmap_kblocks(&mB, w, g.N, g.K, g.K, FP_COLS, FP_KPS)) return false;
+    const int ra = g.num_m > 1 ? BM / 2 : (g.M + 15) / 16 * 8;      // rows of a CTA: half of the tile's, in eights
+    int stages = FP_ROOM / fp_stage_bytes(ra);
+    if (stages > FP_MAX_STAGES) stages = FP_MAX_STAGES;
+    if (!cached_tmap_kblocks(&mA, x, g.M, g.K, ldx, ra, FP_KPS) || !cached_tmap_kblocks(&mB, w, g.N, g.K, g.K, FP_COLS, FP_KPS)) return false;
     g.num_n = (g.N + 2 * FP_COLS - 1) / (2 * FP_COLS);
     g.prefetch = SK_PREFETCH;
     prof_before(EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : (EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID ? (int)EPI_RESID : EPI),
                 2.0 * g.M * (double)g.N * g.K, st);
-    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(SK_THREADS), FP_SMEM, st, 2, g.M, mA, mB, g);
+    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(SK_THREADS), FP_SMEM, st, 2, g.M, mA, mB, g, ra, stages);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (few tiles, pairs): launch: %s", cudaGetErrorString(e)); return false; }
