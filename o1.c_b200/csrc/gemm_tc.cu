@@ -989,23 +989,23 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 }
 
 // ---------------------------------------------------------------- narrow tiles on CTA pairs
-// The 32-column form with two CTAs to a tile of 128 rows x 64 columns: each has 64 rows of the activations, 32 of the weights and,
-// in its tensor memory, 64 rows of the result; and four K blocks to a copy.  What bounds the narrow tiles is the thread that issues the
-// copies, some 145 cycles for each whatever its size (two for a K block, and one for L2), and shared memory: an MMA of 128 x 32 x 16
+// The 32-column form with two CTAs to a tile of 128 rows x 64 to 128 columns: each has half of the rows of the activations, half of the weights
+// and, in its tensor memory, its rows of the result; and four K blocks to a copy.  What bounds the narrow tiles is the thread that
+// issues the copies, some 145 cycles for each whatever its size (two for a K block, and one for L2), and shared memory: an MMA of 128 x 32 x 16
 // reads 5 KB while the copies write as much, the pair's of 128 x 64 x 16 reads and writes 3 KB on an SM.  Same order of the
-// sum, so the same bits.  fewpair_pays() has both sides' times.
+// sum, so the same bits.  fewpair_cols() has both sides' times.
 // How many bytes of weights are on their way decides the time (77 x 4096 x 4096: two stages of four K blocks 16.6 us, four 11.3), so a stage
 // holds no more rows of the activations than there are: a tile of up to 128 rows is shared evenly, `ra` rows (a multiple of eight)
 // to a CTA.  The MMA reads 64, the others from whatever lies behind: their results are not used.
-static constexpr int FP_KPS = 4, FP_COLS = 32;      // K blocks a stage and copy; columns of a CTA
+static constexpr int FP_KPS = 4;      // K blocks a stage and copy
 static constexpr int FP_MAX_STAGES = 12, FP_ROOM = 216 * 1024;
 static constexpr int FP_SMEM = FP_ROOM + 1024 /*align*/ + 256 /*barriers*/;
-static constexpr int fp_stage_bytes(int ra) { return FP_KPS * (ra + FP_COLS) * BK * 2; }
+__host__ __device__ constexpr int fp_stage_bytes(int ra, int fc) { return FP_KPS * (ra + fc) * BK * 2; }
 
 template <int EPI>
 __global__ void __launch_bounds__(SK_THREADS, 1)
 gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g,
-                     const int ra, const int stages) {
+                     const int ra, const int fc, const int stages) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + FP_ROOM);
@@ -1017,8 +1017,8 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     const uint32_t rank = cluster_rank();
     const int tile = (int)(blockIdx.x >> 1);
     const int nb = tile / g.num_m, mb = tile - nb * g.num_m;      // CTAs that share weights run next to each other
-    const int stage_bytes = fp_stage_bytes(ra), a_bytes = ra * BK * 2;
-    const int a_row = mb * 2 * ra + (int)rank * ra, b_row = nb * 2 * FP_COLS + (int)rank * FP_COLS;
+    const int stage_bytes = fp_stage_bytes(ra, fc), a_bytes = ra * BK * 2;
+    const int a_row = mb * 2 * ra + (int)rank * ra, b_row = nb * 2 * fc + (int)rank * fc;
 
     if (threadIdx.x == 64) *s_abort = error_word(g.err);
     if (threadIdx.x == 96) {
@@ -1026,7 +1026,7 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         mbar_init(acc_done, 1);
         fence_mbar_init();
     }
-    if (warp == 1) { tmem_alloc_pair(tmem_slot, 32); tmem_relinquish_pair(); }
+    if (warp == 1) { tmem_alloc_pair(tmem_slot, 64); tmem_relinquish_pair(); }
     const int kblocks = (g.K + BK - 1) / BK;
     const bool ahead = mb == 0 && g.prefetch > 0;     // the other row tiles find the weights in L2
     if (warp == 0 && elect_one()) {
@@ -1057,7 +1057,7 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
     } else if (live && warp == 1) {
         if (rank == 0 && elect_one()) {
-            constexpr uint32_t idesc = umma_idesc_bf16(BM, 2 * FP_COLS, 0, 0);
+            const uint32_t idesc = umma_idesc_bf16(BM, 2 * fc, 0, 0);
             bool good = true;
             uint32_t phase = 0;
             for (int i = 0, s = 0; i < kblocks && good; i += FP_KPS) {
@@ -1068,7 +1068,7 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 for (int u = 0; u < FP_KPS; ++u) {
                     if (i + u >= kblocks) break;
                     const uint64_t ad = umma_desc_sw128(a_addr + u * a_bytes, 16, 1024);
-                    const uint64_t bd = umma_desc_sw128(a_addr + FP_KPS * a_bytes + u * FP_COLS * BK * 2, 16, 1024);
+                    const uint64_t bd = umma_desc_sw128(a_addr + FP_KPS * a_bytes + u * fc * BK * 2, 16, 1024);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) umma_ss_pair(tmem_base, ad + 2 * k, bd + 2 * k, idesc, (i | u | k) != 0);
                 }
@@ -1078,10 +1078,11 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             umma_commit_pair(acc_done);
         }
     } else if (live) {
-        // With 64 rows to a CTA the lanes 0..63 of its tensor memory hold the tile's first 32 columns, 64..127 the other 32 of the same rows.
+        // With 64 rows to a CTA the lanes 0..63 of its tensor memory hold the first half of the tile's columns, 64..127 the other half of
+        // the same rows.
         const int q = warp & 3, failed = error_word(g.err);
         const int row0 = a_row + (q & 1) * 32;
-        const int col0 = nb * 2 * FP_COLS + (q >> 1) * FP_COLS, cols = g.N - col0 < FP_COLS ? g.N - col0 : FP_COLS;
+        const int col0 = nb * 2 * fc + (q >> 1) * fc, cols = g.N - col0 < fc ? g.N - col0 : fc;
         PlainEpilogue<EPI, true> plain;
         plain.row_end = a_row + ra < g.M ? a_row + ra : g.M;
         if (cols > 0) plain.ahead(g, row0, col0, cols, 0, lane);
@@ -1090,13 +1091,13 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         // (all MMAs are through with the stages, which serve as staging)
-        if (ok && cols > 0) plain.run(g, tmem_base + ((uint32_t)(q * 32) << 16), row0, col0, cols, 0, FP_COLS, smem + (warp - 2) * EPI_SLICE, lane, failed);
+        if (ok && cols > 0) plain.run(g, tmem_base + ((uint32_t)(q * 32) << 16), row0, col0, cols, 0, 32, smem + (warp - 2) * EPI_SLICE, lane, failed);
     }
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still signal it or feed an MMA
     tc_fence_after();
-    if (warp == 1) tmem_dealloc_pair(tmem_base, 32);
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 64);
 }
 
 // ---------------------------------------------------------------- tiles fitted to the number of SMs
@@ -2089,29 +2090,36 @@ static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmAr
     return true;
 }
 
-// Narrow tiles on CTA pairs: whole K blocks, from 256 columns on.  One CTA per 32 columns / pairs of 64 with stages of 128 rows / of the rows
-// there are, us: 77 x 4096 x 4096 13.2 / 11.2 / 10.4, 16 x 4096 x 4096 13.0 / 11.0 / 10.0, 128 x 4096 x 4096 13.4 / 11.3 / 11.3, 77 x 1024 x 4096
-// 11.5 / 7.8 / 7.8, 300 x 1024 x 4096 11.9 / 8.8, 77 x 3072 x 4096 12.8 / 10.4 / 9.9, 8 x 1024 x 4096 13.5 / 8.2 / 7.6, 77 x 1024 x 3072 9.4 / 6.7, 16 x
-// 4096 x 1024 8.3 / 6.2 / 5.0, 77 x 4096 x 1024 6.1 / 6.1, 77 x 4096 x 256 6.1 / 6.0.  Pairs with a copy for each K block 12.7 and 11.4 (the first and
-// the fourth of these); eight K blocks to a copy and two stages 12.3 and 8.8, two and eight 11.7 and 9.7.
-static bool fewpair_pays(const GemmArgs& g) {
-    return pair_wanted() && g.num_m * ((g.N + 31) / 32) <= sm_count() && g.K >= 256 && g.K % BK == 0 && !g.a_kblk;
+// Narrow tiles on CTA pairs: columns of a CTA, or 0 for the one-CTA forms; whole K blocks, K from 256 on.  32 columns where that makes at most
+// one CTA per SM; 48 or 64 where 32 make up to two (two CTAs on an SM have half the room each for weights on their way).  One CTA
+// per 32 columns / pairs with stages of 128 rows / of the rows there are, us: 77 x 4096 x 4096 13.2 / 11.2 / 10.4, 16 x 4096 x 4096 13.0 / 11.0 / 10.0,
+// 128 x 4096 x 4096 13.4 / 11.3 / 11.3, 77 x 1024 x 4096 11.5 / 7.8 / 7.8, 300 x 1024 x 4096 11.9 / 8.8, 77 x 3072 x 4096 12.8 / 10.4 / 9.9, 8 x 1024 x
+// 4096 13.5 / 8.2 / 7.6, 16 x 4096 x 1024 8.3 / 6.2 / 5.0, 77 x 4096 x 1024 6.1 / 6.1, 77 x 4096 x 256 6.1 / 6.0.  Pairs with a copy for each K
+// block 12.7 and 11.4 (the first and the fourth of these); eight K blocks to a copy and two stages 12.3 and 8.8, two and eight 11.7 and
+// 9.7.  Two CTAs of 32 columns on an SM / pairs of 48 or 64: 130 x 4096 x 4096 16.9 / 13.5, 256 x 4096 x 4096 18.3 / 14.3, 520 x 1024 x 4096 17.4 / 11.5,
+// 300 x 3072 x 4096 17.3 / 13.2, 256 x 4608 x 4608 21.9 / 16.2, 520 x 1152 x 1152 7.3 / 6.0, 256 x 4096 x 1024 6.8 / 6.2.  The 96-column form with 96
+// columns of a pair tile to a CTA (two CTAs per SM, five stages of one block): 520 x 4304 x 1152 11.9 / 11.5, x 512 8.5 / 8.9: left alone.
+static int fewpair_cols(const GemmArgs& g) {
+    if (!pair_wanted() || g.K < 256 || g.K % BK != 0 || g.a_kblk) return 0;
+    for (int fc = 32; fc <= 64; fc += 16)
+        if (2 * g.num_m * ((g.N + 2 * fc - 1) / (2 * fc)) <= sm_count()) return fc;
+    return 0;
 }
 template <int EPI>
-static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, cudaStream_t st) {
+static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, int fc, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
     auto kern = gemm_few_pair_kernel<EPI>;
     if (!func_attr_once(attr_done, (const void*)kern, FP_SMEM, "gemm (few tiles, pairs)")) return false;
     CUtensorMap mA, mB;
     const int ra = g.num_m > 1 ? BM / 2 : (g.M + 15) / 16 * 8;      // rows of a CTA: half of the tile's, in eights
-    int stages = FP_ROOM / fp_stage_bytes(ra);
+    int stages = FP_ROOM / fp_stage_bytes(ra, fc);
     if (stages > FP_MAX_STAGES) stages = FP_MAX_STAGES;
-    if (!cached_tmap_kblocks(&mA, x, g.M, g.K, ldx, ra, FP_KPS) || !cached_tmap_kblocks(&mB, w, g.N, g.K, g.K, FP_COLS, FP_KPS)) return false;
-    g.num_n = (g.N + 2 * FP_COLS - 1) / (2 * FP_COLS);
+    if (!cached_tmap_kblocks(&mA, x, g.M, g.K, ldx, ra, FP_KPS) || !cached_tmap_kblocks(&mB, w, g.N, g.K, g.K, fc, FP_KPS)) return false;
+    g.num_n = (g.N + 2 * fc - 1) / (2 * fc);
     g.prefetch = SK_PREFETCH;
     prof_before(EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : (EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID ? (int)EPI_RESID : EPI),
                 2.0 * g.M * (double)g.N * g.K, st);
-    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(SK_THREADS), FP_SMEM, st, 2, g.M, mA, mB, g, ra, stages);
+    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(SK_THREADS), FP_SMEM, st, 2, g.M, mA, mB, g, ra, fc, stages);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (few tiles, pairs): launch: %s", cudaGetErrorString(e)); return false; }
@@ -2124,7 +2132,7 @@ static bool launch_split(const CUtensorMap* tA, const void* x, int ldx, const vo
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, p.bn)) return false;
     switch (p.bn) {
         case 32:
-            if (fewpair_pays(g)) return launch_few_pair<EPI>(x, ldx, w, g, st);
+            if (const int fc = fewpair_cols(g)) return launch_few_pair<EPI>(x, ldx, w, g, fc, st);
             if (g.num_m * ((g.N + 31) / 32) <= sm_count()) return launch_split_bn<EPI, 32, 2>(tA, &mB, g, p.ks, st);
             return launch_split_bn<EPI, 32>(tA, &mB, g, p.ks, st);
         case 96: return launch_split_bn<EPI, 96>(tA, &mB, g, p.ks, st);

@@ -540,10 +540,10 @@ def gemm_form(pkg, M, N, K, epi, bn):
 
 
 @pytest.mark.parametrize("M,N,K", [(8, 72, 256), (77, 4096, 320), (16, 1032, 4096), (17, 512, 832), (33, 1024, 640), (100, 768, 1024), (113, 640, 384), (64, 1024, 576), (65, 3072, 512), (128, 4608, 1152),
-                                   (129, 2048, 448), (300, 1024, 4096), (520, 896, 2048), (1000, 512, 1024)])
+                                   (129, 2048, 448), (300, 1024, 4096), (520, 896, 2048), (1000, 512, 1024), (256, 4608, 704), (130, 3072, 448), (520, 1152, 1152), (300, 1160, 640)])
 @pytest.mark.parametrize("epi", [0, 1, 2, 7, 8, 9])
 def test_narrow_tiles_on_pairs_give_the_bits_of_single_ctas(pkg, dev, M, N, K, epi):
-    """The 32-column form with two CTAs per 128 x 64 tile and four K blocks to a copy against the one-CTA form (pair mode 0), every
+    """The 32-column form with two CTAs per tile of 128 x 64, 96 or 128 and four K blocks to a copy against the one-CTA form (pair mode 0), every
     epilogue: rows shared by the two CTAs in eights, row tiles whose second half has no rows or few, a ragged last column tile, K blocks
     that are no whole number of copies."""
     if epi in (2, 8, 9) and N % 128:
