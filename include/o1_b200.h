@@ -475,8 +475,9 @@ int o1_gemm(const void *x, int ldx, const void *w, const void *w2, void *y, int 
 /* The form o1_gemm gives a problem on the current device (no launch): 0 = a warp per column (*width: rows that share it), 1 =
  * one CTA per tile of 128 rows x *width columns, 2 = two CTAs per 256 x 256 tile (SwiGLU from K = 2048 on also per 256 weight
  * rows x 64 to 256 rows of x, as many as fit their number), 3 = one CTA per tile of a *width fitted to
- * the number of SMs, 4 = the kernel for few tiles of *width columns, *ctas of a cluster sharing the K of each; -1 = not
- * supported.  1 and 3 with *ctas = 2: a CTA pair per tile of 256 rows.  force_bn -1 (which o1_gemm takes too): as 0, and K may
+ * the number of SMs, 4 = the kernels for few tiles: *width = 32 (from K = 256 on two CTAs per 64 to 128 columns where that is the better
+ * way) or 96 columns, or *width = 128 and K summed in *ctas parts (that many CTAs of a cluster, or that many accumulators of a CTA
+ * pair); -1 = not supported.  1 and 3 with *ctas = 2: a CTA pair per tile of 256 rows.  force_bn -1 (which o1_gemm takes too): as 0, and K may
  * be shared; -2 (the vision tower's linears): as -1, and a pair tile of 96 to 256 columns from 257 rows on where K >= 2048 (in
  * place of narrow tiles), from 1025 rows on where 1024 <= K < 2048 and N is no multiple of 256, if that takes fewer rounds. */
 int o1_gemm_form(int M, int N, int K, int epi, int force_bn, int *width, int *ctas);

@@ -125,15 +125,15 @@ static constexpr bool epi_has_resid(int e) { return e == EPI_RESID || e == EPI_B
 static constexpr bool epi_plain(int e) { return e == EPI_STORE || epi_has_bias(e) || epi_has_resid(e); }
 
 // Groups of 32 columns at c_first, c_first + c_step, ... of a tile, plain row-major output (or column blocks, see GemmArgs).
-// LIMIT: rows from row_end on are another CTA's (row_end <= M).
-template <int EPI, bool LIMIT = false>
+// LIMIT: rows from row_end on are another CTA's (row_end <= M).  PARTS: the sum lies in `parts` accumulators, part_cols columns apart.
+template <int EPI, bool LIMIT = false, bool PARTS = false>
 struct PlainEpilogue {
     static_assert(epi_plain(EPI), "this epilogue has no operands by column and element");
     static constexpr bool HAS_BIAS = epi_has_bias(EPI), HAS_RESID = epi_has_resid(EPI);
     // what the next group needs, requested one group ahead: the residual, eight rows of four 16-byte pieces at a time, and the bias
     // (or gate), a piece by each of four lanes
     uint4 rn[4] = {}, bq = {};
-    int row_end = 0;
+    int row_end = 0, parts = 1, part_cols = 0;
     // row0: first of the warp's rows; cols: columns of the tile that exist (a multiple of eight)
     __device__ __forceinline__ void ahead(const GemmArgs& g, int row0, int col0, int cols, int c, int lane) {
         if (HAS_BIAS && lane < 4 && c + lane * 8 < cols) bq = *reinterpret_cast<const uint4*>(g.bias + col0 + c + lane * 8);
@@ -165,6 +165,19 @@ struct PlainEpilogue {
                 __syncwarp();
             }
             tmem_ld_wait();
+            if (PARTS) {
+                // (from zero on, in the order of the parts, as the CTAs of a cluster add theirs)
+#pragma unroll
+                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__fadd_rn(0.f, __uint_as_float(r[j])));
+#pragma unroll 1
+                for (int p = 1; p < parts; ++p) {
+                    uint32_t r2[32];
+                    tmem_ld32(t_row + p * part_cols + c, r2);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(r2[j])));
+                }
+            }
             float v[32];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -666,17 +679,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // ---------------------------------------------------------------- few tiles
 // A problem with few output tiles leaves most SMs idle in the persistent kernel: a 77-row projection is 32 tiles of 128
-// columns, the tower's fc2 at 520 rows 45 tiles of 68 K blocks.  This kernel takes one tile per CTA, two CTAs per SM (one's
-// epilogue runs under the other's main loop), and makes more of them in one of two ways:
-//  * narrower tiles (32 or 96 columns): the same sum for every element, for callers that rely on it;
-//  * the K blocks of a 128-column tile shared by the `ks` CTAs of a cluster.  Each accumulates its part in its own tensor
-//    memory; then CTA r takes over the 16-column units [8r/ks, 8(r+1)/ks): the others write those FP32 columns straight
-//    into its shared memory (one thread per row: consecutive 16-byte pieces, no bank conflicts) and it adds them in rank
-//    order, so the result does not depend on timing and no workspace, atomic or second launch is needed.
-static constexpr int SK_BN = 128;
+// columns, the tower's fc2 at 520 rows 45 tiles of 68 K blocks.  This kernel takes one narrower tile (32 or 96 columns) per CTA, two CTAs
+// per SM (one's epilogue runs under the other's main loop): the same sum for every element, for callers that rely on it.
+// gemm_few_pair_kernel is its form on CTA pairs, and the one that sums a long K in parts.
 // K blocks of weights requested into L2 ahead of their load, before the wait for the previous grid to begin with: three to
-// five stages do not cover the way from memory (1152 x 4304 at 520 rows, five CTAs per tile: 21.0 -> 19.0 us; the
-// persistent kernel's six stages do, and there the requests only cost: 24 -> 32 us at 77 x 4096 x 4096).
+// five stages do not cover the way from memory (the persistent kernel's six do, and there the requests only cost: 24 -> 32 us at
+// 77 x 4096 x 4096).
 static constexpr int SK_PREFETCH = 24;
 // KPS: K blocks per stage.  Two where an SM has one CTA anyway: the trip through a stage's barriers then counts half (a K
 // block of a 32-column tile takes 290 cycles instead of 390-430; 77 x 4096 x 4096 17.8 -> 12.7 us).
@@ -693,15 +701,9 @@ struct SplitCfg {
 static constexpr int VQ_BN = 144;
 static constexpr int VQ_PITCH = 168;     // bytes of a staged row of one head: 16 lanes' 8-byte pieces meet 32 different banks
 
-__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d)
-                 : "memory");
-}
-
 template <int EPI, int BN, int KPS>
 __global__ void __launch_bounds__(SplitCfg<BN, KPS>::THREADS, KPS == 1 ? 2 : 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g,
-                  const int ks) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g) {
     constexpr int SK_STAGE_BYTES = SplitCfg<BN, KPS>::STAGE_BYTES, SK_STAGES = SplitCfg<BN, KPS>::STAGES, NU = BN / 16;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -712,8 +714,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     __shared__ uint4 bias_s[BN / 8];
     const int warp = warp_index(), lane = threadIdx.x & 31;
-    const int rank = (int)(blockIdx.x % ks), tile = (int)(blockIdx.x / ks);
-    const int nb = tile / g.num_m, mb = tile - nb * g.num_m;      // CTAs that share weights run next to each other
+    const int nb = (int)(blockIdx.x / g.num_m), mb = (int)blockIdx.x - nb * g.num_m;      // CTAs that share weights run next to each other
 
     if (threadIdx.x == 64) *s_abort = error_word(g.err);
     if (threadIdx.x == 0) {
@@ -725,10 +726,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     if (warp == 1) { tmem_alloc(tmem_slot, SplitCfg<BN, KPS>::TMEM_COLS); tmem_relinquish(); }
     const int kblocks = (g.K + BK - 1) / BK;
-    const int kb0 = rank * kblocks / ks, nkb = (rank + 1) * kblocks / ks - kb0;
     const bool ahead = mb == 0 && g.prefetch > 0;     // the other row tiles find the weights in L2
     if (ahead && warp == 0 && elect_one())
-        for (int i = 0; i < g.prefetch && i < nkb; ++i) tma_prefetch_2d(&tmB, (kb0 + i) * BK, nb * BN);
+        for (int i = 0; i < g.prefetch && i < kblocks; ++i) tma_prefetch_2d(&tmB, i * BK, nb * BN);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -742,21 +742,21 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
     if (ok && warp == 0) {
         if (elect_one()) {
-            for (int i = 0, it = 0; i < nkb; i += KPS, ++it) {
-                const int s = it % SK_STAGES, n = nkb - i < KPS ? nkb - i : KPS;
+            for (int i = 0, it = 0; i < kblocks; i += KPS, ++it) {
+                const int s = it % SK_STAGES, n = kblocks - i < KPS ? kblocks - i : KPS;
                 if (!mbar_wait(&empty[s], ((it / SK_STAGES) & 1) ^ 1)) { atomicExch(g.err, 51); break; }
                 uint8_t* a_s = smem + s * SK_STAGE_BYTES;
                 mbar_expect_tx(&full[s], n * (SK_STAGE_BYTES / KPS));
                 for (int u = 0; u < n; ++u) {
-                    if (ahead && i + u + g.prefetch < nkb) tma_prefetch_2d(&tmB, (kb0 + i + u + g.prefetch) * BK, nb * BN);
-                    int a_c0 = (kb0 + i + u) * BK, a_c1 = mb * BM;
+                    if (ahead && i + u + g.prefetch < kblocks) tma_prefetch_2d(&tmB, (i + u + g.prefetch) * BK, nb * BN);
+                    int a_c0 = (i + u) * BK, a_c1 = mb * BM;
                     if (g.a_kblk > 0) {
                         const int blk = a_c0 / g.a_kblk;
                         a_c0 -= blk * g.a_kblk;
                         a_c1 += blk * g.a_rows;
                     }
                     tma_load_2d(a_s + u * BM * BK * 2, &tmA, &full[s], a_c0, a_c1);
-                    tma_load_2d(a_s + KPS * BM * BK * 2 + u * BN * BK * 2, &tmB, &full[s], (kb0 + i + u) * BK, nb * BN);
+                    tma_load_2d(a_s + KPS * BM * BK * 2 + u * BN * BK * 2, &tmB, &full[s], (i + u) * BK, nb * BN);
                 }
             }
         }
@@ -764,14 +764,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, 0, 0);
             bool good = true;
-            for (int i = 0, it = 0; i < nkb && good; i += KPS, ++it) {
+            for (int i = 0, it = 0; i < kblocks && good; i += KPS, ++it) {
                 const int s = it % SK_STAGES;
                 if (!mbar_wait(&full[s], (it / SK_STAGES) & 1)) { atomicExch(g.err, 52); good = false; break; }
                 tc_fence_after();
                 const uint32_t a_addr = smem_u32(smem + s * SK_STAGE_BYTES);
 #pragma unroll
                 for (int u = 0; u < KPS; ++u) {
-                    if (i + u >= nkb) break;
+                    if (i + u >= kblocks) break;
                     const uint64_t ad = umma_desc_sw128(a_addr + u * BM * BK * 2, 16, 1024);
                     const uint64_t bd = umma_desc_sw128(a_addr + KPS * BM * BK * 2 + u * BN * BK * 2, 16, 1024);
 #pragma unroll
@@ -807,7 +807,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     constexpr bool HAS_BIAS = epi_has_bias(EPI) || EPI == EPI_VROPE, HAS_RESID = epi_has_resid(EPI);
     const int q = warp & 3;       // TMEM lane quadrant this warp may access
     const int trow = q * 32 + lane;
-    const int u0 = rank * NU / ks, u1 = (rank + 1) * NU / ks;     // this CTA's share of the tile's 16-column units
     const int row = mb * BM + trow;
     const bool row_ok = row < g.M;
     uint4 res[HAS_RESID ? 2 * NU : 1];
@@ -831,8 +830,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
             for (int h = 0; h < 2 * NU; ++h) {
                 const int col = nb * BN + h * 8;
-                res[h] = row_ok && col < g.N && h >= 2 * u0 && h < 2 * u1
-                             ? *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col) : make_uint4(0, 0, 0, 0);
+                res[h] = row_ok && col < g.N ? *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col) : make_uint4(0, 0, 0, 0);
             }
         }
         if (HAS_BIAS) asm volatile("bar.sync 1, 128;" ::: "memory");      // the four epilogue warps
@@ -904,35 +902,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN, KPS>::TMEM_COLS);
         return;
     }
-    const int mu = (NU + ks - 1) / ks;                            // most units a CTA owns
-    if (ks > 1) {
-        // every CTA's MMAs are through with its stages, which now receive the others' columns:
-        // [source][unit][4 columns][row] of 16 bytes: (ks - 1) x mu units of 8 KB, see split_exchange_fits()
-        __syncwarp();
-        cluster_sync_all();
-        if (ok && warp >= 2) {
-            for (int dst = 0; dst < ks; ++dst) {
-                if (dst == rank) continue;
-                const uint32_t base = map_to_rank(smem_u32(smem), dst);
-                const int slot = rank < dst ? rank : rank - 1, d0 = dst * NU / ks, d1 = (dst + 1) * NU / ks;
-                for (int u = d0; u < d1; ++u) {
-                    uint32_t r[16];
-                    tmem_ld16(t_row + u * 16, r);
-                    tmem_ld_wait();
-                    const uint32_t at = base + (uint32_t)((((slot * mu + u - d0) * 4) * BM + trow) * 16);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        st_cluster_v4(at + c * BM * 16, r[c * 4], r[c * 4 + 1], r[c * 4 + 2], r[c * 4 + 3]);
-                }
-            }
-        }
-        __syncwarp();
-        cluster_sync_all();
-    }
     if (ok && warp >= 2) {
 #pragma unroll
         for (int u = 0; u < NU; ++u) {
-            if (u < u0 || u >= u1) continue;
             const int col = nb * BN + u * 16;
             // (N is a multiple of eight: a unit is whole, its first half, or outside)
             const bool h0 = store && col < g.N, h1 = store && col + 8 < g.N;
@@ -941,21 +913,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             tmem_ld_wait();
             float v[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = 0.f;
-            for (int src = 0; src < ks; ++src) {
-                if (src == rank) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
-                } else {
-                    const int slot = src < rank ? src : src - 1;
-                    const uint8_t* at = smem + (size_t)((((slot * mu + u - u0) * 4) * BM + trow) * 16);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const float4 f = *reinterpret_cast<const float4*>(at + c * BM * 16);
-                        v[c * 4] += f.x; v[c * 4 + 1] += f.y; v[c * 4 + 2] += f.z; v[c * 4 + 3] += f.w;
-                    }
-                }
-            }
+            for (int j = 0; j < 16; ++j) v[j] = __fadd_rn(0.f, __uint_as_float(r[j]));
             // the rounding points of gemm_tc_kernel's epilogues
             float b[16], rs[16];
 #pragma unroll
@@ -993,7 +951,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // and, in its tensor memory, its rows of the result; and four K blocks to a copy.  What bounds the narrow tiles is the thread that
 // issues the copies, some 145 cycles for each whatever its size (two for a K block, and one for L2), and shared memory: an MMA of 128 x 32 x 16
 // reads 5 KB while the copies write as much, the pair's of 128 x 64 x 16 reads and writes 3 KB on an SM.  Same order of the
-// sum, so the same bits.  fewpair_cols() has both sides' times.
+// sum, so the same bits.
+// PARTS: so too where the K of a tile is to be summed in parts.  The parts, which a cluster's CTAs share in gemm_split_kernel, follow one
+// another here, each in an accumulator of its own, and the epilogue adds them in their order.  (At 520 x 1152 x 4304 the exchange
+// took 13,000 of that kernel's 33,000 cycles, the main loop 11,000.)  fewpair_cols() has both sides' times.
 // How many bytes of weights are on their way decides the time (77 x 4096 x 4096: two stages of four K blocks 16.6 us, four 11.3), so a stage
 // holds no more rows of the activations than there are: a tile of up to 128 rows is shared evenly, `ra` rows (a multiple of eight)
 // to a CTA.  The MMA reads 64, the others from whatever lies behind: their results are not used.
@@ -1002,13 +963,14 @@ static constexpr int FP_MAX_STAGES = 12, FP_ROOM = 216 * 1024;
 static constexpr int FP_SMEM = FP_ROOM + 1024 /*align*/ + 256 /*barriers*/;
 __host__ __device__ constexpr int fp_stage_bytes(int ra, int fc) { return FP_KPS * (ra + fc) * BK * 2; }
 
-template <int EPI>
+template <int EPI, bool PARTS>
 __global__ void __launch_bounds__(SK_THREADS, 1)
-gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g,
-                     const int ra, const int fc, const int stages) {
+gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2, const GemmArgs g, const int ra, const int fc,
+                     const int stages, const int parts) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + FP_ROOM);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + stages * fp_stage_bytes(ra, fc));
     uint64_t* empty = full + FP_MAX_STAGES;
     uint64_t* acc_done = empty + FP_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
@@ -1026,13 +988,14 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         mbar_init(acc_done, 1);
         fence_mbar_init();
     }
-    if (warp == 1) { tmem_alloc_pair(tmem_slot, 64); tmem_relinquish_pair(); }
-    const int kblocks = (g.K + BK - 1) / BK;
+    if (warp == 1) { tmem_alloc_pair(tmem_slot, PARTS ? 512 : 64); tmem_relinquish_pair(); }
+    // whole K blocks come FP_KPS to a copy, a ragged last one by itself (tmA2, tmB2)
+    const int kblocks = (g.K + BK - 1) / BK, kwhole = g.K / BK;
     const bool ahead = mb == 0 && g.prefetch > 0;     // the other row tiles find the weights in L2
     if (warp == 0 && elect_one()) {
         tma_prefetch_desc(&tmB);
         tma_prefetch_desc(&tmA);
-        if (ahead) for (int i = 0; i < g.prefetch && i < kblocks; i += FP_KPS) tma_prefetch_3d(&tmB, 0, b_row, i);
+        if (ahead) for (int i = 0; i < g.prefetch && i < kwhole; i += FP_KPS) tma_prefetch_3d(&tmB, 0, b_row, i);
     }
     tc_fence_before();
     __syncthreads();
@@ -1046,32 +1009,45 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (live && warp == 0) {
         if (elect_one()) {
             uint32_t phase = 0;
-            for (int i = 0, s = 0; i < kblocks; i += FP_KPS) {
+            for (int i = 0, s = 0; i < kblocks;) {
                 if (!mbar_wait(&empty[s], phase ^ 1)) { atomicExch(g.err, 91); break; }
                 uint8_t* a_s = smem + s * stage_bytes;
-                if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes);      // both CTAs' halves
-                tma_load_3d_pair(a_s, &tmA, &full[s], 0, a_row, i);
-                tma_load_3d_pair(a_s + FP_KPS * a_bytes, &tmB, &full[s], 0, b_row, i);
+                if (i < kwhole) {
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes);      // both CTAs' halves
+                    tma_load_3d_pair(a_s, &tmA, &full[s], 0, a_row, i);
+                    tma_load_3d_pair(a_s + FP_KPS * a_bytes, &tmB, &full[s], 0, b_row, i);
+                    i = i + FP_KPS < kwhole ? i + FP_KPS : kwhole;
+                } else {
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes / FP_KPS);
+                    tma_load_2d_pair(a_s, &tmA2, &full[s], i * BK, a_row);
+                    tma_load_2d_pair(a_s + FP_KPS * a_bytes, &tmB2, &full[s], i * BK, b_row);
+                    ++i;
+                }
                 if (++s == stages) { s = 0; phase ^= 1; }
             }
         }
     } else if (live && warp == 1) {
         if (rank == 0 && elect_one()) {
             const uint32_t idesc = umma_idesc_bf16(BM, 2 * fc, 0, 0);
-            bool good = true;
-            uint32_t phase = 0;
-            for (int i = 0, s = 0; i < kblocks && good; i += FP_KPS) {
-                if (!mbar_wait(&full[s], phase)) { atomicExch(g.err, 92); good = false; break; }
+            uint32_t phase = 0, d = tmem_base;
+            int p = 0, p_end = kblocks / parts;      // K part, first K block of the next one
+            bool fresh = true;                       // nothing in its accumulator yet
+            for (int i = 0, s = 0; i < kblocks;) {
+                if (!mbar_wait(&full[s], phase)) { atomicExch(g.err, 92); break; }
                 tc_fence_after();
                 const uint32_t a_addr = smem_u32(smem + s * stage_bytes);
+                const int n = i < kwhole ? (kwhole - i < FP_KPS ? kwhole - i : FP_KPS) : 1;
 #pragma unroll
                 for (int u = 0; u < FP_KPS; ++u) {
-                    if (i + u >= kblocks) break;
+                    if (u >= n) break;
+                    if (PARTS && i + u == p_end && p + 1 < parts) { ++p; p_end = (p + 1) * kblocks / parts; d += fc; fresh = true; }
                     const uint64_t ad = umma_desc_sw128(a_addr + u * a_bytes, 16, 1024);
                     const uint64_t bd = umma_desc_sw128(a_addr + FP_KPS * a_bytes + u * fc * BK * 2, 16, 1024);
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) umma_ss_pair(tmem_base, ad + 2 * k, bd + 2 * k, idesc, (i | u | k) != 0);
+                    for (int k = 0; k < BK / 16; ++k) umma_ss_pair(d, ad + 2 * k, bd + 2 * k, idesc, k != 0 || !fresh);
+                    fresh = false;
                 }
+                i += n;
                 umma_commit_pair(&empty[s]);
                 if (++s == stages) { s = 0; phase ^= 1; }
             }
@@ -1083,8 +1059,9 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int q = warp & 3, failed = error_word(g.err);
         const int row0 = a_row + (q & 1) * 32;
         const int col0 = nb * 2 * fc + (q >> 1) * fc, cols = g.N - col0 < fc ? g.N - col0 : fc;
-        PlainEpilogue<EPI, true> plain;
+        PlainEpilogue<EPI, true, PARTS> plain;
         plain.row_end = a_row + ra < g.M ? a_row + ra : g.M;
+        if (PARTS) { plain.parts = parts; plain.part_cols = fc; }
         if (cols > 0) plain.ahead(g, row0, col0, cols, 0, lane);
         bool ok = mbar_wait(acc_done, 0);
         if (!ok) atomicExch(g.err, 93);
@@ -1097,7 +1074,7 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     __syncthreads();
     cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still signal it or feed an MMA
     tc_fence_after();
-    if (warp == 1) tmem_dealloc_pair(tmem_base, 64);
+    if (warp == 1) tmem_dealloc_pair(tmem_base, PARTS ? 512 : 64);
 }
 
 // ---------------------------------------------------------------- tiles fitted to the number of SMs
@@ -1973,18 +1950,16 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
     return true;
 }
 
-// Which form of gemm_split_kernel a problem takes: tile width and CTAs per tile; width 0: the persistent kernel is the
+// Which form for few tiles a problem takes: tile width and parts of K; width 0: the persistent kernel is the
 // better one.  Times in us, persistent kernel with 128-column tiles against this one:
 //  * 32 columns where that makes at most two CTAs per SM: 77 x 4096 x 4096 19.4 / 12.7, 520 x 1152 x 1152 11.1 / 8.7,
 //    130 x 4608 x 4608 23.9 / 20.0; beyond, the activations are read too often: 296 x 4096 x 4096 19.6 / 31.6
 //  * 96 columns where the wider tiles need a second round and these do not, and K is short: 2916 x 1152 x 1152 16.0 / 12.5,
 //    520 x 4304 x 1152 16.4 / 14.1; 593 x 4096 x 12288 86 / 84, where CTA pairs take 72
-//  * K over a cluster where even narrow tiles leave a long main loop: 520 x 1152 x 4304 23.5 / 18.7 (five CTAs, 32 columns
-//    27.2), 96 x 1152 x 4304 22.2 / 12.9 (six; 16.2); with 64 tiles and more 32 columns are as good (130 x 4096 x 4608).
-//    (Narrow tiles have become faster since, with two K blocks a stage and the epilogue through shared memory: where there is at most
-//    one for each SM they are ahead of the shared K, 160 to 512 x 1152 x 4304 15 / 18-19, 128 x 4608 x 4608 15.1 / 19.2,
-//    256 x 2048 x 4096 11.9 / 17.0; not with one row tile of 36 narrow ones, 96 x 1152 x 4304 14.0 / 12.2, nor beyond one per SM,
-//    520 x 1152 x 4304 26.8 / 18.7.  The order of those sums, hence the tower's bits, hangs on this rule.)
+//  * a long K in parts (bn 128, ks parts), for callers that allow that order of the sum: what once went over the CTAs of a cluster, where
+//    even narrow tiles left a long main loop (520 x 1152 x 4304 23.5 / 18.7, five CTAs; 96 x 1152 x 4304 22.2 / 12.9, six).  Narrow pair
+//    tiles take it now with an accumulator for each part (13.5, 10.4), and take half the time whole or in parts; the parts stay, for the
+//    tower's bits, and because shorter chains of sums misround less (7,883 of 13.6 M results of the tower's linears against 37,310).
 // But few rows of a long K (small_rows()) are read by fewer SMs in wider tiles: by at most half of them from K = 2048 on, by no
 // more than all from K = 512 on.  Narrow / 128 columns / before there were narrow ones: 10 x 4096 x 4096 27.4 / 22.5 / 24.6,
 // 10 x 6144 x 4096 52.0 / 26.5 / 26.3, 12 x 8192 x 2048 28.7 / 18.3 / 19.7, 33 x 8192 x 1024 13.7 / 9.8 / 12.3, 12 x 8192 x 512
@@ -1993,11 +1968,7 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
 // / 1.93 / 3.15 ms.  K of no whole 64 columns, whose rows lie across the memory's lines, gains nothing from two CTAs per SM
 // (640 x 1152 x 4304 27.0 / 22.5 / 26.7) except where a residual is added (the tower of 832 patches 2.66 / 2.70 ms).
 struct SplitPlan { int bn, ks; };
-static constexpr int MAX_SPLIT = 6;
-// A CTA's stages have to hold the columns it takes over from the ks - 1 others (six CTAs: 5 x 2 units of 8 KB in 96 KB).
-static constexpr bool split_exchange_fits(int bn, int ks, int stage_total) {
-    return (ks - 1) * ((bn / 16 + ks - 1) / ks) * 8192 <= stage_total;
-}
+static constexpr int MAX_SPLIT = 6;      // (accumulators of 64 columns at most: 384 of tensor memory's 512)
 static SplitPlan split_plan(int M, int N, int K, bool may_split, bool resid) {
     const int sms = sm_count(), kblocks = (K + BK - 1) / BK;
     const long num_m = (M + BM - 1) / BM;
@@ -2069,13 +2040,9 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
 }
 
 template <int EPI, int BN, int KPS = 1>
-static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmArgs& g, int ks, cudaStream_t st) {
+static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmArgs& g, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
     constexpr int SMEM = SplitCfg<BN, KPS>::SMEM;
-    if (ks < 1 || ks > MAX_SPLIT || !split_exchange_fits(BN, ks, SplitCfg<BN, KPS>::STAGES * SplitCfg<BN, KPS>::STAGE_BYTES)) {
-        set_error("gemm (few tiles): %d CTAs cannot share a %d-column tile", ks, BN);
-        return false;
-    }
     auto kern = gemm_split_kernel<EPI, BN, KPS>;
     if (!func_attr_once(attr_done, (const void*)kern, SMEM, "gemm (few tiles)")) return false;
     g.num_n = (g.N + BN - 1) / BN;
@@ -2083,43 +2050,53 @@ static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmAr
     prof_before((EPI == EPI_BIAS_GELU || EPI == EPI_VROPE) ? (int)EPI_BIAS
                                                            : ((EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID) ? (int)EPI_RESID : EPI),
                 2.0 * g.M * (double)g.N * g.K, st);
-    cudaError_t e = launch_chained(kern, dim3(g.num_m * g.num_n * ks), dim3(SplitCfg<BN, KPS>::THREADS), SMEM, st, ks, g.M, *tA, *tB, g, ks);
+    cudaError_t e = launch_chained(kern, dim3(g.num_m * g.num_n), dim3(SplitCfg<BN, KPS>::THREADS), SMEM, st, 1, g.M, *tA, *tB, g);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (few tiles): launch: %s", cudaGetErrorString(e)); return false; }
     return true;
 }
 
-// Narrow tiles on CTA pairs: columns of a CTA, or 0 for the one-CTA forms; whole K blocks, K from 256 on.  32 columns where that makes at most
-// one CTA per SM; 48 or 64 where 32 make up to two (two CTAs on an SM have half the room each for weights on their way).  One CTA
-// per 32 columns / pairs with stages of 128 rows / of the rows there are, us: 77 x 4096 x 4096 13.2 / 11.2 / 10.4, 16 x 4096 x 4096 13.0 / 11.0 / 10.0,
-// 128 x 4096 x 4096 13.4 / 11.3 / 11.3, 77 x 1024 x 4096 11.5 / 7.8 / 7.8, 300 x 1024 x 4096 11.9 / 8.8, 77 x 3072 x 4096 12.8 / 10.4 / 9.9, 8 x 1024 x
-// 4096 13.5 / 8.2 / 7.6, 16 x 4096 x 1024 8.3 / 6.2 / 5.0, 77 x 4096 x 1024 6.1 / 6.1, 77 x 4096 x 256 6.1 / 6.0.  Pairs with a copy for each K
-// block 12.7 and 11.4 (the first and the fourth of these); eight K blocks to a copy and two stages 12.3 and 8.8, two and eight 11.7 and
-// 9.7.  Two CTAs of 32 columns on an SM / pairs of 48 or 64: 130 x 4096 x 4096 16.9 / 13.5, 256 x 4096 x 4096 18.3 / 14.3, 520 x 1024 x 4096 17.4 / 11.5,
-// 300 x 3072 x 4096 17.3 / 13.2, 256 x 4608 x 4608 21.9 / 16.2, 520 x 1152 x 1152 7.3 / 6.0, 256 x 4096 x 1024 6.8 / 6.2.  The 96-column form with 96
-// columns of a pair tile to a CTA (two CTAs per SM, five stages of one block): 520 x 4304 x 1152 11.9 / 11.5, x 512 8.5 / 8.9: left alone.
-static int fewpair_cols(const GemmArgs& g) {
-    if (!pair_wanted() || g.K < 256 || g.K % BK != 0 || g.a_kblk) return 0;
+// Narrow tiles on CTA pairs: columns of a CTA, or 0 for the one-CTA forms; K from 256 on.  32 columns where that makes at most one CTA per
+// SM, else 48 or 64 (two CTAs of 32 columns on an SM have half the room each for weights on their way).  One CTA per 32 columns / pairs,
+// us: 77 x 4096 x 4096 13.2 / 10.2, 16 x 4096 x 4096 13.0 / 10.0, 128 x 4096 x 4096 13.4 / 11.3, 77 x 1024 x 4096 11.5 / 7.8, 300 x 1024 x 4096
+// 11.9 / 8.8, 77 x 1024 x 3072 9.4 / 6.7, 16 x 4096 x 1024 8.5 / 4.4, 77 x 4096 x 1024 4.95 / 4.95, 77 x 4096 x 256 3.5 / 3.3, 256 x 1152 x 1152 4.85 / 4.26;
+// a short K of more than two row tiles only where 32 columns do not fit: 300 x 1152 x 1152 5.07 / 5.11, 512 x 1152 x 1152 5.26 / 5.61.  (A copy
+// for each K block: 77 x 4096 x 4096 12.7, 77 x 1024 x 4096 11.4; stages of 128 rows: 11.2 and 7.8; eight K blocks to a copy and two stages
+// 12.3 and 8.8, two and eight 11.7 and 9.7.)  Two CTAs of 32 columns on an SM / pairs of 48 or 64: 130 x 4096 x 4096 16.9 / 13.5, 256 x 4096 x
+// 4096 18.3 / 14.3, 520 x 1024 x 4096 17.4 / 11.5, 300 x 3072 x 4096 17.3 / 13.2, 256 x 4608 x 4608 21.9 / 16.2, 520 x 1152 x 1152 6.8 / 6.1, 200 x
+// 4096 x 1024 6.3 / 5.8.  K shared by the CTAs of a cluster / the parts' accumulators in one pair: 520 x 1152 x 4304 18.4 / 13.5, 160 x 1152 x
+// 4304 17.6 / 11.0, 96 x 1152 x 4304 12.1 / 10.4, 128 x 4608 x 4608 19.3 / 13.4, 128 x 4096 x 4608 18.1 / 12.2, 300 x 1024 x 2112 14.4 / 7.5, 9 x 4096
+// x 4104 23.5 / 12.4.  The 96-column form with 96 columns of a pair tile to a CTA (two CTAs per SM, five stages of one block): 520 x 4304 x 1152
+// 11.9 / 11.5, x 512 8.5 / 8.9: left alone.
+static int fewpair_cols(const GemmArgs& g, int parts) {
+    if (!pair_wanted() || g.K < 256 || g.a_kblk) return 0;
     for (int fc = 32; fc <= 64; fc += 16)
-        if (2 * g.num_m * ((g.N + 2 * fc - 1) / (2 * fc)) <= sm_count()) return fc;
+        if (2 * g.num_m * ((g.N + 2 * fc - 1) / (2 * fc)) <= sm_count()) return fc == 32 && g.num_m > 2 && g.K < LONG_K && parts == 1 ? 0 : fc;
     return 0;
 }
-template <int EPI>
-static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, int fc, cudaStream_t st) {
+template <int EPI, bool PARTS>
+static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, int fc, int parts, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
-    auto kern = gemm_few_pair_kernel<EPI>;
+    auto kern = gemm_few_pair_kernel<EPI, PARTS>;
     if (!func_attr_once(attr_done, (const void*)kern, FP_SMEM, "gemm (few tiles, pairs)")) return false;
     CUtensorMap mA, mB;
     const int ra = g.num_m > 1 ? BM / 2 : (g.M + 15) / 16 * 8;      // rows of a CTA: half of the tile's, in eights
     int stages = FP_ROOM / fp_stage_bytes(ra, fc);
     if (stages > FP_MAX_STAGES) stages = FP_MAX_STAGES;
-    if (!cached_tmap_kblocks(&mA, x, g.M, g.K, ldx, ra, FP_KPS) || !cached_tmap_kblocks(&mB, w, g.N, g.K, g.K, fc, FP_KPS)) return false;
+    // no more room than the K blocks take: a short K leaves some for the next kernel's CTAs
+    const int copies = (g.K / BK + FP_KPS - 1) / FP_KPS + (g.K % BK != 0);
+    if (stages > copies) stages = copies;
+    const int smem = stages * fp_stage_bytes(ra, fc) + 1024 /*align*/ + 256 /*barriers*/;
+    const int kw = g.K / BK * BK;
+    if (!cached_tmap_kblocks(&mA, x, g.M, kw, ldx, ra, FP_KPS) || !cached_tmap_kblocks(&mB, w, g.N, kw, g.K, fc, FP_KPS)) return false;
+    CUtensorMap mA2 = mA, mB2 = mB;
+    if (kw != g.K && (!cached_tmap(&mA2, x, g.M, g.K, ldx, ra) || !cached_tmap(&mB2, w, g.N, g.K, g.K, fc))) return false;
     g.num_n = (g.N + 2 * fc - 1) / (2 * fc);
     g.prefetch = SK_PREFETCH;
     prof_before(EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : (EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID ? (int)EPI_RESID : EPI),
                 2.0 * g.M * (double)g.N * g.K, st);
-    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(SK_THREADS), FP_SMEM, st, 2, g.M, mA, mB, g, ra, fc, stages);
+    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(SK_THREADS), smem, st, 2, g.M, mA, mB, mA2, mB2, g, ra, fc, stages, parts);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (few tiles, pairs): launch: %s", cudaGetErrorString(e)); return false; }
@@ -2128,16 +2105,14 @@ static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, 
 
 template <int EPI>
 static bool launch_split(const CUtensorMap* tA, const void* x, int ldx, const void* w, GemmArgs& g, const GemmPlan& p, cudaStream_t st) {
+    if (p.bn != 96)
+        if (const int fc = fewpair_cols(g, p.ks)) return p.ks > 1 ? launch_few_pair<EPI, true>(x, ldx, w, g, fc, p.ks, st) : launch_few_pair<EPI, false>(x, ldx, w, g, fc, 1, st);
     CUtensorMap mB;
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, p.bn)) return false;
-    switch (p.bn) {
-        case 32:
-            if (const int fc = fewpair_cols(g)) return launch_few_pair<EPI>(x, ldx, w, g, fc, st);
-            if (g.num_m * ((g.N + 31) / 32) <= sm_count()) return launch_split_bn<EPI, 32, 2>(tA, &mB, g, p.ks, st);
-            return launch_split_bn<EPI, 32>(tA, &mB, g, p.ks, st);
-        case 96: return launch_split_bn<EPI, 96>(tA, &mB, g, p.ks, st);
-        default: return launch_split_bn<EPI, 128>(tA, &mB, g, p.ks, st);
-    }
+    if (p.bn == 96) return launch_split_bn<EPI, 96>(tA, &mB, g, st);
+    if (p.bn == 32) return g.num_m * ((g.N + 31) / 32) <= sm_count() ? launch_split_bn<EPI, 32, 2>(tA, &mB, g, st) : launch_split_bn<EPI, 32>(tA, &mB, g, st);
+    set_error("gemm (few tiles): no kernel for %d columns and %d parts of K", p.bn, p.ks);
+    return false;
 }
 
 // Rows that share a warp of gemm_simt_kernel, which then reads a weight once for all of them; equal groups of at most four.
@@ -2271,7 +2246,7 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
         set_error("gemm: BN=256 needs N (and the output column block) %% 256 == 0");
         return false;
     }
-    const GemmPlan p = gemm_plan(M, N, K, epi, force_bn, !o_cb && !o_tab, wide_ok);
+    const GemmPlan p = gemm_plan(M, N, K, epi, a_kblk && force_bn < 0 ? 0 : force_bn, !o_cb && !o_tab, wide_ok);     // (K in parts: plain rows)
     if (epi == EPI_SWIGLU) {
         const int bn = force_bn == 0 && !a_kblk ? swiglu_rows_width(M, N, K) : 0;
         if (bn) {
@@ -2419,8 +2394,8 @@ bool gemm_vision_qkv(const void* x, const void* w, const void* b, void* y, int M
     CUtensorMap mA, mB;
     if (!cached_tmap(&mA, x, M, K, K, 128) || !cached_tmap(&mB, w, N, K, K, VQ_BN)) return false;
     // (with one CTA per SM, two K blocks a stage, see SplitCfg: the tower at 520 patches 2155 -> 2058 us)
-    if (g.num_m * (N / VQ_BN) <= sm_count()) return launch_split_bn<EPI_VROPE, VQ_BN, 2>(&mA, &mB, g, 1, st);
-    return launch_split_bn<EPI_VROPE, VQ_BN>(&mA, &mB, g, 1, st);
+    if (g.num_m * (N / VQ_BN) <= sm_count()) return launch_split_bn<EPI_VROPE, VQ_BN, 2>(&mA, &mB, g, st);
+    return launch_split_bn<EPI_VROPE, VQ_BN>(&mA, &mB, g, st);
 }
 
 }  // namespace o1

@@ -36,8 +36,8 @@ void prof_after(cudaStream_t st);
 // gemm_pair_mode).  GEMM_TOWER = the same for the vision tower's linears, whose long K takes pair tiles of any width.
 enum { GEMM_SPLIT_K = -1, GEMM_TOWER = -2 };
 // The form a problem takes: GEMM_ROWS = warps (bn: rows that share one), GEMM_TILE = one CTA per 128 x bn tile, GEMM_PAIR = two
-// per 256 x 256 tile (SwiGLU: or 256 weight rows x a fitted number of rows), GEMM_FIT = one per tile of a width fitted to the SMs, GEMM_FEW = tiles for problems that have few (ks CTAs of
-// a cluster share a tile's K).  GEMM_TILE and GEMM_FIT with ks = 2: a CTA pair per 256 x bn tile.
+// per 256 x 256 tile (SwiGLU: or 256 weight rows x a fitted number of rows), GEMM_FIT = one per tile of a width fitted to the SMs,
+// GEMM_FEW = tiles for problems that have few (a tile's K is summed in ks parts).  GEMM_TILE and GEMM_FIT with ks = 2: a CTA pair per 256 x bn tile.
 enum GemmForm { GEMM_ROWS = 0, GEMM_TILE = 1, GEMM_PAIR = 2, GEMM_FIT = 3, GEMM_FEW = 4 };
 struct GemmPlan { int form, bn, ks; };
 GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok);

@@ -569,6 +569,29 @@ def test_narrow_tiles_on_pairs_give_the_bits_of_single_ctas(pkg, dev, M, N, K, e
     assert pkg.lib.o1_device_error() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(520, 1152, 4304), (9, 72, 2120), (96, 1152, 4304), (128, 4608, 2048), (257, 1160, 2112), (640, 1024, 2000),
+                                   (300, 128, 4104)])
+def test_k_in_parts_is_added_in_the_order_of_the_parts(pkg, dev, M, N, K):
+    """A K that is summed in parts: a part's first product is all there is in it, 2^24, 1, -2^24, 1, .., so that the FP32 sum of the parts from
+    zero on is 1 or 2 more where their order is another (2^24 + 1 is 2^24 there)."""
+    form = gemm_form(pkg, M, N, K, 0, -1)
+    if pkg.lib.o1_sm_count() == 148:
+        assert form[:2] == (4, 128) and form[2] > 1
+    x, w = (torch.zeros(r, K, dtype=torch.bfloat16, device=dev) for r in (M, N))
+    kb, want = (K + 63) // 64, np.float32(0)
+    for p in range(form[2]):
+        big = {0: 4096.0, 2: -4096.0}.get(p)
+        x[:, p * kb // form[2] * 64] = big or 1.0
+        w[:, p * kb // form[2] * 64] = 4096.0 if big else 1.0
+        want = np.float32(want + np.float32(4096.0 * big if big else 1.0))
+    y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
+    assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N + 8, M, N, K, 0, None, None, N, 0.0, -1) == 0, pkg.last_error()
+    done(pkg, "K in parts")
+    assert (y[:M, :N] == float(want)).all(), (y[0, 0].item(), want)
+    assert (y[M:] == 777.0).all() and (y[:, N:] == 777.0).all(), "written beyond the matrix"
+    assert pkg.lib.o1_device_error() == 0
+
+
 def gelu_tanh_f64(v):
     """0.5 v (1 + tanh u) = v / (1 + e^-2u): in 64 bits too, 1 + tanh u has no digits left where u is far below zero."""
     return v / (1 + torch.exp(-2 * 0.7978845608028654 * (v + 0.044715 * v ** 3)))
