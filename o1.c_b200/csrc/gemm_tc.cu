@@ -694,7 +694,8 @@ struct SplitCfg {
     static constexpr int STAGE_BYTES = KPS * (BM + BN) * BK * 2;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
     static constexpr int TMEM_COLS = BN <= 32 ? 32 : (BN <= 128 ? 128 : 256);
-    static constexpr int THREADS = BN == 96 ? GEMM_THREADS : SK_THREADS;     // (32 columns are one group for each quadrant)
+    // (32 columns are one group for each quadrant; two CTAs of 144 have no registers for more)
+    static constexpr int THREADS = BN == 96 || (BN == 144 && KPS == 2) ? GEMM_THREADS : SK_THREADS;
 };
 // The tower's q | k | v projection takes the same kernel unsplit with tiles of 144 columns, two whole heads of 72: a
 // thread then holds both halves of its row's heads and the rotary is part of the epilogue (3456 = 24 tiles exactly).
@@ -833,7 +834,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 res[h] = row_ok && col < g.N ? *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col) : make_uint4(0, 0, 0, 0);
             }
         }
-        if (HAS_BIAS) asm volatile("bar.sync 1, 128;" ::: "memory");      // the four epilogue warps
+        if (HAS_BIAS) asm volatile("bar.sync 1, %0;" ::"n"(SplitCfg<BN, KPS>::THREADS - 64) : "memory");      // the epilogue warps
     }
     if (ok && warp >= 2) {
         if (!mbar_wait(acc_done, 0)) { atomicExch(g.err, 53); ok = false; }
@@ -848,9 +849,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         // loaded per head and every thread storing its own row, 32 lines to an instruction, this epilogue took three times the
         // main loop's time: the launch 21.4 -> 14.6 us at 520 rows and 60.8 -> 43.8 us at 4096.
         if (ok && warp >= 2) {
-            uint8_t* stg = smem + q * (32 * VQ_PITCH);
+            // (with one CTA on an SM a head for each of eight warps)
+            uint8_t* stg = smem + (warp - 2) * (32 * VQ_PITCH);
 #pragma unroll 1
-            for (int hh = 0; hh < 2; ++hh) {
+            for (int hh = (warp - 2) >> 2; hh < 2; hh += SplitCfg<BN, KPS>::THREADS == GEMM_THREADS ? 2 : 1) {
                 const int col = nb * VQ_BN + hh * 72, which = col / 1152, h = (col - which * 1152) / 72;
                 const uint2* bs = reinterpret_cast<const uint2*>(bias_s) + hh * 18;
                 __syncwarp();
@@ -964,7 +966,7 @@ static constexpr int FP_SMEM = FP_ROOM + 1024 /*align*/ + 256 /*barriers*/;
 __host__ __device__ constexpr int fp_stage_bytes(int ra, int fc) { return FP_KPS * (ra + fc) * BK * 2; }
 
 template <int EPI, bool PARTS>
-__global__ void __launch_bounds__(SK_THREADS, 1)
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2, const GemmArgs g, const int ra, const int fc,
                      const int stages, const int parts) {
@@ -1062,13 +1064,14 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         PlainEpilogue<EPI, true, PARTS> plain;
         plain.row_end = a_row + ra < g.M ? a_row + ra : g.M;
         if (PARTS) { plain.parts = parts; plain.part_cols = fc; }
-        if (cols > 0) plain.ahead(g, row0, col0, cols, 0, lane);
+        const int c_first = ((warp - 2) >> 2) * 32, c_step = ((int)blockDim.x - 64) >> 2;     // four or eight warps
+        if (cols > c_first) plain.ahead(g, row0, col0, cols, c_first, lane);
         bool ok = mbar_wait(acc_done, 0);
         if (!ok) atomicExch(g.err, 93);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         // (all MMAs are through with the stages, which serve as staging)
-        if (ok && cols > 0) plain.run(g, tmem_base + ((uint32_t)(q * 32) << 16), row0, col0, cols, 0, 32, smem + (warp - 2) * EPI_SLICE, lane, failed);
+        if (ok && cols > c_first) plain.run(g, tmem_base + ((uint32_t)(q * 32) << 16), row0, col0, cols, c_first, c_step, smem + (warp - 2) * EPI_SLICE, lane, failed);
     }
     tc_fence_before();
     __syncthreads();
@@ -2096,7 +2099,7 @@ static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, 
     g.prefetch = SK_PREFETCH;
     prof_before(EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : (EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID ? (int)EPI_RESID : EPI),
                 2.0 * g.M * (double)g.N * g.K, st);
-    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(SK_THREADS), smem, st, 2, g.M, mA, mB, mA2, mB2, g, ra, fc, stages, parts);
+    cudaError_t e = launch_chained(kern, dim3(2 * g.num_m * g.num_n), dim3(fc > 32 ? GEMM_THREADS : SK_THREADS), smem, st, 2, g.M, mA, mB, mA2, mB2, g, ra, fc, stages, parts);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (few tiles, pairs): launch: %s", cudaGetErrorString(e)); return false; }
