@@ -684,7 +684,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // gemm_few_pair_kernel is its form on CTA pairs, and the one that sums a long K in parts.
 // K blocks of weights requested into L2 ahead of their load, before the wait for the previous grid to begin with: three to
 // five stages do not cover the way from memory (the persistent kernel's six do, and there the requests only cost: 24 -> 32 us at
-// 77 x 4096 x 4096).
+// 77 x 4096 x 4096).  The row tiles of a column share them: the thread of the first one alone took 18 x 145 cycles for a K of 1152, and
+// found room for them only where the kernel before left some (the tower of 520 patches 1777 -> 1764 us).
 static constexpr int SK_PREFETCH = 24;
 // KPS: K blocks per stage.  Two where an SM has one CTA anyway: the trip through a stage's barriers then counts half (a K
 // block of a 32-column tile takes 290 cycles instead of 390-430; 77 x 4096 x 4096 17.8 -> 12.7 us).
@@ -727,9 +728,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     if (warp == 1) { tmem_alloc(tmem_slot, SplitCfg<BN, KPS>::TMEM_COLS); tmem_relinquish(); }
     const int kblocks = (g.K + BK - 1) / BK;
-    const bool ahead = mb == 0 && g.prefetch > 0;     // the other row tiles find the weights in L2
-    if (ahead && warp == 0 && elect_one())
-        for (int i = 0; i < g.prefetch && i < kblocks; ++i) tma_prefetch_2d(&tmB, i * BK, nb * BN);
+    // the row tiles share the requests for the weights they all read
+    const int span = g.prefetch * g.num_m;
+    if (warp == 0 && elect_one())
+        for (int i = mb; i < span && i < kblocks; i += g.num_m) tma_prefetch_2d(&tmB, i * BK, nb * BN);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -749,7 +751,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 uint8_t* a_s = smem + s * SK_STAGE_BYTES;
                 mbar_expect_tx(&full[s], n * (SK_STAGE_BYTES / KPS));
                 for (int u = 0; u < n; ++u) {
-                    if (ahead && i + u + g.prefetch < kblocks) tma_prefetch_2d(&tmB, (i + u + g.prefetch) * BK, nb * BN);
+                    if (mb == 0 && span > 0 && i + u + span < kblocks) tma_prefetch_2d(&tmB, (i + u + span) * BK, nb * BN);
                     int a_c0 = (i + u) * BK, a_c1 = mb * BM;
                     if (g.a_kblk > 0) {
                         const int blk = a_c0 / g.a_kblk;
@@ -993,11 +995,12 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (warp == 1) { tmem_alloc_pair(tmem_slot, PARTS ? 512 : 64); tmem_relinquish_pair(); }
     // whole K blocks come FP_KPS to a copy, a ragged last one by itself (tmA2, tmB2)
     const int kblocks = (g.K + BK - 1) / BK, kwhole = g.K / BK;
-    const bool ahead = mb == 0 && g.prefetch > 0;     // the other row tiles find the weights in L2
     if (warp == 0 && elect_one()) {
         tma_prefetch_desc(&tmB);
         tma_prefetch_desc(&tmA);
-        if (ahead) for (int i = 0; i < g.prefetch && i < kwhole; i += FP_KPS) tma_prefetch_3d(&tmB, 0, b_row, i);
+        // the row tiles share the requests for the weights they all read; for a long K (PARTS) all of them make as many as one would
+        const int most = PARTS ? g.prefetch * g.num_m : g.prefetch;
+        for (int i = mb * FP_KPS; i < most && i < kwhole; i += g.num_m * FP_KPS) tma_prefetch_3d(&tmB, 0, b_row, i);
     }
     tc_fence_before();
     __syncthreads();

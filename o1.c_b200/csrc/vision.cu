@@ -114,6 +114,13 @@ layernorm_reg_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict_
                      uint16_t* __restrict__ y, int rows, int cols, float eps) {
     if (FEW) {
         grid_dep_launch();
+        // weight and bias on their way to L2 while the kernel before still runs (1794 -> 1777 us for the tower of 520 patches)
+        if (blockIdx.x == 0) {
+            for (int i = threadIdx.x * 64; i < cols; i += LN_WARPS * 32 * 64) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(w + i));
+                if (b) asm volatile("prefetch.global.L2 [%0];" ::"l"(b + i));
+            }
+        }
         grid_dep_wait();
     }
     const int row = blockIdx.x * LN_WARPS + (threadIdx.x >> 5);
