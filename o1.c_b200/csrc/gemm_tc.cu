@@ -45,6 +45,7 @@ struct GemmArgs {
     const float* rope_sin; // EPI_VROPE: sin [M,72]
     float scale;
     int num_m, num_n, group_m;
+    int halves_from;       // gate | up on pairs: the first tile that is taken as two halves
     int prefetch;          // K blocks of weights requested into L2 ahead of their load (0: none)
     // Output column blocks: column c lives at out + (c / o_cb) * o_cb_stride + row * ldo + c % o_cb
     // (o_cb == 0: plain row-major).  Lets a projection write its head groups into per-destination
@@ -366,8 +367,11 @@ __device__ __forceinline__ void head_epilogue(const GemmArgs& g, uint32_t t_head
 template <int EPI, int BN, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmB3, const GemmArgs g) {
+               const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmB3, const __grid_constant__ CUtensorMap tmB4,
+               const GemmArgs g) {
     using Cfg = GemmCfg<BN, PAIR>;
+    // gate | up on pairs: the last tiles as halves of 64 columns of each (tmB3, tmB4: boxes of 64 rows), see launch_tc_pair()
+    constexpr bool HALVES = PAIR && EPI == EPI_SWIGLU;
     static_assert(!PAIR || BN == 256, "the pair form splits a 256-wide B tile");
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -420,7 +424,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // the pair form walks tiles of 256 rows: row tile 2 * mb2 + rank of each belongs to this CTA
     const int sched_m = PAIR ? (g.num_m + 1) / 2 : g.num_m;
     const int sched_group = PAIR ? (g.group_m + 1) / 2 : g.group_m;
-    const int num_tiles = sched_m * g.num_n;
+    // (HALVES: units from halves_from on are halves, two to a tile)
+    const int halves_from = HALVES ? g.halves_from : 0;
+    const int num_tiles = sched_m * g.num_n + (HALVES ? sched_m * g.num_n - halves_from : 0);
     const int tile0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const int tile_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     const int kblocks = (g.K + BK - 1) / BK;   // a ragged last K block is zero-filled by TMA in both operands
@@ -435,14 +441,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             bool ok = true;
             for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
                 int mb, nb;
-                tile_coords(tile, sched_m, g.num_n, sched_group, mb, nb);
+                const bool is_half = HALVES && tile >= halves_from;
+                tile_coords(is_half ? halves_from + ((tile - halves_from) >> 1) : tile, sched_m, g.num_n, sched_group, mb, nb);
                 if (PAIR) mb = mb * 2 + (int)rank;
+                const uint32_t pair_bytes = 2 * (is_half ? Cfg::STAGE_BYTES - 64 * BK * 2 : Cfg::STAGE_BYTES);      // both CTAs' halves
                 for (int kb = 0; kb < kblocks; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1)) { ok = false; atomicExch(g.err, 1); break; }
                     uint8_t* a_s = smem + stage * Cfg::STAGE_BYTES;
                     uint8_t* b_s = a_s + Cfg::A_BYTES;
                     if (!PAIR) mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-                    else if (rank == 0) mbar_expect_tx(&full[stage], 2 * Cfg::STAGE_BYTES);   // both CTAs' halves
+                    else if (rank == 0) mbar_expect_tx(&full[stage], pair_bytes);
                     int a_c0 = kb * BK, a_c1 = mb * BM;
                     if (g.a_kblk > 0) {
                         const int blk = a_c0 / g.a_kblk;
@@ -452,7 +460,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if (PAIR) {
                         // this CTA's 128 rows of A and its 128 of the tile's 256 B rows (second half for the second CTA)
                         tma_load_2d_pair(a_s, &tmA, &full[stage], a_c0, a_c1);
-                        if (EPI == EPI_SWIGLU) {
+                        if (is_half) {
+                            tma_load_2d_pair(b_s, rank == 0 ? &tmB3 : &tmB4, &full[stage], kb * BK, nb * 128 + ((tile - halves_from) & 1) * 64);
+                        } else if (EPI == EPI_SWIGLU) {
                             tma_load_2d_pair(b_s, rank == 0 ? &tmB : &tmB2, &full[stage], kb * BK, nb * 128);
                         } else if (EPI == EPI_QKV) {
                             const int col0 = nb * BN;
@@ -493,13 +503,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     } else if (warp == 1) {
         // ------------------------------------------------------ MMA issuer
         if (rank == 0 && elect_one()) {
-            constexpr uint32_t idesc = umma_idesc_bf16(PAIR ? 2 * BM : BM, BN, 0, 0);
+            constexpr uint32_t idesc_full = umma_idesc_bf16(PAIR ? 2 * BM : BM, BN, 0, 0), idesc_half = umma_idesc_bf16(2 * BM, BN / 2, 0, 0);
             int stage = 0;
             uint32_t phase = 0;
             int as = 0;
             uint32_t aphase = 0;
             bool ok = true;
             for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+                const uint32_t idesc = HALVES && tile >= halves_from ? idesc_half : idesc_full;
                 if (!mbar_wait(&tempty[as], aphase ^ 1)) { atomicExch(g.err, 2); break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * BN;
@@ -533,7 +544,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int failed = error_word(g.err);
         for (int tile = tile0; tile < num_tiles; tile += tile_step) {
             int mb, nb;
-            tile_coords(tile, sched_m, g.num_n, sched_group, mb, nb);
+            const bool is_half = HALVES && tile >= halves_from;
+            tile_coords(is_half ? halves_from + ((tile - halves_from) >> 1) : tile, sched_m, g.num_n, sched_group, mb, nb);
             if (PAIR) mb = mb * 2 + (int)rank;
             const int rows = failed ? 0 : g.M;
             const int row0 = mb * BM + q * 32;
@@ -560,16 +572,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             const int epi_eff = (EPI == EPI_QKV) ? (seg < 2 ? (int)EPI_QKNORM : (int)EPI_STORE) : EPI;
             if (EPI == EPI_SWIGLU) {
+                const int width = is_half ? 64 : 128, col0 = nb * 128 + (is_half ? ((tile - halves_from) & 1) * 64 : 0);
 #pragma unroll 1
-                for (int c = half * 32; c < 128; c += 64) {
+                for (int c = half * 32; c < width; c += 64) {
                     uint32_t rg[32], ru[32];
                     tmem_ld32(t_row + c, rg);
-                    tmem_ld32(t_row + 128 + c, ru);
+                    tmem_ld32(t_row + width + c, ru);
                     tmem_ld_wait();
                     float v[32];
                     swiglu_all(rg, ru, v);
                     __syncwarp();
-                    PlainEpilogue<EPI_STORE>::store_group(g, v, stg, row0, nb * 128 + c, 32, lane, failed);
+                    PlainEpilogue<EPI_STORE>::store_group(g, v, stg, row0, col0 + c, 32, lane, failed);
                 }
             } else if (epi_eff == EPI_STORE && g.o_tab_n) {
                 // Blocks of the output live in other GPUs' memory.  One thread per row would put 16-byte
@@ -1729,19 +1742,26 @@ static int pair_capacity(const void* kern, int threads, int smem) {
     return n;
 }
 
+// gate | up: where at most half of the pairs have a tile in the last round, its tiles are taken as two halves of 64 gate and 64 up columns.
+// A half takes some 0.6 of a tile's time (it loads 24 KB for each K block, the tile 32).  Whole tiles / with halves, 12288 columns of each, K =
+// 4096, us: 256 rows (1.3 rounds) 71 / 55, 1024 rows 174 / 162, 1280 rows 211 / 195 (170 / 161 at the full clock), 1792 rows 285 / 270, 2048 rows
+// 307 / 293, 3500 rows 549 / 532, 4352 rows 650 / 642; last rounds that more than half of the pairs have stay whole (two rounds of halves).
+// A block that runs at the power cap gains less (1280 rows: nothing beyond 1 %).
 template <int EPI>
 static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2, GemmArgs& g,
-                           cudaStream_t st, const CUtensorMap* tB3) {
+                           cudaStream_t st, const CUtensorMap* tB3, const CUtensorMap* tB4 = nullptr) {
     using Cfg = GemmCfg<256, true>;
     static std::atomic<uint64_t> attr_done{0};
     auto kern = gemm_tc_kernel<EPI, 256, true>;
     if (!func_attr_once(attr_done, (const void*)kern, Cfg::SMEM_BYTES, "gemm (pair)")) return false;
     const int tiles = ((g.num_m + 1) / 2) * g.num_n;
     int pairs = pair_capacity((const void*)kern, GEMM_THREADS, Cfg::SMEM_BYTES);
+    g.halves_from = tiles;
+    if (EPI == EPI_SWIGLU && tiles > pairs && 2 * (tiles % pairs) <= pairs) g.halves_from = tiles - tiles % pairs;
     if (pairs > tiles) pairs = tiles;
     prof_before(EPI == EPI_QKV ? (int)EPI_STORE : EPI, 2.0 * g.M * (double)g.N * g.K * (EPI == EPI_SWIGLU ? 2.0 : 1.0), st);
     cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 2, overlap_rows(g), *tA, *tB, *tB2,
-                                   tB3 ? *tB3 : *tB2, g);
+                                   tB3 ? *tB3 : *tB2, tB4 ? *tB4 : *tB2, g);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (pair): launch: %s", cudaGetErrorString(e)); return false; }
@@ -1949,7 +1969,7 @@ static bool launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
     if (grid > tiles) grid = tiles;
     prof_before((EPI == EPI_QKNORM || EPI == EPI_QKV) ? (int)EPI_STORE : (EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : ((EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID) ? (int)EPI_RESID : EPI)), 2.0 * g.M * (double)g.N * g.K * (EPI == EPI_SWIGLU ? 2.0 : 1.0), st);
     cudaError_t e = launch_chained(kern, dim3(grid), dim3(GEMM_THREADS), Cfg::SMEM_BYTES, st, 1, overlap_rows(g), *tA, *tB, *tB2,
-                                   tB3 ? *tB3 : *tB2, g);
+                                   tB3 ? *tB3 : *tB2, *tB2, g);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm: launch: %s", cudaGetErrorString(e)); return false; }
@@ -2261,7 +2281,10 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
             return launch_rows<EPI_SWIGLU>(x, ldx, &mG, &mU, &mU, g, bn, st);
         }
         g.num_n = N / 128;
-        return p.form == GEMM_PAIR ? launch_tc_pair<EPI_SWIGLU>(tA, tB, tB2, g, st, nullptr) : launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
+        if (p.form != GEMM_PAIR) return launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
+        CUtensorMap hG, hU;      // (of half tiles)
+        if (!cached_tmap(&hG, w, N, K, K, 64) || !cached_tmap(&hU, w2, N, K, K, 64)) return false;
+        return launch_tc_pair<EPI_SWIGLU>(tA, tB, tB2, g, st, &hG, &hU);
     }
     if (p.form == GEMM_FEW) switch (epi) {
         case EPI_STORE: return launch_split<EPI_STORE>(tA, x, ldx, w, g, p, st);

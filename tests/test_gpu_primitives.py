@@ -505,6 +505,28 @@ def test_pairs_with_tokens_as_columns(pkg, dev, M, K):
     assert pkg.lib.o1_device_error() == 0
 
 
+@pytest.mark.parametrize("M,K", [(130, 72), (256, 192), (100, 64)])
+@pytest.mark.parametrize("blocks", [149, 185, 186, 259, 295])
+def test_last_tiles_as_halves(pkg, dev, M, K, blocks):
+    """gate | up + SwiGLU on CTA pairs (blocks of 128 columns, 74 pairs): the tiles of a last round that at most half of the pairs have,
+    1 and 37 of them, are taken as two halves, more of them whole; the bits of one-CTA tiles, nothing written beside the result."""
+    N = blocks * 128
+    x, wg, wu = (dv(seeded_bf16((r, K), 80 + i, 0.0, 1.0 if i == 0 else 0.05), dev) for i, r in enumerate((M, N, N)))
+    ys = []
+    try:
+        for on in (1, 0):
+            pkg.lib.o1_gemm_pair_mode(on)
+            y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
+            assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(wg), pkg.ptr(wu), pkg.ptr(y), N + 8, M, N, K, 3, None, None, 0, 0.0, -1) == 0, pkg.last_error()
+            done(pkg, "swiglu")
+            assert (y[M:] == 777.0).all() and (y[:, N:] == 777.0).all(), "written beside the matrix"
+            ys.append(y)
+    finally:
+        pkg.lib.o1_gemm_pair_mode(1)
+    assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
+    assert pkg.lib.o1_device_error() == 0
+
+
 def check_linear_f64(y, x, w, bias, what):
     """y against 64 bits: an FP32 sum of K products in any order is within K * 2^-23 * sum|x||w| of the exact one, and the
     two bf16 roundings (of the sum, of the sum plus bias) are monotonic, so the result lies between the rounded ends."""
