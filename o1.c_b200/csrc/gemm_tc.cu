@@ -716,6 +716,63 @@ struct SplitCfg {
 static constexpr int VQ_BN = 144;
 static constexpr int VQ_PITCH = 168;     // bytes of a staged row of one head: 16 lanes' 8-byte pieces meet 32 different banks
 
+// Bias, rotary and the spacing of the tower's heads, for one head of 72 columns and the 32 rows of a warp.  bs: the head's bias; vcs, vsn: cos and
+// sin of this thread's row; stg: 32 x VQ_PITCH bytes of the warp's own.
+__device__ __forceinline__ void vrope_head(const GemmArgs& g, uint32_t t_head, int col, const uint2* bs, const float (&vcs)[36], const float (&vsn)[36],
+                                           uint8_t* stg, int row0, bool failed, int lane) {
+    const int which = col / 1152, h = (col - which * 1152) / 72;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {      // twelve columns and their partners 36 further
+        uint32_t rl[3][4], rh[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            tmem_ld4(t_head + k * 12 + i * 4, rl[i]);
+            tmem_ld4(t_head + 36 + k * 12 + i * 4, rh[i]);
+        }
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const uint2 bl = bs[k * 3 + i], bh = bs[9 + k * 3 + i];
+            const float b0[4] = {bf16lo(bl.x), bf16hi(bl.x), bf16lo(bl.y), bf16hi(bl.y)};
+            const float b1[4] = {bf16lo(bh.x), bf16hi(bh.x), bf16lo(bh.y), bf16hi(bh.y)};
+            float lo[4], hi[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float x = bf16_round(bf16_round(__uint_as_float(rl[i][j])) + b0[j]);
+                const float y = bf16_round(bf16_round(__uint_as_float(rh[i][j])) + b1[j]);
+                const float c = vcs[(k * 3 + i) * 4 + j], sn = vsn[(k * 3 + i) * 4 + j];
+                // fp32 rotary, one rounding (src/cuda/rope.cu:155-178); the table repeats after 36
+                lo[j] = which < 2 ? rope_f32(x, c, -y, sn) : x;
+                hi[j] = which < 2 ? rope_f32(y, c, x, sn) : y;
+            }
+            uint2* d = reinterpret_cast<uint2*>(stg + lane * VQ_PITCH) + k * 3 + i;
+            d[0] = make_uint2(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]));
+            d[9] = make_uint2(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]));
+        }
+    }
+    __syncwarp();
+    const int rows = failed ? 0 : g.M - row0;
+    uint16_t* out = g.out + (size_t)row0 * g.ldo + (which * 16 + h) * 128;
+#pragma unroll
+    for (int i = 0; i < 10; ++i) {
+        const int p = i * 32 + lane, r = p / 10, c = p - r * 10;
+        const uint2* sp = reinterpret_cast<const uint2*>(stg + r * VQ_PITCH) + c * 2;
+        uint4 o = make_uint4(0, 0, 0, 0);          // columns 72..79
+        if (c < 9) { const uint2 o0 = sp[0], o1 = sp[1]; o = make_uint4(o0.x, o0.y, o1.x, o1.y); }
+        if (r < rows) *reinterpret_cast<uint4*>(out + (size_t)r * g.ldo + c * 8) = o;
+    }
+}
+__device__ __forceinline__ void vrope_tables(const GemmArgs& g, int row, float (&vcs)[36], float (&vsn)[36]) {
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+        const float4 c4 = *reinterpret_cast<const float4*>(g.rope + (size_t)row * 72 + c * 4);
+        const float4 s4 = *reinterpret_cast<const float4*>(g.rope_sin + (size_t)row * 72 + c * 4);
+        vcs[c * 4] = c4.x; vcs[c * 4 + 1] = c4.y; vcs[c * 4 + 2] = c4.z; vcs[c * 4 + 3] = c4.w;
+        vsn[c * 4] = s4.x; vsn[c * 4 + 1] = s4.y; vsn[c * 4 + 2] = s4.z; vsn[c * 4 + 3] = s4.w;
+    }
+}
+
 template <int EPI, int BN, int KPS>
 __global__ void __launch_bounds__(SplitCfg<BN, KPS>::THREADS, KPS == 1 ? 2 : 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g) {
@@ -829,14 +886,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     float vcs[36], vsn[36];      // (EPI_VROPE)
     if (ok && warp >= 2) {
         if (EPI == EPI_VROPE) {
-            const int r = row_ok ? row : 0;
-#pragma unroll
-            for (int c = 0; c < 9; ++c) {
-                const float4 c4 = *reinterpret_cast<const float4*>(g.rope + (size_t)r * 72 + c * 4);
-                const float4 s4 = *reinterpret_cast<const float4*>(g.rope_sin + (size_t)r * 72 + c * 4);
-                vcs[c * 4] = c4.x; vcs[c * 4 + 1] = c4.y; vcs[c * 4 + 2] = c4.z; vcs[c * 4 + 3] = c4.w;
-                vsn[c * 4] = s4.x; vsn[c * 4 + 1] = s4.y; vsn[c * 4 + 2] = s4.z; vsn[c * 4 + 3] = s4.w;
-            }
+            vrope_tables(g, row_ok ? row : 0, vcs, vsn);
         }
         if (HAS_BIAS && trow * 8 < BN) {
             const int col = nb * BN + trow * 8;
@@ -868,49 +918,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             uint8_t* stg = smem + (warp - 2) * (32 * VQ_PITCH);
 #pragma unroll 1
             for (int hh = (warp - 2) >> 2; hh < 2; hh += SplitCfg<BN, KPS>::THREADS == GEMM_THREADS ? 2 : 1) {
-                const int col = nb * VQ_BN + hh * 72, which = col / 1152, h = (col - which * 1152) / 72;
-                const uint2* bs = reinterpret_cast<const uint2*>(bias_s) + hh * 18;
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {      // twelve columns and their partners 36 further
-                    uint32_t rl[3][4], rh[3][4];
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        tmem_ld4(t_row + hh * 72 + k * 12 + i * 4, rl[i]);
-                        tmem_ld4(t_row + hh * 72 + 36 + k * 12 + i * 4, rh[i]);
-                    }
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        const uint2 bl = bs[k * 3 + i], bh = bs[9 + k * 3 + i];
-                        const float b0[4] = {bf16lo(bl.x), bf16hi(bl.x), bf16lo(bl.y), bf16hi(bl.y)};
-                        const float b1[4] = {bf16lo(bh.x), bf16hi(bh.x), bf16lo(bh.y), bf16hi(bh.y)};
-                        float lo[4], hi[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float x = bf16_round(bf16_round(__uint_as_float(rl[i][j])) + b0[j]);
-                            const float y = bf16_round(bf16_round(__uint_as_float(rh[i][j])) + b1[j]);
-                            const float c = vcs[(k * 3 + i) * 4 + j], sn = vsn[(k * 3 + i) * 4 + j];
-                            // fp32 rotary, one rounding (src/cuda/rope.cu:155-178); the table repeats after 36
-                            lo[j] = which < 2 ? rope_f32(x, c, -y, sn) : x;
-                            hi[j] = which < 2 ? rope_f32(y, c, x, sn) : y;
-                        }
-                        uint2* d = reinterpret_cast<uint2*>(stg + lane * VQ_PITCH) + k * 3 + i;
-                        d[0] = make_uint2(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]));
-                        d[9] = make_uint2(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]));
-                    }
-                }
-                __syncwarp();
-                const int rows = failed ? 0 : g.M - mb * BM - q * 32;
-                uint16_t* out = g.out + (size_t)(mb * BM + q * 32) * g.ldo + (which * 16 + h) * 128;
-#pragma unroll
-                for (int i = 0; i < 10; ++i) {
-                    const int p = i * 32 + lane, r = p / 10, c = p - r * 10;
-                    const uint2* sp = reinterpret_cast<const uint2*>(stg + r * VQ_PITCH) + c * 2;
-                    uint4 o = make_uint4(0, 0, 0, 0);          // columns 72..79
-                    if (c < 9) { const uint2 o0 = sp[0], o1 = sp[1]; o = make_uint4(o0.x, o0.y, o1.x, o1.y); }
-                    if (r < rows) *reinterpret_cast<uint4*>(out + (size_t)r * g.ldo + c * 8) = o;
-                }
+                vrope_head(g, t_row + hh * 72, nb * VQ_BN + hh * 72, reinterpret_cast<const uint2*>(bias_s) + hh * 18, vcs, vsn, stg, mb * BM + q * 32,
+                           failed, lane);
             }
         }
         tc_fence_before();
@@ -1216,11 +1225,14 @@ gemm_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
 // ---------------------------------------------------------------- CTA pairs with a tile width chosen at run time
 // The pair form (256 rows over two CTAs, each with half of the B tile) for any width that is a multiple of 16, any N and every
-// epilogue with plain row-major output.  Narrower tiles pay where they make fewer or fuller rounds: a one-CTA tile of 128 x 128
+// epilogue with plain row-major output, and for the tower's q | k | v (EPI_VROPE).  Narrower tiles pay where they make fewer or fuller rounds: a one-CTA tile of 128 x 128
 // brings 32 KB into an SM per K block and is bound by that (70 bytes a clock); half a pair tile of 256 x 128 brings 24 KB for the
 // same products.
 static constexpr int PF_MAX_STAGES = 8, PF_STAGE_ROOM = 192 * 1024, PF_STORE = EPI_WARPS * EPI_SLICE;
 static constexpr int PF_SMEM = PF_STAGE_ROOM + PF_STORE + 1024 /*align*/ + 256 /*barriers*/;
+// EPI_VROPE: two heads to a tile, one for each of a quadrant's two warps, whose slice holds 32 staged rows of it and its bias.
+static constexpr int PFV_STAGES = 7, PFV_ROOM = PFV_STAGES * (BM + VQ_BN / 2) * BK * 2, PFV_SLICE = 32 * VQ_PITCH + 160, PFV_STORE = EPI_WARPS * PFV_SLICE;
+static constexpr int PFV_SMEM = PFV_ROOM + PFV_STORE + 1024 /*align*/ + 256 /*barriers*/;
 
 template <int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -1229,8 +1241,8 @@ gemm_pair_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int stage_bytes = (BM + bn / 2) * BK * 2;      // (bn is a multiple of 16: the stages stay 1024-byte aligned)
-    uint8_t* store_s = smem + PF_STAGE_ROOM;
-    uint64_t* full = reinterpret_cast<uint64_t*>(store_s + PF_STORE);
+    uint8_t* store_s = smem + (EPI == EPI_VROPE ? PFV_ROOM : PF_STAGE_ROOM);
+    uint64_t* full = reinterpret_cast<uint64_t*>(store_s + (EPI == EPI_VROPE ? PFV_STORE : PF_STORE));
     uint64_t* empty = full + PF_MAX_STAGES;
     uint64_t* tfull = empty + PF_MAX_STAGES;
     uint64_t* tempty = tfull + 2;
@@ -1310,20 +1322,35 @@ gemm_pair_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
     } else if (live) {
         const int q = warp & 3, half = (warp - 2) >> 2;       // (as in gemm_tc_kernel)
-        uint8_t* stg = store_s + (warp - 2) * EPI_SLICE;
+        uint8_t* stg = store_s + (warp - 2) * (EPI == EPI_VROPE ? PFV_SLICE : EPI_SLICE);
         int as = 0;
         uint32_t aphase = 0;
         const int failed = error_word(g.err);
         for (int tile = tile0; tile < num_tiles; tile += tile_step) {
             int mb, nb;
             tile_coords(tile, num_m, g.num_n, group_m, mb, nb);
-            const int row0 = (mb * 2 + (int)rank) * BM + q * 32, col0 = nb * bn, cols = g.N - col0 < bn ? g.N - col0 : bn;
-            PlainEpilogue<EPI> plain;
-            plain.ahead(g, row0, col0, cols, half * 32, lane);
-            const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase));
-            if (!got) { atomicExch(g.err, 74); break; }
-            tc_fence_after();
-            plain.run(g, tmem_base + as * 256 + ((uint32_t)(q * 32) << 16), row0, col0, cols, half * 32, 64, stg, lane, failed);
+            const int row0 = (mb * 2 + (int)rank) * BM + q * 32;
+            const uint32_t t_row = tmem_base + as * 256 + ((uint32_t)(q * 32) << 16);
+            if constexpr (EPI == EPI_VROPE) {
+                const int col0 = nb * VQ_BN + half * 72;
+                float vcs[36], vsn[36];
+                vrope_tables(g, row0 + lane < g.M ? row0 + lane : 0, vcs, vsn);
+                uint2* bs = reinterpret_cast<uint2*>(stg + 32 * VQ_PITCH);
+                if (lane < 18) bs[lane] = *reinterpret_cast<const uint2*>(g.bias + col0 + lane * 4);
+                const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase));
+                if (!got) { atomicExch(g.err, 74); break; }
+                tc_fence_after();
+                vrope_head(g, t_row + half * 72, col0, bs, vcs, vsn, stg, row0, failed, lane);
+                __syncwarp();      // (the bias and the staged rows have been read)
+            } else {
+                const int col0 = nb * bn, cols = g.N - col0 < bn ? g.N - col0 : bn;
+                PlainEpilogue<EPI> plain;
+                plain.ahead(g, row0, col0, cols, half * 32, lane);
+                const bool got = __all_sync(0xffffffffu, mbar_wait(&tfull[as], aphase));
+                if (!got) { atomicExch(g.err, 74); break; }
+                tc_fence_after();
+                plain.run(g, t_row, row0, col0, cols, half * 32, 64, stg, lane, failed);
+            }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&tempty[as]), 0));
@@ -1772,18 +1799,19 @@ template <int EPI>
 static bool launch_pair_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, int bn, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
     auto kern = gemm_pair_fit_kernel<EPI>;
-    if (!func_attr_once(attr_done, (const void*)kern, PF_SMEM, "gemm (pair, fitted)")) return false;
+    constexpr int SMEM = EPI == EPI_VROPE ? PFV_SMEM : PF_SMEM, ROOM = EPI == EPI_VROPE ? PFV_ROOM : PF_STAGE_ROOM;
+    if (!func_attr_once(attr_done, (const void*)kern, SMEM, "gemm (pair, fitted)")) return false;
     CUtensorMap mB;
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, bn / 2)) return false;
     g.num_n = (g.N + bn - 1) / bn;
-    int stages = PF_STAGE_ROOM / ((BM + bn / 2) * BK * 2);
+    int stages = ROOM / ((BM + bn / 2) * BK * 2);
     if (stages > PF_MAX_STAGES) stages = PF_MAX_STAGES;
     const int tiles = (g.num_m + 1) / 2 * g.num_n;
-    int pairs = pair_capacity((const void*)kern, GEMM_THREADS, PF_SMEM);
+    int pairs = pair_capacity((const void*)kern, GEMM_THREADS, SMEM);
     if (pairs > tiles) pairs = tiles;
-    prof_before(EPI == EPI_BIAS_GELU ? (int)EPI_BIAS : (EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID ? (int)EPI_RESID : EPI),
+    prof_before(EPI == EPI_BIAS_GELU || EPI == EPI_VROPE ? (int)EPI_BIAS : (EPI == EPI_BIAS_RESID || EPI == EPI_GATE_RESID ? (int)EPI_RESID : EPI),
                 2.0 * g.M * (double)g.N * g.K, st);
-    cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), PF_SMEM, st, 2, overlap_rows(g), *tA, mB, g, bn, stages);
+    cudaError_t e = launch_chained(kern, dim3(2 * pairs), dim3(GEMM_THREADS), SMEM, st, 2, overlap_rows(g), *tA, mB, g, bn, stages);
     prof_after(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("gemm (pair, fitted): launch: %s", cudaGetErrorString(e)); return false; }
@@ -2421,9 +2449,18 @@ bool gemm_vision_qkv(const void* x, const void* w, const void* b, void* y, int M
     g.num_m = (M + BM - 1) / BM;
     g.err = device_error_word();
     CUtensorMap mA, mB;
-    if (!cached_tmap(&mA, x, M, K, K, 128) || !cached_tmap(&mB, w, N, K, K, VQ_BN)) return false;
-    // (with one CTA per SM, two K blocks a stage, see SplitCfg: the tower at 520 patches 2155 -> 2058 us)
-    if (g.num_m * (N / VQ_BN) <= sm_count()) return launch_split_bn<EPI_VROPE, VQ_BN, 2>(&mA, &mB, g, st);
+    if (!cached_tmap(&mA, x, M, K, K, 128)) return false;
+    // One CTA per SM: two K blocks a stage, see SplitCfg (the tower at 520 patches 2155 -> 2058 us).  More tiles than that: CTA pairs, which
+    // bring three quarters of the bytes into their SMs and have the next tile's products under their epilogue.  Two CTAs of one tile each on an SM /
+    // pairs, us: 832 rows 15.2 / 14.1, 1600 rows 25.1 / 18.8, 3024 rows 32.5 / 26.9, 4096 rows 47.0 / 37.4, 8192 rows 94.5 / 70.9; below, one CTA
+    // per SM / pairs: 128 rows 8.4 / 9.1, 520 rows 9.1 / 9.8, 768 rows 9.3 / 9.8.
+    const bool one_each = g.num_m * (N / VQ_BN) <= sm_count();
+    if (!one_each && pair_wanted()) {
+        g.group_m = 32;
+        return launch_pair_fit<EPI_VROPE>(&mA, w, g, VQ_BN, st);
+    }
+    if (!cached_tmap(&mB, w, N, K, K, VQ_BN)) return false;
+    if (one_each) return launch_split_bn<EPI_VROPE, VQ_BN, 2>(&mA, &mB, g, st);
     return launch_split_bn<EPI_VROPE, VQ_BN>(&mA, &mB, g, st);
 }
 

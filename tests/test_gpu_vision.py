@@ -416,3 +416,37 @@ def test_workspace_tensors_are_those_of_the_layout(pkg, dev, tower, gh, gw):
     assert ((norm(a) - norm(b)).abs() <= 2.0 ** -7 * norm(b) + 1e-6).all()
     want = run_tower(pkg, dev, binding, px, gh, gw, snaps=False)[0]
     assert torch.equal(bits(emb), bits(want))
+
+
+@pytest.mark.parametrize("M", [768, 769, 833, 1297, 2048, 4100])
+def test_qkv_rotary_projection_on_cta_pairs(pkg, dev, M):
+    """The tower's q | k | v launch around the row counts where it goes from a tile for each SM to CTA pairs (tiles with no row of the second
+    CTA, with one, more than a round): the bits of single CTAs, columns 72..79 of a head zero, nothing else written."""
+    fn = pkg.lib._ZN2o115gemm_vision_qkvEPKvS1_S1_PviPKfS4_P11CUstream_st      # o1::gemm_vision_qkv
+    fn.argtypes, fn.restype = [C.c_void_p] * 4 + [C.c_int] + [C.c_void_p] * 3, C.c_bool
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(M)
+    n_ = lambda *s: torch.empty(*s, device=dev).normal_(0, 1, generator=gen)  # noqa: E731
+    x, w, b = n_(M, 1152).bfloat16(), (n_(3456, 1152) * 0.03).bfloat16(), n_(3456).bfloat16()
+    cos, sin = (torch.cat([h, h], 1).contiguous() for h in (n_(M, 36).cos(), n_(M, 36).sin()))
+    outs = []
+    try:
+        for on in (1, 0):
+            pkg.lib.o1_gemm_pair_mode(on)
+            y = torch.full((M + 1, 6144), 777.0, dtype=torch.bfloat16, device=dev)
+            torch.cuda.synchronize()
+            assert fn(pkg.ptr(x), pkg.ptr(w), pkg.ptr(b), pkg.ptr(y), M, pkg.ptr(cos), pkg.ptr(sin), None), pkg.last_error()
+            torch.cuda.synchronize()
+            outs.append(y)
+    finally:
+        pkg.lib.o1_gemm_pair_mode(1)
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
+    heads = outs[0][:M].view(M, 3, 16, 128)
+    assert (outs[0][M:] == 777.0).all() and (heads[..., 80:] == 777.0).all() and (heads[..., 72:80] == 0).all()
+    v = ((x.float() @ w.float().t()).bfloat16().float() + b.float()).bfloat16().float().view(M, 3, 16, 72)
+    c, s = cos[:, None, None, :], sin[:, None, None, :]
+    turned = v * c + torch.cat([-v[..., 36:], v[..., :36]], -1) * s
+    ref = torch.cat([turned[:, :2], v[:, 2:]], 1)
+    # one ulp of the projection (its sum in another order) through the rotation, and the last rounding
+    assert (heads[..., :72].float() - ref).abs().max().item() <= 3 * 2.0 ** -8 * v.abs().max().item()
+    assert pkg.lib.o1_device_error() == 0
