@@ -476,9 +476,8 @@ int o1_gemm(const void *x, int ldx, const void *w, const void *w2, void *y, int 
  * one CTA per tile of 128 rows x *width columns, 2 = two CTAs per 256 x 256 tile (SwiGLU from K = 2048 on also per 256 weight
  * rows x 64 to 256 rows of x, as many as fit their number), 3 = one CTA per tile of a *width fitted to
  * the number of SMs, 4 = the kernels for few tiles: *width = 32 (from K = 256 on two CTAs per 64 to 128 columns where that is the better
- * way) or 96 columns, or *width = 128 and K summed in *ctas parts (that many CTAs of a cluster, or that many accumulators of a CTA
- * pair); -1 = not supported.  1 and 3 with *ctas = 2: a CTA pair per tile of 256 rows.  force_bn -1 (which o1_gemm takes too): as 0, and K may
- * be shared; -2 (the vision tower's linears): as -1, and a pair tile of 96 to 256 columns from 257 rows on where K >= 2048 (in
+ * way) or 96 columns, or *width = 128 and K summed in *ctas parts (as many accumulators of a CTA pair); -1 = not supported.  1 and 3 with *ctas = 2: a CTA pair per tile of 256 rows.  force_bn -1 (which o1_gemm takes too): as 0, and K may
+ * be summed in parts; -2 (the vision tower's linears): as -1, and a pair tile of 96 to 256 columns from 257 rows on where K >= 2048 (in
  * place of narrow tiles), from 1025 rows on where 1024 <= K < 2048 and N is no multiple of 256, if that takes fewer rounds. */
 int o1_gemm_form(int M, int N, int K, int epi, int force_bn, int *width, int *ctas);
 /* The q, k and v projections of a decoder block (src/model/block.c:257-265) with the per-head RMSNorm + rotary of
@@ -511,8 +510,8 @@ void o1_attention_tile_mode(int mode);
  * of the accumulator and half of the B tile: 256 columns in the plain, bias, residual, SwiGLU and grouped q|k|v families (in
  * the last two also 256 weight rows by a fitted number of rows), 96
  * to 256 (see o1_gemm_form) in every epilogue of one weight matrix but the per-head norm and LoRA; and a
- * linear of the vision tower that has few tiles shares the K of a tile among up to six CTAs. 0 = always one CTA per tile, no
- * cluster is launched.  The pairs add a row's K products in the order of single CTAs: same bits.  The shared K is another
+ * linear of the vision tower that has few tiles sums a long K in up to six parts. 0 = always one CTA per tile, no
+ * cluster is launched.  The pairs add a row's K products in the order of single CTAs: same bits.  K in parts is another
  * order of the fp32 sum, so the tower's outputs (hd_vision_forward) at small images depend on the mode within rounding;
  * those of the decoder do not.  No reference counterpart (cuBLASLt picks its own kernels there, src/cuda/gemm.cu:413-461). */
 void o1_gemm_pair_mode(int mode);

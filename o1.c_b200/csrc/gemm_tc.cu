@@ -32,7 +32,7 @@ static constexpr int BK = 64;
 static constexpr int EPI_WARPS = 8;                       // two per quadrant of tensor memory
 static constexpr int EPI_SLICE = 2048 + 64;               // shared memory of a warp: 32 rows x 32 columns, and their bias
 static constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
-static constexpr int SK_THREADS = 192;                    // gemm_split_kernel's 32-column and shared tiles: four epilogue warps
+static constexpr int SK_THREADS = 192;                    // narrow tiles: four epilogue warps
 
 struct GemmArgs {
     int M, N, K;
@@ -167,7 +167,7 @@ struct PlainEpilogue {
             }
             tmem_ld_wait();
             if (PARTS) {
-                // (from zero on, in the order of the parts, as the CTAs of a cluster add theirs)
+                // (from zero on, in the order of the parts)
 #pragma unroll
                 for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__fadd_rn(0.f, __uint_as_float(r[j])));
 #pragma unroll 1
@@ -808,8 +808,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     grid_dep_launch();
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
-    // after a failure no loads and no results, but the cluster's barriers below are passed all the same (the CTAs of a cluster
-    // may read the word at different times)
+    // (after a failure no loads and no results)
     bool ok = *s_abort == 0;
     const int failed = warp >= 2 ? error_word(g.err) : 0;
 
@@ -978,9 +977,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // issues the copies, some 145 cycles for each whatever its size (two for a K block, and one for L2), and shared memory: an MMA of 128 x 32 x 16
 // reads 5 KB while the copies write as much, the pair's of 128 x 64 x 16 reads and writes 3 KB on an SM.  Same order of the
 // sum, so the same bits.
-// PARTS: so too where the K of a tile is to be summed in parts.  The parts, which a cluster's CTAs share in gemm_split_kernel, follow one
-// another here, each in an accumulator of its own, and the epilogue adds them in their order.  (At 520 x 1152 x 4304 the exchange
-// took 13,000 of that kernel's 33,000 cycles, the main loop 11,000.)  fewpair_cols() has both sides' times.
+// PARTS: so too where the K of a tile is to be summed in parts.  The parts follow one another, each in an accumulator of its
+// own, and the epilogue adds them in their order.  (When the CTAs of a cluster shared them, the exchange took 13,000 of 33,000 cycles at
+// 520 x 1152 x 4304, the main loop 11,000.)  fewpair_cols() has both sides' times.
 // How many bytes of weights are on their way decides the time (77 x 4096 x 4096: two stages of four K blocks 16.6 us, four 11.3), so a stage
 // holds no more rows of the activations than there are: a tile of up to 128 rows is shared evenly, `ra` rows (a multiple of eight)
 // to a CTA.  The MMA reads 64, the others from whatever lies behind: their results are not used.
@@ -1725,7 +1724,7 @@ bool func_attr_once(std::atomic<uint64_t>& done, const void* func, int smem_byte
 }
 
 // 0: single CTAs only, no cluster is launched; else CTA pairs where tile_form() finds them the better form and, for callers
-// that allow it, K split over a cluster (the default)
+// that allow it, a long K of few tiles in parts (the default)
 static int g_pair_mode = -1;
 void gemm_pair_mode(int mode) { g_pair_mode = mode; }
 static bool pair_wanted() {

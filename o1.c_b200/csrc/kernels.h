@@ -32,7 +32,7 @@ void prof_after(cudaStream_t st);
 // force_bn: 0 = tile chosen by shape, 128 / 256 = that tile width; every output element is summed by one CTA in the order
 // of k, so that a row's result does not depend on the tile or on how many other rows the call has (the decoder's layers
 // rely on that: a row is the same in a sharded, a cached or a paired pass).  GEMM_SPLIT_K = chosen by shape, and a problem
-// of few tiles may share a tile's K among the CTAs of a cluster, which is another order of the FP32 sum (not in mode 0 of
+// of few tiles may sum a tile's K in parts, which is another order of the FP32 sum (not in mode 0 of
 // gemm_pair_mode).  GEMM_TOWER = the same for the vision tower's linears, whose long K takes pair tiles of any width.
 enum { GEMM_SPLIT_K = -1, GEMM_TOWER = -2 };
 // The form a problem takes: GEMM_ROWS = warps (bn: rows that share one), GEMM_TILE = one CTA per 128 x bn tile, GEMM_PAIR = two
@@ -99,7 +99,7 @@ void attention_tail_ways(int ways);
 bool attention_two_tile_only();       // mode 1 is set
 void attention_tile_mode(int mode);   // 0, 2: one query tile per CTA; 1: two
 int gemm_pair_capacity();
-void gemm_pair_mode(int mode);   // 0: single CTAs only; else clusters (CTA pairs, K split) where they are the better form
+void gemm_pair_mode(int mode);   // 0: single CTAs only; else CTA pairs, and K in parts, where they are the better form
 // seq-major operands; output rows [b*out_rows, (b+1)*out_rows) go to out_tab[b] (row-major, leading
 // dimension ldo), which may be peer-mapped memory of another GPU
 bool flash_attention_tab(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,
