@@ -391,6 +391,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __shared__ int s_abort;
     if (threadIdx.x == 64) s_abort = error_word(g.err);
     const uint32_t rank = PAIR ? cluster_rank() : 0u;    // 0: the CTA that issues the pair's MMAs
+    if (PAIR) cluster_arrive();
 
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
@@ -407,14 +408,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         fence_mbar_init();
     }
+    if (PAIR) cluster_wait();
     if (warp == 1) {
-        if (PAIR) { tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish_pair(); }
+        if (PAIR) tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
         else { tmem_alloc(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish(); }
     }
     tc_fence_before();
     __syncthreads();
     if (PAIR) cluster_sync_all();           // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
+    if (PAIR && warp == 1) tmem_relinquish_pair();
     grid_dep_launch();
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
@@ -1002,6 +1005,7 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
+    cluster_arrive();
     const int tile = (int)(blockIdx.x >> 1);
     const int nb = tile / g.num_m, mb = tile - nb * g.num_m;      // CTAs that share weights run next to each other
     const int stage_bytes = fp_stage_bytes(ra, fc), a_bytes = ra * BK * 2;
@@ -1013,7 +1017,8 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         mbar_init(acc_done, 1);
         fence_mbar_init();
     }
-    if (warp == 1) { tmem_alloc_pair(tmem_slot, PARTS ? 512 : 64); tmem_relinquish_pair(); }
+    cluster_wait();
+    if (warp == 1) tmem_alloc_pair(tmem_slot, PARTS ? 512 : 64);
     // whole K blocks come FP_KPS to a copy, a ragged last one by itself (tmA2, tmB2)
     const int kblocks = (g.K + BK - 1) / BK, kwhole = g.K / BK;
     if (warp == 0 && elect_one()) {
@@ -1027,6 +1032,7 @@ gemm_few_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     __syncthreads();
     cluster_sync_all();           // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
+    if (warp == 1) tmem_relinquish_pair();
     grid_dep_launch();
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
@@ -1249,6 +1255,7 @@ gemm_pair_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
+    cluster_arrive();
     if (threadIdx.x == 64) *s_abort = error_word(g.err);
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
@@ -1257,7 +1264,8 @@ gemm_pair_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 2 * EPI_WARPS); }
         fence_mbar_init();
     }
-    if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+    cluster_wait();
+    if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
     const int num_m = (g.num_m + 1) / 2, group_m = (g.group_m + 1) / 2;
     const int num_tiles = num_m * g.num_n, kblocks = (g.K + BK - 1) / BK;
     const int tile0 = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
@@ -1265,6 +1273,7 @@ gemm_pair_fit_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     __syncthreads();
     cluster_sync_all();           // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
+    if (warp == 1) tmem_relinquish_pair();
     grid_dep_launch();
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
@@ -1392,6 +1401,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
+    cluster_arrive();
     if (threadIdx.x == 64) *s_abort = error_word(g.err);
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmX);
@@ -1402,13 +1412,15 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 2 * EPI_WARPS); }
         fence_mbar_init();
     }
-    if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+    cluster_wait();
+    if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
     const int num_tiles = g.num_m * g.num_n, kblocks = (g.K + BK - 1) / BK;
     const int tile0 = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();           // both CTAs' barriers exist before either signals the other's
     tc_fence_after();
+    if (warp == 1) tmem_relinquish_pair();
     grid_dep_launch();
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;

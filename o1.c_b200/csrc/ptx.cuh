@@ -241,7 +241,18 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorM
         "l"(map), "r"(map_to_rank(smem_u32(bar), 0)), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
-// both CTAs of the pair execute these (same warp index in each)
+// Tensor memory of a pair.  Both CTAs execute these with the same warp, between cluster barriers:
+//     cluster_arrive(); .. cluster_wait();      both CTAs run
+//     tmem_alloc_pair(..);  __syncthreads();  cluster_sync_all();      both have their columns
+//     tmem_relinquish_pair();
+// The allocation is one of both CTAs.  A CTA that comes to it on its own gets its columns all the same, and if it also gives up the permit before the
+// other has come, the other's allocation never ends: with the allocation and the relinquishment behind one another and no barrier in front, a pair whose
+// second CTA had started 0.6 us late (the SM's slots were still full of the norm's blocks) hung, one of some 10^6 launches.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(ncols)
                  : "memory");

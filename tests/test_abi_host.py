@@ -421,3 +421,15 @@ def test_only_plain_epilogues_read_operands_by_column(tmp_path):
                        capture_output=True, text=True)
     assert r.returncode != 0
     assert r.stderr.count("error: static assertion failed") == len(others), r.stderr[-2000:]
+
+
+def test_a_pair_takes_tensor_memory_between_cluster_barriers():
+    """tcgen05.alloc of a CTA pair is one allocation of both: each kernel with one lets both CTAs arrive before it and gives up the
+    permit only behind a second barrier of both (otherwise one that comes late may wait without a limit, which no healthy run shows)."""
+    text = open(os.path.join(ROOT, "o1.c_b200", "csrc", "gemm_tc.cu")).read()
+    kernels = [k for k in text.split("__global__ void")[1:] if "tmem_alloc_pair(" in k]
+    assert len(kernels) == 4 and text.count("tmem_alloc_pair(") == 4
+    for k in kernels:
+        assert k.count("tmem_relinquish_pair(") == 1
+        at = [k.index(c) for c in ("cluster_arrive()", "cluster_wait()", "tmem_alloc_pair(", "cluster_sync_all()", "tmem_relinquish_pair(", "grid_dep_launch()")]
+        assert at == sorted(at), k[:200]

@@ -492,3 +492,36 @@ def test_guided_step_stays_inside_the_workspace_it_was_given(pkg, dev, room):
     xp = eng.xp[:(Sc + Su) * 3072].view(-1, 3072)
     assert torch.equal(xp[:Sc].view(torch.int16), xs[0].view(torch.int16))
     assert torch.equal(xp[Sc:].view(torch.int16), xs[1].view(torch.int16))
+
+
+@pytest.mark.parametrize("rows", [(600, 724, 1100), (513, 650, 768)])
+def test_states_in_turn_without_a_wait(pkg, dev, rows):
+    """Conditioned forwards of three states, some hundred passes behind one another with nothing that waits between them: the bits of
+    the first pass, no wait that ran out."""
+    T, L, V = 60, 3, 40
+    w = pkg.Weights(n_layers=L, seed=1234, weight_set="B", device=dev)
+    states = []
+    for k, I in enumerate(rows):
+        pos, ar = pkg.seq_t2i(T, I, 1)
+        mask = torch.zeros(T + I, dtype=torch.uint8)
+        mask[5:5 + V] = 1
+        vis = (mask.to(dev), u16_to_torch(seeded_bf16((V, 4096), 20 + k), dev),
+               [u16_to_torch(seeded_bf16((V, 4096), 30 + 3 * k + i), dev) for i in range(3)])
+        states.append((pkg.Engine(w, T, I, ar_len=ar), torch.from_numpy(make_ids(T, k)).to(dev), pos.to(dev),
+                       u16_to_torch(seeded_bf16((I, 3072), 40 + k), dev), vis,
+                       torch.empty(T + I, 3072, dtype=torch.bfloat16, device=dev)))
+
+    def one_pass(i):
+        e, ids, pos, vin, vis, out = states[i % 3]
+        e.forward(ids, pos, vin, 0.3, out=out, visual=vis)
+
+    for i in range(3):
+        one_pass(i)
+        torch.cuda.synchronize()
+    outs = [s[-1] for s in states]
+    first = [o.clone() for o in outs]
+    for i in range(300):
+        one_pass(i)
+    torch.cuda.synchronize()
+    pkg.check_cuda_errbuf("passes")
+    assert all(torch.equal(a.view(torch.int16), b.view(torch.int16)) for a, b in zip(first, outs))
