@@ -290,8 +290,11 @@ def last_error():
 
 
 def check(status, what=""):
+    """Raises for a failed call, with the library's texts.  They are taken: a later check_cuda_errbuf() is about later calls."""
     if status != HD_OK:
-        raise O1Error(f"{what} failed with hd_status {status}: {last_error()}")
+        text = last_error()
+        lib.hd_cuda_clear_error()
+        raise O1Error(f"{what} failed with hd_status {status}: {text}")
 
 
 def check_cuda_errbuf(what=""):

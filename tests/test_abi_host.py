@@ -91,6 +91,15 @@ def test_argument_checks_fail_closed_without_touching_the_gpu(pkg):
     assert lib.hd_lora_merge_gpu(None, 0, None) == 0
 
 
+def test_a_failure_is_named_once(pkg):
+    """The text of a call that check() has reported is not found again by the next call's check_cuda_errbuf()."""
+    pkg.lib.hd_cuda_clear_error()
+    pkg.lib.hd_linear(None, None, None, None, 4, 4, 4, 1)
+    with pytest.raises(pkg.O1Error, match="linear: bad args"):
+        pkg.check(1, "a call")
+    pkg.check_cuda_errbuf("the next call")
+
+
 def test_host_bf16_helpers(pkg):
     lib = pkg.lib
     assert lib.hd_f32_to_bf16(1.0) == 0x3F80 and lib.hd_f32_to_bf16(1.01171875) == 0x3F82
