@@ -33,6 +33,7 @@ static constexpr int EPI_WARPS = 8;                       // two per quadrant of
 static constexpr int EPI_SLICE = 2048 + 64;               // shared memory of a warp: 32 rows x 32 columns, and their bias
 static constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS;
 static constexpr int SK_THREADS = 192;                    // narrow tiles: four epilogue warps
+static constexpr int PAIR_ALONE = 116 * 1024;             // least shared memory of a CTA of a pair: more than half of an SM's 228 KB, see pair_capacity()
 
 struct GemmArgs {
     int M, N, K;
@@ -1758,7 +1759,11 @@ static long overlap_rows(const GemmArgs& g) {
 }
 
 // A persistent grid must be co-resident: as many pairs as the device can hold at once (a GPC with an odd number of SMs leaves one
-// without a partner), asked once per device.  (Every pair kernel fills an SM with one CTA.)
+// without a partner), asked once per device.
+// Every pair kernel takes more than half of an SM's shared memory (PAIR_ALONE), so that no two CTAs of pairs are ever on an SM, of
+// one grid, of the next one in a chain or of another stream.  tcgen05.alloc of a pair needs a turn on both of its SMs (a CTA has it until it gives up its
+// permit), and nothing in its definition orders two pairs that begin on the same two SMs: each might have the turn on one of them and
+// wait for the other, without a limit.  A single CTA's allocation waits on its own SM only, for CTAs that do not wait for it.
 static int pair_capacity(const void* kern, int threads, int smem) {
     static std::atomic<int> max_pairs[64];
     int dev = 0;
@@ -1789,6 +1794,7 @@ template <int EPI>
 static bool launch_tc_pair(const CUtensorMap* tA, const CUtensorMap* tB, const CUtensorMap* tB2, GemmArgs& g,
                            cudaStream_t st, const CUtensorMap* tB3, const CUtensorMap* tB4 = nullptr) {
     using Cfg = GemmCfg<256, true>;
+    static_assert(Cfg::SMEM_BYTES >= PAIR_ALONE, "see pair_capacity()");
     static std::atomic<uint64_t> attr_done{0};
     auto kern = gemm_tc_kernel<EPI, 256, true>;
     if (!func_attr_once(attr_done, (const void*)kern, Cfg::SMEM_BYTES, "gemm (pair)")) return false;
@@ -1811,6 +1817,7 @@ static bool launch_pair_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, i
     static std::atomic<uint64_t> attr_done{0};
     auto kern = gemm_pair_fit_kernel<EPI>;
     constexpr int SMEM = EPI == EPI_VROPE ? PFV_SMEM : PF_SMEM, ROOM = EPI == EPI_VROPE ? PFV_ROOM : PF_STAGE_ROOM;
+    static_assert(SMEM >= PAIR_ALONE, "see pair_capacity()");
     if (!func_attr_once(attr_done, (const void*)kern, SMEM, "gemm (pair, fitted)")) return false;
     CUtensorMap mB;
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, bn / 2)) return false;
@@ -1833,6 +1840,7 @@ static bool launch_pair_fit(const CUtensorMap* tA, const void* w, GemmArgs& g, i
 template <int EPI>
 static bool launch_rows(const void* x, int ldx, const CUtensorMap* mW, const CUtensorMap* mW2, const CUtensorMap* mW3, GemmArgs& g, int bn,
                         cudaStream_t st) {
+    static_assert(RW_SMEM >= PAIR_ALONE, "see pair_capacity()");
     static std::atomic<uint64_t> attr_done{0};
     auto kern = gemm_rows_kernel<EPI>;
     if (!func_attr_once(attr_done, (const void*)kern, RW_SMEM, "gemm (pair, rows)")) return false;
@@ -2124,18 +2132,24 @@ static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmAr
 
 // Narrow tiles on CTA pairs: columns of a CTA, or 0 for the one-CTA forms; K from 256 on.  32 columns where that makes at most one CTA per
 // SM, else 48 or 64 (two CTAs of 32 columns on an SM have half the room each for weights on their way).  One CTA per 32 columns / pairs,
-// us: 77 x 4096 x 4096 13.2 / 10.2, 16 x 4096 x 4096 13.0 / 10.0, 128 x 4096 x 4096 13.4 / 11.3, 77 x 1024 x 4096 11.5 / 7.8, 300 x 1024 x 4096
-// 11.9 / 8.8, 77 x 1024 x 3072 9.4 / 6.7, 16 x 4096 x 1024 8.5 / 4.4, 77 x 4096 x 1024 4.95 / 4.95, 77 x 4096 x 256 3.5 / 3.3, 256 x 1152 x 1152 4.85 / 4.26;
+// us: 77 x 4096 x 4096 13.2 / 10.1, 16 x 4096 x 4096 13.0 / 9.3, 128 x 4096 x 4096 13.4 / 11.0, 77 x 1024 x 4096 11.5 / 7.4, 300 x 1024 x 4096
+// 11.9 / 8.7, 77 x 1024 x 3072 9.4 / 6.0, 16 x 4096 x 1024 8.5 / 4.8, 256 x 1152 x 1152 4.6 / 3.9;
 // a short K of more than two row tiles only where 32 columns do not fit: 300 x 1152 x 1152 5.07 / 5.11, 512 x 1152 x 1152 5.26 / 5.61.  (A copy
 // for each K block: 77 x 4096 x 4096 12.7, 77 x 1024 x 4096 11.4; stages of 128 rows: 11.2 and 7.8; eight K blocks to a copy and two stages
-// 12.3 and 8.8, two and eight 11.7 and 9.7.)  Two CTAs of 32 columns on an SM / pairs of 48 or 64: 130 x 4096 x 4096 16.9 / 13.5, 256 x 4096 x
-// 4096 18.3 / 14.3, 520 x 1024 x 4096 17.4 / 11.5, 300 x 3072 x 4096 17.3 / 13.2, 256 x 4608 x 4608 21.9 / 16.2, 520 x 1152 x 1152 6.8 / 6.1, 200 x
-// 4096 x 1024 6.3 / 5.8.  K shared by the CTAs of a cluster / the parts' accumulators in one pair: 520 x 1152 x 4304 18.4 / 13.5, 160 x 1152 x
-// 4304 17.6 / 11.0, 96 x 1152 x 4304 12.1 / 10.4, 128 x 4608 x 4608 19.3 / 13.4, 128 x 4096 x 4608 18.1 / 12.2, 300 x 1024 x 2112 14.4 / 7.5, 9 x 4096
+// 12.3 and 8.8, two and eight 11.7 and 9.7.)  Two CTAs of 32 columns on an SM / pairs of 48 or 64: 130 x 4096 x 4096 16.9 / 12.7, 256 x 4096 x
+// 4096 18.3 / 14.3, 520 x 1024 x 4096 17.4 / 10.9, 300 x 3072 x 4096 17.3 / 13.2, 256 x 4608 x 4608 21.9 / 16.2, 520 x 1152 x 1152 6.8 / 5.4, 200 x
+// 4096 x 1024 6.2 / 6.0.  K shared by the CTAs of a cluster / the parts' accumulators in one pair: 520 x 1152 x 4304 18.4 / 12.8, 160 x 1152 x
+// 4304 17.6 / 11.0, 96 x 1152 x 4304 12.1 / 9.3, 128 x 4608 x 4608 19.3 / 12.3, 128 x 4096 x 4608 18.1 / 12.2, 300 x 1024 x 2112 14.4 / 7.5, 9 x 4096
 // x 4104 23.5 / 12.4.  The 96-column form with 96 columns of a pair tile to a CTA (two CTAs per SM, five stages of one block): 520 x 4304 x 1152
 // 11.9 / 11.5, x 512 8.5 / 8.9: left alone.
+// A short K ends before the pair's set-up (two cluster barriers, and no other pair beside it) has paid: from eight K a row on, up to K = 1024 for 128
+// rows and more, and from K = 384 on where the one-CTA tiles leave half of the SMs idle.  One CTA / pairs, 4096 columns: 16 rows K = 256 3.70
+// / 3.54, 40 rows K = 384 4.11 / 3.81, 77 rows K = 256 3.05 / 3.70, K = 640 4.50 / 4.43, 128 rows K = 768 4.12 / 4.65, K = 1024 5.00 / 5.16 (3072 columns
+// 4.81 / 4.51), 256 rows K = 512 4.25 / 4.56, K = 1024 6.28 / 5.97; 1152 columns: 128 rows K = 256 2.78 / 2.78, K = 384 3.10 / 2.97, K = 768 4.01 / 3.39.
 static int fewpair_cols(const GemmArgs& g, int parts) {
     if (!pair_wanted() || g.K < 256 || g.a_kblk) return 0;
+    const bool idle = 2 * g.num_m * ((g.N + 31) / 32) <= sm_count();
+    if (parts == 1 && g.K < 8 * (g.M < 128 ? g.M : 128) && !(idle && g.K >= 384)) return 0;
     for (int fc = 32; fc <= 64; fc += 16)
         if (2 * g.num_m * ((g.N + 2 * fc - 1) / (2 * fc)) <= sm_count()) return fc == 32 && g.num_m > 2 && g.K < LONG_K && parts == 1 ? 0 : fc;
     return 0;
@@ -2149,10 +2163,11 @@ static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, 
     const int ra = g.num_m > 1 ? BM / 2 : (g.M + 15) / 16 * 8;      // rows of a CTA: half of the tile's, in eights
     int stages = FP_ROOM / fp_stage_bytes(ra, fc);
     if (stages > FP_MAX_STAGES) stages = FP_MAX_STAGES;
-    // no more room than the K blocks take: a short K leaves some for the next kernel's CTAs
+    // no more stages than the K blocks take: a short K leaves room for the next kernel's CTAs, but not for another one of this grid
     const int copies = (g.K / BK + FP_KPS - 1) / FP_KPS + (g.K % BK != 0);
     if (stages > copies) stages = copies;
-    const int smem = stages * fp_stage_bytes(ra, fc) + 1024 /*align*/ + 256 /*barriers*/;
+    int smem = stages * fp_stage_bytes(ra, fc) + 1024 /*align*/ + 256 /*barriers*/;
+    if (smem < PAIR_ALONE) smem = PAIR_ALONE;
     const int kw = g.K / BK * BK;
     if (!cached_tmap_kblocks(&mA, x, g.M, kw, ldx, ra, FP_KPS) || !cached_tmap_kblocks(&mB, w, g.N, kw, g.K, fc, FP_KPS)) return false;
     CUtensorMap mA2 = mA, mB2 = mB;

@@ -496,11 +496,11 @@ def test_guided_step_stays_inside_the_workspace_it_was_given(pkg, dev, room):
 
 @pytest.mark.parametrize("rows", [(600, 724, 1100), (513, 650, 768)])
 def test_states_in_turn_without_a_wait(pkg, dev, rows):
-    """Conditioned forwards of three states, some hundred passes behind one another with nothing that waits between them: the bits of
-    the first pass, no wait that ran out."""
+    """Conditioned forwards of three states and linears of few rows and a short K (several launches of CTA pairs on their way at once), some
+    hundred passes behind one another with nothing that waits between them: the bits of the first pass, no wait that ran out."""
     T, L, V = 60, 3, 40
     w = pkg.Weights(n_layers=L, seed=1234, weight_set="B", device=dev)
-    states = []
+    states, lins = [], []
     for k, I in enumerate(rows):
         pos, ar = pkg.seq_t2i(T, I, 1)
         mask = torch.zeros(T + I, dtype=torch.uint8)
@@ -510,16 +510,23 @@ def test_states_in_turn_without_a_wait(pkg, dev, rows):
         states.append((pkg.Engine(w, T, I, ar_len=ar), torch.from_numpy(make_ids(T, k)).to(dev), pos.to(dev),
                        u16_to_torch(seeded_bf16((I, 3072), 40 + k), dev), vis,
                        torch.empty(T + I, 3072, dtype=torch.bfloat16, device=dev)))
+    for i, (m, n, k) in enumerate((m, n, k) for n, k in ((4096, 256), (4096, 1024)) for m in (8, 16, 45, 77, 128, 256)):
+        lins.append((u16_to_torch(seeded_bf16((m, k), 100 + i), dev), u16_to_torch(seeded_bf16((n, k), 120 + i, 0.0, 0.05), dev),
+                     torch.empty(m, n, dtype=torch.bfloat16, device=dev)))
 
     def one_pass(i):
         e, ids, pos, vin, vis, out = states[i % 3]
         e.forward(ids, pos, vin, 0.3, out=out, visual=vis)
+        for x, wt, y in lins:
+            pkg.lib.hd_linear(pkg.ptr(x), pkg.ptr(wt), None, pkg.ptr(y), x.shape[0], wt.shape[0], x.shape[1], 1)
 
     for i in range(3):
         one_pass(i)
         torch.cuda.synchronize()
-    outs = [s[-1] for s in states]
+    outs = [s[-1] for s in states] + [y for _, _, y in lins]
     first = [o.clone() for o in outs]
+    for x, wt, y in lins:
+        assert (y.float() - x.float() @ wt.float().t()).abs().max().item() <= 2.0 ** -7 * y.float().abs().max().item()
     for i in range(300):
         one_pass(i)
     torch.cuda.synchronize()
