@@ -480,6 +480,11 @@ int o1_gemm(const void *x, int ldx, const void *w, const void *w2, void *y, int 
  * be summed in parts; -2 (the vision tower's linears): as -1, and a pair tile of 96 to 256 columns from 257 rows on where K >= 2048 (in
  * place of narrow tiles), from 1025 rows on where 1024 <= K < 2048 and N is no multiple of 256, if that takes fewer rounds. */
 int o1_gemm_form(int M, int N, int K, int epi, int force_bn, int *width, int *ctas);
+/* Which of a form's two kernels that is.  Form 4: the columns of w that each CTA of a pair has (32, 48 or 64), form 2 with SwiGLU: the
+ * rows of x in a tile of 256 weight rows; 0: one CTA per narrow tile, tiles of 256 x 256.  The second one: the same number of rows for
+ * o1_gemm_qkv. */
+int o1_gemm_pair_tile(int M, int N, int K, int epi, int force_bn);
+int o1_gemm_qkv_pair_rows(int M, int qc, int kc, int K);
 /* The q, k and v projections of a decoder block (src/model/block.c:257-265) with the per-head RMSNorm + rotary of
  * q and k (:266-289) as ONE launch over the three weight tensors: y [M, qc | kc | kc] (row pitch ldy) =
  * norm_rope(x wq^T) | norm_rope(x wk^T) | x wv^T.  q_norm / k_norm [128] bf16, cs [M,128] fp32 (o1_mrope_table),

@@ -248,6 +248,8 @@ _sig("o1_launch_count", c_int64, c_int)
 _sig("o1_gemm", c_int, _P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, c_int,
      c_float, c_int)
 _sig("o1_gemm_form", c_int, c_int, c_int, c_int, c_int, c_int, C.POINTER(c_int), C.POINTER(c_int))
+_sig("o1_gemm_pair_tile", c_int, c_int, c_int, c_int, c_int, c_int)
+_sig("o1_gemm_qkv_pair_rows", c_int, c_int, c_int, c_int, c_int)
 _sig("o1_gemm_qkv", c_int, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, _P, c_float)
 _sig("o1_flash_attention", c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, c_int, c_int, c_int,
      c_int, c_float)

@@ -931,6 +931,11 @@ int o1_gemm_form(int M, int N, int K, int epi, int force_bn, int* width, int* ct
     if (ctas) *ctas = p.ks;
     return p.form;
 }
+int o1_gemm_pair_tile(int M, int N, int K, int epi, int force_bn) {
+    if (o1_gemm_form(M, N, K, epi, force_bn, nullptr, nullptr) < 0) return 0;
+    return gemm_plan(M, N, K, epi, force_bn, true, (N % 256) == 0).pair;
+}
+int o1_gemm_qkv_pair_rows(int M, int qc, int kc, int K) { return M < 8 || qc <= 0 || kc <= 0 || K <= 0 ? 0 : gemm_qkv_rows(M, qc, kc, K); }
 int o1_gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void* wv, void* y, int ldy, int M, int qc,
                 int kc, int K, const void* q_norm, const void* k_norm, const float* cs, float eps) {
     if (!gemm_qkv(x, ldx, wq, wk, wv, y, ldy, M, qc, kc, K, q_norm, k_norm, cs, eps, 0, nullptr, nullptr, nullptr, g_stream))

@@ -2059,6 +2059,31 @@ static SplitPlan split_plan(int M, int N, int K, bool may_split, bool resid) {
     return {0, 0};
 }
 
+// Narrow tiles on CTA pairs: columns of a CTA, or 0 for the one-CTA forms; K from 256 on.  32 columns where that makes at most one CTA per
+// SM, else 48 or 64 (two CTAs of 32 columns on an SM have half the room each for weights on their way).  One CTA per 32 columns / pairs,
+// us: 77 x 4096 x 4096 13.2 / 10.1, 16 x 4096 x 4096 13.0 / 9.3, 128 x 4096 x 4096 13.4 / 11.0, 77 x 1024 x 4096 11.5 / 7.4, 300 x 1024 x 4096
+// 11.9 / 8.7, 77 x 1024 x 3072 9.4 / 6.0, 16 x 4096 x 1024 8.5 / 4.8, 256 x 1152 x 1152 4.6 / 3.9;
+// a short K of more than two row tiles only where 32 columns do not fit: 300 x 1152 x 1152 5.07 / 5.11, 512 x 1152 x 1152 5.26 / 5.61.  (A copy
+// for each K block: 77 x 4096 x 4096 12.7, 77 x 1024 x 4096 11.4; stages of 128 rows: 11.2 and 7.8; eight K blocks to a copy and two stages
+// 12.3 and 8.8, two and eight 11.7 and 9.7.)  Two CTAs of 32 columns on an SM / pairs of 48 or 64: 130 x 4096 x 4096 16.9 / 12.7, 256 x 4096 x
+// 4096 18.3 / 14.3, 520 x 1024 x 4096 17.4 / 10.9, 300 x 3072 x 4096 17.3 / 13.2, 256 x 4608 x 4608 21.9 / 16.2, 520 x 1152 x 1152 6.8 / 5.4, 200 x
+// 4096 x 1024 6.2 / 6.0.  K shared by the CTAs of a cluster / the parts' accumulators in one pair: 520 x 1152 x 4304 18.4 / 12.8, 160 x 1152 x
+// 4304 17.6 / 11.0, 96 x 1152 x 4304 12.1 / 9.3, 128 x 4608 x 4608 19.3 / 12.3, 128 x 4096 x 4608 18.1 / 12.2, 300 x 1024 x 2112 14.4 / 7.5, 9 x 4096
+// x 4104 23.5 / 12.4.  The 96-column form with 96 columns of a pair tile to a CTA (two CTAs per SM, five stages of one block): 520 x 4304 x 1152
+// 11.9 / 11.5, x 512 8.5 / 8.9: left alone.
+// A short K ends before the pair's set-up (two cluster barriers, and no other pair beside it) has paid: from eight K a row on, up to K = 1024 for 128
+// rows and more, and from K = 384 on where the one-CTA tiles leave half of the SMs idle.  One CTA / pairs, 4096 columns: 16 rows K = 256 3.70
+// / 3.54, 40 rows K = 384 4.11 / 3.81, 77 rows K = 256 3.05 / 3.70, K = 640 4.50 / 4.43, 128 rows K = 768 4.12 / 4.65, K = 1024 5.00 / 5.16 (3072 columns
+// 4.81 / 4.51), 256 rows K = 512 4.25 / 4.56, K = 1024 6.28 / 5.97; 1152 columns: 128 rows K = 256 2.78 / 2.78, K = 384 3.10 / 2.97, K = 768 4.01 / 3.39.
+static int fewpair_cols(int M, int N, int K, int parts) {
+    if (!pair_wanted() || K < 256) return 0;
+    const long num_m = (M + BM - 1) / BM;
+    const bool idle = 2 * num_m * ((N + 31) / 32) <= sm_count();
+    if (parts == 1 && K < 8 * (M < 128 ? M : 128) && !(idle && K >= 384)) return 0;
+    for (int fc = 32; fc <= 64; fc += 16)
+        if (2 * num_m * ((N + 2 * fc - 1) / (2 * fc)) <= sm_count()) return fc == 32 && num_m > 2 && K < LONG_K && parts == 1 ? 0 : fc;
+    return 0;
+}
 static int swiglu_rows_width(int M, int N, int K) {
     long units = 0;
     tile_form((M + BM - 1) / BM, 2 * N, K, true, true, &units);
@@ -2066,12 +2091,13 @@ static int swiglu_rows_width(int M, int N, int K) {
 }
 static int simt_rows(int M, int N, int K);
 // The form a GEMM takes.  plain: row-major output; wide_ok: 256-column tiles fit it.
-GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok) {
+GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok, bool blocked_a) {
     if (!gemm_tc_supported(M, N, K, epi)) return {GEMM_ROWS, simt_rows(M, N, K), 1};
     const int num_m = (M + BM - 1) / BM;
     if (epi == EPI_SWIGLU) {     // (2N columns of gate and up; pairs of 256 x 256 or gemm_rows_kernel's of 256 x any)
-        const bool pair = force_bn <= 0 && (tile_form(num_m, 2 * N, K, true, true) == TILE_PAIR || (force_bn == 0 && swiglu_rows_width(M, N, K)));
-        return {pair ? GEMM_PAIR : GEMM_TILE, 256, pair ? 2 : 1};
+        const int rows = force_bn == 0 && !blocked_a ? swiglu_rows_width(M, N, K) : 0;
+        const bool pair = force_bn <= 0 && (rows || tile_form(num_m, 2 * N, K, true, true) == TILE_PAIR);
+        return {pair ? GEMM_PAIR : GEMM_TILE, 256, pair ? 2 : 1, rows};
     }
     const bool pair_ok = epi == EPI_STORE || epi == EPI_BIAS || epi == EPI_RESID;
     if (force_bn == 128) return {GEMM_TILE, 128, 1};
@@ -2086,7 +2112,8 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
     if (small) {
         const SplitPlan p = split_plan(M, N, K, (tower || force_bn == GEMM_SPLIT_K) && pair_wanted(), resid);
         // the tower's long K (the MLP's second linear, the mergers): pair tiles of any width instead of narrow ones, from 257 rows on
-        if (p.ks > 1 || (p.bn > 0 && !(tower && pair_wanted() && K >= LONG_K && num_m > 2))) return {GEMM_FEW, p.bn, p.ks};
+        if (p.ks > 1 || (p.bn > 0 && !(tower && pair_wanted() && K >= LONG_K && num_m > 2)))
+            return {GEMM_FEW, p.bn, p.ks, p.bn == 96 || blocked_a ? 0 : fewpair_cols(M, N, K, p.ks)};
         // (From 1025 rows on a K of 1024 and more too: the tower of 1200 / 3024 / 4096 patches 2800 / 5600 / 8100 -> 2700 / 5370 / 7820
         // us, but of 832 patches 2165 -> 2197.  Only where 256 does not divide N: with the 256-column forms to choose from, a
         // pair width loses as often as it gains, 1600 x 2304 x 1152 13.5 / 14.5, 1100 x 4096 x 1024 12.6 / 13.7, 4096 rows
@@ -2130,30 +2157,6 @@ static bool launch_split_bn(const CUtensorMap* tA, const CUtensorMap* tB, GemmAr
     return true;
 }
 
-// Narrow tiles on CTA pairs: columns of a CTA, or 0 for the one-CTA forms; K from 256 on.  32 columns where that makes at most one CTA per
-// SM, else 48 or 64 (two CTAs of 32 columns on an SM have half the room each for weights on their way).  One CTA per 32 columns / pairs,
-// us: 77 x 4096 x 4096 13.2 / 10.1, 16 x 4096 x 4096 13.0 / 9.3, 128 x 4096 x 4096 13.4 / 11.0, 77 x 1024 x 4096 11.5 / 7.4, 300 x 1024 x 4096
-// 11.9 / 8.7, 77 x 1024 x 3072 9.4 / 6.0, 16 x 4096 x 1024 8.5 / 4.8, 256 x 1152 x 1152 4.6 / 3.9;
-// a short K of more than two row tiles only where 32 columns do not fit: 300 x 1152 x 1152 5.07 / 5.11, 512 x 1152 x 1152 5.26 / 5.61.  (A copy
-// for each K block: 77 x 4096 x 4096 12.7, 77 x 1024 x 4096 11.4; stages of 128 rows: 11.2 and 7.8; eight K blocks to a copy and two stages
-// 12.3 and 8.8, two and eight 11.7 and 9.7.)  Two CTAs of 32 columns on an SM / pairs of 48 or 64: 130 x 4096 x 4096 16.9 / 12.7, 256 x 4096 x
-// 4096 18.3 / 14.3, 520 x 1024 x 4096 17.4 / 10.9, 300 x 3072 x 4096 17.3 / 13.2, 256 x 4608 x 4608 21.9 / 16.2, 520 x 1152 x 1152 6.8 / 5.4, 200 x
-// 4096 x 1024 6.2 / 6.0.  K shared by the CTAs of a cluster / the parts' accumulators in one pair: 520 x 1152 x 4304 18.4 / 12.8, 160 x 1152 x
-// 4304 17.6 / 11.0, 96 x 1152 x 4304 12.1 / 9.3, 128 x 4608 x 4608 19.3 / 12.3, 128 x 4096 x 4608 18.1 / 12.2, 300 x 1024 x 2112 14.4 / 7.5, 9 x 4096
-// x 4104 23.5 / 12.4.  The 96-column form with 96 columns of a pair tile to a CTA (two CTAs per SM, five stages of one block): 520 x 4304 x 1152
-// 11.9 / 11.5, x 512 8.5 / 8.9: left alone.
-// A short K ends before the pair's set-up (two cluster barriers, and no other pair beside it) has paid: from eight K a row on, up to K = 1024 for 128
-// rows and more, and from K = 384 on where the one-CTA tiles leave half of the SMs idle.  One CTA / pairs, 4096 columns: 16 rows K = 256 3.70
-// / 3.54, 40 rows K = 384 4.11 / 3.81, 77 rows K = 256 3.05 / 3.70, K = 640 4.50 / 4.43, 128 rows K = 768 4.12 / 4.65, K = 1024 5.00 / 5.16 (3072 columns
-// 4.81 / 4.51), 256 rows K = 512 4.25 / 4.56, K = 1024 6.28 / 5.97; 1152 columns: 128 rows K = 256 2.78 / 2.78, K = 384 3.10 / 2.97, K = 768 4.01 / 3.39.
-static int fewpair_cols(const GemmArgs& g, int parts) {
-    if (!pair_wanted() || g.K < 256 || g.a_kblk) return 0;
-    const bool idle = 2 * g.num_m * ((g.N + 31) / 32) <= sm_count();
-    if (parts == 1 && g.K < 8 * (g.M < 128 ? g.M : 128) && !(idle && g.K >= 384)) return 0;
-    for (int fc = 32; fc <= 64; fc += 16)
-        if (2 * g.num_m * ((g.N + 2 * fc - 1) / (2 * fc)) <= sm_count()) return fc == 32 && g.num_m > 2 && g.K < LONG_K && parts == 1 ? 0 : fc;
-    return 0;
-}
 template <int EPI, bool PARTS>
 static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, int fc, int parts, cudaStream_t st) {
     static std::atomic<uint64_t> attr_done{0};
@@ -2185,8 +2188,7 @@ static bool launch_few_pair(const void* x, int ldx, const void* w, GemmArgs& g, 
 
 template <int EPI>
 static bool launch_split(const CUtensorMap* tA, const void* x, int ldx, const void* w, GemmArgs& g, const GemmPlan& p, cudaStream_t st) {
-    if (p.bn != 96)
-        if (const int fc = fewpair_cols(g, p.ks)) return p.ks > 1 ? launch_few_pair<EPI, true>(x, ldx, w, g, fc, p.ks, st) : launch_few_pair<EPI, false>(x, ldx, w, g, fc, 1, st);
+    if (p.pair) return p.ks > 1 ? launch_few_pair<EPI, true>(x, ldx, w, g, p.pair, p.ks, st) : launch_few_pair<EPI, false>(x, ldx, w, g, p.pair, 1, st);
     CUtensorMap mB;
     if (!cached_tmap(&mB, w, g.N, g.K, g.K, p.bn)) return false;
     if (p.bn == 96) return launch_split_bn<EPI, 96>(tA, &mB, g, st);
@@ -2326,13 +2328,12 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
         set_error("gemm: BN=256 needs N (and the output column block) %% 256 == 0");
         return false;
     }
-    const GemmPlan p = gemm_plan(M, N, K, epi, a_kblk && force_bn < 0 ? 0 : force_bn, !o_cb && !o_tab, wide_ok);     // (K in parts: plain rows)
+    const GemmPlan p = gemm_plan(M, N, K, epi, a_kblk && force_bn < 0 ? 0 : force_bn, !o_cb && !o_tab, wide_ok, a_kblk != 0);     // (K in parts: plain rows)
     if (epi == EPI_SWIGLU) {
-        const int bn = force_bn == 0 && !a_kblk ? swiglu_rows_width(M, N, K) : 0;
-        if (bn) {
+        if (p.pair) {
             CUtensorMap mG, mU;
             if (!cached_tmap(&mG, w, N, K, K, 64) || !cached_tmap(&mU, w2, N, K, K, 64)) return false;
-            return launch_rows<EPI_SWIGLU>(x, ldx, &mG, &mU, &mU, g, bn, st);
+            return launch_rows<EPI_SWIGLU>(x, ldx, &mG, &mU, &mU, g, p.pair, st);
         }
         g.num_n = N / 128;
         if (p.form != GEMM_PAIR) return launch_tc<EPI_SWIGLU, 256>(tA, tB, tB2, g, st);
@@ -2394,6 +2395,14 @@ bool gemm_bf16_ex(const void* x, int ldx, const void* w, const void* w2, void* y
     return false;
 }
 
+int gemm_qkv_rows(int M, int qc, int kc, int K) {
+    const int N = qc + 2 * kc;
+    if (N % 256) return 0;
+    long units = 0;
+    tile_form((M + BM - 1) / BM, N, K, (qc % 256) == 0 && (kc % 256) == 0, true, &units);
+    return rows_width(M, N / 256, K, (double)units);
+}
+
 // q | k | v projections of one activation matrix as ONE launch: y[M, qc | kc | kc] (row pitch ldy) = x wq^T | x wk^T |
 // x wv^T, the per-head RMSNorm + rotary applied to the q and k columns in the epilogue (norm weights q_norm / k_norm
 // [128], cos|sin table cs [M,128] fp32).  Three launches of 14.05 + 3.5 + 3.5 waves of tiles (at 16640 rows) become
@@ -2450,10 +2459,9 @@ bool gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const void
     // 256-wide tiles need every segment (and every destination block) to be a multiple of 256 columns
     bool wide = (qc % 256) == 0 && (kc % 256) == 0;
     if (tabs && (((qc / n_dst) % 256) != 0 || ((kc / n_dst) % 256) != 0)) wide = false;
-    long units = 0;
-    const TileForm form = tile_form(g.num_m, N, K, wide, true, &units);
-    const int bn = !tabs && (N % 256) == 0 && K >= LONG_K && (ldy % 8) == 0 && (((uintptr_t)y) & 15) == 0 ? rows_width(M, N / 256, K, (double)units) : 0;
+    const int bn = !tabs && (ldy % 8) == 0 && (((uintptr_t)y) & 15) == 0 ? gemm_qkv_rows(M, qc, kc, K) : 0;
     if (bn) return launch_rows<EPI_QKV>(x, ldx, &mQ, &mK, &mV, g, bn, st);
+    const TileForm form = tile_form(g.num_m, N, K, wide, true);
     g.num_n = N / (form == TILE_128 ? 128 : 256);
     if (form == TILE_PAIR) return launch_tc_pair<EPI_QKV>(&mA, &mQ, &mK, g, st, &mV);
     return form == TILE_256 ? launch_tc<EPI_QKV, 256>(&mA, &mQ, &mK, g, st, &mV) : launch_tc<EPI_QKV, 128>(&mA, &mQ, &mK, g, st, &mV);

@@ -38,9 +38,12 @@ enum { GEMM_SPLIT_K = -1, GEMM_TOWER = -2 };
 // The form a problem takes: GEMM_ROWS = warps (bn: rows that share one), GEMM_TILE = one CTA per 128 x bn tile, GEMM_PAIR = two
 // per 256 x 256 tile (SwiGLU: or 256 weight rows x a fitted number of rows), GEMM_FIT = one per tile of a width fitted to the SMs,
 // GEMM_FEW = tiles for problems that have few (a tile's K is summed in ks parts).  GEMM_TILE and GEMM_FIT with ks = 2: a CTA pair per 256 x bn tile.
+// pair: GEMM_FEW: columns of a CTA of gemm_few_pair_kernel, GEMM_PAIR: rows of x in a tile of gemm_rows_kernel; 0: the other kernel of that form.
 enum GemmForm { GEMM_ROWS = 0, GEMM_TILE = 1, GEMM_PAIR = 2, GEMM_FIT = 3, GEMM_FEW = 4 };
-struct GemmPlan { int form, bn, ks; };
-GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok);
+struct GemmPlan { int form, bn, ks, pair = 0; };
+GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool wide_ok, bool blocked_a = false);
+// rows of x in a tile of gemm_rows_kernel for q | k | v with plain rows, 0: another kernel
+int gemm_qkv_rows(int M, int qc, int kc, int K);
 bool gemm_bf16(const void* x, const void* w, const void* w2, void* y, int M, int N, int K, int epi,
                const void* bias, const void* resid, float scale, int force_bn, cudaStream_t st);
 // Same, with explicit row pitches (elements) for x and y so that a GEMM can

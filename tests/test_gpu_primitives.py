@@ -433,7 +433,8 @@ def test_qkv_projections_as_one_launch(pkg, dev, M, qc, kc, K):
 
 @pytest.mark.parametrize("M,N,K,epi", [(4352, 4096, 512, 0), (4115, 4096, 256, 2), (4200, 3072, 320, 1), (8320, 4096, 192, 2),
                                        (1280, 4096, 2048, 3), (1400, 4096, 2056, 3), (2304, 4096, 2048, 0), (2561, 4096, 2104, 2),
-                                       (2048, 4096, 512, 1), (1921, 4096, 1032, 2), (2304, 4096, 1024, 0)])
+                                       (2048, 4096, 512, 1), (1921, 4096, 1032, 2), (2304, 4096, 1024, 0),
+                                       (2242, 4096, 2048, 3)])
 def test_gemm_on_cta_pairs_equals_single_cta_tiles(pkg, dev, M, N, K, epi):
     """The cta_group::2 form (two CTAs per 256 x 256 tile, each with half of the B tile) adds a row's K products in the
     same order as the one-CTA form: same bits, for an even and an odd number of row tiles, a partly filled last row
@@ -470,13 +471,19 @@ def test_gemm_on_cta_pairs_equals_single_cta_tiles(pkg, dev, M, N, K, epi):
     assert err < 1e-2, err     # the pair form really computed the product (fp32 reference, bf16 rounding of the result)
 
 
-@pytest.mark.parametrize("M", [77, 129, 144, 257, 296, 513, 592, 785, 1030, 1300])
+@pytest.mark.parametrize("M,N,qc,kc", [(77, 1536, 512, 256), (129, 1536, 512, 256), (144, 1536, 512, 256), (257, 1536, 512, 256), (296, 1536, 512, 256),
+                                       (513, 1536, 512, 256), (592, 1536, 512, 256), (785, 1536, 512, 256), (1030, 1536, 512, 256), (1300, 1536, 512, 256),
+                                       (300, 12288, 4096, 1024), (785, 12288, 4096, 1024), (1300, 12288, 4096, 1024)])
 @pytest.mark.parametrize("K", [2048, 2104])
-def test_pairs_with_tokens_as_columns(pkg, dev, M, K):
+def test_pairs_with_tokens_as_columns(pkg, dev, M, N, qc, kc, K):
     """gate | up + SwiGLU and q | k | v with the weights as the MMA's rows (tiles of 256 weight rows and a number of tokens that fits)
-    give the bits of one-CTA tiles: partly filled token tiles, fewer and more than a round of tiles, a ragged last K block, q, k and v tiles of
-    one launch; nothing is written beside the result."""
-    N, qc, kc = 1536, 512, 256
+    give the bits of one-CTA tiles: partly filled token tiles, fewer than a round of tiles and up to eight of them for a pair, a ragged last K
+    block, q, k and v tiles of one launch; nothing is written beside the result.  (77 rows of gate | up and q | k | v of 1030 and 1300 rows and
+    1024 columns are left to other kernels.)"""
+    if pkg.lib.o1_sm_count() == 148:
+        assert (pkg.lib.o1_gemm_pair_tile(M, N, K, 3, 0) >= 64) == (M != 77)
+        assert (pkg.lib.o1_gemm_qkv_pair_rows(M, qc, kc, K) >= 64) == (qc != 512 or M < 1030)
+        assert pkg.lib.o1_gemm_pair_tile(M, N, K, 3, 256) == 0
     x, wg, wu = (dv(seeded_bf16((r, K), 60 + i, 0.0, 1.0 if i == 0 else 0.05), dev) for i, r in enumerate((M, N, N)))
     ys = []
     for bn in (0, 256):
@@ -505,7 +512,7 @@ def test_pairs_with_tokens_as_columns(pkg, dev, M, K):
     assert pkg.lib.o1_device_error() == 0
 
 
-@pytest.mark.parametrize("M,K", [(130, 72), (256, 192), (100, 64)])
+@pytest.mark.parametrize("M,K", [(130, 72), (256, 192), (200, 64)])
 @pytest.mark.parametrize("blocks", [149, 185, 186, 259, 295])
 def test_last_tiles_as_halves(pkg, dev, M, K, blocks):
     """gate | up + SwiGLU on CTA pairs (blocks of 128 columns, 74 pairs): the tiles of a last round that at most half of the pairs have,
@@ -516,6 +523,8 @@ def test_last_tiles_as_halves(pkg, dev, M, K, blocks):
     try:
         for on in (1, 0):
             pkg.lib.o1_gemm_pair_mode(on)
+            if pkg.lib.o1_sm_count() == 148:
+                assert gemm_form(pkg, M, N, K, 3, -1)[2] == 1 + on and pkg.lib.o1_gemm_pair_tile(M, N, K, 3, -1) == 0
             y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
             assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(wg), pkg.ptr(wu), pkg.ptr(y), N + 8, M, N, K, 3, None, None, 0, 0.0, -1) == 0, pkg.last_error()
             done(pkg, "swiglu")
@@ -525,6 +534,23 @@ def test_last_tiles_as_halves(pkg, dev, M, K, blocks):
         pkg.lib.o1_gemm_pair_mode(1)
     assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
     assert pkg.lib.o1_device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1280, 12288, 2048), (1280, 12288, 2104), (2048, 12288, 4096), (2242, 12288, 2048), (1400, 1536, 2104)])
+def test_gate_up_on_whole_pair_tiles_of_a_long_k(pkg, dev, M, N, K):
+    """gate | up + SwiGLU on tiles of 256 x 256, more K blocks to a tile than there are stages: last rounds of halves (36 and 28 of 74 pairs), a whole
+    one (50), a single round, ragged K and rows; the bits of one-CTA tiles, nothing written beside the result."""
+    if pkg.lib.o1_sm_count() == 148:
+        assert gemm_form(pkg, M, N, K, 3, 0) == (2, 256, 2) and pkg.lib.o1_gemm_pair_tile(M, N, K, 3, 0) == 0
+    x, wg, wu = (dv(seeded_bf16((r, K), 50 + i, 0.0, 1.0 if i == 0 else 0.05), dev) for i, r in enumerate((M, N, N)))
+    ys = []
+    for bn in (0, 256):
+        y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
+        assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(wg), pkg.ptr(wu), pkg.ptr(y), N + 8, M, N, K, 3, None, None, 0, 0.0, bn) == 0, pkg.last_error()
+        done(pkg, "swiglu")
+        assert (y[M:] == 777.0).all() and (y[:, N:] == 777.0).all(), "written beside the matrix"
+        ys.append(y)
+    assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
 
 
 def check_linear_f64(y, x, w, bias, what):
@@ -561,10 +587,12 @@ def gemm_form(pkg, M, N, K, epi, bn):
     return pkg.lib.o1_gemm_form(M, N, K, epi, bn, C.byref(width), C.byref(ctas)), width.value, ctas.value
 
 
-@pytest.mark.parametrize("M,N,K", [(8, 72, 256), (77, 4096, 320), (16, 1032, 4096), (17, 512, 832), (33, 1024, 640), (100, 768, 1024), (113, 640, 384), (64, 1024, 576), (65, 3072, 512), (128, 4608, 1152),
-                                   (129, 2048, 448), (300, 1024, 4096), (520, 896, 2048), (1000, 512, 1024), (256, 4608, 704), (130, 3072, 448), (520, 1152, 1152), (300, 1160, 640)])
+@pytest.mark.parametrize("M,N,K,cols", [(8, 72, 256, 32), (77, 4096, 632, 32), (40, 4096, 320, 32), (16, 1032, 4096, 32), (17, 512, 832, 32), (33, 1024, 640, 32),
+                                        (100, 768, 1024, 32), (113, 640, 384, 32), (64, 1024, 576, 32), (65, 3072, 520, 32), (128, 4608, 1152, 32),
+                                        (129, 2048, 1032, 32), (300, 1024, 4096, 32), (520, 896, 2048, 32), (256, 4608, 1088, 64), (130, 3072, 1088, 48),
+                                        (520, 1152, 1152, 48), (300, 1160, 2056, 32)])
 @pytest.mark.parametrize("epi", [0, 1, 2, 7, 8, 9])
-def test_narrow_tiles_on_pairs_give_the_bits_of_single_ctas(pkg, dev, M, N, K, epi):
+def test_narrow_tiles_on_pairs_give_the_bits_of_single_ctas(pkg, dev, M, N, K, cols, epi):
     """The 32-column form with two CTAs per tile of 128 x 64, 96 or 128 and four K blocks to a copy against the one-CTA form (pair mode 0), every
     epilogue: rows shared by the two CTAs in eights, row tiles whose second half has no rows or few, a ragged last column tile, K blocks
     that are no whole number of copies."""
@@ -579,6 +607,7 @@ def test_narrow_tiles_on_pairs_give_the_bits_of_single_ctas(pkg, dev, M, N, K, e
             pkg.lib.o1_gemm_pair_mode(mode)
             if pkg.lib.o1_sm_count() == 148:
                 assert gemm_form(pkg, M, N, K, epi, 0) == (4, 32, 1)
+                assert pkg.lib.o1_gemm_pair_tile(M, N, K, epi, 0) == (cols if mode else 0)
             y = torch.full((M + 1, N + 8), 777.0, dtype=torch.bfloat16, device=dev)
             assert pkg.lib.o1_gemm(pkg.ptr(x), K, pkg.ptr(w), None, pkg.ptr(y), N + 8, M, N, K, epi, pkg.ptr(b), pkg.ptr(r), N, 0.0, 0) == 0, pkg.last_error()
             done(pkg, "narrow tiles")
