@@ -2095,7 +2095,7 @@ GemmPlan gemm_plan(int M, int N, int K, int epi, int force_bn, bool plain, bool 
     if (!gemm_tc_supported(M, N, K, epi)) return {GEMM_ROWS, simt_rows(M, N, K), 1};
     const int num_m = (M + BM - 1) / BM;
     if (epi == EPI_SWIGLU) {     // (2N columns of gate and up; pairs of 256 x 256 or gemm_rows_kernel's of 256 x any)
-        const int rows = force_bn == 0 && !blocked_a ? swiglu_rows_width(M, N, K) : 0;
+        const int rows = force_bn <= 0 && !blocked_a ? swiglu_rows_width(M, N, K) : 0;
         const bool pair = force_bn <= 0 && (rows || tile_form(num_m, 2 * N, K, true, true) == TILE_PAIR);
         return {pair ? GEMM_PAIR : GEMM_TILE, 256, pair ? 2 : 1, rows};
     }

@@ -481,6 +481,7 @@ def test_pairs_with_tokens_as_columns(pkg, dev, M, N, qc, kc, K):
     block, q, k and v tiles of one launch; nothing is written beside the result.  (77 rows of gate | up and q | k | v of 1030 and 1300 rows and
     1024 columns are left to other kernels.)"""
     if pkg.lib.o1_sm_count() == 148:
+        assert pkg.lib.o1_gemm_pair_tile(M, N, K, 3, 0) == pkg.lib.o1_gemm_pair_tile(M, N, K, 3, -1)
         assert (pkg.lib.o1_gemm_pair_tile(M, N, K, 3, 0) >= 64) == (M != 77)
         assert (pkg.lib.o1_gemm_qkv_pair_rows(M, qc, kc, K) >= 64) == (qc != 512 or M < 1030)
         assert pkg.lib.o1_gemm_pair_tile(M, N, K, 3, 256) == 0
