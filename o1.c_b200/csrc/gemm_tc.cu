@@ -711,7 +711,7 @@ struct SplitCfg {
     static constexpr int STAGES = BN <= 32 ? 5 : 3;      // with KPS = 1 as many as leave room for a second CTA
     static constexpr int STAGE_BYTES = KPS * (BM + BN) * BK * 2;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
-    static constexpr int TMEM_COLS = BN <= 32 ? 32 : (BN <= 128 ? 128 : 256);
+    static constexpr int TMEM_COLS = BN == 32 ? 32 : (BN == 96 ? 128 : 256);
     // (32 columns are one group for each quadrant; two CTAs of 144 have no registers for more)
     static constexpr int THREADS = BN == 96 || (BN == 144 && KPS == 2) ? GEMM_THREADS : SK_THREADS;
 };
@@ -780,6 +780,7 @@ __device__ __forceinline__ void vrope_tables(const GemmArgs& g, int row, float (
 template <int EPI, int BN, int KPS>
 __global__ void __launch_bounds__(SplitCfg<BN, KPS>::THREADS, KPS == 1 ? 2 : 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g) {
+    static_assert(BN == 32 || BN == 96 || (BN == VQ_BN && EPI == EPI_VROPE), "the tiles there are");
     constexpr int SK_STAGE_BYTES = SplitCfg<BN, KPS>::STAGE_BYTES, SK_STAGES = SplitCfg<BN, KPS>::STAGES, NU = BN / 16;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -878,14 +879,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (warp == 1) tmem_dealloc(tmem_base, SplitCfg<BN, KPS>::TMEM_COLS);
         return;
     }
-    // The epilogue's other operands are requested while the main loop runs: this thread's residual row into registers, the
-    // tile's bias into shared memory (each of the eight units of a tile would otherwise wait for its own loads).
-    constexpr bool HAS_BIAS = epi_has_bias(EPI) || EPI == EPI_VROPE, HAS_RESID = epi_has_resid(EPI);
+    // (32 columns without a residual, or the tower's 144.)  The tile's bias comes into shared memory while the main loop runs: each of
+    // its units of 16 columns would otherwise wait for its own loads.
+    constexpr bool HAS_BIAS = epi_has_bias(EPI) || EPI == EPI_VROPE;
     const int q = warp & 3;       // TMEM lane quadrant this warp may access
     const int trow = q * 32 + lane;
     const int row = mb * BM + trow;
     const bool row_ok = row < g.M;
-    uint4 res[HAS_RESID ? 2 * NU : 1];
     float vcs[36], vsn[36];      // (EPI_VROPE)
     if (ok && warp >= 2) {
         if (EPI == EPI_VROPE) {
@@ -894,13 +894,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (HAS_BIAS && trow * 8 < BN) {
             const int col = nb * BN + trow * 8;
             bias_s[trow] = col < g.N ? *reinterpret_cast<const uint4*>(g.bias + col) : make_uint4(0, 0, 0, 0);
-        }
-        if (HAS_RESID) {
-#pragma unroll
-            for (int h = 0; h < 2 * NU; ++h) {
-                const int col = nb * BN + h * 8;
-                res[h] = row_ok && col < g.N ? *reinterpret_cast<const uint4*>(g.resid + (size_t)row * g.ldr + col) : make_uint4(0, 0, 0, 0);
-            }
         }
         if (HAS_BIAS) asm volatile("bar.sync 1, %0;" ::"n"(SplitCfg<BN, KPS>::THREADS - 64) : "memory");      // the epilogue warps
     }
@@ -944,19 +937,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = __fadd_rn(0.f, __uint_as_float(r[j]));
             // the rounding points of gemm_tc_kernel's epilogues
-            float b[16], rs[16];
+            float b[16];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < 2; ++h)
                 if (HAS_BIAS) unpack8_bf16(bias_s[2 * u + h], b + h * 8);
-                if (HAS_RESID) unpack8_bf16(res[HAS_RESID ? 2 * u + h : 0], rs + h * 8);
-            }
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 if (EPI == EPI_BIAS) v[j] = bf16_round(v[j]) + b[j];
                 if (EPI == EPI_BIAS_GELU) v[j] = bf16_round(bf16_round(v[j]) + b[j]);
-                if (EPI == EPI_RESID) v[j] = bf16_round(v[j]) + rs[j];
-                if (EPI == EPI_BIAS_RESID) v[j] = rs[j] + bf16_round(bf16_round(v[j]) + b[j]);
-                if (EPI == EPI_GATE_RESID) v[j] = rs[j] + bf16_round(b[j] * bf16_round(v[j]));
             }
             if (EPI == EPI_BIAS_GELU) gelu_all(v, g.scale != 0.f);
 #pragma unroll
