@@ -491,6 +491,9 @@ int o1_gemm_qkv_pair_rows(int M, int qc, int kc, int K);
  * qc and kc multiples of 128, M >= 8.  Bit-identical to three o1_gemm calls (epilogues 6, 6, 0). */
 int o1_gemm_qkv(const void *x, int ldx, const void *wq, const void *wk, const void *wv, void *y, int ldy, int M,
                 int qc, int kc, int K, const void *q_norm, const void *k_norm, const float *cs, float eps);
+/* The same of a block of the vision tower (width 1152, 16 heads of 72; src/model/vision.c): y [M, 3 x 16 x 128], a head's 72 columns
+ * and eight zeros at the beginning of its 128, q and k rotated by cos / sin [M,72] fp32; M >= 8. */
+int o1_gemm_vision_qkv(const void *x, const void *w, const void *b, void *y, int M, const float *cos, const float *sin);
 /* Prefix-causal flash attention on seq-major operands: q [S, ldq], k [S, ldk],
  * v [S, ldv], out [S, ldo]; head h at columns [128h, 128h+128). */
 int o1_flash_attention(const void *q, int ldq, const void *k, int ldk, const void *v, int ldv,

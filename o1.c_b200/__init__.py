@@ -251,6 +251,7 @@ _sig("o1_gemm_form", c_int, c_int, c_int, c_int, c_int, c_int, C.POINTER(c_int),
 _sig("o1_gemm_pair_tile", c_int, c_int, c_int, c_int, c_int, c_int)
 _sig("o1_gemm_qkv_pair_rows", c_int, c_int, c_int, c_int, c_int)
 _sig("o1_gemm_qkv", c_int, _P, c_int, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, _P, _P, c_float)
+_sig("o1_gemm_vision_qkv", c_int, _P, _P, _P, _P, c_int, _P, _P)
 _sig("o1_flash_attention", c_int, _P, c_int, _P, c_int, _P, c_int, _P, c_int, c_int, c_int, c_int,
      c_int, c_float)
 _sig("o1_attention_tail_ways", None, c_int)

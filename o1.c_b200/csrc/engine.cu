@@ -943,6 +943,11 @@ int o1_gemm_qkv(const void* x, int ldx, const void* wq, const void* wk, const vo
     count();
     return 0;
 }
+int o1_gemm_vision_qkv(const void* x, const void* w, const void* b, void* y, int M, const float* cos, const float* sin) {
+    if (!gemm_vision_qkv(x, w, b, y, M, cos, sin, g_stream)) return 1;
+    count();
+    return 0;
+}
 int o1_flash_attention(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, void* out,
                        int ldo, int S, int heads, int kv_heads, int ar_len, float scale) {
     if (!flash_attention(q, ldq, k, ldk, v, ldv, out, ldo, S, heads, kv_heads, ar_len, scale, g_stream))

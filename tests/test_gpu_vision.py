@@ -422,8 +422,6 @@ def test_workspace_tensors_are_those_of_the_layout(pkg, dev, tower, gh, gw):
 def test_qkv_rotary_projection_on_cta_pairs(pkg, dev, M):
     """The tower's q | k | v launch around the row counts where it goes from a tile for each SM to CTA pairs (tiles with no row of the second
     CTA, with one, more than a round): the bits of single CTAs, columns 72..79 of a head zero, nothing else written."""
-    fn = pkg.lib._ZN2o115gemm_vision_qkvEPKvS1_S1_PviPKfS4_P11CUstream_st      # o1::gemm_vision_qkv
-    fn.argtypes, fn.restype = [C.c_void_p] * 4 + [C.c_int] + [C.c_void_p] * 3, C.c_bool
     gen = torch.Generator(device=dev)
     gen.manual_seed(M)
     n_ = lambda *s: torch.empty(*s, device=dev).normal_(0, 1, generator=gen)  # noqa: E731
@@ -435,7 +433,7 @@ def test_qkv_rotary_projection_on_cta_pairs(pkg, dev, M):
             pkg.lib.o1_gemm_pair_mode(on)
             y = torch.full((M + 1, 6144), 777.0, dtype=torch.bfloat16, device=dev)
             torch.cuda.synchronize()
-            assert fn(pkg.ptr(x), pkg.ptr(w), pkg.ptr(b), pkg.ptr(y), M, pkg.ptr(cos), pkg.ptr(sin), None), pkg.last_error()
+            assert pkg.lib.o1_gemm_vision_qkv(pkg.ptr(x), pkg.ptr(w), pkg.ptr(b), pkg.ptr(y), M, pkg.ptr(cos), pkg.ptr(sin)) == 0, pkg.last_error()
             torch.cuda.synchronize()
             outs.append(y)
     finally:
