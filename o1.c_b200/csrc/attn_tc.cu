@@ -532,7 +532,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // leaves this unit's rows in its Q tile, from where another warp takes them to memory.  What stays between two units is the
 // accumulator, which PV of the next one may only overwrite once it has been read.
 // A CTA for each item (barriers, tensor memory, first copies and the way out for each) / units in a stream, 32 / 8 heads, us: 592
-// rows 18.8 / 14.9, 1280 rows 39.2 / 31.9, 3157 rows 175 / 152, 8000 rows 960 / 852, 16640 rows 3853 / 3721 (power cap), all rows
+// rows 18.8 / 14.9, 1280 rows 39.2 / 31.9, 3157 rows 175 / 152, 8000 rows 960 / 852, 16640 rows alike (3.7 to 3.9 ms at the power cap), all rows
 // causal 1280 rows 29.6 / 20.5, 3157 rows 115 / 88; the tower's 16 heads of 72 at 4096 patches 124 / 107; one unit for each CTA (200
 // rows) 6.5 / 6.5.  The same bits.  A key tile takes 1340 to 1410 cycles (1560 before), 1250 of which shared memory needs for the
 // operands (160 KB: Q and K 64, V 32, the copies 64); storing the rows by the set itself cost 2 to 5 % of these times.
@@ -1144,18 +1144,18 @@ __global__ void __launch_bounds__(AD) attn_merge_kernel(const AttnArgs a, int n_
     dst[col] = f32_to_bf16(v);
 }
 
-// Number of key-range parts for the tail items: the last (total % SMs) items would otherwise occupy a wave
-// of CTAs alone.  Cost of the tail in item durations: rounds of CTAs it needs, ceil(rem * w / SMs), times the
-// duration of a part, 1/w plus a fixed share for its prologue, Q load, fp32 epilogue and the merge launch.  With 128-row items that
-// share is some twelve key tiles' worth (4 heads, 5500 rows: a key tile is 0.95 us, a wave of items of 43 key tiles 40, the tail of 24
-// items 40 unsplit and 29 in parts of 7 key tiles).  After full waves the SMs have drifted apart and a tail of a few items costs
-// next to nothing: split from a fifth of a wave on, or after one wave at most.  Unsplit / split, us: 4 heads 10496
-// rows (32 tail items after two waves) 231 / 194, 16640 rows (76 after three, two rounds of parts) 509 / 501, 8 heads 8192 rows
-// 270 / 252, 12356 rows (36 after five) 585 / 541, 16 heads 12356 rows 1082 / 1061; left alone: 8 heads 16640 rows (4 after
-// seven) 933 / 937, 16 heads 8192 rows 485 / 522.
+// Number of key-range parts for the tail items: the last (total % SMs) items would otherwise be a round of their own.  Cost of the tail in
+// item durations: rounds it needs, ceil(rem * w / SMs), times the duration of a part, 1/w plus a fixed share, which the rule
+// takes as twelve key tiles' worth for 128-row items.  That share was measured with a CTA for each item (its set-up, copies, drain and the
+// merge launch); as units of a stream the parts have less of it, and the rule is right more often than it thinks.  After full rounds the
+// SMs have drifted apart and a tail of a few items costs next to nothing: split from a fifth of a round on, or after one round at
+// most.  Unsplit / split, units in a stream, us: 4 heads 10496 rows (32 tail items after two rounds) 193 / 171, 16640 rows (76 after three)
+// 476 / 462, 8 heads 8192 rows (68 after three) 248 / 236, 12356 rows (36 after five) 555 / 504, 16 heads 12356 rows (72 after
+// ten) 1027 / 999; left alone: 8 heads 16640 rows (4 after seven) 990, 16 heads 8192 rows (136 after six) 426.
 // Below T1_EXACT_ROWS rows the share is four key tiles, as measured with the two-tile kernel's 256-row items (which keep it),
-// and the tail a quarter of a wave: like the max there, the choice decides the bits of a forward.  The figure above would be the
-// better one there too, 16 heads 1280 rows 27.0 / 20.5 us, 32 heads 3157 rows 169 / 164, 8 heads 6000 rows 154 / 142.
+// and the tail a quarter of a round: like the max there, the choice decides the bits of a forward, so it stays although most tails are better left
+// whole now: 4 heads 5500 rows (24 after one) 71.9 / 60.7 us, but 16 heads 1280 rows (12 after one) 22.3 / 24.6, 8 heads 6000 rows (80 after
+// two) 143 / 156, 32 heads 3157 rows (60 after five) 132 / 137, 8000 rows (92 after thirteen) 823 / 831.
 // Every part keeps at least two key tiles.
 static int g_tail_ways = 0;   // 0: choose; 1: never split; n > 1: n parts whenever they fit
 void attention_tail_ways(int ways) { g_tail_ways = ways < 0 ? 0 : ways; }

@@ -247,7 +247,7 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorM
 //     tmem_relinquish_pair();
 // The allocation is one of both CTAs.  A CTA that comes to it on its own gets its columns all the same, and if it also gives up the permit before the
 // other has come, the other's allocation never ends: with the allocation and the relinquishment behind one another and no barrier in front, a pair whose
-// second CTA had started 0.6 us late (the SM's slots were still full of the norm's blocks) hung, one of some 10^6 launches.
+// second CTA had started 0.6 us late hung, one of some 10^6 launches.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() {
     __syncwarp();
