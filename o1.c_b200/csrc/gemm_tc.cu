@@ -1675,10 +1675,12 @@ static bool make_tmap_kblocks(CUtensorMap* out, const void* base, uint64_t rows,
     return true;
 }
 
+// What a map is of: rows x cols; `parts` heads, hoff elements apart; rows x cols in boxes of `parts` K blocks.
+enum TmapKind { TMAP_MATRIX, TMAP_HEADS, TMAP_KBLOCKS };
 struct TmapKey {
-    const void* p; uint64_t rows, cols, ld, heads, hoff; uint32_t box;     // heads == 0: a plain matrix; hoff == 0: K blocks, heads of them a box
+    TmapKind kind; const void* p; uint64_t rows, cols, ld; uint32_t box; uint64_t parts, hoff;
     bool operator<(const TmapKey& o) const {
-        return std::tie(p, rows, cols, ld, heads, hoff, box) < std::tie(o.p, o.rows, o.cols, o.ld, o.heads, o.hoff, o.box);
+        return std::tie(kind, p, rows, cols, ld, box, parts, hoff) < std::tie(o.kind, o.p, o.rows, o.cols, o.ld, o.box, o.parts, o.hoff);
     }
 };
 // Encoding a tensor map costs a few microseconds on the host; weights and
@@ -1692,20 +1694,22 @@ static bool cached(CUtensorMap* out, const TmapKey& k) {
     auto it = cache.find(k);
     if (it != cache.end()) { *out = it->second; return true; }
     if (cache.size() > 8192) cache.clear();
-    if (!(k.heads && !k.hoff ? make_tmap_kblocks(out, k.p, k.rows, k.cols, k.ld, k.box, (uint32_t)k.heads) : k.heads ? make_tmap_heads(out, k.p, k.cols, k.rows, k.heads, k.ld, k.hoff, k.box) : make_tmap_bf16(out, k.p, k.rows, k.cols, k.ld, k.box)))
-        return false;
+    const bool made = k.kind == TMAP_MATRIX ? make_tmap_bf16(out, k.p, k.rows, k.cols, k.ld, k.box)
+                      : k.kind == TMAP_HEADS ? make_tmap_heads(out, k.p, k.cols, k.rows, k.parts, k.ld, k.hoff, k.box)
+                                             : make_tmap_kblocks(out, k.p, k.rows, k.cols, k.ld, k.box, (uint32_t)k.parts);
+    if (!made) return false;
     cache.emplace(k, *out);
     return true;
 }
 bool cached_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
-    return cached(out, TmapKey{base, rows, cols, ld, 0, 0, box_rows});
+    return cached(out, TmapKey{TMAP_MATRIX, base, rows, cols, ld, box_rows, 0, 0});
 }
 static bool cached_tmap_kblocks(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t blocks) {
-    return cached(out, TmapKey{base, rows, cols, ld, blocks, 0, box_rows});
+    return cached(out, TmapKey{TMAP_KBLOCKS, base, rows, cols, ld, box_rows, blocks, 0});
 }
 bool cached_tmap_heads(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t heads, uint64_t ld, uint64_t hoff,
                        uint32_t box_rows) {
-    return cached(out, TmapKey{base, rows, cols, ld, heads, hoff, box_rows});
+    return cached(out, TmapKey{TMAP_HEADS, base, rows, cols, ld, box_rows, heads, hoff});
 }
 
 // cudaFuncSetAttribute is per device: remember, per kernel instantiation, on which devices it was done.
